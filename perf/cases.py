@@ -131,7 +131,7 @@ def _draw(rng: random.Random) -> dict:
     hidden = rng.choice([2048, 4096])
     return dict(kind="llama", layers=rng.choice([1, 2]), hidden=hidden, heads=hidden // D,
                 kv_heads=rng.choice([8, hidden // D]), ffn=rng.choice([5632, 11008, 14336]), vocab=32000,
-                seq=4 * _log(rng, 256, 2048))
+                seq=8 * _log(rng, 128, 1024))      # the weight gradients need a multiple of 8 tokens
 
 
 # ------------------------------------------------------------------------------------------------
