@@ -150,12 +150,16 @@ static_assert(sizeof(BwdSmem) <= 232448, "BwdSmem exceeds the 227 KB a CTA may u
 
 // First 128-query tile of a segment that can see the key tile starting at column c0.
 __device__ __forceinline__ int seg_first_qt(const AttnSeg& sg, int c0) {
-  if (!sg.causal) return 0;
+  if (!(sg.causal & SEG_UPPER)) return 0;
   const int r_min = c0 - sg.diag;   // smallest query index that sees key c0
   return r_min <= 0 ? 0 : r_min / BWD_QT;
 }
-__device__ __forceinline__ int seg_num_qt(const AttnSeg& sg) {
-  return (sg.len + BWD_QT - 1) / BWD_QT;
+// One past the last 128-query tile of a segment that can see it.
+__device__ __forceinline__ int seg_num_qt(const AttnSeg& sg, int c0) {
+  const int n = (sg.len + BWD_QT - 1) / BWD_QT;
+  if (!(sg.causal & SEG_LOWER)) return n;
+  const int r_max = c0 + ATTN_TILE - 1 - sg.lo;   // largest query index that sees the tile's last key
+  return r_max < 0 ? 0 : min(n, r_max / BWD_QT + 1);
 }
 
 
@@ -179,7 +183,7 @@ struct BwdStepIter {
     // (g, e) valid; find the next segment with work from here on
     for (;;) {
       sg = p.segs[e];
-      nq = seg_num_qt(sg);
+      nq = seg_num_qt(sg, c0);
       t = seg_first_qt(sg, c0);
       if (t < nq) return;
       if (++e >= col.seg_end) { e = col.seg_begin; ++g; }
@@ -209,7 +213,7 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 // of the tensor core, packed to bf16 pairs. MASK applies the causal / key-tail mask (tiles that
 // need none skip the compares).
 template <bool MASK>
-__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, bool key_ok, int r_first,
+__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, bool key_ok, int r_first, int r_last,
                                             uint32_t (&pk)[32]) {
   float sv[2][32];
   tmem_ld_x32(t_st, reinterpret_cast<uint32_t(&)[32]>(sv[0]));
@@ -226,8 +230,8 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, boo
       // instruction issue, not by the special-function unit), so the default is none
       const float p0 = (c & 7) < BWD_POLY_EXP_OF_8 ? poly_exp2(x0) : fast_exp2(x0);
       const float p1 = ((c + 1) & 7) < BWD_POLY_EXP_OF_8 ? poly_exp2(x1) : fast_exp2(x1);
-      sv[h][c] = (!MASK || (key_ok && (h * 32 + c) >= r_first)) ? p0 : 0.f;
-      sv[h][c + 1] = (!MASK || (key_ok && (h * 32 + c + 1) >= r_first)) ? p1 : 0.f;
+      sv[h][c] = (!MASK || (key_ok && (h * 32 + c) >= r_first && (h * 32 + c) <= r_last)) ? p0 : 0.f;
+      sv[h][c + 1] = (!MASK || (key_ok && (h * 32 + c + 1) >= r_first && (h * 32 + c + 1) <= r_last)) ? p1 : 0.f;
     }
 #pragma unroll
     for (int c = 0; c < 16; ++c) pk[h * 16 + c] = pack_bf16x2(sv[h][2 * c], sv[h][2 * c + 1]);
@@ -313,7 +317,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   int steps_per_head = 0;
   for (int e = col.seg_begin; e < col.seg_end; ++e) {
     const AttnSeg sg = p.segs[e];
-    const int n = seg_num_qt(sg) - seg_first_qt(sg, c0);
+    const int n = seg_num_qt(sg, c0) - seg_first_qt(sg, c0);
     steps_per_head += n > 0 ? n : 0;
   }
   const int n_steps = steps_per_head * p.kv_group;
@@ -341,7 +345,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         const int head = kv_head * p.kv_group + g;
         for (int e = col.seg_begin; e < col.seg_end && ok; ++e) {
           const AttnSeg sg = p.segs[e];
-          const int nq = seg_num_qt(sg);
+          const int nq = seg_num_qt(sg, c0);
           if (seg_first_qt(sg, c0) < nq &&
               !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
             report_error(wc, UA_ERR_FLAG_TIMEOUT, 121, sg.wait_flag);
@@ -570,7 +574,10 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       if (i + 1 < n_steps) write_aug((i + 1) & 1, lv, dv);
       BWD_PROF(prof, pslot + 7);
       // visible iff key_c <= r + diag  <=>  r >= key_c - diag   (r relative to this half)
-      const int r_first = sg.causal ? (key_c - sg.diag - cur.t * BWD_QT - wg * 64) : 0;
+      const int r_half = cur.t * BWD_QT + wg * 64;
+      const int r_first = (sg.causal & SEG_UPPER) ? key_c - sg.diag - r_half : 0;
+      // ... and key_c >= r + lo  <=>  r <= key_c - lo
+      const int r_last = (sg.causal & SEG_LOWER) ? key_c - sg.lo - r_half : 63;
       // the row terms of step i+2 travel while this step computes
       if (i + 2 < n_steps) {
         fut.next(p, col, c0);
@@ -583,10 +590,10 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       BWD_PROF(prof, pslot + 2);
       tc_fence_after_sync();
       uint32_t pk[32];                 // this thread's 64 probabilities, packed; kept for phase B
-      if (__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0))
-        bwd_phase_a<false>(t_st, p.scale_log2, key_ok, r_first, pk);
+      if (__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63))
+        bwd_phase_a<false>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
       else
-        bwd_phase_a<true>(t_st, p.scale_log2, key_ok, r_first, pk);
+        bwd_phase_a<true>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
       // packed P^T of this half goes to the first 32 columns of this half's own S^T columns
       // (the other warpgroup may still be reading its fp32 half)
       BWD_PROF(prof, pslot + 3);
@@ -696,7 +703,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       const int head = kv_head * p.kv_group + g;
       for (int e = col.seg_begin; e < col.seg_end && ok; ++e) {
         const AttnSeg sg = p.segs[e];
-        const int nq = seg_num_qt(sg);
+        const int nq = seg_num_qt(sg, c0);
         const CUtensorMap* tdq = &p.tmdQ[sg.src];
         const long rs = p.dq_row_stride[sg.src];
         float* dq_col = p.dq_ptr[sg.src] + batch * p.dq_batch_stride[sg.src] +
@@ -954,7 +961,7 @@ __global__ void noalloc_fill_tables(BwdCol* col, AttnSeg* seg, int2* tiles, int 
     *col = c;
     AttnSeg s;
     s.src = 0; s.start = 0; s.len = tokens; s.causal = causal; s.diag = 0;
-    s.wait_flag = 0; s.wait_count = 0; s.pad2 = 0;
+    s.wait_flag = 0; s.wait_count = 0; s.lo = 0;
     *seg = s;
   }
   // key tile t of a causal problem is visited by all query sub-tiles at or below it, so the

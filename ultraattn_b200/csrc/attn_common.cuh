@@ -26,12 +26,15 @@ struct AttnSeg {
   int src;      // source slot
   int start;    // first token inside the source buffer
   int len;      // tokens
-  int causal;   // 0: every (q,k) pair allowed; 1: key c allowed for query r iff c <= r + diag
+  int causal;   // bit set of SEG_*: 0 = every (q, k) pair allowed; SEG_UPPER: key c allowed for query r
+                // only if c <= r + diag; SEG_LOWER: only if c >= r + lo (both set: a band)
   int diag;     // (r and c are 0-based inside the query block / the segment)
   int wait_flag;   // 0: data is in place; f > 0: wait until stage_flags[f - 1] >= wait_count
   int wait_count;
-  int pad2;
+  int lo;
 };
+constexpr int SEG_UPPER = 1;
+constexpr int SEG_LOWER = 2;
 
 // One chunk of the in-kernel staging prologue: copy n_vec16 16-byte vectors from src (usually a
 // peer GPU's memory, read with plain peer loads over NVLink) to dst (this GPU's staging mirror),

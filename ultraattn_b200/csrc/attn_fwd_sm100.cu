@@ -107,17 +107,18 @@ struct __align__(1024) FwdSmem {
 };
 static_assert(sizeof(FwdSmem) + 1024 <= 232448, "FwdSmem exceeds the 227 KB a CTA may use");
 
-// Number of 128-key tiles of a segment that the 256-row tile starting at block-relative row r0
-// has to visit (tiles entirely above the causal diagonal for both sub-tiles are skipped).
-__device__ __forceinline__ int seg_tiles(const AttnSeg& sg, int r0, int rows_here) {
-  int n = (sg.len + ATTN_TILE - 1) / ATTN_TILE;
-  if (sg.causal) {
+// 128-key tiles [first, end) of a segment that the 256-row tile starting at block-relative row r0
+// has to visit (tiles that neither sub-tile can see, above the upper or below the lower bound, are
+// skipped).
+struct TileRange { int first, end; };
+__device__ __forceinline__ TileRange seg_tiles(const AttnSeg& sg, int r0, int rows_here) {
+  TileRange tr{0, (sg.len + ATTN_TILE - 1) / ATTN_TILE};
+  if (sg.causal & SEG_UPPER) {
     const int last = r0 + rows_here - 1 + sg.diag;  // largest allowed key index
-    if (last < 0) return 0;
-    const int nc = last / ATTN_TILE + 1;
-    n = nc < n ? nc : n;
+    tr.end = last < 0 ? 0 : min(tr.end, last / ATTN_TILE + 1);
   }
-  return n;
+  if (sg.causal & SEG_LOWER) tr.first = min(tr.end, max(0, r0 + sg.lo) / ATTN_TILE);
+  return tr;
 }
 
 // Optional pipeline trace (compile with -DUA_FWD_PROF): CTA (0, 0) records clock64() at the
@@ -189,7 +190,10 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
 
   // total number of key tiles this CTA visits (identical in every role)
   int n_total = 0;
-  for (int e = row.seg_begin; e < row.seg_end; ++e) n_total += seg_tiles(p.segs[e], r0, rows_here);
+  for (int e = row.seg_begin; e < row.seg_end; ++e) {
+    const TileRange tr = seg_tiles(p.segs[e], r0, rows_here);
+    n_total += tr.end - tr.first;
+  }
 
   if (warp >= Cfg::SOFTMAX_WARPS) {
   // 20 warps are launched with 96 registers per thread, and that launch-time total (5 x 96 per
@@ -218,15 +222,15 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       uint32_t j = 0;
       for (int e = row.seg_begin; e < row.seg_end && ok; ++e) {
         const AttnSeg sg = p.segs[e];
-        const int nt = seg_tiles(sg, r0, rows_here);
+        const TileRange tr = seg_tiles(sg, r0, rows_here);
         const CUtensorMap* tk = &p.tmK[sg.src];
         const CUtensorMap* tv = &p.tmV[sg.src];
-        if (nt > 0 && !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
+        if (tr.first < tr.end && !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
           report_error(wc, UA_ERR_FLAG_TIMEOUT, 111, sg.wait_flag);
           ok = false;
           break;
         }
-        for (int t = 0; t < nt; ++t, ++j) {
+        for (int t = tr.first; t < tr.end; ++t, ++j) {
           const int st = j % FWD_KV_STAGES;
           const uint32_t ph = (j / FWD_KV_STAGES) & 1;
           const int krow = sg.start + t * ATTN_TILE;
@@ -344,8 +348,8 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     uint32_t j = 0;
     for (int e = row.seg_begin; e < row.seg_end && ok; ++e) {
       const AttnSeg sg = p.segs[e];
-      const int nt = seg_tiles(sg, r0, rows_here);
-      for (int t = 0; t < nt; ++t, ++j) {
+      const TileRange tr = seg_tiles(sg, r0, rows_here);
+      for (int t = tr.first; t < tr.end; ++t, ++j) {
         const bool prof = (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0 && part == 0;
         const int pslot = 8 + w * 24 + (static_cast<int>(j) - FWD_PROF_TILE) * 8;
         (void)prof; (void)pslot;
@@ -362,13 +366,20 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           tmem_wait_ld();
         }
         FWD_PROF(prof, pslot + 2);
-        // masking: key index c (segment-relative) allowed iff c < len and (c <= r + diag)
+        // masking: key index c (segment-relative) allowed iff c < len, c <= r + diag and c >= r + lo
         const int c0 = t * ATTN_TILE + part * NC;
         int limit = sg.len - c0;                               // columns < limit are in range
-        if (sg.causal) limit = min(limit, r_blk + sg.diag - c0 + 1);
+        if (sg.causal & SEG_UPPER) limit = min(limit, r_blk + sg.diag - c0 + 1);
         if (limit < NC) {
 #pragma unroll
           for (int i = 0; i < NC; ++i) sv[i] = (i < limit) ? sv[i] : NEG_INF;
+        }
+        if (sg.causal & SEG_LOWER) {
+          const int first = r_blk + sg.lo - c0;                // columns >= first are in range
+          if (first > 0) {
+#pragma unroll
+            for (int i = 0; i < NC; ++i) sv[i] = (i >= first) ? sv[i] : NEG_INF;
+          }
         }
         // eight independent running maxima, two new values per instruction: one dependent chain of
         // compares would cost more than the exponentials

@@ -35,7 +35,8 @@ class Seg:
     """A run of tokens in source slot ``src`` starting at ``start``.
 
     ``causal``: key c of the segment is visible to query r of the block iff ``c <= r + diag``
-    (both 0-based inside their block / segment).
+    (both 0-based inside their block / segment). ``lo``: additionally only iff ``c >= r + lo`` (with
+    ``causal`` the two bounds make a band).
     """
     src: int
     start: int
@@ -44,6 +45,7 @@ class Seg:
     diag: int = 0
     wait_flag: int = 0       # 0: in place; f > 0: wait for staging flag f - 1 to reach wait_count
     wait_count: int = 0
+    lo: int | None = None
 
 
 @dataclass
@@ -114,7 +116,15 @@ def _seg_tiles(seg: Seg, r0: int, rows_here: int) -> int:
         if last < 0:
             return 0
         n = min(n, last // TILE + 1)
+    if seg.lo is not None:
+        n -= min(n, max(0, r0 + seg.lo) // TILE)
     return n
+
+
+def _seg_entry(s: Seg) -> tuple:
+    """The device form of a segment (struct AttnSeg of csrc/attn_common.cuh)."""
+    return (s.src, s.start, s.length, int(s.causal) | (2 if s.lo is not None else 0), s.diag, s.wait_flag, s.wait_count,
+            0 if s.lo is None else s.lo)
 
 
 class FwdPlan:
@@ -128,7 +138,7 @@ class FwdPlan:
         for ri, r in enumerate(self.rows):
             b = len(segs)
             for s in r.segs:
-                segs.append((s.src, s.start, s.length, int(s.causal), s.diag, s.wait_flag, s.wait_count, 0))
+                segs.append(_seg_entry(s))
             row_arr[ri] = (r.q_src, r.q_start, r.q_len, b, len(segs), r.o_slot, r.o_start,
                            int(r.accumulate), r.q_wait_flag, r.q_wait_count)
             for t in range((r.q_len + CTA_ROWS - 1) // CTA_ROWS):
@@ -349,11 +359,21 @@ def _stage_args(stage):
 
 
 def _mask_for(seg: Seg, q_len: int, device) -> torch.Tensor | None:
-    if not seg.causal:
+    """Visible pairs [queries, keys] of a forward segment; None: all of them."""
+    return _visible(q_len, seg.length, seg, device)
+
+
+def _visible(n_q: int, n_k: int, seg: Seg, device) -> torch.Tensor | None:
+    if not seg.causal and seg.lo is None:
         return None
-    r = torch.arange(q_len, device=device)[:, None]
-    c = torch.arange(seg.length, device=device)[None, :]
-    return c <= r + seg.diag
+    r = torch.arange(n_q, device=device)[:, None]
+    c = torch.arange(n_k, device=device)[None, :]
+    m = torch.ones(n_q, n_k, dtype=torch.bool, device=device)
+    if seg.causal:
+        m &= c <= r + seg.diag
+    if seg.lo is not None:
+        m &= c >= r + seg.lo
+    return m
 
 
 def attn_fwd_reference(q_srcs, k_srcs, v_srcs, outs, rows: Sequence[Row],
@@ -448,6 +468,9 @@ def _col_steps(c: Col, c0: int) -> int:
         if s.causal:
             r_min = c0 - s.diag
             first = 0 if r_min <= 0 else r_min // BWD_QT
+        if s.lo is not None:
+            r_max = c0 + TILE - 1 - s.lo
+            nq = 0 if r_max < 0 else min(nq, r_max // BWD_QT + 1)
         n += max(0, nq - first)
     return n
 
@@ -463,7 +486,7 @@ class BwdPlan:
         for ci, c in enumerate(self.cols):
             b = len(segs)
             for s in c.segs:
-                segs.append((s.src, s.start, s.length, int(s.causal), s.diag, s.wait_flag, s.wait_count, 0))
+                segs.append(_seg_entry(s))
             col_arr[ci] = (c.kv_src, c.kv_start, c.kv_len, b, len(segs), c.g_slot, c.g_start, 0,
                            c.kv_wait_flag, c.kv_wait_count)
             for t in range((c.kv_len + TILE - 1) // TILE):
@@ -560,10 +583,9 @@ def attn_bwd_reference(q_sides: Sequence[BwdQSide], k_srcs, v_srcs, kv_outs: Seq
             sc = torch.einsum("bqhd,bkhd->bhqk", q, kk) * scale
             lse_safe = torch.where(torch.isfinite(lse), lse, torch.full_like(lse, float("inf")))
             p = torch.exp(sc - lse_safe[..., None])
-            if s.causal:
-                r = torch.arange(s.length, device=q.device)[:, None]
-                cc = torch.arange(c.kv_len, device=q.device)[None, :]
-                p = p * (cc <= r + s.diag)[None, None].to(p.dtype)
+            m = _visible(s.length, c.kv_len, s, q.device)
+            if m is not None:
+                p = p * m[None, None].to(p.dtype)
             dp = torch.einsum("bqhd,bkhd->bhqk", do, vv)
             ds = p * (dp - dvec[..., None])
             dv += torch.einsum("bhqk,bqhd->bkhd", p, do)
