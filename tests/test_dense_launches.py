@@ -1,0 +1,90 @@
+"""Dense launches (no tables; packed query heads, keys split over CTAs) against float64 attention; the dense
+backward against the table launch."""
+import math
+
+import pytest
+import torch
+
+from ultraattn_b200.ops import attention as A
+
+pytestmark = pytest.mark.gpu
+
+# (batch, queries, keys, query heads, kv heads, causal, key splits): one query and a full / overfull 128-row tile
+# of packed rows, ungrouped heads, a group that is no power of two, fewer keys than one tile, more splits than
+# key tiles, rows that see no key (more queries than keys under a causal mask), ragged everything
+CASES = [(2, 1, 1000, 8, 2, True, 0), (1, 1, 513, 4, 4, True, 3), (3, 1, 4096, 16, 2, False, 7), (1, 1, 100, 8, 8, True, 0),
+         (1, 32, 900, 8, 2, True, 0), (1, 33, 900, 8, 2, True, 5), (1, 128, 640, 2, 2, True, 2), (1, 129, 640, 2, 2, True, 2),
+         (2, 17, 700, 6, 2, True, 0), (1, 40, 700, 12, 2, False, 4), (1, 300, 1111, 8, 1, True, 0), (1, 257, 257, 4, 2, True, 3),
+         (1, 1000, 1000, 8, 2, True, 0), (1, 1000, 1000, 8, 2, True, 1), (1, 700, 300, 4, 2, True, 2), (1, 5, 1, 2, 1, False, 9),
+         (1, 512, 4100, 4, 1, True, 0), (2, 260, 260, 2, 2, False, 1), (1, 64, 60, 2, 1, True, 1), (1, 1, 70000, 2, 1, True, 0)]
+
+
+@pytest.mark.parametrize("B,Sq,Skv,H,Hk,causal,n_split", CASES)
+def test_dense_forward_matches_float64(B, Sq, Skv, H, Hk, causal, n_split):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    g = torch.Generator(device="cuda").manual_seed(Sq * 7 + Skv)
+    mk = lambda s, h: torch.randn(B, s, h, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, k, v = mk(Sq, H), mk(Skv, Hk), mk(Skv, Hk)
+    o = torch.full_like(q, 7.0)
+    lse = torch.full((B, H, Sq), 7.0, device="cuda")
+    A.attn_fwd_dense(q, k, v, (o, lse), causal, None, n_split)
+    A.check_status()
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double().repeat_interleave(H // Hk, 2)) / math.sqrt(128)
+    if causal:
+        r, c = torch.arange(Sq, device="cuda")[:, None], torch.arange(Skv, device="cuda")[None, :]
+        s = s.masked_fill(c > r + Skv - Sq, float("-inf"))
+    ref_lse = torch.logsumexp(s, -1)
+    p = torch.exp(s - ref_lse.masked_fill(ref_lse == float("-inf"), 0.0)[..., None])
+    ref = torch.einsum("bhqk,bkhd->bqhd", p, v.double().repeat_interleave(H // Hk, 2))
+    seen = torch.isfinite(ref_lse)
+    assert torch.equal(torch.isfinite(lse), seen)
+    assert (lse[seen] - ref_lse[seen]).abs().max() < 1e-3
+    # P and O are rounded to bf16 (2^-9 each), rows without keys are exactly zero
+    assert (o.double() - ref).norm() <= 4 * 2 ** -9 * ref.norm()
+    assert (o.transpose(1, 2)[~seen] == 0).all()
+
+
+def test_dense_forward_writes_into_strided_outputs_and_reads_strided_inputs():
+    """K / V as views of a packed projection, O as a slice of a larger buffer."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    torch.manual_seed(0)
+    kv = torch.randn(1, 900, 2, 2, 128, device="cuda", dtype=torch.bfloat16)
+    q = torch.randn(1, 9, 8, 128, device="cuda", dtype=torch.bfloat16)
+    big = torch.zeros(1, 9, 12, 128, device="cuda", dtype=torch.bfloat16)
+    lse = torch.empty(1, 8, 9, device="cuda")
+    A.attn_fwd_dense(q, kv[:, :, 0], kv[:, :, 1], (big[:, :, 2:10], lse), True)
+    o2, lse2 = torch.empty_like(q), torch.empty_like(lse)
+    A.attn_fwd_dense(q, kv[:, :, 0].contiguous(), kv[:, :, 1].contiguous(), (o2, lse2), True)
+    assert torch.equal(big[:, :, 2:10], o2) and torch.equal(lse, lse2)
+    assert (big[:, :, :2] == 0).all() and (big[:, :, 10:] == 0).all()
+
+
+@pytest.mark.parametrize("B,Sq,Skv,H,Hk,causal", [(2, 300, 300, 4, 2, True), (1, 129, 700, 4, 1, True), (3, 200, 77, 2, 2, True),
+                                                  (2, 128, 129, 4, 4, False), (1, 1, 130, 2, 1, True), (1, 1000, 1000, 8, 2, False)])
+def test_dense_backward_equals_the_table_launch(B, Sq, Skv, H, Hk, causal):
+    """Same kernel, same order of work: dK and dV bit for bit; dQ is summed in arrival order (fp32)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    from ultraattn_b200.ops import elementwise as E
+    g = torch.Generator(device="cuda").manual_seed(Sq + Skv)
+    mk = lambda s, h: torch.randn(B, s, h, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, k, v, d_o = mk(Sq, H), mk(Skv, Hk), mk(Skv, Hk), mk(Sq, H)
+    o, lse = torch.empty_like(q), torch.empty(B, H, Sq, device="cuda")
+    A.attn_fwd_dense(q, k, v, (o, lse), causal)
+    dvec, zero = E.bwd_prepare(o, d_o)
+    assert (zero == 0).all()
+    assert (dvec - (o.double() * d_o.double()).sum(-1).transpose(1, 2)).abs().max() < 1e-3
+    res = []
+    for dense in (True, False):
+        dq, out = torch.zeros_like(zero), A.BwdKvOut(torch.empty_like(k), torch.empty_like(v))
+        side = A.BwdQSide(q, d_o, lse, dvec, dq)
+        if dense:
+            A.attn_bwd_dense(side, k, v, out, causal)
+        else:
+            A.attn_bwd([side], [k], [v], [out], A.BwdPlan([A.Col(0, 0, Skv, (A.Seg(0, 0, Sq, causal, Skv - Sq),))], "cuda"))
+        res.append((out.dk, out.dv, dq))
+    A.check_status()
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    assert (res[0][2] - res[1][2]).norm() <= 1e-6 * res[1][2].norm()

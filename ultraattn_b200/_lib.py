@@ -47,9 +47,12 @@ def _declare(lib):
                          vp],
         "ua_attn_fwd": [POINTER(UaTensorSrc), i, POINTER(UaTensorSrc), POINTER(UaTensorSrc), i,
                         POINTER(UaOutDst), i, vp, vp, vp, i, i, i, i, f, vp, vp, i, i, vp, i, vp, vp],
+        "ua_attn_fwd_dense_parts": [i, i, i, i, i, i, i],
+        "ua_attn_fwd_dense": [POINTER(UaTensorSrc), POINTER(UaTensorSrc), POINTER(UaTensorSrc), POINTER(UaOutDst), i, f,
+                              i, vp, vp, vp],
         "ua_attn_bwd": [POINTER(UaTensorSrc), POINTER(UaTensorSrc), POINTER(UaBwdQSide), i,
                         POINTER(UaTensorSrc), POINTER(UaTensorSrc), i, POINTER(UaBwdKvOut), i,
-                        vp, vp, vp, i, i, i, i, f, vp, vp, i, i, vp, i, vp, vp],
+                        vp, vp, vp, i, i, i, i, i, f, vp, vp, i, i, vp, i, vp, vp],
         "ua_barrier": [POINTER(vp), i, i, i, ctypes.c_uint, ctypes.c_double, vp, vp],
         "ua_xent_fwd": [vp, vp, vp, vp, l, l, i, vp],
         "ua_xent_bwd": [vp, vp, vp, vp, l, l, i, vp],
@@ -61,6 +64,7 @@ def _declare(lib):
         "ua_lse_merge": [POINTER(vp), POINTER(vp), POINTER(l), POINTER(l), i, vp, vp, l, l, i, i,
                          vp],
         "ua_rowdot": [vp, vp, vp, l, l, l, i, i, vp],
+        "ua_bwd_prepare": [vp, vp, vp, vp, l, l, l, l, i, i, i, vp],
         "ua_cast_scale": [vp, vp, l, f, i, vp],
         "ua_rmsnorm_fwd": [vp, vp, vp, vp, i, i, f, vp],
         "ua_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, i, i, vp],

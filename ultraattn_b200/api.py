@@ -32,39 +32,52 @@ def local_plans(pattern: BSA_Repr, seq_len: int, device) -> tuple:
     return _plan_cache[key]
 
 
+def _dense_kind(pattern: BSA_Repr, q, k, v) -> int:
+    """1 / 2: the pattern is one full / causal block over all tokens, which the kernels run without
+    launch tables; 0: anything else."""
+    tab = pattern.block_table_int
+    one = tab.shape == (1, 1) and q.is_cuda and q.shape[1] == k.shape[1] == v.shape[1]
+    return int(tab[0, 0]) if one else 0
+
+
 class _LocalAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, pattern, softmax_scale):
-        fplan, bplan = local_plans(pattern, q.shape[1], q.device)
         o = torch.empty_like(q)
         lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
-        A.attn_fwd([q], [k], [v], [(o, lse)], fplan, softmax_scale)
+        ctx.dense = _dense_kind(pattern, q, k, v)
+        if ctx.dense:
+            ctx.bplan = None
+            A.attn_fwd_dense(q, k, v, (o, lse), ctx.dense == 2, softmax_scale)
+        else:
+            fplan, ctx.bplan = local_plans(pattern, q.shape[1], q.device)
+            A.attn_fwd([q], [k], [v], [(o, lse)], fplan, softmax_scale)
         ctx.save_for_backward(q, k, v, o, lse)
-        ctx.bplan = bplan
         ctx.scale = softmax_scale
         return o
 
     @staticmethod
     def backward(ctx, d_o):
         q, k, v, o, lse = ctx.saved_tensors
-        dq, dk, dv = local_backward(q, k, v, o, lse, d_o.contiguous(), ctx.bplan, ctx.scale)
+        dq, dk, dv = local_backward(q, k, v, o, lse, d_o.contiguous(), ctx.bplan, ctx.scale, ctx.dense)
         return dq, dk, dv, None, None
 
 
-def local_backward(q, k, v, o, lse, d_o, bplan, softmax_scale=None):
-    """dQ, dK, dV of the single-device operator (bf16 on CUDA, input dtype on CPU)."""
-    B, S, H, D = q.shape
-    dvec = torch.empty(B, H, S, dtype=torch.float32, device=q.device)
-    for b in range(B):
-        E.rowdot(o[b], d_o[b], dvec[b])
-    dq32 = torch.zeros(B, S, H, D, dtype=torch.float32, device=q.device)
+def local_backward(q, k, v, o, lse, d_o, bplan, softmax_scale=None, dense: int = 0):
+    """dQ, dK, dV of the single-device operator (bf16 on CUDA, input dtype on CPU). ``dense`` = 1 / 2:
+    full / causal attention over all tokens; ``bplan`` is not read."""
+    dvec, dq32 = E.bwd_prepare(o, d_o)
     if q.is_cuda:
         dk = torch.empty_like(k)
         dv = torch.empty_like(v)
     else:
         dk = torch.zeros(k.shape, dtype=torch.float32, device=q.device)
         dv = torch.zeros(v.shape, dtype=torch.float32, device=q.device)
-    A.attn_bwd([A.BwdQSide(q, d_o, lse, dvec, dq32)], [k], [v], [A.BwdKvOut(dk, dv)], bplan, softmax_scale)
+    side, kv_out = A.BwdQSide(q, d_o, lse, dvec, dq32), A.BwdKvOut(dk, dv)
+    if dense:
+        A.attn_bwd_dense(side, k, v, kv_out, dense == 2, softmax_scale)
+    else:
+        A.attn_bwd([side], [k], [v], [kv_out], bplan, softmax_scale)
     if q.is_cuda:
         dq = torch.empty_like(q)
         E.cast_scale(dq32, dq)

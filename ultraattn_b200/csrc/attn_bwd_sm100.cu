@@ -105,6 +105,9 @@ struct BwdParams {
   float scale;                      // softmax scale
   float scale_log2;
   int* status;
+  // dense launches (cols == nullptr): one column, one query segment, no tables
+  BwdCol dense_col;
+  AttnSeg dense_seg;
   StageParams stage;                // optional in-kernel staging of remote blocks
   KernelTrace trace;                // optional per-CTA time stamps
 };
@@ -175,6 +178,9 @@ constexpr int BWD_PROF_STEP = 8;
 
 // Walks the (query head of the group, query segment, 128-query tile) steps of one key tile in the
 // order every role of the CTA uses.
+__device__ __forceinline__ AttnSeg bwd_seg(const BwdParams& p, int e) {
+  return p.cols == nullptr ? p.dense_seg : p.segs[e];
+}
 struct BwdStepIter {
   int g, e, t, nq;
   bool new_seg;      // first step of a (head, segment) pair
@@ -182,7 +188,7 @@ struct BwdStepIter {
   __device__ __forceinline__ void seek(const BwdParams& p, const BwdCol& col, int c0) {
     // (g, e) valid; find the next segment with work from here on
     for (;;) {
-      sg = p.segs[e];
+      sg = bwd_seg(p, e);
       nq = seg_num_qt(sg, c0);
       t = seg_first_qt(sg, c0);
       if (t < nq) return;
@@ -255,16 +261,20 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   const int lane = threadIdx.x & 31;
 
   const int kv_head = blockIdx.x / p.n_tiles;
-  const int2 tl = p.tiles[blockIdx.x % p.n_tiles];
+  // (dense: the first key tiles are seen by the most queries under a causal mask, so the natural order
+  // is heaviest first)
+  const bool dense = p.cols == nullptr;
+  const int item = blockIdx.x % p.n_tiles;
+  const int2 tl = dense ? make_int2(0, item) : p.tiles[item];
   const int batch = blockIdx.y;
-  const BwdCol col = p.cols[tl.x];
+  const BwdCol col = dense ? p.dense_col : p.cols[tl.x];
   const int cta_linear = blockIdx.y * gridDim.x + blockIdx.x;
   trace_stamp(p.trace, cta_linear, 0);
   trace_ident(p.trace, cta_linear, tl.x);
   {
     // does this CTA read a staged block? then it first helps to empty the copy queue
     bool waits = col.kv_wait_flag != 0;
-    for (int e = col.seg_begin; e < col.seg_end && !waits; ++e) waits = p.segs[e].wait_flag != 0;
+    for (int e = col.seg_begin; e < col.seg_end && !waits; ++e) waits = bwd_seg(p, e).wait_flag != 0;
     drain_stage_queue(p.stage, waits, cta_linear, &s.stage_slot);
   }
   trace_stamp(p.trace, cta_linear, 1);
@@ -316,7 +326,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   // number of (head, segment, query tile) steps; identical in every role
   int steps_per_head = 0;
   for (int e = col.seg_begin; e < col.seg_end; ++e) {
-    const AttnSeg sg = p.segs[e];
+    const AttnSeg sg = bwd_seg(p, e);
     const int n = seg_num_qt(sg, c0) - seg_first_qt(sg, c0);
     steps_per_head += n > 0 ? n : 0;
   }
@@ -344,7 +354,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       for (int g = 0; g < p.kv_group && ok; ++g) {
         const int head = kv_head * p.kv_group + g;
         for (int e = col.seg_begin; e < col.seg_end && ok; ++e) {
-          const AttnSeg sg = p.segs[e];
+          const AttnSeg sg = bwd_seg(p, e);
           const int nq = seg_num_qt(sg, c0);
           if (seg_first_qt(sg, c0) < nq &&
               !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
@@ -702,7 +712,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     for (int g = 0; g < p.kv_group && ok; ++g) {
       const int head = kv_head * p.kv_group + g;
       for (int e = col.seg_begin; e < col.seg_end && ok; ++e) {
-        const AttnSeg sg = p.segs[e];
+        const AttnSeg sg = bwd_seg(p, e);
         const int nq = seg_num_qt(sg, c0);
         const CUtensorMap* tdq = &p.tmdQ[sg.src];
         const long rs = p.dq_row_stride[sg.src];
@@ -836,16 +846,19 @@ static int encode_src_box(CUtensorMap* tm, const UaTensorSrc& t, uint32_t rows) 
 
 static int g_bwd_smem_set[64] = {0};
 
+// dense = 0: tables; 1 / 2: all queries of source 0 against all its keys, without a mask / causal (key c is
+// visible to query r iff c <= r + skv - sq); the table arguments are then not read.
 extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
                            const UaBwdQSide* q_side, int n_q, const UaTensorSrc* k_src,
                            const UaTensorSrc* v_src, int n_kv, const UaBwdKvOut* kv_out, int n_out,
                            const void* cols_dev, const void* segs_dev, const void* tiles_dev,
-                           int n_tiles, int n_heads, int n_kv_heads, int batch,
+                           int n_tiles, int dense, int n_heads, int n_kv_heads, int batch,
                            float softmax_scale, int* status, const void* copy_tasks_dev,
                            int n_copy_tasks, int n_copy_ctas, unsigned int* stage_flags,
                            int stage_epoch, unsigned int* stage_ticket, cudaStream_t stream) {
   if (n_q > ATTN_MAX_SRC || n_kv > ATTN_MAX_SRC || n_out > ATTN_MAX_SRC)
     UA_FAIL("ua_attn_bwd: too many sources (max %d)", ATTN_MAX_SRC);
+  if (dense) n_tiles = static_cast<int>((k_src[0].tokens + ATTN_TILE - 1) / ATTN_TILE);
   if (n_tiles <= 0) return 0;
   BwdParams p;
   memset(&p, 0, sizeof(p));
@@ -882,6 +895,15 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
     p.dkv_row_stride[i] = kv_out[i].row_stride;
     p.dkv_batch_stride[i] = kv_out[i].batch_stride;
     p.dkv_add_f32[i] = kv_out[i].add_f32;
+  }
+  if (dense) {
+    const int sq = static_cast<int>(q_src[0].tokens), skv = static_cast<int>(k_src[0].tokens);
+    p.dense_col.kv_len = skv;
+    p.dense_col.seg_end = 1;
+    p.dense_seg.len = sq;
+    p.dense_seg.causal = dense == 2 ? SEG_UPPER : 0;
+    p.dense_seg.diag = skv - sq;
+    cols_dev = nullptr;
   }
   p.cols = static_cast<const BwdCol*>(cols_dev);
   p.segs = static_cast<const AttnSeg*>(segs_dev);

@@ -10,42 +10,40 @@
 // through a unicast TMA tensor map), and the epilogue can either overwrite (O, lse) or merge into
 // an existing partial (O, lse) — possibly a mailbox in a peer GPU's memory.
 //
-// CTA = 256 query rows x 1 head: two 128-row sub-tiles processed ping-pong so that the tensor
-// core works on one sub-tile while the softmax warps work on the other. TPR = threads per query
-// row (template parameter):
-//   TPR = 1 (320 threads, default): warps 0-3 softmax / correction / epilogue for sub-tile 0 (one thread per
-//            query row, 128 score columns each), warps 4-7 the same for sub-tile 1
-//   TPR = 2 (640 threads, UA_FWD_TPR=2): two warpgroups per sub-tile; the two threads of a row take 64
-//            score columns each (both can reach the row's TMEM lane), exchange their row maxima
-//            through shared memory once per tile and each keep a partial row sum. The softmax of
-//            a 128 x 128 tile is a chain of dependent latencies (TMEM load, max, exp2, pack, TMEM
-//            store) that one warp per scheduler cannot hide; four warps per scheduler can. As
-//            measured (S = 16k, 32 heads) this form is slower than TPR = 1 all the same, 876 against
-//            1192 TFLOP/s: 104 registers per softmax thread leave spills in its inner loop and
-//            the exchange adds a barrier per tile. It is kept as a tested variant.
-//   then one TMA producer warp (Q once, then the K and V rings) and one tcgen05.mma issuer warp
-//   (one elected thread; it also owns the TMEM allocation)
+// CTA: warps 0-3 softmax / correction / epilogue of sub-tile 0 (one thread per query
+// row, 128 score columns each), warps 4-7 the same for sub-tile 1, then one TMA producer warp and
+// one tcgen05.mma issuer warp (one elected thread; it also owns the TMEM allocation). The two
+// sub-tiles run ping-pong, so that the tensor core works on one while the softmax warps work on
+// the other:
+//   FEW = false: 256 query rows, 128 per sub-tile; both sub-tiles visit every key tile
+//   FEW = true:  up to 128 query rows, the same ones in both sub-tiles, which take the key tiles in
+//                turn (decoding: a handful of rows behind a long cache)
 // TMEM (512 columns): S0 | S1 | O0 | O1, 128 fp32 columns each; P (bf16) overwrites the first
 // 64 columns of its S region and is consumed from TMEM as the A operand of the PV product.
+//
+// Two kinds of launches use the kernel. Table launches (ua_attn_fwd) read rows, segments and tiles
+// from device tables. Dense launches (ua_attn_fwd_dense: all queries against all keys, causal or
+// not) carry their one row and segment in the kernel parameters, so that nothing is uploaded, and
+//   * pack the query heads of a key/value head: row r of a tile is query token r / G, head r % G
+//     (G heads of a group, a power of two), so that a decoding step reads its cache once per
+//     key/value head and not once per query head;
+//   * split the keys over several CTAs when the rows alone leave SMs idle: every part writes its
+//     normalised fp32 O and lse, and combine_kernel merges them (see plan_dense).
 #include "attn_common.cuh"
 #include "host_common.cuh"
 #include "ptx.cuh"
 
 namespace ua {
 
-constexpr int FWD_KV_STAGES = 2;
-template <int TPR> struct FwdCfg {
-  static constexpr int SOFTMAX_WARPS = 8 * TPR;
-  static constexpr int TMA_WARP = SOFTMAX_WARPS;
-  static constexpr int MMA_WARP = SOFTMAX_WARPS + 1;
-  // TPR = 2: five warpgroups (the last one: TMA, MMA and two idle warps), so that every scheduler
-  // hosts the same number of warps and the register file can be re-balanced by warpgroup
-  static constexpr int THREADS = TPR == 2 ? 640 : 32 * (SOFTMAX_WARPS + 2);
-  static constexpr int NC = ATTN_TILE / TPR;      // score columns per thread
-  // register split of the TPR = 2 form (see the role dispatch in the kernel)
-  static constexpr int REGS_LAUNCH = 96, REGS_LOAD = 64, REGS_SOFTMAX = 104;
-  static_assert(4 * REGS_SOFTMAX + REGS_LOAD <= 5 * REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
-};
+constexpr int FWD_SOFTMAX_WARPS = 8;
+constexpr int FWD_TMA_WARP = 8;
+constexpr int FWD_MMA_WARP = 9;
+// three warpgroups (the last one: TMA, MMA and two idle warps), so that the register file can be
+// re-balanced by warpgroup: a softmax thread holds its row's 128 scores besides everything else and
+// spilled at the 168 registers an even split leaves; 2 x 216 + 64 <= 3 x 168
+constexpr int FWD_THREADS = 384;
+constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 64, FWD_REGS_SOFTMAX = 216;
+static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
 #ifndef UA_FWD_POLY_EXP_PERIOD
 #define UA_FWD_POLY_EXP_PERIOD 0
 #endif
@@ -83,41 +81,53 @@ struct FwdParams {
   int kv_group;        // query heads per key/value head
   float scale_log2;    // softmax scale * log2(e)
   int* status;
+  // dense launches (rows == nullptr)
+  FwdRow dense_row;
+  AttnSeg dense_seg;
+  int pack_shift;      // log2 of the query heads packed into the rows of a tile (0 in table launches)
+  int n_split;         // CTAs that share the keys of a tile
+  float* part_o;       // not null: fp32 partial results [batch, parts, tokens, heads, 128] ...
+  float* part_lse;     // ... and [batch, parts, tokens, heads]; parts = n_split (x 2 if FEW)
+  int n_parts;
   StageParams stage;   // optional in-kernel staging of remote K/V (and Q) blocks
   KernelTrace trace;   // optional per-CTA time stamps
 };
 
+template <bool FEW>
 struct __align__(1024) FwdSmem {
-  uint8_t q[2][FWD_TILE_BYTES];
-  uint8_t k[FWD_KV_STAGES][FWD_TILE_BYTES];
-  uint8_t v[FWD_KV_STAGES][FWD_TILE_BYTES];
+  static constexpr int STAGES = FEW ? 3 : 2;      // (the second Q tile's room goes to the rings)
+  uint8_t q[FEW ? 1 : 2][FWD_TILE_BYTES];
+  uint8_t k[STAGES][FWD_TILE_BYTES];
+  uint8_t v[STAGES][FWD_TILE_BYTES];
   uint64_t q_full[2];
-  uint64_t k_full[FWD_KV_STAGES];
-  uint64_t k_empty[FWD_KV_STAGES];
-  uint64_t v_full[FWD_KV_STAGES];
-  uint64_t v_empty[FWD_KV_STAGES];
+  uint64_t k_full[STAGES];
+  uint64_t k_empty[STAGES];
+  uint64_t v_full[STAGES];
+  uint64_t v_empty[STAGES];
   uint64_t s_full[2];
   uint64_t p_full[2];
   uint64_t o_full;
   uint32_t tmem_base;
   int abort_flag;
   int stage_slot;
-  float xchg[2][2][ATTN_TILE];    // [sub-tile][column half][row]: row maxima / row sums exchanged between the two threads of a row
-  uint64_t xbar[2];               // the 8 warps of a sub-tile meet here (an mbarrier, so that the wait is bounded)
 };
-static_assert(sizeof(FwdSmem) + 1024 <= 232448, "FwdSmem exceeds the 227 KB a CTA may use");
+static_assert(sizeof(FwdSmem<false>) + 1024 <= 232448, "FwdSmem exceeds the 227 KB a CTA may use");
+static_assert(sizeof(FwdSmem<true>) + 1024 <= 232448, "FwdSmem exceeds the 227 KB a CTA may use");
 
-// 128-key tiles [first, end) of a segment that the 256-row tile starting at block-relative row r0
-// has to visit (tiles that neither sub-tile can see, above the upper or below the lower bound, are
-// skipped).
+// 128-key tiles [first, end) of a segment that the query tokens [t0, t_last] have to visit (tiles
+// above the upper or below the lower bound of all of them are skipped).
 struct TileRange { int first, end; };
-__device__ __forceinline__ TileRange seg_tiles(const AttnSeg& sg, int r0, int rows_here) {
+__host__ __device__ __forceinline__ TileRange seg_tiles(const AttnSeg& sg, int t0, int t_last) {
   TileRange tr{0, (sg.len + ATTN_TILE - 1) / ATTN_TILE};
   if (sg.causal & SEG_UPPER) {
-    const int last = r0 + rows_here - 1 + sg.diag;  // largest allowed key index
-    tr.end = last < 0 ? 0 : min(tr.end, last / ATTN_TILE + 1);
+    const int last = t_last + sg.diag;  // largest allowed key index
+    const int nc = last < 0 ? 0 : last / ATTN_TILE + 1;
+    tr.end = nc < tr.end ? nc : tr.end;
   }
-  if (sg.causal & SEG_LOWER) tr.first = min(tr.end, max(0, r0 + sg.lo) / ATTN_TILE);
+  if (sg.causal & SEG_LOWER) {
+    const int lo = t0 + sg.lo < 0 ? 0 : (t0 + sg.lo) / ATTN_TILE;
+    tr.first = lo < tr.end ? lo : tr.end;
+  }
   return tr;
 }
 
@@ -132,43 +142,63 @@ __device__ long long g_fwd_prof[64];
 constexpr int FWD_PROF_TILE = 8;
 
 
-template <int TPR>
-__global__ void __launch_bounds__(FwdCfg<TPR>::THREADS, 1)
+template <bool FEW>
+__global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ FwdParams p) {
-  using Cfg = FwdCfg<TPR>;
-  constexpr int NC = Cfg::NC;
+  constexpr int STAGES = FwdSmem<FEW>::STAGES;
   extern __shared__ uint8_t smem_raw[];
-  FwdSmem& s = *reinterpret_cast<FwdSmem*>(
+  FwdSmem<FEW>& s = *reinterpret_cast<FwdSmem<FEW>*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  // (packed launches: `head` is the key/value head and stands for all its query heads)
+  const bool dense = p.rows == nullptr;
   const int head = blockIdx.x / p.n_tiles;
-  const int2 tl = p.tiles[blockIdx.x % p.n_tiles];
+  const int item = blockIdx.x % p.n_tiles;
+  // dense tiles run from the last rows to the first: under a causal mask the heaviest ones come first
+  const int2 tl = dense ? make_int2(0, (p.n_tiles - 1 - item) / p.n_split) : p.tiles[item];
+  const int split = dense ? (p.n_tiles - 1 - item) % p.n_split : 0;
   const int batch = blockIdx.y;
-  const FwdRow row = p.rows[tl.x];
+  const FwdRow row = dense ? p.dense_row : p.rows[tl.x];
+  auto seg_at = [&](int e) { return dense ? p.dense_seg : p.segs[e]; };
   const int cta_linear = blockIdx.y * gridDim.x + blockIdx.x;
   trace_stamp(p.trace, cta_linear, 0);
   trace_ident(p.trace, cta_linear, tl.x);
   {
     // does this CTA read a staged block? then it first helps to empty the copy queue
     bool waits = row.q_wait_flag != 0;
-    for (int e = row.seg_begin; e < row.seg_end && !waits; ++e) waits = p.segs[e].wait_flag != 0;
+    for (int e = row.seg_begin; e < row.seg_end && !waits; ++e) waits = seg_at(e).wait_flag != 0;
     drain_stage_queue(p.stage, waits, cta_linear, &s.stage_slot);
   }
   trace_stamp(p.trace, cta_linear, 1);
-  const int r0 = tl.y * 256;                                    // block-relative first row
-  const int rows_here = min(256, row.q_len - r0);               // valid query rows of this CTA
-  const int kv_head = head / p.kv_group;
+  constexpr int CTA_ROWS = FEW ? ATTN_TILE : 2 * ATTN_TILE;
+  const int psh = p.pack_shift;
+  const int r0 = tl.y * CTA_ROWS;                               // block-relative first (packed) row
+  const int rows_here = min(CTA_ROWS, (row.q_len << psh) - r0); // valid rows of this CTA
+  const int tok0 = r0 >> psh, tok_last = (r0 + rows_here - 1) >> psh;
+  const int q_head = head << psh;                               // query head of packed row 0
+  const int kv_head = q_head / p.kv_group;
+  // key tiles of segment e that this CTA visits: all of them, or its share of a split launch
+  auto cta_tiles = [&](const AttnSeg& sg) {
+    TileRange tr = seg_tiles(sg, tok0, tok_last);
+    if (p.n_split > 1) {
+      const int n = tr.end - tr.first, base = tr.first;
+      tr.first = base + static_cast<int>(static_cast<long>(n) * split / p.n_split);
+      tr.end = base + static_cast<int>(static_cast<long>(n) * (split + 1) / p.n_split);
+    }
+    return tr;
+  };
+  // FEW: warps without a valid row have nothing to do (their scores are never read back)
+  const int act_warps = FEW ? (rows_here + 31) / 32 : 4;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.s_full[i], 1);
-      mbar_init(&s.p_full[i], 4 * TPR);     // one arrival per softmax warp
-      mbar_init(&s.xbar[i], 8);
+      mbar_init(&s.p_full[i], act_warps);   // one arrival per softmax warp
     }
-    for (int i = 0; i < FWD_KV_STAGES; ++i) {
+    for (int i = 0; i < STAGES; ++i) {
       mbar_init(&s.k_full[i], 1);
       mbar_init(&s.k_empty[i], 1);
       mbar_init(&s.v_full[i], 1);
@@ -178,7 +208,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     s.abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == Cfg::MMA_WARP) {
+  if (warp == FWD_MMA_WARP) {
     tmem_alloc(&s.tmem_base, 512);
     tmem_relinquish();
   }
@@ -191,19 +221,13 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
   // total number of key tiles this CTA visits (identical in every role)
   int n_total = 0;
   for (int e = row.seg_begin; e < row.seg_end; ++e) {
-    const TileRange tr = seg_tiles(p.segs[e], r0, rows_here);
+    const TileRange tr = cta_tiles(seg_at(e));
     n_total += tr.end - tr.first;
   }
 
-  if (warp >= Cfg::SOFTMAX_WARPS) {
-  // 20 warps are launched with 96 registers per thread, and that launch-time total (5 x 96 per
-  // scheduler lane) is the whole pool that setmaxnreg can redistribute: an increase that asks for
-  // more than the decreases have returned never completes. The last warpgroup (TMA, MMA, two idle
-  // warps) goes down to 64 and the four softmax warpgroups, which hold 64 scores per thread, go up
-  // to 104: 4 x 104 + 64 = 5 x 96. (The instruction sits inside the role's branch so that the
-  // compiler budgets each role separately.)
-  if constexpr (TPR == 2) reg_dealloc<FwdCfg<2>::REGS_LOAD>();
-  if (warp == Cfg::TMA_WARP) {
+  if (warp >= FWD_SOFTMAX_WARPS) {
+  reg_dealloc<FWD_REGS_LOAD>();
+  if (warp == FWD_TMA_WARP) {
     // =============================== TMA producer ===========================================
     if (lane == 0 && n_total > 0) {
       const CUtensorMap* tq = &p.tmQ[row.q_src];
@@ -213,16 +237,16 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         report_error(wc, UA_ERR_FLAG_TIMEOUT, 110, row.q_wait_flag);
         ok = false;
       }
-      for (int w = 0; w < 2 && ok; ++w) {
+      for (int w = 0; w < (FEW ? 1 : 2) && ok; ++w) {
         mbar_arrive_expect_tx(&s.q_full[w], FWD_TILE_BYTES);
-        const int qrow = row.q_start + r0 + w * ATTN_TILE;
-        tma_load_4d(s.q[w], tq, &s.q_full[w], 0, head, qrow, batch);
-        tma_load_4d(s.q[w] + 16384, tq, &s.q_full[w], 64, head, qrow, batch);
+        const int qrow = row.q_start + tok0 + ((w * ATTN_TILE) >> psh);
+        tma_load_4d(s.q[w], tq, &s.q_full[w], 0, q_head, qrow, batch);
+        tma_load_4d(s.q[w] + 16384, tq, &s.q_full[w], 64, q_head, qrow, batch);
       }
       uint32_t j = 0;
       for (int e = row.seg_begin; e < row.seg_end && ok; ++e) {
-        const AttnSeg sg = p.segs[e];
-        const TileRange tr = seg_tiles(sg, r0, rows_here);
+        const AttnSeg sg = seg_at(e);
+        const TileRange tr = cta_tiles(sg);
         const CUtensorMap* tk = &p.tmK[sg.src];
         const CUtensorMap* tv = &p.tmV[sg.src];
         if (tr.first < tr.end && !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
@@ -231,8 +255,8 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           break;
         }
         for (int t = tr.first; t < tr.end; ++t, ++j) {
-          const int st = j % FWD_KV_STAGES;
-          const uint32_t ph = (j / FWD_KV_STAGES) & 1;
+          const int st = j % STAGES;
+          const uint32_t ph = (j / STAGES) & 1;
           const int krow = sg.start + t * ATTN_TILE;
           if (!mbar_wait(&s.k_empty[st], ph ^ 1, wc, 100)) { ok = false; break; }
           mbar_arrive_expect_tx(&s.k_full[st], FWD_TILE_BYTES);
@@ -245,7 +269,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         }
       }
     }
-  } else if (warp == Cfg::MMA_WARP) {
+  } else if (warp == FWD_MMA_WARP) {
     // =============================== MMA issuer =============================================
     if (lane == 0 && n_total > 0) {
       const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S = Q K^T, both K-major
@@ -253,7 +277,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       const uint32_t tS[2] = {tmem_base + 0, tmem_base + 128};
       const uint32_t tO[2] = {tmem_base + 256, tmem_base + 384};
       auto issue_s = [&](int w, int st) {
-        const uint32_t qa = smem_u32(s.q[w]);
+        const uint32_t qa = smem_u32(s.q[FEW ? 0 : w]);
         const uint32_t ka = smem_u32(s.k[st]);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
@@ -274,6 +298,29 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       bool ok = true;
       do {
         if (!mbar_wait(&s.q_full[0], 0, wc, 200)) { ok = false; break; }
+        if constexpr (FEW) {
+          // key tile j belongs to sub-tile j & 1; its scores are issued two tiles ahead
+          auto next_s = [&](int j) -> bool {
+            if (!mbar_wait(&s.k_full[j % STAGES], (j / STAGES) & 1, wc, 201)) return false;
+            tc_fence_after_sync();
+            issue_s(j & 1, j % STAGES);
+            tc_commit(&s.s_full[j & 1]);
+            tc_commit(&s.k_empty[j % STAGES]);
+            return true;
+          };
+          ok = next_s(0) && (n_total < 2 || next_s(1));
+          for (int j = 0; j < n_total && ok; ++j) {
+            const int w = j & 1, st = j % STAGES;
+            if (!mbar_wait(&s.v_full[st], (j / STAGES) & 1, wc, 203)) { ok = false; break; }
+            if (!mbar_wait(&s.p_full[w], (j >> 1) & 1, wc, 204)) { ok = false; break; }
+            tc_fence_after_sync();
+            issue_pv(w, st, j >= 2);
+            tc_commit(&s.v_empty[st]);
+            if (j + 2 < n_total) ok = next_s(j + 2);
+          }
+          if (ok) tc_commit(&s.o_full);
+          break;
+        }
         if (!mbar_wait(&s.k_full[0], 0, wc, 201)) { ok = false; break; }
         tc_fence_after_sync();
         issue_s(0, 0);
@@ -284,10 +331,10 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         tc_commit(&s.s_full[1]);
         tc_commit(&s.k_empty[0]);
         for (int j = 0; j < n_total; ++j) {
-          const int st = j % FWD_KV_STAGES;
-          const uint32_t ph = (j / FWD_KV_STAGES) & 1;
-          const int stn = (j + 1) % FWD_KV_STAGES;
-          const uint32_t phn = ((j + 1) / FWD_KV_STAGES) & 1;
+          const int st = j % STAGES;
+          const uint32_t ph = (j / STAGES) & 1;
+          const int stn = (j + 1) % STAGES;
+          const uint32_t phn = ((j + 1) / STAGES) & 1;
           const bool more = (j + 1 < n_total);
           FWD_PROF(j == FWD_PROF_TILE, 0);
           if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
@@ -320,65 +367,57 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     }
   }
   } else {
+  reg_alloc<FWD_REGS_SOFTMAX>();
+  if ((warp & 3) < act_warps) {
     // =============================== softmax + epilogue =====================================
-    if constexpr (TPR == 2) reg_alloc<FwdCfg<2>::REGS_SOFTMAX>();
-    const int w = warp / (4 * TPR);          // sub-tile
-    const int part = (warp >> 2) % TPR;      // which NC-column slice of the row this thread handles
+    const int w = warp >> 2;                 // sub-tile
     const int quad = warp & 3;               // TMEM lane quadrant of this warp
     const int r_tile = quad * 32 + lane;     // row inside the 128-row sub-tile
-    const int r_blk = r0 + w * ATTN_TILE + r_tile;   // row inside the query block
+    const int r_cta = (FEW ? 0 : w * ATTN_TILE) + r_tile;   // row inside the CTA's tile
+    const int r_blk = (r0 + r_cta) >> psh;                  // query token inside the query block
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t tS = tmem_base + lane_base + w * 128;
-    const uint32_t tSp = tS + part * NC;             // this thread's score columns
-    const uint32_t tPp = tS + part * (NC / 2);       // ... and where its packed probabilities go
     const uint32_t tO = tmem_base + lane_base + 256 + w * 128;
     const float NEG_INF = -INFINITY;
 
-    uint32_t xph = 0;        // phase of the sub-tile's exchange barrier
-    // all 256 threads of the sub-tile have passed this point (bounded like every other wait)
-    auto subtile_sync = [&]() -> bool {
-      mbar_arrive_warp(&s.xbar[w]);
-      const bool good = mbar_wait(&s.xbar[w], xph & 1, wc, 330 + w);
-      ++xph;
-      return good;
-    };
-    float m_use = NEG_INF;   // running reference max, log2 units (already scaled); identical in both threads of a row
-    float l = 0.f;           // row sum over this thread's columns
+    float m_use = NEG_INF;   // running reference max, log2 units (already scaled)
+    float l = 0.f;           // row sum
     bool ok = true;
     uint32_t j = 0;
     for (int e = row.seg_begin; e < row.seg_end && ok; ++e) {
-      const AttnSeg sg = p.segs[e];
-      const TileRange tr = seg_tiles(sg, r0, rows_here);
+      const AttnSeg sg = seg_at(e);
+      const TileRange tr = cta_tiles(sg);
       for (int t = tr.first; t < tr.end; ++t, ++j) {
-        const bool prof = (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0 && part == 0;
+        if (FEW && (j & 1) != static_cast<uint32_t>(w)) continue;
+        const bool prof = (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0;
         const int pslot = 8 + w * 24 + (static_cast<int>(j) - FWD_PROF_TILE) * 8;
         (void)prof; (void)pslot;
         FWD_PROF(prof, pslot + 0);
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full[w], j & 1, wc, 300 + w))) { ok = false; break; }
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full[w], (FEW ? j >> 1 : j) & 1, wc, 300 + w))) { ok = false; break; }
         FWD_PROF(prof, pslot + 1);
         tc_fence_after_sync();
-        float sv[NC];
+        float sv[ATTN_TILE];
         {
-          uint32_t(&raw)[NC] = reinterpret_cast<uint32_t(&)[NC]>(sv);
+          uint32_t(&raw)[ATTN_TILE] = reinterpret_cast<uint32_t(&)[ATTN_TILE]>(sv);
 #pragma unroll
-          for (int c = 0; c < NC / 32; ++c)
-            tmem_ld_x32(tSp + c * 32, reinterpret_cast<uint32_t(&)[32]>(raw[c * 32]));
+          for (int c = 0; c < 4; ++c)
+            tmem_ld_x32(tS + c * 32, reinterpret_cast<uint32_t(&)[32]>(raw[c * 32]));
           tmem_wait_ld();
         }
         FWD_PROF(prof, pslot + 2);
         // masking: key index c (segment-relative) allowed iff c < len, c <= r + diag and c >= r + lo
-        const int c0 = t * ATTN_TILE + part * NC;
+        const int c0 = t * ATTN_TILE;
         int limit = sg.len - c0;                               // columns < limit are in range
         if (sg.causal & SEG_UPPER) limit = min(limit, r_blk + sg.diag - c0 + 1);
-        if (limit < NC) {
+        if (limit < ATTN_TILE) {
 #pragma unroll
-          for (int i = 0; i < NC; ++i) sv[i] = (i < limit) ? sv[i] : NEG_INF;
+          for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i < limit) ? sv[i] : NEG_INF;
         }
         if (sg.causal & SEG_LOWER) {
           const int first = r_blk + sg.lo - c0;                // columns >= first are in range
           if (first > 0) {
 #pragma unroll
-            for (int i = 0; i < NC; ++i) sv[i] = (i >= first) ? sv[i] : NEG_INF;
+            for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i >= first) ? sv[i] : NEG_INF;
           }
         }
         // eight independent running maxima, two new values per instruction: one dependent chain of
@@ -387,33 +426,24 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(sv[i], sv[8 + i]);
 #pragma unroll
-        for (int i = 16; i < NC; i += 16)
+        for (int i = 16; i < ATTN_TILE; i += 16)
 #pragma unroll
           for (int k = 0; k < 8; ++k) mx8[k] = fmax3(mx8[k], sv[i + k], sv[i + 8 + k]);
         float mx = fmaxf(fmax3(mx8[0], mx8[1], mx8[2]), fmax3(mx8[3], mx8[4], mx8[5]));
         mx = fmax3(mx, mx8[6], mx8[7]);
-        if constexpr (TPR == 2) {
-          // the row maximum over all 128 columns: exchange with the thread that holds the other half.
-          // (The slot is free again: its reader of the previous tile arrived at p_full before the
-          // products this tile's scores waited for could be issued.)
-          s.xchg[w][part][r_tile] = mx;
-          if (!__all_sync(0xFFFFFFFFu, subtile_sync())) { ok = false; break; }
-          mx = fmaxf(mx, s.xchg[w][part ^ 1][r_tile]);
-        }
         mx *= p.scale_log2;
         const float m_new = fmaxf(m_use, mx);
         // lazy rescale: only when the running max grew by more than 2^8 (warp-uniform branch,
         // because the TMEM accesses below are warp-collective)
         const bool need = (m_new - m_use > 8.0f) || (m_use == NEG_INF && m_new > NEG_INF);
-        if (j == 0) {
+        if (j < (FEW ? 2u : 1u)) {
           m_use = m_new;
         } else if (__any_sync(0xFFFFFFFFu, need)) {
           const float alpha = need ? fast_exp2(m_use - m_new) : 1.0f;
           if (need) m_use = m_new;
           l *= alpha;
-          // each thread of the row rescales its share of the 128 output columns
 #pragma unroll 1
-          for (int c = part * (4 / TPR); c < (part + 1) * (4 / TPR); ++c) {
+          for (int c = 0; c < 4; ++c) {
             uint32_t ov[32];
             tmem_ld_x32(tO + c * 32, ov);
             tmem_wait_ld();
@@ -431,7 +461,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) ls2[k] = f2_pack(0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < NC / 32; ++c) {
+        for (int c = 0; c < 4; ++c) {
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -449,7 +479,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
             ls2[i & 3] = f2_add(ls2[i & 3], f2_pack(p0, p1));
             pk[i] = pack_bf16x2(p0, p1);
           }
-          tmem_st_x16(tPp + c * 16, pk);
+          tmem_st_x16(tS + c * 16, pk);
         }
         float ls4[4];
 #pragma unroll
@@ -466,39 +496,29 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         FWD_PROF(prof, pslot + 5);
       }
     }
-    if constexpr (TPR == 2) {
-      // the row sum over all columns (m_use is the same in both threads)
-      if (ok) ok = __all_sync(0xFFFFFFFFu, subtile_sync());      // the last exchange of maxima has been read
-      s.xchg[w][part][r_tile] = l;
-      if (ok) ok = __all_sync(0xFFFFFFFFu, subtile_sync());
-      l += s.xchg[w][part ^ 1][r_tile];
-    }
-
     // ---------------------------------- epilogue --------------------------------------------
-    const bool valid_row = (w * ATTN_TILE + r_tile) < rows_here;
+    const bool valid_row = r_cta < rows_here;
+    const int qh = q_head + ((r0 + r_cta) & ((1 << psh) - 1));       // query head of this row
+    const bool any = FEW ? n_total > w : n_total > 0;                // this sub-tile has seen a key tile
     const long orow = static_cast<long>(row.o_start + r_blk);
     __nv_bfloat16* optr = p.o_ptr[row.o_slot] + batch * p.o_batch_stride[row.o_slot] +
-                          orow * p.o_row_stride[row.o_slot] + static_cast<long>(head) * ATTN_D;
+                          orow * p.o_row_stride[row.o_slot] + static_cast<long>(qh) * ATTN_D;
     float* lptr = p.lse_ptr[row.o_slot] + batch * p.lse_batch_stride[row.o_slot] +
-                  head * p.lse_head_stride[row.o_slot] + orow;
+                  qh * p.lse_head_stride[row.o_slot] + orow;
     if (n_total > 0 && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full, 0, wc, 310 + w));
     tc_fence_after_sync();
     float lse = NEG_INF;
     float inv = 0.f;
     // (a row whose keys were all masked has m_use = -inf; the polynomial exponential leaves about
     // 2^-126 per masked entry in l, which must not count as probability mass)
-    if (n_total > 0 && l > 0.f && m_use > NEG_INF) {
+    if (any && l > 0.f && m_use > NEG_INF) {
       lse = (m_use + log2f(l)) * 0.6931471805599453f;
       inv = 1.0f / l;
     }
     float w_old = 0.f, w_new = 1.f;
     float lse_old = NEG_INF;
-    if (row.accumulate) {
-      if (valid_row) lse_old = *lptr;
-      // (both threads of a row have read the old lse before one of them overwrites it below)
-      if constexpr (TPR == 2) { if (ok) ok = __all_sync(0xFFFFFFFFu, subtile_sync()); }
-    }
     if (row.accumulate && valid_row) {
+      lse_old = *lptr;
       const float mx = fmaxf(lse_old, lse);
       if (mx == NEG_INF) {
         w_old = 0.f; w_new = 0.f;
@@ -510,17 +530,33 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       }
     }
     const float fnew = inv * w_new;
+    float* pptr = nullptr;               // fp32 partial result of a split launch
+    if (p.part_o != nullptr) {
+      const int part = FEW ? 2 * split + w : split;
+      const long prow = ((static_cast<long>(batch) * p.n_parts + part) * row.q_len + r_blk) * p.n_heads + qh;
+      pptr = p.part_o + prow * ATTN_D;
+      lptr = p.part_lse + prow;
+    }
 #pragma unroll 1
-    for (int c = part * (4 / TPR); c < (part + 1) * (4 / TPR); ++c) {
+    for (int c = 0; c < 4; ++c) {
       uint32_t ov[32];
-      if (n_total > 0) {
+      if (any) {
         tmem_ld_x32(tO + c * 32, ov);
         tmem_wait_ld();
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) ov[i] = 0u;
       }
-      if (valid_row) {
+      if (valid_row && pptr != nullptr) {
+        float4* d4 = reinterpret_cast<float4*>(pptr + c * 32);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          float f[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 4 + i]) * fnew;
+          d4[q] = make_float4(f[0], f[1], f[2], f[3]);
+        }
+      } else if (valid_row) {
         uint4* d4 = reinterpret_cast<uint4*>(optr + c * 32);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -547,16 +583,60 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         }
       }
     }
-    if (valid_row && part == 0) *lptr = lse;
+    if (valid_row) *lptr = lse;
+  }
   }
 
   tc_fence_before_sync();
   __syncthreads();
   trace_stamp(p.trace, cta_linear, 2);
-  if (warp == Cfg::MMA_WARP) {
+  if (warp == FWD_MMA_WARP) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
+}
+
+// Merge the parts of a split dense launch: O = sum_i w_i O_i with w_i = exp(lse_i - lse), fp32 throughout,
+// one warp per (token, head) row, 4 head-dim elements per lane. Bound by reading the parts (they
+// mostly sit in L2: 0.5 KB per row and part).
+__global__ void __launch_bounds__(256)
+combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, int n_parts, int tokens, int heads,
+               __nv_bfloat16* __restrict__ o, long o_row_stride, long o_batch_stride, float* __restrict__ lse,
+               long lse_head_stride, long lse_batch_stride, long n_rows) {
+  const long r = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= n_rows) return;
+  const long per_part = static_cast<long>(tokens) * heads;
+  const long batch = r / per_part, in = r % per_part;           // in = token * heads + head
+  const long first = batch * n_parts * per_part + in;
+  float mx = -INFINITY;
+  for (int i = lane; i < n_parts; i += 32) mx = fmaxf(mx, part_lse[first + i * per_part]);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
+  float tot = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (mx > -INFINITY) {
+#pragma unroll 4
+    for (int i = 0; i < n_parts; ++i) {
+      const float w = __expf(part_lse[first + i * per_part] - mx);
+      const float4 v = *reinterpret_cast<const float4*>(part_o + (first + i * per_part) * ATTN_D + lane * 4);
+      tot += w;
+      if (w != 0.f) {
+        acc.x += w * v.x;
+        acc.y += w * v.y;
+        acc.z += w * v.z;
+        acc.w += w * v.w;
+      }
+    }
+  }
+  const float inv = tot > 0.f ? 1.f / tot : 0.f;
+  const long tok = in / heads, head = in % heads;
+  uint2 ov;
+  ov.x = pack_bf16x2(acc.x * inv, acc.y * inv);
+  ov.y = pack_bf16x2(acc.z * inv, acc.w * inv);
+  *reinterpret_cast<uint2*>(o + batch * o_batch_stride + tok * o_row_stride + head * ATTN_D + lane * 4) = ov;
+  if (lane == 0)
+    lse[batch * lse_batch_stride + head * lse_head_stride + tok] = tot > 0.f ? mx + __logf(tot) : -INFINITY;
 }
 
 }  // namespace ua
@@ -610,17 +690,41 @@ struct UaOutDst {
   long lse_batch_stride;
 };
 
-static int encode_src(CUtensorMap* tm, const UaTensorSrc& t) {
+// rows_head / rows_tok: heads and tokens per 128-row tile (1 x 128, or a packed group of heads)
+static int encode_src(CUtensorMap* tm, const UaTensorSrc& t, uint32_t rows_head = 1) {
   uint64_t dims[4] = {ATTN_D, static_cast<uint64_t>(t.heads), static_cast<uint64_t>(t.tokens),
                       static_cast<uint64_t>(t.batch)};
   uint64_t str[3] = {static_cast<uint64_t>(t.head_stride) * 2,
                      static_cast<uint64_t>(t.token_stride) * 2,
                      static_cast<uint64_t>(t.batch_stride > 0 ? t.batch_stride : t.token_stride * t.tokens) * 2};
-  uint32_t box[4] = {64, 1, ATTN_TILE, 1};
+  uint32_t box[4] = {64, rows_head, ATTN_TILE / rows_head, 1};
   return make_tmap_2byte(tm, t.ptr, 4, dims, str, box);
 }
 
-static int g_fwd_smem_set[2][64] = {{0}};
+template <bool FEW>
+static int launch_fwd(const FwdParams& p, int heads, int batch, cudaStream_t stream) {
+  static int smem_set[64] = {0};
+  const int smem_bytes = sizeof(FwdSmem<FEW>) + 1024;
+  int dev = 0;
+  UA_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !smem_set[dev]) {
+    UA_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+    if (dev < 64) smem_set[dev] = 1;
+  }
+  dim3 grid(p.n_tiles * heads, batch, 1);
+  attn_fwd_kernel<FEW><<<grid, FWD_THREADS, smem_bytes, stream>>>(p);
+  UA_CUDA(cudaGetLastError());
+  return 0;
+}
+
+static int set_trace(FwdParams& p) {
+  int dev = 0;
+  UA_CUDA(cudaGetDevice(&dev));
+  const TraceSlot ts = dev < 64 ? trace_registry()[0 * 64 + dev] : TraceSlot{nullptr, 0};
+  p.trace.buf = ts.buf;
+  p.trace.cap = ts.cap;
+  return 0;
+}
 
 // rows / segs / tiles are device pointers (prepared once per plan); q/k/v/out tables are host
 // arrays of n_q / n_kv / n_out entries.
@@ -667,35 +771,170 @@ extern "C" int ua_attn_fwd(const UaTensorSrc* q_src, int n_q, const UaTensorSrc*
   p.stage.flags = stage_flags;
   p.stage.epoch = stage_epoch;
   p.stage.ticket = stage_ticket;
-  {
-    int tdev = 0;
-    UA_CUDA(cudaGetDevice(&tdev));
-    const TraceSlot ts = tdev < 64 ? trace_registry()[0 * 64 + tdev] : TraceSlot{nullptr, 0};
-    p.trace.buf = ts.buf;
-    p.trace.cap = ts.cap;
-  }
+  if (set_trace(p)) return -1;
   if (n_copy_tasks > 0) {
     if (stage_ticket == nullptr) UA_FAIL("ua_attn_fwd: copy tasks need a ticket counter");
     UA_CUDA(cudaMemsetAsync(stage_ticket, 0, sizeof(unsigned int), stream));
   }
-  const int smem_bytes = sizeof(FwdSmem) + 1024;
-  int dev = 0;
-  UA_CUDA(cudaGetDevice(&dev));
-  // UA_FWD_TPR = 1 / 2: softmax threads per query row (see the top of this file)
-  const char* env = getenv("UA_FWD_TPR");
-  const int tpr = (env != nullptr && atoi(env) == 2) ? 2 : 1;
-  if (dev < 64 && !g_fwd_smem_set[tpr - 1][dev]) {
-    if (tpr == 2)
-      UA_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    else
-      UA_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    g_fwd_smem_set[tpr - 1][dev] = 1;
+  p.n_split = 1;
+  return launch_fwd<false>(p, n_heads, batch, stream);
+}
+
+// ---- dense launches -------------------------------------------------------------------------------
+namespace ua {
+
+// Rates of the estimate below, measured on a B200 (us, bytes per us).
+constexpr int FEW_MIN_KEY_TILES = 4;
+constexpr int MAX_SPLIT = 64;
+constexpr double TILE_US = 1.9;               // one 128-key tile of a 256-row CTA
+constexpr double CTA_US = 6.0;                // start, first loads, epilogue
+constexpr double FEW_TILE_US = 0.75;          // one 128-key tile of a FEW CTA that has the memory to itself
+constexpr double FEW_BYTES_PER_US = 6.5e6;
+constexpr double COMBINE_US = 3.0;
+constexpr double COMBINE_BYTES_PER_US = 3.0e6;
+
+struct DensePlan {
+  bool few;
+  int pack_shift;
+  int heads;       // head indices of the grid: query heads, or key/value heads when packed
+  int q_tiles;
+  int n_split;
+  int n_parts;     // partial results per row (0: written directly)
+};
+
+// How a dense problem is cut into CTAs. Rows first (query heads of a group packed when their number
+// is a power of two: at 1000 tokens, 32 / 8 heads, a tile then spans 64 tokens instead of 256 and wastes
+// less under the diagonal); then, if those leave SMs idle or the last wave nearly empty, the keys.
+// The estimate of one choice: CTAs of equal cost run in whole waves, unequal ones (causal, heaviest
+// first) fill up to about half a CTA of tail, whichever is shorter; plus what the extra fp32 parts
+// cost to write and merge.
+// Measured (us, unpacked and unsplit -> as planned here): 16 sequences, 1 query behind 8123 keys, 32 / 8
+// heads 528 -> 107 (cold L2; 82 is the time of the bytes); 1 sequence behind 8192 keys 138 -> 26; 512 queries
+// behind 32768 keys, 32 / 8 heads, 520 -> 292; 8192 causal tokens, 32 / 8 heads, 589 -> 517 (packing alone).
+// On the other side of the line: 1000 causal tokens, 32 / 8 heads, run 32 unsplit and 62 split in two.
+static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_heads, int causal, int n_split, int sms) {
+  DensePlan d{};
+  const int group = n_heads / n_kv_heads;
+  int sh = 0;
+  while ((1 << sh) < group) ++sh;
+  if ((1 << sh) != group || group > ATTN_TILE) sh = 0;
+  d.pack_shift = sh;
+  d.heads = sh > 0 ? n_kv_heads : n_heads;
+  const long rows = static_cast<long>(sq) << sh;
+  const int key_tiles = (skv + ATTN_TILE - 1) / ATTN_TILE;
+  d.few = rows <= ATTN_TILE && key_tiles >= FEW_MIN_KEY_TILES;
+  const int cta_rows = d.few ? ATTN_TILE : 2 * ATTN_TILE;
+  d.q_tiles = static_cast<int>((rows + cta_rows - 1) / cta_rows);
+  // key tiles of the heaviest tile and of all tiles together
+  double total = 0;
+  const AttnSeg sg{0, 0, skv, causal ? SEG_UPPER : 0, skv - sq, 0, 0, 0};
+  if (causal && d.q_tiles > 1) {
+    for (int t = 0; t < d.q_tiles; ++t) {
+      const long last = ((static_cast<long>(t) + 1) * cta_rows < rows ? (static_cast<long>(t) + 1) * cta_rows : rows) - 1;
+      total += seg_tiles(sg, 0, static_cast<int>(last >> sh)).end;
+    }
+  } else {
+    total = static_cast<double>(key_tiles) * d.q_tiles;
   }
-  dim3 grid(n_tiles * n_heads, batch, 1);
-  if (tpr == 2)
-    attn_fwd_kernel<2><<<grid, FwdCfg<2>::THREADS, smem_bytes, stream>>>(p);
-  else
-    attn_fwd_kernel<1><<<grid, FwdCfg<1>::THREADS, smem_bytes, stream>>>(p);
-  UA_CUDA(cudaGetLastError());
+  const double per_head = static_cast<double>(d.heads) * batch;
+  total *= per_head;
+  const double base = d.q_tiles * per_head;
+  double best = 0;
+  int best_z = 1;
+  const int max_z = n_split > 0 ? 1 : (key_tiles < MAX_SPLIT ? key_tiles : MAX_SPLIT);
+  for (int z = 1; z <= max_z; ++z) {
+    const double ctas = base * z;
+    const double active = ctas < sms ? ctas : sms;
+    double tile_us = TILE_US;
+    if (d.few) {
+      const double mem_us = active * (2.0 * FWD_TILE_BYTES) / FEW_BYTES_PER_US;
+      tile_us = mem_us > FEW_TILE_US ? mem_us : FEW_TILE_US;
+    }
+    const double heavy = CTA_US + (static_cast<double>(key_tiles) / z) * tile_us;
+    const double waves = static_cast<double>(static_cast<long>((ctas + sms - 1) / sms)) * heavy;
+    const double filled = (ctas * CTA_US + total * tile_us) / sms + 0.5 * heavy;
+    double us = ctas <= sms ? heavy : (waves < filled ? waves : filled);
+    const int parts = d.few ? 2 * z : (z > 1 ? z : 0);
+    if (parts > 0)
+      us += COMBINE_US + static_cast<double>(parts) * batch * sq * n_heads * (2.0 * ATTN_D * 4) / COMBINE_BYTES_PER_US;
+    if (z == 1 || us < best) {
+      best = us;
+      best_z = z;
+    }
+  }
+  d.n_split = n_split > 0 ? (n_split < key_tiles ? n_split : key_tiles) : best_z;
+  d.n_parts = d.few ? 2 * d.n_split : (d.n_split > 1 ? d.n_split : 0);
+  return d;
+}
+
+static int sm_count() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if (dev < 64 && cached[dev] > 0) return cached[dev];
+  int n = 148;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  if (dev < 64) cached[dev] = n;
+  return n;
+}
+
+}  // namespace ua
+
+// Partial results per (batch, token, head) that ua_attn_fwd_dense needs room for: the caller's
+// workspace holds n * batch * sq * n_heads rows of 129 floats. n_split = 0 leaves the choice here.
+extern "C" int ua_attn_fwd_dense_parts(int batch, int sq, int skv, int n_heads, int n_kv_heads, int causal, int n_split) {
+  if (batch <= 0 || sq <= 0 || skv <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return 0;
+  return plan_dense(batch, sq, skv, n_heads, n_kv_heads, causal, n_split, sm_count()).n_parts;
+}
+
+// All queries of `q` against all keys: O and lse of softmax(scale Q K^T) V; causal: key c is visible
+// to query r iff c <= r + skv - sq.
+extern "C" int ua_attn_fwd_dense(const UaTensorSrc* q, const UaTensorSrc* k, const UaTensorSrc* v, const UaOutDst* out,
+                                 int causal, float softmax_scale, int n_split, float* workspace, int* status,
+                                 cudaStream_t stream) {
+  const int batch = static_cast<int>(q->batch), sq = static_cast<int>(q->tokens), skv = static_cast<int>(k->tokens);
+  const int n_heads = static_cast<int>(q->heads), n_kv_heads = static_cast<int>(k->heads);
+  if (sq <= 0 || batch <= 0) return 0;
+  if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0)
+    UA_FAIL("ua_attn_fwd_dense: %d query heads do not divide into %d key/value heads", n_heads, n_kv_heads);
+  const DensePlan d = plan_dense(batch, sq, skv, n_heads, n_kv_heads, causal, n_split, sm_count());
+  if (d.n_parts > 0 && workspace == nullptr) UA_FAIL("ua_attn_fwd_dense: a split launch needs a workspace");
+  FwdParams p;
+  memset(&p, 0, sizeof(p));
+  if (encode_src(&p.tmQ[0], *q, 1u << d.pack_shift)) return -1;
+  if (encode_src(&p.tmK[0], *k) || encode_src(&p.tmV[0], *v)) return -1;
+  p.o_ptr[0] = static_cast<__nv_bfloat16*>(out->o_ptr);
+  p.lse_ptr[0] = out->lse_ptr;
+  p.o_row_stride[0] = out->o_row_stride;
+  p.o_batch_stride[0] = out->o_batch_stride;
+  p.lse_head_stride[0] = out->lse_head_stride;
+  p.lse_batch_stride[0] = out->lse_batch_stride;
+  p.dense_row.q_len = sq;
+  p.dense_row.seg_end = 1;
+  p.dense_seg.len = skv;
+  p.dense_seg.causal = causal ? SEG_UPPER : 0;
+  p.dense_seg.diag = skv - sq;
+  p.pack_shift = d.pack_shift;
+  p.n_split = d.n_split;
+  p.n_tiles = d.q_tiles * d.n_split;
+  p.n_heads = n_heads;
+  p.kv_group = n_heads / n_kv_heads;
+  p.scale_log2 = softmax_scale * 1.4426950408889634f;
+  p.status = status;
+  p.stage.epoch = 1;
+  const long n_rows = static_cast<long>(batch) * sq * n_heads;
+  if (d.n_parts > 0) {
+    p.n_parts = d.n_parts;
+    p.part_o = workspace;
+    p.part_lse = workspace + static_cast<long>(d.n_parts) * n_rows * ATTN_D;
+  }
+  if (set_trace(p)) return -1;
+  if (d.few ? launch_fwd<true>(p, d.heads, batch, stream) : launch_fwd<false>(p, d.heads, batch, stream)) return -1;
+  if (d.n_parts > 0) {
+    combine_kernel<<<static_cast<unsigned>((n_rows + 7) / 8), 256, 0, stream>>>(
+        p.part_o, p.part_lse, d.n_parts, sq, n_heads, p.o_ptr[0], p.o_row_stride[0], p.o_batch_stride[0], p.lse_ptr[0],
+        p.lse_head_stride[0], p.lse_batch_stride[0], n_rows);
+    UA_CUDA(cudaGetLastError());
+  }
   return 0;
 }

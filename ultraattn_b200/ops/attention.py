@@ -349,6 +349,34 @@ def attn_fwd_cuda(q_srcs: Sequence[torch.Tensor], k_srcs: Sequence[torch.Tensor]
     _lib.check(rc, "ua_attn_fwd")
 
 
+def attn_fwd_dense(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tuple[torch.Tensor, torch.Tensor],
+                   causal: bool, softmax_scale: float | None = None, n_split: int = 0) -> None:
+    """All queries against all keys, written into ``out = (O, lse)``; ``causal``: key c is visible to
+    query r iff ``c <= r + Skv - Sq``. On CUDA the launch needs no tables; the library packs the query
+    heads of a group into a tile's rows and splits the keys over several CTAs (``n_split`` of them; 0:
+    its own choice) where the rows alone would leave SMs idle."""
+    B, sq, H, D = q.shape
+    skv = k.shape[1]
+    if not q.is_cuda or debug_bounds_enabled():
+        rows = [Row(0, 0, sq, (Seg(0, 0, skv, bool(causal), skv - sq),), 0, 0, False)]
+        if debug_bounds_enabled():
+            _raise_if_bad("forward", check_fwd_tables(rows, [q], [k], [v], [out]))
+        if not q.is_cuda:
+            return attn_fwd_reference([q], [k], [v], [out], rows, softmax_scale)
+    lib = _lib.load()
+    o, lse = out
+    assert o.dtype == torch.bfloat16 and lse.dtype == torch.float32 and o.stride(3) == 1
+    assert o.stride(2) == 128 and lse.stride(2) == 1
+    scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
+    parts = lib.ua_attn_fwd_dense_parts(B, sq, skv, H, k.shape[2], int(causal), n_split)
+    ws = torch.empty(parts * B * sq * H * 129, dtype=torch.float32, device=q.device) if parts else None
+    dst = _lib.UaOutDst(o.data_ptr(), lse.data_ptr(), o.stride(1), o.stride(0), lse.stride(1), lse.stride(0))
+    rc = lib.ua_attn_fwd_dense(_src_struct(q), _src_struct(k), _src_struct(v), dst, int(causal), scale, n_split,
+                               ws.data_ptr() if parts else None, status_buffer(q.device).data_ptr(),
+                               torch.cuda.current_stream(q.device).cuda_stream)
+    _lib.check(rc, "ua_attn_fwd_dense")
+
+
 def _stage_args(stage):
     if stage is None:
         return (None, 0, 0, None, 1, None)
@@ -526,7 +554,9 @@ class BwdKvOut:
 
 
 def attn_bwd_cuda(q_sides: Sequence[BwdQSide], k_srcs, v_srcs, kv_outs: Sequence[BwdKvOut],
-                  plan: BwdPlan, softmax_scale: float | None = None, stage=None) -> None:
+                  plan: BwdPlan | None, softmax_scale: float | None = None, stage=None, dense: int = 0) -> None:
+    """``dense`` = 1 / 2: no plan; all queries of the one source against all its keys, without a mask /
+    causal (see :func:`attn_bwd_dense`)."""
     lib = _lib.load()
     q0 = q_sides[0].q
     n_heads = q0.shape[2]
@@ -552,9 +582,9 @@ def attn_bwd_cuda(q_sides: Sequence[BwdQSide], k_srcs, v_srcs, kv_outs: Sequence
                                   int(o.add_f32), 0))
     kos = (_lib.UaBwdKvOut * len(ko))(*ko)
     st = status_buffer(q0.device)
-    rc = lib.ua_attn_bwd(qs, dos, sides, nq, ks, vs, len(k_srcs), kos, len(ko),
-                         plan.cols_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(),
-                         plan.n_tiles, n_heads, n_kv_heads, q0.shape[0], scale, st.data_ptr(),
+    tables = (None, None, None, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(),
+                                                  plan.tiles_t.data_ptr(), plan.n_tiles)
+    rc = lib.ua_attn_bwd(qs, dos, sides, nq, ks, vs, len(k_srcs), kos, len(ko), *tables, dense, n_heads, n_kv_heads, q0.shape[0], scale, st.data_ptr(),
                          *_stage_args(stage),
                          torch.cuda.current_stream(q0.device).cuda_stream)
     _lib.check(rc, "ua_attn_bwd")
@@ -612,6 +642,18 @@ def attn_bwd(q_sides, k_srcs, v_srcs, kv_outs, plan: BwdPlan, softmax_scale=None
         attn_bwd_cuda(q_sides, k_srcs, v_srcs, kv_outs, plan, softmax_scale, stage)
     else:
         attn_bwd_reference(q_sides, k_srcs, v_srcs, kv_outs, plan.cols, softmax_scale)
+
+
+def attn_bwd_dense(q_side: BwdQSide, k, v, kv_out: BwdKvOut, causal: bool, softmax_scale=None) -> None:
+    """The backward of :func:`attn_fwd_dense`; on CUDA without tables."""
+    sq, skv = q_side.q.shape[1], k.shape[1]
+    if not q_side.q.is_cuda or debug_bounds_enabled():
+        cols = [Col(0, 0, skv, (Seg(0, 0, sq, bool(causal), skv - sq),), 0, 0)]
+        if debug_bounds_enabled():
+            _raise_if_bad("backward", check_bwd_tables(cols, [q_side], [k], [v], [kv_out]))
+        if not q_side.q.is_cuda:
+            return attn_bwd_reference([q_side], [k], [v], [kv_out], cols, softmax_scale)
+    attn_bwd_cuda([q_side], [k], [v], [kv_out], None, softmax_scale, None, 2 if causal else 1)
 
 
 def cols_from_block_table(table: np.ndarray, block: int, kv_block: int | None = None) -> list[Col]:

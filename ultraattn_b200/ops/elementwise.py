@@ -65,6 +65,22 @@ def rowdot(o: torch.Tensor, d_o: torch.Tensor, out: torch.Tensor | None = None) 
     return out
 
 
+def bwd_prepare(o: torch.Tensor, d_o: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """(D, dq) of a backward over ``[batch, tokens, heads, head_dim]``: D = rowdot(O, dO) ``[batch, heads,
+    tokens]`` fp32 and a zeroed fp32 dQ accumulator, in one launch."""
+    B, S, H, D = o.shape
+    dvec = torch.empty(B, H, S, dtype=torch.float32, device=o.device)
+    if not o.is_cuda:
+        for b in range(B):
+            rowdot(o[b], d_o[b], dvec[b])
+        return dvec, torch.zeros(B, S, H, D, dtype=torch.float32, device=o.device)
+    dq = torch.empty(B, S, H, D, dtype=torch.float32, device=o.device)
+    rc = _lib.load().ua_bwd_prepare(o.data_ptr(), d_o.data_ptr(), dvec.data_ptr(), dq.data_ptr(), o.stride(0),
+                                    o.stride(1), d_o.stride(0), d_o.stride(1), B, S, H, _stream(o))
+    _lib.check(rc, "ua_bwd_prepare")
+    return dvec, dq
+
+
 def cast_scale(src: torch.Tensor, dst: torch.Tensor, scale: float = 1.0, accumulate: bool = False):
     """dst(bf16) (+)= scale * src(fp32); both contiguous."""
     if not src.is_cuda:

@@ -56,19 +56,22 @@ def _forward(q, k, v, rows, out, softmax_scale):
     return o, lse
 
 
-def _backward(dout, q, k, v, out, lse, dq, dk, dv, cols, softmax_scale, softmax_d):
+def _backward(dout, q, k, v, out, lse, dq, dk, dv, cols, softmax_scale, softmax_d, causal=False):
+    """``cols``: the work items of a packed batch, or None: all queries against all keys (``causal``)."""
     B, S, H, D = q.shape
     if softmax_d is None:
-        softmax_d = torch.empty(B, H, S, dtype=torch.float32, device=q.device)
-        for b in range(B):
-            E.rowdot(out[b], dout[b], softmax_d[b])
-    dq32 = torch.zeros(B, S, H, D, dtype=torch.float32, device=q.device)
+        softmax_d, dq32 = E.bwd_prepare(out, dout)
+    else:
+        dq32 = torch.zeros(B, S, H, D, dtype=torch.float32, device=q.device)
     if q.is_cuda:
         dkv = A.BwdKvOut(dk, dv)                   # bf16 destinations are written directly
     else:
         dkv = A.BwdKvOut(torch.zeros(k.shape, dtype=torch.float32), torch.zeros(v.shape, dtype=torch.float32))
-    A.attn_bwd([A.BwdQSide(q, dout.contiguous(), lse, softmax_d.float(), dq32)], [k], [v], [dkv],
-               A.BwdPlan(cols, q.device), softmax_scale)
+    side = A.BwdQSide(q, dout.contiguous(), lse, softmax_d.float(), dq32)
+    if cols is None:
+        A.attn_bwd_dense(side, k, v, dkv, causal, softmax_scale)
+    else:
+        A.attn_bwd([side], [k], [v], [dkv], A.BwdPlan(cols, q.device), softmax_scale)
     if q.is_cuda:
         E.cast_scale(dq32, dq)
     else:
@@ -87,8 +90,9 @@ def _flash_attn_forward(q, k, v, dropout_p, softmax_scale, causal, window_size=(
     if _windowed(window_size):
         o, lse = W.window_forward(q, k, v, window_size, bool(causal), _scale(q, softmax_scale), out)
         return o, q, k, v, o, lse, None, None
-    rows = [A.Row(0, 0, sq, (A.Seg(0, 0, skv, bool(causal), skv - sq),), 0, 0, False)]
-    o, lse = _forward(q, k, v, rows, out, _scale(q, softmax_scale))
+    o = out if out is not None else torch.empty_like(q)
+    lse = torch.empty(q.shape[0], q.shape[2], sq, dtype=torch.float32, device=q.device)
+    A.attn_fwd_dense(q, k, v, (o, lse), bool(causal), _scale(q, softmax_scale))
     return o, q, k, v, o, lse, None, None
 
 
@@ -109,8 +113,7 @@ def _flash_attn_backward(dout, q, k, v, out, softmax_lse, dq, dk, dv, dropout_p,
         for dst, src in zip((dq, dk, dv), g):
             dst.copy_(src)
         return dq, dk, dv, softmax_d
-    cols = [A.Col(0, 0, skv, (A.Seg(0, 0, sq, bool(causal), skv - sq),), 0, 0)]
-    d = _backward(dout, q, k, v, out, softmax_lse, dq, dk, dv, cols, _scale(q, softmax_scale), softmax_d)
+    d = _backward(dout, q, k, v, out, softmax_lse, dq, dk, dv, None, _scale(q, softmax_scale), softmax_d, bool(causal))
     return dq, dk, dv, d
 
 

@@ -267,10 +267,9 @@ def _cuda_forward(q, k, v, out, fplan, full: bool, scale):
     return o, lse
 
 
-def _cuda_backward(d_o, q, k, v, lse, softmax_d, bplan, sink_idx, full: bool, scale):
-    """One launch: fp32 dQ accumulator, dK / dV written in the inputs' type by their only producer (the
+def _cuda_backward(d_o, q, k, v, lse, softmax_d, dq32, bplan, sink_idx, full: bool, scale):
+    """One launch: fp32 dQ accumulator (zeroed ``dq32``), dK / dV written in the inputs' type by their only producer (the
     sink keys', which have several, go through a small fp32 buffer)."""
-    dq32 = torch.zeros(q.shape, dtype=torch.float32, device=q.device)
     new = torch.empty_like if full else torch.zeros_like
     dk, dv = new(k), new(v)
     outs = [A.BwdKvOut(dk, dv)]
@@ -397,20 +396,21 @@ def window_backward(d_o, q, k, v, o, lse, window_size, causal: bool = False,
     B, S, H, D = q.shape
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     q, k, v, d_o = q.contiguous(), k.contiguous(), v.contiguous(), d_o.contiguous()
+    dq32 = None
     if softmax_d is None:
-        softmax_d = torch.empty(B, H, S, dtype=torch.float32, device=q.device)
-        for b in range(B):
-            E.rowdot(o[b], d_o[b], softmax_d[b])
+        softmax_d, dq32 = E.bwd_prepare(o, d_o)
+    elif q.is_cuda:
+        dq32 = torch.zeros(q.shape, dtype=torch.float32, device=q.device)
     lse = lse.float().contiguous()
     softmax_d = softmax_d.float().contiguous()
     f32 = lambda t: torch.zeros(t.shape, dtype=torch.float32, device=t.device)
     whole = _whole_sequence_plans(S, k.shape[1], window_size, causal, q.device, cu_seqlens, q_offset)
     if q.is_cuda:
         if whole is not None:
-            return _cuda_backward(d_o, q, k, v, lse, softmax_d, whole[1], None, _covers(_seq_bounds(cu_seqlens, S), S), scale)
+            return _cuda_backward(d_o, q, k, v, lse, softmax_d, dq32, whole[1], None, _covers(_seq_bounds(cu_seqlens, S), S), scale)
         _, bplan, idx, full = _pick_band_plans(S, k.shape[1], window_size, causal, q.device, cu_seqlens, sink_tokens,
                                                q_offset)
-        return _cuda_backward(d_o, q, k, v, lse, softmax_d, bplan, idx, full, scale)
+        return _cuda_backward(d_o, q, k, v, lse, softmax_d, dq32, bplan, idx, full, scale)
     if whole is not None:
         dq32, kv = f32(q), A.BwdKvOut(f32(k), f32(v))
         A.attn_bwd([A.BwdQSide(q, d_o, lse, softmax_d, dq32)], [k], [v], [kv], whole[1], scale)
