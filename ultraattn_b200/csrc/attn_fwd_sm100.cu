@@ -40,9 +40,9 @@ constexpr int FWD_TMA_WARP = 8;
 constexpr int FWD_MMA_WARP = 9;
 // three warpgroups (the last one: TMA, MMA and two idle warps), so that the register file can be
 // re-balanced by warpgroup: a softmax thread holds its row's 128 scores besides everything else and
-// spilled at the 168 registers an even split leaves; 2 x 216 + 64 <= 3 x 168
+// spills at the 168 registers an even split leaves; 2 x 200 + 104 <= 3 x 168
 constexpr int FWD_THREADS = 384;
-constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 64, FWD_REGS_SOFTMAX = 216;
+constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 104, FWD_REGS_SOFTMAX = 200;
 static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
 #ifndef UA_FWD_POLY_EXP_PERIOD
 #define UA_FWD_POLY_EXP_PERIOD 0
@@ -89,8 +89,21 @@ struct FwdParams {
   float* part_o;       // not null: fp32 partial results [batch, parts, tokens, heads, 128] ...
   float* part_lse;     // ... and [batch, parts, tokens, heads]; parts = n_split (x 2 if FEW)
   int n_parts;
+  int persist;         // CTAs take over further items (0: one item per CTA)
   StageParams stage;   // optional in-kernel staging of remote K/V (and Q) blocks
   KernelTrace trace;   // optional per-CTA time stamps
+};
+
+// One work item of a launch: what a CTA of a grid without cancellation would have been.
+struct FwdItem {
+  FwdRow row;
+  int row_idx;
+  int batch, split;
+  int q_head, kv_head;       // query head of packed row 0, key/value head
+  int r0, rows_here;         // first (packed) row inside the block row, valid rows
+  int tok0, tok_last;        // their query tokens
+  int linear;                // index in the grid (time stamps)
+  int exists;                // 0: there is no further item
 };
 
 template <bool FEW>
@@ -106,7 +119,13 @@ struct __align__(1024) FwdSmem {
   uint64_t v_empty[STAGES];
   uint64_t s_full[2];
   uint64_t p_full[2];
+  uint64_t q_empty;
   uint64_t o_full;
+  uint4 clc;             // response of a cancellation request
+  uint64_t clc_full;
+  FwdItem item[2];       // item number n in slot n & 1
+  uint64_t item_full[2];
+  uint64_t item_empty[2];
   uint32_t tmem_base;
   int abort_flag;
   int stage_slot;
@@ -143,6 +162,62 @@ constexpr int FWD_PROF_TILE = 8;
 
 
 template <bool FEW>
+__device__ __forceinline__ FwdItem fwd_item(const FwdParams& p, int bx, int by) {
+  FwdItem it;
+  constexpr int CTA_ROWS = FEW ? ATTN_TILE : 2 * ATTN_TILE;
+  const bool dense = p.rows == nullptr;
+  // (packed launches: `head` is the key/value head and stands for all its query heads)
+  const int head = bx / p.n_tiles;
+  const int i = bx % p.n_tiles;
+  // dense tiles run from the last rows to the first: under a causal mask the heaviest ones come first
+  const int2 tl = dense ? make_int2(0, (p.n_tiles - 1 - i) / p.n_split) : p.tiles[i];
+  it.split = dense ? (p.n_tiles - 1 - i) % p.n_split : 0;
+  it.batch = by;
+  it.row = dense ? p.dense_row : p.rows[tl.x];
+  it.row_idx = tl.x;
+  it.q_head = head << p.pack_shift;
+  it.kv_head = it.q_head / p.kv_group;
+  it.r0 = tl.y * CTA_ROWS;
+  it.rows_here = min(CTA_ROWS, (it.row.q_len << p.pack_shift) - it.r0);
+  it.tok0 = it.r0 >> p.pack_shift;
+  it.tok_last = (it.r0 + it.rows_here - 1) >> p.pack_shift;
+  it.linear = by * gridDim.x + bx;
+  it.exists = 1;
+  return it;
+}
+__device__ __forceinline__ AttnSeg fwd_seg(const FwdParams& p, int e) {
+  return p.rows == nullptr ? p.dense_seg : p.segs[e];
+}
+// key tiles of a segment that the item visits: all of them, or its share of a split launch
+__device__ __forceinline__ TileRange fwd_tiles(const FwdParams& p, const FwdItem& it, const AttnSeg& sg) {
+  TileRange tr = seg_tiles(sg, it.tok0, it.tok_last);
+  if (p.n_split > 1) {
+    const int n = tr.end - tr.first, base = tr.first;
+    tr.first = base + static_cast<int>(static_cast<long>(n) * it.split / p.n_split);
+    tr.end = base + static_cast<int>(static_cast<long>(n) * (it.split + 1) / p.n_split);
+  }
+  return tr;
+}
+__device__ __forceinline__ int fwd_total(const FwdParams& p, const FwdItem& it) {
+  int n = 0;
+  for (int e = it.row.seg_begin; e < it.row.seg_end; ++e) {
+    const TileRange tr = fwd_tiles(p, it, fwd_seg(p, e));
+    n += tr.end - tr.first;
+  }
+  return n;
+}
+
+// Persistent CTAs: the grid has one CTA per work item, and a CTA that is done with an item cancels one
+// that has not started yet and takes its place (cluster launch control), so that the hardware's own
+// dispatch order stays the schedule. The TMA warp runs ahead: it takes over the next item as soon as
+// the loads of this one are issued, its Q and first K / V tiles arrive while the softmax warps write
+// this item's output, and the MMA warp issues its first scores. TMEM, barriers and descriptors are
+// set up once. One item per CTA -> this (B200, us): 64
+// sequences of 512 keys, one query, 32 heads 184 -> 143; 12 documents in 16k tokens 599 -> 546; window
+// 4096 in 16k tokens 1140 -> 1090; 4 x 2000 tokens 192 -> 182; causal 8k 609 -> 588, 16k 2010 -> 1978.
+// Launches that stage peers' blocks run one item per CTA (p.persist = 0): their CTAs must be able to
+// wait for each other's copies.
+template <bool FEW>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ FwdParams p) {
   constexpr int STAGES = FwdSmem<FEW>::STAGES;
@@ -151,52 +226,27 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const int psh = p.pack_shift;
 
-  // (packed launches: `head` is the key/value head and stands for all its query heads)
-  const bool dense = p.rows == nullptr;
-  const int head = blockIdx.x / p.n_tiles;
-  const int item = blockIdx.x % p.n_tiles;
-  // dense tiles run from the last rows to the first: under a causal mask the heaviest ones come first
-  const int2 tl = dense ? make_int2(0, (p.n_tiles - 1 - item) / p.n_split) : p.tiles[item];
-  const int split = dense ? (p.n_tiles - 1 - item) % p.n_split : 0;
-  const int batch = blockIdx.y;
-  const FwdRow row = dense ? p.dense_row : p.rows[tl.x];
-  auto seg_at = [&](int e) { return dense ? p.dense_seg : p.segs[e]; };
-  const int cta_linear = blockIdx.y * gridDim.x + blockIdx.x;
-  trace_stamp(p.trace, cta_linear, 0);
-  trace_ident(p.trace, cta_linear, tl.x);
+  const FwdItem item0 = fwd_item<FEW>(p, blockIdx.x, blockIdx.y);
+  trace_stamp(p.trace, item0.linear, 0);
   {
     // does this CTA read a staged block? then it first helps to empty the copy queue
-    bool waits = row.q_wait_flag != 0;
-    for (int e = row.seg_begin; e < row.seg_end && !waits; ++e) waits = seg_at(e).wait_flag != 0;
-    drain_stage_queue(p.stage, waits, cta_linear, &s.stage_slot);
+    bool waits = item0.row.q_wait_flag != 0;
+    for (int e = item0.row.seg_begin; e < item0.row.seg_end && !waits; ++e) waits = fwd_seg(p, e).wait_flag != 0;
+    drain_stage_queue(p.stage, waits, item0.linear, &s.stage_slot);
   }
-  trace_stamp(p.trace, cta_linear, 1);
-  constexpr int CTA_ROWS = FEW ? ATTN_TILE : 2 * ATTN_TILE;
-  const int psh = p.pack_shift;
-  const int r0 = tl.y * CTA_ROWS;                               // block-relative first (packed) row
-  const int rows_here = min(CTA_ROWS, (row.q_len << psh) - r0); // valid rows of this CTA
-  const int tok0 = r0 >> psh, tok_last = (r0 + rows_here - 1) >> psh;
-  const int q_head = head << psh;                               // query head of packed row 0
-  const int kv_head = q_head / p.kv_group;
-  // key tiles of segment e that this CTA visits: all of them, or its share of a split launch
-  auto cta_tiles = [&](const AttnSeg& sg) {
-    TileRange tr = seg_tiles(sg, tok0, tok_last);
-    if (p.n_split > 1) {
-      const int n = tr.end - tr.first, base = tr.first;
-      tr.first = base + static_cast<int>(static_cast<long>(n) * split / p.n_split);
-      tr.end = base + static_cast<int>(static_cast<long>(n) * (split + 1) / p.n_split);
-    }
-    return tr;
-  };
-  // FEW: warps without a valid row have nothing to do (their scores are never read back)
-  const int act_warps = FEW ? (rows_here + 31) / 32 : 4;
+  // FEW: warps without a valid row have nothing to do (their scores are never read back). The
+  // launch has one row tile, so the number is the same for all its items.
+  const int act_warps = FEW ? (item0.rows_here + 31) / 32 : 4;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.s_full[i], 1);
       mbar_init(&s.p_full[i], act_warps);   // one arrival per softmax warp
+      mbar_init(&s.item_full[i], 1);
+      mbar_init(&s.item_empty[i], 1 + 2 * act_warps);   // MMA warp and softmax warps
     }
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&s.k_full[i], 1);
@@ -204,7 +254,10 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       mbar_init(&s.v_full[i], 1);
       mbar_init(&s.v_empty[i], 1);
     }
+    mbar_init(&s.q_empty, 1);
+    mbar_init(&s.clc_full, 1);
     mbar_init(&s.o_full, 1);
+    s.item[0] = item0;
     s.abort_flag = 0;
     fence_mbar_init();
   }
@@ -218,60 +271,89 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
   const uint32_t tmem_base = s.tmem_base;
   WaitCtx wc{&s.abort_flag, p.status, 4000000000ull};
 
-  // total number of key tiles this CTA visits (identical in every role)
-  int n_total = 0;
-  for (int e = row.seg_begin; e < row.seg_end; ++e) {
-    const TileRange tr = cta_tiles(seg_at(e));
-    n_total += tr.end - tr.first;
-  }
+  // Consumers: done with item n; true once item n + 1 is in its slot (false: there is none, or a wait
+  // gave up). One thread calls it.
+  auto next_item = [&](uint32_t n) -> bool {
+    if (!p.persist) return false;
+    mbar_arrive(&s.item_empty[n & 1]);
+    const uint32_t m = n + 1;
+    if (!mbar_wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, wc, 120)) return false;
+    return s.item[m & 1].exists != 0;
+  };
 
   if (warp >= FWD_SOFTMAX_WARPS) {
   reg_dealloc<FWD_REGS_LOAD>();
   if (warp == FWD_TMA_WARP) {
-    // =============================== TMA producer ===========================================
-    if (lane == 0 && n_total > 0) {
-      const CUtensorMap* tq = &p.tmQ[row.q_src];
-      tma_prefetch_desc(tq);
+    // =============================== TMA producer and scheduler ==============================
+    if (lane == 0) {
       bool ok = true;
-      if (!wait_staged(p.stage.flags, row.q_wait_flag, row.q_wait_count * p.stage.epoch, wc.budget_ns)) {
-        report_error(wc, UA_ERR_FLAG_TIMEOUT, 110, row.q_wait_flag);
-        ok = false;
-      }
-      for (int w = 0; w < (FEW ? 1 : 2) && ok; ++w) {
-        mbar_arrive_expect_tx(&s.q_full[w], FWD_TILE_BYTES);
-        const int qrow = row.q_start + tok0 + ((w * ATTN_TILE) >> psh);
-        tma_load_4d(s.q[w], tq, &s.q_full[w], 0, q_head, qrow, batch);
-        tma_load_4d(s.q[w] + 16384, tq, &s.q_full[w], 64, q_head, qrow, batch);
-      }
-      uint32_t j = 0;
-      for (int e = row.seg_begin; e < row.seg_end && ok; ++e) {
-        const AttnSeg sg = seg_at(e);
-        const TileRange tr = cta_tiles(sg);
-        const CUtensorMap* tk = &p.tmK[sg.src];
-        const CUtensorMap* tv = &p.tmV[sg.src];
-        if (tr.first < tr.end && !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
-          report_error(wc, UA_ERR_FLAG_TIMEOUT, 111, sg.wait_flag);
-          ok = false;
-          break;
+      FwdItem it = item0;
+      uint32_t j = 0;          // K / V tiles loaded so far
+      uint32_t live = 0;       // items with keys so far
+      for (uint32_t n = 0; ok; ++n) {
+        if (fwd_total(p, it) > 0) {
+          const CUtensorMap* tq = &p.tmQ[it.row.q_src];
+          tma_prefetch_desc(tq);
+          if (!wait_staged(p.stage.flags, it.row.q_wait_flag, it.row.q_wait_count * p.stage.epoch, wc.budget_ns)) {
+            report_error(wc, UA_ERR_FLAG_TIMEOUT, 110, it.row.q_wait_flag);
+            ok = false;
+          }
+          // the previous item's last scores have been computed
+          if (ok && live > 0 && !mbar_wait(&s.q_empty, (live - 1) & 1, wc, 102)) ok = false;
+          for (int w = 0; w < (FEW ? 1 : 2) && ok; ++w) {
+            mbar_arrive_expect_tx(&s.q_full[w], FWD_TILE_BYTES);
+            const int qrow = it.row.q_start + it.tok0 + ((w * ATTN_TILE) >> psh);
+            tma_load_4d(s.q[w], tq, &s.q_full[w], 0, it.q_head, qrow, it.batch);
+            tma_load_4d(s.q[w] + 16384, tq, &s.q_full[w], 64, it.q_head, qrow, it.batch);
+          }
+          ++live;
+          for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
+            const AttnSeg sg = fwd_seg(p, e);
+            const TileRange tr = fwd_tiles(p, it, sg);
+            const CUtensorMap* tk = &p.tmK[sg.src];
+            const CUtensorMap* tv = &p.tmV[sg.src];
+            if (tr.first < tr.end &&
+                !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
+              report_error(wc, UA_ERR_FLAG_TIMEOUT, 111, sg.wait_flag);
+              ok = false;
+              break;
+            }
+            for (int t = tr.first; t < tr.end; ++t, ++j) {
+              const int st = j % STAGES;
+              const uint32_t ph = (j / STAGES) & 1;
+              const int krow = sg.start + t * ATTN_TILE;
+              if (!mbar_wait(&s.k_empty[st], ph ^ 1, wc, 100)) { ok = false; break; }
+              mbar_arrive_expect_tx(&s.k_full[st], FWD_TILE_BYTES);
+              tma_load_4d(s.k[st], tk, &s.k_full[st], 0, it.kv_head, krow, it.batch);
+              tma_load_4d(s.k[st] + 16384, tk, &s.k_full[st], 64, it.kv_head, krow, it.batch);
+              if (!mbar_wait(&s.v_empty[st], ph ^ 1, wc, 101)) { ok = false; break; }
+              mbar_arrive_expect_tx(&s.v_full[st], FWD_TILE_BYTES);
+              tma_load_4d(s.v[st], tv, &s.v_full[st], 0, it.kv_head, krow, it.batch);
+              tma_load_4d(s.v[st] + 16384, tv, &s.v_full[st], 64, it.kv_head, krow, it.batch);
+            }
+          }
         }
-        for (int t = tr.first; t < tr.end; ++t, ++j) {
-          const int st = j % STAGES;
-          const uint32_t ph = (j / STAGES) & 1;
-          const int krow = sg.start + t * ATTN_TILE;
-          if (!mbar_wait(&s.k_empty[st], ph ^ 1, wc, 100)) { ok = false; break; }
-          mbar_arrive_expect_tx(&s.k_full[st], FWD_TILE_BYTES);
-          tma_load_4d(s.k[st], tk, &s.k_full[st], 0, kv_head, krow, batch);
-          tma_load_4d(s.k[st] + 16384, tk, &s.k_full[st], 64, kv_head, krow, batch);
-          if (!mbar_wait(&s.v_empty[st], ph ^ 1, wc, 101)) { ok = false; break; }
-          mbar_arrive_expect_tx(&s.v_full[st], FWD_TILE_BYTES);
-          tma_load_4d(s.v[st], tv, &s.v_full[st], 0, kv_head, krow, batch);
-          tma_load_4d(s.v[st] + 16384, tv, &s.v_full[st], 64, kv_head, krow, batch);
-        }
+        if (!ok || !p.persist) break;
+        // everything of this item is on its way: take over the next one
+        mbar_arrive_expect_tx(&s.clc_full, 16);
+        clc_try_cancel(&s.clc, &s.clc_full);
+        if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
+        int bx, by;
+        const bool got = clc_read(&s.clc, bx, by);
+        fence_proxy_async_smem();               // read before the next response may overwrite it
+        if (got) it = fwd_item<FEW>(p, bx, by);
+        else it.exists = 0;
+        // the slot's previous item (n - 1) is done with
+        const uint32_t slot = (n + 1) & 1;
+        if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
+        s.item[slot] = it;
+        mbar_arrive(&s.item_full[slot]);
+        if (!got) break;
       }
     }
   } else if (warp == FWD_MMA_WARP) {
     // =============================== MMA issuer =============================================
-    if (lane == 0 && n_total > 0) {
+    if (lane == 0) {
       const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S = Q K^T, both K-major
       const uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);   // O += P V, V is N-major
       const uint32_t tS[2] = {tmem_base + 0, tmem_base + 128};
@@ -296,74 +378,90 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         }
       };
       bool ok = true;
-      do {
-        if (!mbar_wait(&s.q_full[0], 0, wc, 200)) { ok = false; break; }
-        if constexpr (FEW) {
-          // key tile j belongs to sub-tile j & 1; its scores are issued two tiles ahead
-          auto next_s = [&](int j) -> bool {
-            if (!mbar_wait(&s.k_full[j % STAGES], (j / STAGES) & 1, wc, 201)) return false;
+      uint32_t kv = 0;                  // K / V tiles of the items before this one
+      uint32_t live = 0;
+      uint32_t p_cnt[2] = {0, 0};       // FEW: tiles of each sub-tile so far
+      for (uint32_t n = 0; ok; ++n) {
+        const int n_total = fwd_total(p, s.item[n & 1]);
+        if (n_total > 0) {
+          // (that O of the previous item has been read out is implied by p_full of this one's first tile:
+          // the same warps arrive there after their epilogue)
+          if (!mbar_wait(&s.q_full[0], live & 1, wc, 200)) break;
+          if constexpr (FEW) {
+            // key tile j belongs to sub-tile j & 1; its scores are issued two tiles ahead
+            auto next_s = [&](int j) -> bool {
+              const uint32_t g = kv + j;
+              if (!mbar_wait(&s.k_full[g % STAGES], (g / STAGES) & 1, wc, 201)) return false;
+              tc_fence_after_sync();
+              issue_s(j & 1, g % STAGES);
+              tc_commit(&s.s_full[j & 1]);
+              tc_commit(&s.k_empty[g % STAGES]);
+              if (j + 1 == n_total) tc_commit(&s.q_empty);
+              return true;
+            };
+            ok = next_s(0) && (n_total < 2 || next_s(1));
+            for (int j = 0; j < n_total && ok; ++j) {
+              const int w = j & 1, st = (kv + j) % STAGES;
+              if (!mbar_wait(&s.v_full[st], ((kv + j) / STAGES) & 1, wc, 203)) { ok = false; break; }
+              if (!mbar_wait(&s.p_full[w], p_cnt[w] & 1, wc, 204)) { ok = false; break; }
+              ++p_cnt[w];
+              tc_fence_after_sync();
+              issue_pv(w, st, j >= 2);
+              tc_commit(&s.v_empty[st]);
+              if (j + 2 < n_total) ok = next_s(j + 2);
+            }
+          } else {
+            if (!mbar_wait(&s.k_full[kv % STAGES], (kv / STAGES) & 1, wc, 201)) break;
             tc_fence_after_sync();
-            issue_s(j & 1, j % STAGES);
-            tc_commit(&s.s_full[j & 1]);
-            tc_commit(&s.k_empty[j % STAGES]);
-            return true;
-          };
-          ok = next_s(0) && (n_total < 2 || next_s(1));
-          for (int j = 0; j < n_total && ok; ++j) {
-            const int w = j & 1, st = j % STAGES;
-            if (!mbar_wait(&s.v_full[st], (j / STAGES) & 1, wc, 203)) { ok = false; break; }
-            if (!mbar_wait(&s.p_full[w], (j >> 1) & 1, wc, 204)) { ok = false; break; }
-            tc_fence_after_sync();
-            issue_pv(w, st, j >= 2);
-            tc_commit(&s.v_empty[st]);
-            if (j + 2 < n_total) ok = next_s(j + 2);
-          }
-          if (ok) tc_commit(&s.o_full);
-          break;
-        }
-        if (!mbar_wait(&s.k_full[0], 0, wc, 201)) { ok = false; break; }
-        tc_fence_after_sync();
-        issue_s(0, 0);
-        tc_commit(&s.s_full[0]);
-        if (!mbar_wait(&s.q_full[1], 0, wc, 202)) { ok = false; break; }
-        tc_fence_after_sync();
-        issue_s(1, 0);
-        tc_commit(&s.s_full[1]);
-        tc_commit(&s.k_empty[0]);
-        for (int j = 0; j < n_total; ++j) {
-          const int st = j % STAGES;
-          const uint32_t ph = (j / STAGES) & 1;
-          const int stn = (j + 1) % STAGES;
-          const uint32_t phn = ((j + 1) / STAGES) & 1;
-          const bool more = (j + 1 < n_total);
-          FWD_PROF(j == FWD_PROF_TILE, 0);
-          if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
-          if (!mbar_wait(&s.p_full[0], j & 1, wc, 204)) { ok = false; break; }
-          FWD_PROF(j == FWD_PROF_TILE, 1);
-          tc_fence_after_sync();
-          issue_pv(0, st, j > 0);
-          if (more) {
-            if (!mbar_wait(&s.k_full[stn], phn, wc, 205)) { ok = false; break; }
-            tc_fence_after_sync();
-            issue_s(0, stn);
+            issue_s(0, kv % STAGES);
             tc_commit(&s.s_full[0]);
-          }
-          FWD_PROF(j == FWD_PROF_TILE, 2);
-          if (!mbar_wait(&s.p_full[1], j & 1, wc, 206)) { ok = false; break; }
-          FWD_PROF(j == FWD_PROF_TILE, 3);
-          tc_fence_after_sync();
-          issue_pv(1, st, j > 0);
-          tc_commit(&s.v_empty[st]);
-          if (more) {
-            issue_s(1, stn);
+            if (!mbar_wait(&s.q_full[1], live & 1, wc, 202)) break;
+            tc_fence_after_sync();
+            issue_s(1, kv % STAGES);
             tc_commit(&s.s_full[1]);
-            tc_commit(&s.k_empty[stn]);
+            tc_commit(&s.k_empty[kv % STAGES]);
+            if (n_total == 1) tc_commit(&s.q_empty);
+            for (int j = 0; j < n_total; ++j) {
+              const uint32_t g = kv + j;
+              const int st = g % STAGES;
+              const uint32_t ph = (g / STAGES) & 1;
+              const int stn = (g + 1) % STAGES;
+              const uint32_t phn = ((g + 1) / STAGES) & 1;
+              const bool more = (j + 1 < n_total);
+              FWD_PROF(g == FWD_PROF_TILE, 0);
+              if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
+              if (!mbar_wait(&s.p_full[0], g & 1, wc, 204)) { ok = false; break; }
+              FWD_PROF(g == FWD_PROF_TILE, 1);
+              tc_fence_after_sync();
+              issue_pv(0, st, j > 0);
+              if (more) {
+                if (!mbar_wait(&s.k_full[stn], phn, wc, 205)) { ok = false; break; }
+                tc_fence_after_sync();
+                issue_s(0, stn);
+                tc_commit(&s.s_full[0]);
+              }
+              FWD_PROF(g == FWD_PROF_TILE, 2);
+              if (!mbar_wait(&s.p_full[1], g & 1, wc, 206)) { ok = false; break; }
+              FWD_PROF(g == FWD_PROF_TILE, 3);
+              tc_fence_after_sync();
+              issue_pv(1, st, j > 0);
+              tc_commit(&s.v_empty[st]);
+              if (more) {
+                issue_s(1, stn);
+                tc_commit(&s.s_full[1]);
+                tc_commit(&s.k_empty[stn]);
+                if (j + 2 == n_total) tc_commit(&s.q_empty);
+              }
+              FWD_PROF(g == FWD_PROF_TILE, 4);
+            }
           }
-          FWD_PROF(j == FWD_PROF_TILE, 4);
+          if (!ok) break;
+          tc_commit(&s.o_full);
+          kv += n_total;
+          ++live;
         }
-        if (ok) tc_commit(&s.o_full);
-      } while (false);
-      (void)ok;
+        if (!next_item(n)) break;
+      }
     }
   }
   } else {
@@ -374,27 +472,34 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     const int quad = warp & 3;               // TMEM lane quadrant of this warp
     const int r_tile = quad * 32 + lane;     // row inside the 128-row sub-tile
     const int r_cta = (FEW ? 0 : w * ATTN_TILE) + r_tile;   // row inside the CTA's tile
-    const int r_blk = (r0 + r_cta) >> psh;                  // query token inside the query block
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t tS = tmem_base + lane_base + w * 128;
     const uint32_t tO = tmem_base + lane_base + 256 + w * 128;
     const float NEG_INF = -INFINITY;
-
+    uint32_t cnt = 0;                        // score tiles of this sub-tile so far
+    uint32_t live = 0;
+    for (uint32_t n = 0;; ++n) {
+    const FwdItem& it = s.item[n & 1];       // (stays in shared memory: the score loop needs the registers)
+    const int r_blk = (it.r0 + r_cta) >> psh;               // query token inside the query block
+    if (n > 0) trace_stamp(p.trace, it.linear, 0);
+    trace_stamp(p.trace, it.linear, 1);
+    trace_ident(p.trace, it.linear, it.row_idx);
     float m_use = NEG_INF;   // running reference max, log2 units (already scaled)
     float l = 0.f;           // row sum
     bool ok = true;
     uint32_t j = 0;
-    for (int e = row.seg_begin; e < row.seg_end && ok; ++e) {
-      const AttnSeg sg = seg_at(e);
-      const TileRange tr = cta_tiles(sg);
+    for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
+      const AttnSeg sg = fwd_seg(p, e);
+      const TileRange tr = fwd_tiles(p, it, sg);
       for (int t = tr.first; t < tr.end; ++t, ++j) {
         if (FEW && (j & 1) != static_cast<uint32_t>(w)) continue;
-        const bool prof = (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0;
+        const bool prof = (n == 0) && (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0;
         const int pslot = 8 + w * 24 + (static_cast<int>(j) - FWD_PROF_TILE) * 8;
         (void)prof; (void)pslot;
         FWD_PROF(prof, pslot + 0);
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full[w], (FEW ? j >> 1 : j) & 1, wc, 300 + w))) { ok = false; break; }
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full[w], cnt & 1, wc, 300 + w))) { ok = false; break; }
         FWD_PROF(prof, pslot + 1);
+        ++cnt;
         tc_fence_after_sync();
         float sv[ATTN_TILE];
         {
@@ -497,15 +602,16 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       }
     }
     // ---------------------------------- epilogue --------------------------------------------
-    const bool valid_row = r_cta < rows_here;
-    const int qh = q_head + ((r0 + r_cta) & ((1 << psh) - 1));       // query head of this row
-    const bool any = FEW ? n_total > w : n_total > 0;                // this sub-tile has seen a key tile
-    const long orow = static_cast<long>(row.o_start + r_blk);
-    __nv_bfloat16* optr = p.o_ptr[row.o_slot] + batch * p.o_batch_stride[row.o_slot] +
-                          orow * p.o_row_stride[row.o_slot] + static_cast<long>(qh) * ATTN_D;
-    float* lptr = p.lse_ptr[row.o_slot] + batch * p.lse_batch_stride[row.o_slot] +
-                  qh * p.lse_head_stride[row.o_slot] + orow;
-    if (n_total > 0 && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full, 0, wc, 310 + w));
+    const uint32_t n_total = j;
+    const bool valid_row = r_cta < it.rows_here;
+    const int qh = it.q_head + ((it.r0 + r_cta) & ((1 << psh) - 1));       // query head of this row
+    const bool any = FEW ? n_total > static_cast<uint32_t>(w) : n_total > 0;                // this sub-tile has seen a key tile
+    const long orow = static_cast<long>(it.row.o_start + r_blk);
+    __nv_bfloat16* optr = p.o_ptr[it.row.o_slot] + it.batch * p.o_batch_stride[it.row.o_slot] +
+                          orow * p.o_row_stride[it.row.o_slot] + static_cast<long>(qh) * ATTN_D;
+    float* lptr = p.lse_ptr[it.row.o_slot] + it.batch * p.lse_batch_stride[it.row.o_slot] +
+                  qh * p.lse_head_stride[it.row.o_slot] + orow;
+    if (n_total > 0 && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full, live & 1, wc, 310 + w));
     tc_fence_after_sync();
     float lse = NEG_INF;
     float inv = 0.f;
@@ -517,7 +623,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     }
     float w_old = 0.f, w_new = 1.f;
     float lse_old = NEG_INF;
-    if (row.accumulate && valid_row) {
+    if (it.row.accumulate && valid_row) {
       lse_old = *lptr;
       const float mx = fmaxf(lse_old, lse);
       if (mx == NEG_INF) {
@@ -530,10 +636,10 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       }
     }
     const float fnew = inv * w_new;
-    float* pptr = nullptr;               // fp32 partial result of a split launch
+    float* pptr = nullptr;               // fp32 partial result of a it.split launch
     if (p.part_o != nullptr) {
-      const int part = FEW ? 2 * split + w : split;
-      const long prow = ((static_cast<long>(batch) * p.n_parts + part) * row.q_len + r_blk) * p.n_heads + qh;
+      const int part = FEW ? 2 * it.split + w : it.split;
+      const long prow = ((static_cast<long>(it.batch) * p.n_parts + part) * it.row.q_len + r_blk) * p.n_heads + qh;
       pptr = p.part_o + prow * ATTN_D;
       lptr = p.part_lse + prow;
     }
@@ -563,7 +669,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           float f[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 8 + i]) * fnew;
-          if (row.accumulate) {
+          if (it.row.accumulate) {
             const uint4 old = d4[q];
             const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
 #pragma unroll
@@ -584,12 +690,19 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       }
     }
     if (valid_row) *lptr = lse;
+    trace_stamp(p.trace, it.linear, 2);
+    if (n_total > 0) ++live;
+    if (!ok) break;
+    __syncwarp();                            // every lane is done reading the item
+    int more = 0;
+    if (lane == 0) more = next_item(n) ? 1 : 0;
+    if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
+    }
   }
   }
 
   tc_fence_before_sync();
   __syncthreads();
-  trace_stamp(p.trace, cta_linear, 2);
   if (warp == FWD_MMA_WARP) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
@@ -777,6 +890,7 @@ extern "C" int ua_attn_fwd(const UaTensorSrc* q_src, int n_q, const UaTensorSrc*
     UA_CUDA(cudaMemsetAsync(stage_ticket, 0, sizeof(unsigned int), stream));
   }
   p.n_split = 1;
+  p.persist = stage_flags == nullptr;
   return launch_fwd<false>(p, n_heads, batch, stream);
 }
 
@@ -922,6 +1036,7 @@ extern "C" int ua_attn_fwd_dense(const UaTensorSrc* q, const UaTensorSrc* k, con
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
   p.stage.epoch = 1;
+  p.persist = 1;
   const long n_rows = static_cast<long>(batch) * sq * n_heads;
   if (d.n_parts > 0) {
     p.n_parts = d.n_parts;

@@ -142,6 +142,39 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
 }
 
 // ----------------------------------------------------------------------------------------------
+// Cluster launch control: take over a CTA of the grid that has not started
+// ----------------------------------------------------------------------------------------------
+// Asks for one; the 16-byte response arrives at `resp` (16-byte aligned) and completes 16 bytes of `bar`.
+__device__ __forceinline__ void clc_try_cancel(void* resp, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(resp)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// The response: true and the CTA's index if one was taken over (after a false no further request may
+// be made).
+__device__ __forceinline__ bool clc_read(const void* resp, int& bx, int& by) {
+  uint32_t ok, x, y;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P1;\n\t"
+      ".reg .b128 R;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "mov.u32 %2, 0;\n\t"
+      "ld.shared.b128 R, [%3];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 P1, R;\n\t"
+      "selp.u32 %0, 1, 0, P1;\n\t"
+      "@P1 clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, _, _}, R;\n\t"
+      "}\n"
+      : "=&r"(ok), "=&r"(x), "=&r"(y)
+      : "r"(smem_u32(resp))
+      : "memory");
+  bx = static_cast<int>(x);
+  by = static_cast<int>(y);
+  return ok != 0;
+}
+
+// ----------------------------------------------------------------------------------------------
 // TMA (unicast loads into this CTA's shared memory; stores from shared memory)
 // ----------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
