@@ -44,10 +44,14 @@ constexpr int FWD_MMA_WARP = 9;
 constexpr int FWD_THREADS = 384;
 constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 104, FWD_REGS_SOFTMAX = 200;
 static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
-#ifndef UA_FWD_POLY_EXP_PERIOD
-#define UA_FWD_POLY_EXP_PERIOD 0
-#endif
-constexpr int FWD_POLY_EXP_PERIOD = UA_FWD_POLY_EXP_PERIOD;   // every n-th pair of exponentials is polynomial (0: none)
+// The MMA warp starts P V on the first 96 keys of a tile while the softmax warps compute the last 32. A
+// tile pair is bound by two chains of the same length, 3350 clocks: the 32 MMAs, which take 89 clocks each
+// with TMA writes and operand reads on one shared-memory port, and one sub-tile's softmax (1950) plus
+// its own 16 MMAs. Measured (us) without -> with: 4 x 2000 tokens 184 -> 180, causal 8k tokens, 32 heads
+// 592 -> 576, full 16k 3630 -> 3560; 32 or 64 keys in front of the hand-over are within 0.5 %. With 128
+// keys' maxima found beside the exponentials of the tile (against the running maximum) the softmax
+// is 100 clocks shorter and nothing faster.
+constexpr int P_PART = 96;
 constexpr int FWD_TILE_BYTES = ATTN_TILE * ATTN_D * 2;  // 32 KB: [2 d-halves][128 rows][128 B]
 
 struct FwdRow {
@@ -119,6 +123,7 @@ struct __align__(1024) FwdSmem {
   uint64_t v_empty[STAGES];
   uint64_t s_full[2];
   uint64_t p_full[2];
+  uint64_t p_part[2];    // the first P_PART keys of P are there
   uint64_t q_empty;
   uint64_t o_full;
   uint4 clc;             // response of a cancellation request
@@ -245,6 +250,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.s_full[i], 1);
       mbar_init(&s.p_full[i], act_warps);   // one arrival per softmax warp
+      mbar_init(&s.p_part[i], act_warps);
       mbar_init(&s.item_full[i], 1);
       mbar_init(&s.item_empty[i], 1 + 2 * act_warps);   // MMA warp and softmax warps
     }
@@ -368,10 +374,11 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
                   make_smem_desc_sw128(ka + off, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
         }
       };
-      auto issue_pv = [&](int w, int st, bool acc) {
+      auto issue_pv = [&](int w, int st, bool acc, int k0, int k1) {
         const uint32_t va = smem_u32(s.v[st]);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
+          if (kk < k0 || kk >= k1) continue;
           // A: 16 keys = 8 packed columns of P; B: 16 key rows = 2048 B, d-halves 16384 B apart
           umma_ts(tO[w], tS[w] + kk * 8, make_smem_desc_sw128(va + kk * 2048, 16384, 1024),
                   idesc_o, (acc || kk > 0) ? 1u : 0u);
@@ -406,7 +413,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               if (!mbar_wait(&s.p_full[w], p_cnt[w] & 1, wc, 204)) { ok = false; break; }
               ++p_cnt[w];
               tc_fence_after_sync();
-              issue_pv(w, st, j >= 2);
+              issue_pv(w, st, j >= 2, 0, 8);
               tc_commit(&s.v_empty[st]);
               if (j + 2 < n_total) ok = next_s(j + 2);
             }
@@ -430,10 +437,13 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               const bool more = (j + 1 < n_total);
               FWD_PROF(g == FWD_PROF_TILE, 0);
               if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
-              if (!mbar_wait(&s.p_full[0], g & 1, wc, 204)) { ok = false; break; }
+              if (!mbar_wait(&s.p_part[0], g & 1, wc, 204)) { ok = false; break; }
               FWD_PROF(g == FWD_PROF_TILE, 1);
               tc_fence_after_sync();
-              issue_pv(0, st, j > 0);
+              issue_pv(0, st, j > 0, 0, P_PART / 16);
+              if (!mbar_wait(&s.p_full[0], g & 1, wc, 207)) { ok = false; break; }
+              tc_fence_after_sync();
+              issue_pv(0, st, j > 0, P_PART / 16, 8);
               if (more) {
                 if (!mbar_wait(&s.k_full[stn], phn, wc, 205)) { ok = false; break; }
                 tc_fence_after_sync();
@@ -441,10 +451,13 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
                 tc_commit(&s.s_full[0]);
               }
               FWD_PROF(g == FWD_PROF_TILE, 2);
-              if (!mbar_wait(&s.p_full[1], g & 1, wc, 206)) { ok = false; break; }
+              if (!mbar_wait(&s.p_part[1], g & 1, wc, 206)) { ok = false; break; }
               FWD_PROF(g == FWD_PROF_TILE, 3);
               tc_fence_after_sync();
-              issue_pv(1, st, j > 0);
+              issue_pv(1, st, j > 0, 0, P_PART / 16);
+              if (!mbar_wait(&s.p_full[1], g & 1, wc, 208)) { ok = false; break; }
+              tc_fence_after_sync();
+              issue_pv(1, st, j > 0, P_PART / 16, 8);
               tc_commit(&s.v_empty[st]);
               if (more) {
                 issue_s(1, stn);
@@ -572,19 +585,16 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           for (int i = 0; i < 16; ++i) {
             float x0, x1;
             f2_unpack(f2_fma(f2_pack(sv[c * 32 + 2 * i], sv[c * 32 + 2 * i + 1]), sc2, nm2), x0, x1);
-            // optionally one pair in every FWD_POLY_EXP_PERIOD runs on the FMA pipe (packed cubic)
-            const bool poly = FWD_POLY_EXP_PERIOD > 0 && (i % (FWD_POLY_EXP_PERIOD > 0 ? FWD_POLY_EXP_PERIOD : 1)) == (FWD_POLY_EXP_PERIOD > 0 ? FWD_POLY_EXP_PERIOD : 1) - 1;
-            float p0, p1;
-            if (poly) {
-              f2_unpack(poly_exp2_x2(x0, x1), p0, p1);
-            } else {
-              p0 = fast_exp2(x0);
-              p1 = fast_exp2(x1);
-            }
+            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
             ls2[i & 3] = f2_add(ls2[i & 3], f2_pack(p0, p1));
             pk[i] = pack_bf16x2(p0, p1);
           }
           tmem_st_x16(tS + c * 16, pk);
+          if (!FEW && c == P_PART / 32 - 1) {      // (FEW is bound by memory, not by this chain)
+            tmem_wait_st();
+            tc_fence_before_sync();
+            mbar_arrive_warp(&s.p_part[w]);
+          }
         }
         float ls4[4];
 #pragma unroll
