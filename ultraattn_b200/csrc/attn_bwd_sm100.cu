@@ -47,23 +47,13 @@
 namespace ua {
 
 constexpr int BWD_THREADS = 512;              // four warpgroups (the last one: TMA, MMA, two idle warps)
+// (the softmax warps keep their launch-time share)
+constexpr int BWD_REGS_LAUNCH = 128, BWD_REGS_SOFTMAX = 128, BWD_REGS_DRAIN = 152, BWD_REGS_LOAD = 104;
+static_assert(2 * BWD_REGS_SOFTMAX + BWD_REGS_DRAIN + BWD_REGS_LOAD <= 4 * BWD_REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
 constexpr int BWD_TMA_WARP = 12;
 constexpr int BWD_MMA_WARP = 13;
 constexpr int BWD_QT = 128;                // queries per step
 constexpr int BWD_TILE_BYTES = ATTN_TILE * ATTN_D * 2;   // 32 KB: [2 halves][128 rows][128 B]
-#ifndef UA_BWD_DQ_DIRECT
-#define UA_BWD_DQ_DIRECT 0
-#endif
-// dQ leaves the CTA through a shared-memory transpose and TMA reduce-add (default), or straight
-// from registers (one warp-wide 128-byte red.global.add per query row and 32 head-dim elements).
-// Measured at S = 16k, 32 heads: 1.03 PFLOP/s with the TMA reduce, 0.88 with the direct form (its
-// 512 reduction instructions per step crowd the load/store queue the softmax warps depend on).
-constexpr bool BWD_DQ_DIRECT = UA_BWD_DQ_DIRECT != 0;
-#ifndef UA_BWD_POLY_EXP_OF_8
-#define UA_BWD_POLY_EXP_OF_8 0
-#endif
-constexpr int BWD_POLY_EXP_OF_8 = UA_BWD_POLY_EXP_OF_8;    // of every 8 exponentials, how many are polynomial
-
 struct BwdCol {
   int kv_src;     // slot in tmK / tmV
   int kv_start;   // first key token inside that source
@@ -77,6 +67,17 @@ struct BwdCol {
   int kv_wait_count;
 };
 
+// One work item of a launch: a 128-key tile of one key/value head.
+struct BwdItem {
+  BwdCol col;
+  int col_idx;
+  int c0;            // column-relative first key
+  int kv_head;
+  int batch;
+  int linear;        // index in the grid (time stamps)
+  int exists;        // 0: there is no further item
+};
+
 struct BwdParams {
   CUtensorMap tmK[ATTN_MAX_SRC];
   CUtensorMap tmV[ATTN_MAX_SRC];
@@ -88,9 +89,6 @@ struct BwdParams {
   long lse_batch_stride[ATTN_MAX_SRC];
   int q_tokens[ATTN_MAX_SRC];       // tokens in each query-side source (bounds for lse / D)
   CUtensorMap tmdQ[ATTN_MAX_SRC];   // fp32 [batch, tokens, q heads, 128] accumulators, box 128x1x16
-  float* dq_ptr[ATTN_MAX_SRC];      // the same accumulators as plain pointers
-  long dq_row_stride[ATTN_MAX_SRC];     // elements between tokens
-  long dq_batch_stride[ATTN_MAX_SRC];
   void* dk_ptr[ATTN_MAX_SRC];       // bf16 (store mode) or fp32 (add mode) [tokens, kv heads, 128]
   void* dv_ptr[ATTN_MAX_SRC];
   long dkv_row_stride[ATTN_MAX_SRC];
@@ -108,6 +106,7 @@ struct BwdParams {
   // dense launches (cols == nullptr): one column, one query segment, no tables
   BwdCol dense_col;
   AttnSeg dense_seg;
+  int persist;                      // CTAs take over further items (0: one item per CTA)
   StageParams stage;                // optional in-kernel staging of remote blocks
   KernelTrace trace;                // optional per-CTA time stamps
 };
@@ -143,7 +142,13 @@ struct __align__(1024) BwdSmem {
   uint64_t dq_full;      // dQ^T ready              (tcgen05.commit)
   uint64_t dq_free;      // dQ^T read out of TMEM   (4 drain warps, one arrival each)
   uint64_t dkv_full;
-  uint64_t aug0_ready;   // the first step's row terms are in shared memory (8 softmax warps, one arrival each)
+  uint64_t kv_empty;     // the item's last product has read K and V (tcgen05.commit)
+  uint64_t aug0_ready;   // an item's first row terms are in shared memory (8 softmax warps, one arrival each)
+  uint4 clc;             // response of a cancellation request
+  uint64_t clc_full;
+  BwdItem item[2];       // item number n in slot n & 1
+  uint64_t item_full[2];
+  uint64_t item_empty[2];
   uint32_t tmem_base;
   int abort_flag;
   int stage_slot;
@@ -178,6 +183,22 @@ constexpr int BWD_PROF_STEP = 8;
 
 // Walks the (query head of the group, query segment, 128-query tile) steps of one key tile in the
 // order every role of the CTA uses.
+__device__ __forceinline__ BwdItem bwd_item(const BwdParams& p, int bx, int by) {
+  BwdItem it;
+  // (dense: the first key tiles are seen by the most queries under a causal mask, so the natural order
+  // is heaviest first)
+  const bool dense = p.cols == nullptr;
+  const int i = bx % p.n_tiles;
+  const int2 tl = dense ? make_int2(0, i) : p.tiles[i];
+  it.col = dense ? p.dense_col : p.cols[tl.x];
+  it.col_idx = tl.x;
+  it.c0 = tl.y * ATTN_TILE;
+  it.kv_head = bx / p.n_tiles;
+  it.batch = by;
+  it.linear = by * gridDim.x + bx;
+  it.exists = 1;
+  return it;
+}
 __device__ __forceinline__ AttnSeg bwd_seg(const BwdParams& p, int e) {
   return p.cols == nullptr ? p.dense_seg : p.segs[e];
 }
@@ -209,6 +230,17 @@ struct BwdStepIter {
   }
 };
 
+// number of (head, segment, query tile) steps of an item; identical in every role
+__device__ __forceinline__ int bwd_steps(const BwdParams& p, const BwdItem& it) {
+  int per_head = 0;
+  for (int e = it.col.seg_begin; e < it.col.seg_end; ++e) {
+    const AttnSeg sg = bwd_seg(p, e);
+    const int n = seg_num_qt(sg, it.c0) - seg_first_qt(sg, it.c0);
+    per_head += n > 0 ? n : 0;
+  }
+  return per_head * p.kv_group;
+}
+
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -232,10 +264,9 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, boo
     for (int c = 0; c < 32; c += 2) {
       float x0, x1;
       f2_unpack(f2_mul(f2_pack(sv[h][c], sv[h][c + 1]), sc2), x0, x1);     // two products per instruction
-      // optionally some exponentials run on the FMA pipe; measured slower (the phase is bound by
-      // instruction issue, not by the special-function unit), so the default is none
-      const float p0 = (c & 7) < BWD_POLY_EXP_OF_8 ? poly_exp2(x0) : fast_exp2(x0);
-      const float p1 = ((c + 1) & 7) < BWD_POLY_EXP_OF_8 ? poly_exp2(x1) : fast_exp2(x1);
+      // (some of them as a polynomial on the FMA pipe is slower: the phase is bound by instruction
+      // issue, not by the special-function unit)
+      const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
       sv[h][c] = (!MASK || (key_ok && (h * 32 + c) >= r_first && (h * 32 + c) <= r_last)) ? p0 : 0.f;
       sv[h][c + 1] = (!MASK || (key_ok && (h * 32 + c + 1) >= r_first && (h * 32 + c + 1) <= r_last)) ? p1 : 0.f;
     }
@@ -260,25 +291,14 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  const int kv_head = blockIdx.x / p.n_tiles;
-  // (dense: the first key tiles are seen by the most queries under a causal mask, so the natural order
-  // is heaviest first)
-  const bool dense = p.cols == nullptr;
-  const int item = blockIdx.x % p.n_tiles;
-  const int2 tl = dense ? make_int2(0, item) : p.tiles[item];
-  const int batch = blockIdx.y;
-  const BwdCol col = dense ? p.dense_col : p.cols[tl.x];
-  const int cta_linear = blockIdx.y * gridDim.x + blockIdx.x;
-  trace_stamp(p.trace, cta_linear, 0);
-  trace_ident(p.trace, cta_linear, tl.x);
+  const BwdItem item0 = bwd_item(p, blockIdx.x, blockIdx.y);
+  trace_stamp(p.trace, item0.linear, 0);
   {
     // does this CTA read a staged block? then it first helps to empty the copy queue
-    bool waits = col.kv_wait_flag != 0;
-    for (int e = col.seg_begin; e < col.seg_end && !waits; ++e) waits = bwd_seg(p, e).wait_flag != 0;
-    drain_stage_queue(p.stage, waits, cta_linear, &s.stage_slot);
+    bool waits = item0.col.kv_wait_flag != 0;
+    for (int e = item0.col.seg_begin; e < item0.col.seg_end && !waits; ++e) waits = bwd_seg(p, e).wait_flag != 0;
+    drain_stage_queue(p.stage, waits, item0.linear, &s.stage_slot);
   }
-  trace_stamp(p.trace, cta_linear, 1);
-  const int c0 = tl.y * ATTN_TILE;              // column-relative first key of this CTA
 
   if (threadIdx.x == 0) {
     mbar_init(&s.kv_full, 1);
@@ -296,6 +316,13 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     mbar_init(&s.dq_free, 4);
     mbar_init(&s.dkv_full, 1);
     mbar_init(&s.aug0_ready, 8);
+    mbar_init(&s.kv_empty, 1);
+    mbar_init(&s.clc_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s.item_full[i], 1);
+      mbar_init(&s.item_empty[i], 13);        // MMA warp, eight softmax warps, four drain warps
+    }
+    s.item[0] = item0;
     s.abort_flag = 0;
     fence_mbar_init();
   }
@@ -323,63 +350,95 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   const uint32_t tmem_base = s.tmem_base;
   WaitCtx wc{&s.abort_flag, p.status, 4000000000ull};
 
-  // number of (head, segment, query tile) steps; identical in every role
-  int steps_per_head = 0;
-  for (int e = col.seg_begin; e < col.seg_end; ++e) {
-    const AttnSeg sg = bwd_seg(p, e);
-    const int n = seg_num_qt(sg, c0) - seg_first_qt(sg, c0);
-    steps_per_head += n > 0 ? n : 0;
-  }
-  const int n_steps = steps_per_head * p.kv_group;
+  // Persistent CTAs (see the forward kernel): a CTA that is done with an item takes over one whose CTA
+  // has not started. Its Q and dO arrive early, K and V as soon as the last product has read the old
+  // ones, and its first scores run while the softmax warps write this item's dK / dV. One item per CTA
+  // -> this (B200, us): 4 x 2000 tokens 371 -> 357, causal 8k tokens, 32 heads 1360 -> 1326, window 512 in
+  // 16k tokens 745 -> 698.
+  // Consumers wait for item m (m >= 1) with item_ready and hand their slot back with item_done.
+  auto item_ready = [&](uint32_t m) -> bool {
+    if (!p.persist) return false;
+    if (!mbar_wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, wc, 130)) return false;
+    return s.item[m & 1].exists != 0;
+  };
 
   if (warp >= BWD_TMA_WARP) {
     // last warpgroup (TMA, MMA, two idle warps): the drain warpgroup takes most of its registers.
     // The instruction sits inside this branch so that the other roles keep their full budget.
-    reg_dealloc<96>();
+    reg_dealloc<BWD_REGS_LOAD>();
   if (warp == BWD_TMA_WARP) {
     // =============================== TMA producer ===========================================
-    if (lane == 0 && n_steps > 0) {
-      const int krow = col.kv_start + c0;
+    if (lane == 0) {
       bool ok = true;
-      if (!wait_staged(p.stage.flags, col.kv_wait_flag, col.kv_wait_count * p.stage.epoch, wc.budget_ns)) {
-        report_error(wc, UA_ERR_FLAG_TIMEOUT, 120, col.kv_wait_flag);
-        ok = false;
-      }
-      mbar_arrive_expect_tx(&s.kv_full, 2 * BWD_TILE_BYTES);
-      tma_load_4d(s.k, &p.tmK[col.kv_src], &s.kv_full, 0, kv_head, krow, batch);
-      tma_load_4d(s.k + 16384, &p.tmK[col.kv_src], &s.kv_full, 64, kv_head, krow, batch);
-      tma_load_4d(s.v, &p.tmV[col.kv_src], &s.kv_full, 0, kv_head, krow, batch);
-      tma_load_4d(s.v + 16384, &p.tmV[col.kv_src], &s.kv_full, 64, kv_head, krow, batch);
-      uint32_t i = 0;
-      for (int g = 0; g < p.kv_group && ok; ++g) {
-        const int head = kv_head * p.kv_group + g;
-        for (int e = col.seg_begin; e < col.seg_end && ok; ++e) {
-          const AttnSeg sg = bwd_seg(p, e);
-          const int nq = seg_num_qt(sg, c0);
-          if (seg_first_qt(sg, c0) < nq &&
-              !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
-            report_error(wc, UA_ERR_FLAG_TIMEOUT, 121, sg.wait_flag);
-            ok = false;
-            break;
-          }
-          for (int t = seg_first_qt(sg, c0); t < nq; ++t, ++i) {
-            const int st = i & 1;
-            const int qrow = sg.start + t * BWD_QT;
-            if (!mbar_wait(&s.q_empty[st], ((i >> 1) & 1) ^ 1, wc, 100)) { ok = false; break; }
-            mbar_arrive_expect_tx(&s.q_full[st], BWD_TILE_BYTES);
-            tma_load_4d(s.q[st], &p.tmQ[sg.src], &s.q_full[st], 0, head, qrow, batch);
-            tma_load_4d(s.q[st] + 16384, &p.tmQ[sg.src], &s.q_full[st], 64, head, qrow, batch);
-            if (!mbar_wait(&s.do_empty, (i & 1) ^ 1, wc, 101)) { ok = false; break; }
-            mbar_arrive_expect_tx(&s.do_full, BWD_TILE_BYTES);
-            tma_load_4d(s.d_o, &p.tmdO[sg.src], &s.do_full, 0, head, qrow, batch);
-            tma_load_4d(s.d_o + 16384, &p.tmdO[sg.src], &s.do_full, 64, head, qrow, batch);
+      BwdItem it = item0;
+      uint32_t i = 0;          // steps loaded so far
+      uint32_t live = 0;       // items with steps so far
+      for (uint32_t n = 0; ok; ++n) {
+        bool first = true;
+        for (int g = 0; g < p.kv_group && ok; ++g) {
+          const int head = it.kv_head * p.kv_group + g;
+          for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
+            const AttnSeg sg = bwd_seg(p, e);
+            const int nq = seg_num_qt(sg, it.c0);
+            if (seg_first_qt(sg, it.c0) < nq &&
+                !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
+              report_error(wc, UA_ERR_FLAG_TIMEOUT, 121, sg.wait_flag);
+              ok = false;
+              break;
+            }
+            for (int t = seg_first_qt(sg, it.c0); t < nq; ++t, ++i) {
+              const int st = i & 1;
+              const int qrow = sg.start + t * BWD_QT;
+              if (!mbar_wait(&s.q_empty[st], ((i >> 1) & 1) ^ 1, wc, 100)) { ok = false; break; }
+              mbar_arrive_expect_tx(&s.q_full[st], BWD_TILE_BYTES);
+              tma_load_4d(s.q[st], &p.tmQ[sg.src], &s.q_full[st], 0, head, qrow, it.batch);
+              tma_load_4d(s.q[st] + 16384, &p.tmQ[sg.src], &s.q_full[st], 64, head, qrow, it.batch);
+              if (first) {
+                first = false;
+                // the previous item's products have read its K and V
+                if (live > 0 && !mbar_wait(&s.kv_empty, (live - 1) & 1, wc, 102)) { ok = false; break; }
+                if (!wait_staged(p.stage.flags, it.col.kv_wait_flag, it.col.kv_wait_count * p.stage.epoch,
+                                 wc.budget_ns)) {
+                  report_error(wc, UA_ERR_FLAG_TIMEOUT, 120, it.col.kv_wait_flag);
+                  ok = false;
+                  break;
+                }
+                const int krow = it.col.kv_start + it.c0;
+                mbar_arrive_expect_tx(&s.kv_full, 2 * BWD_TILE_BYTES);
+                tma_load_4d(s.k, &p.tmK[it.col.kv_src], &s.kv_full, 0, it.kv_head, krow, it.batch);
+                tma_load_4d(s.k + 16384, &p.tmK[it.col.kv_src], &s.kv_full, 64, it.kv_head, krow, it.batch);
+                tma_load_4d(s.v, &p.tmV[it.col.kv_src], &s.kv_full, 0, it.kv_head, krow, it.batch);
+                tma_load_4d(s.v + 16384, &p.tmV[it.col.kv_src], &s.kv_full, 64, it.kv_head, krow, it.batch);
+                ++live;
+              }
+              if (!mbar_wait(&s.do_empty, (i & 1) ^ 1, wc, 101)) { ok = false; break; }
+              mbar_arrive_expect_tx(&s.do_full, BWD_TILE_BYTES);
+              tma_load_4d(s.d_o, &p.tmdO[sg.src], &s.do_full, 0, head, qrow, it.batch);
+              tma_load_4d(s.d_o + 16384, &p.tmdO[sg.src], &s.do_full, 64, head, qrow, it.batch);
+            }
           }
         }
+        if (!ok || !p.persist) break;
+        // everything of this item is on its way: take over the next one
+        mbar_arrive_expect_tx(&s.clc_full, 16);
+        clc_try_cancel(&s.clc, &s.clc_full);
+        if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
+        int bx, by;
+        const bool got = clc_read(&s.clc, bx, by);
+        fence_proxy_async_smem();               // read before the next response may overwrite it
+        if (got) it = bwd_item(p, bx, by);
+        else it.exists = 0;
+        // the slot's previous item (n - 1) is done with
+        const uint32_t slot = (n + 1) & 1;
+        if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
+        s.item[slot] = it;
+        mbar_arrive(&s.item_full[slot]);
+        if (!got) break;
       }
     }
   } else if (warp == BWD_MMA_WARP) {
     // =============================== MMA issuer =============================================
-    if (lane == 0 && n_steps > 0) {
+    if (lane == 0) {
       const uint32_t idesc_kk = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T: both K-major
       const uint32_t idesc_kn = make_idesc_bf16(128, 128, 0, 1);   // dV, dK: B N-major
       const uint32_t idesc_nn = make_idesc_bf16(128, 128, 1, 1);   // dQ^T: A, B MN-major
@@ -422,22 +481,29 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         umma_ss(t_dp, ones_d_d, aug_desc[st], idesc_kk, 1u);       // - D
       };
       bool ok = true;
-      do {
-        if (!mbar_wait(&s.kv_full, 0, wc, 200)) { ok = false; break; }
-        if (!mbar_wait(&s.q_full[0], 0, wc, 201)) { ok = false; break; }
-        if (!mbar_wait(&s.aug0_ready, 0, wc, 208)) { ok = false; break; }
+      uint32_t i = 0;                   // steps so far
+      uint32_t live = 0;
+      for (uint32_t n = 0; ok; ++n) {
+        const int n_steps = bwd_steps(p, s.item[n & 1]);
+        if (n_steps > 0) {
+        if (!mbar_wait(&s.kv_full, live & 1, wc, 200)) break;
+        if (!mbar_wait(&s.q_full[i & 1], (i >> 1) & 1, wc, 201)) break;
+        if (!mbar_wait(&s.aug0_ready, live & 1, wc, 208)) break;
         tc_fence_after_sync();
-        issue_st(0);
+        issue_st(i & 1);
         tc_commit(&s.s_full);
-        if (!mbar_wait(&s.do_full, 0, wc, 202)) { ok = false; break; }
+        if (!mbar_wait(&s.do_full, i & 1, wc, 202)) break;
+        // dP^T lands where the previous item's last dQ^T was. (That dK / dV of that item have been read
+        // out before they are started anew is implied by p_ready: the warps arrive after their epilogue.)
+        if (i > 0 && !mbar_wait(&s.dq_free, (i - 1) & 1, wc, 209)) break;
         tc_fence_after_sync();
-        issue_dp(0);
+        issue_dp(i & 1);
         tc_commit(&s.dp_full);
-        for (int i = 0; i < n_steps; ++i) {
+        for (int k = 0; k < n_steps; ++k, ++i) {
           const int st = i & 1;
           const uint32_t ph = i & 1;
           const uint64_t qn = q_nmaj0 + st * Q_STAGE;
-          const bool more = i + 1 < n_steps;
+          const bool more = k + 1 < n_steps;
           // dV += P^T dO : A = P^T in TMEM (queries 0-63 packed at columns 0-31, 64-127 at 64-95),
           // B = dO as an N-major operand (16 query rows = 2048 B, d-halves 16384 B apart)
           BWD_PROF(i == BWD_PROF_STEP, 0);
@@ -447,7 +513,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
             umma_ts(t_dv, t_st + (kk >> 2) * 64 + (kk & 3) * 8, do_nmaj + noff(kk), idesc_kn,
-                    (i > 0 || kk > 0) ? 1u : 0u);
+                    (k > 0 || kk > 0) ? 1u : 0u);
           tc_commit(&s.do_empty);
           // S^T of the next step right behind it: it overwrites P^T(i), which dV(i) reads first
           // because the tensor pipe executes in issue order
@@ -472,7 +538,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
           // step), B = Q as an N-major operand; runs while the drain warpgroup reads dQ^T
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            umma_ss(t_dk, ds_kmaj + koff(kk), qn + noff(kk), idesc_kn, (i > 0 || kk > 0) ? 1u : 0u);
+            umma_ss(t_dk, ds_kmaj + koff(kk), qn + noff(kk), idesc_kn, (k > 0 || kk > 0) ? 1u : 0u);
           tc_commit(&s.q_empty[st]);
           BWD_PROF(i == BWD_PROF_STEP, 5);
           if (more) {
@@ -487,8 +553,14 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
             BWD_PROF(i == BWD_PROF_STEP, 8);
           }
         }
-        if (ok) tc_commit(&s.dkv_full);
-      } while (false);
+        if (!ok) break;
+        tc_commit(&s.kv_empty);
+        tc_commit(&s.dkv_full);
+        ++live;
+        }
+        if (p.persist) mbar_arrive(&s.item_empty[n & 1]);
+        if (!item_ready(n + 1)) break;
+      }
     }
   }
   } else if (warp < 8) {
@@ -496,8 +568,6 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     const int wg = warp >> 2;                        // which half of the 128 query columns
     const int quad = warp & 3;
     const int key_t = quad * 32 + lane;              // key inside the tile
-    const int key_c = c0 + key_t;                    // key inside the block column
-    const bool key_ok = key_c < col.kv_len;
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t t_st = tmem_base + lane_base + 256 + wg * 64;
     const uint32_t t_dp = tmem_base + lane_base + 384 + wg * 64;
@@ -511,7 +581,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     const float* dv_g = nullptr;
     int row_lim = 0;                     // rows of the segment that exist in its source
     const float inv_scale_log2 = 1.4426950408889634f / p.scale_log2;
-    auto fetch = [&](const BwdStepIter& it, float& lv, float& dv) -> bool {
+    auto fetch = [&](const BwdItem& item, const BwdStepIter& it, float& lv, float& dv) -> bool {
       if (it.new_seg) {
         const AttnSeg& sg = it.sg;
         if (sg.wait_flag != 0) {
@@ -521,8 +591,8 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
           w_ok = __shfl_sync(0xFFFFFFFFu, w_ok, 0);
           if (!w_ok) return false;
         }
-        const int head = kv_head * p.kv_group + it.g;
-        const long off = batch * p.lse_batch_stride[sg.src] + head * p.lse_head_stride[sg.src] + sg.start;
+        const int head = item.kv_head * p.kv_group + it.g;
+        const long off = item.batch * p.lse_batch_stride[sg.src] + head * p.lse_head_stride[sg.src] + sg.start;
         lse_g = p.lse_ptr[sg.src] + off;
         dv_g = p.dvec_ptr[sg.src] + off;
         row_lim = min(sg.len, p.q_tokens[sg.src] - sg.start);
@@ -559,20 +629,33 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     };
     BwdStepIter cur, fut;
     float lv = INFINITY, dv = 0.f;
-    if (n_steps > 0) {
-      cur.first(p, col, c0);
+    uint32_t i = 0;                      // steps so far
+    uint32_t live = 0;
+    // Row terms of an item's first step (the i-th of the CTA) into its operand tile, those of the
+    // second into registers.
+    auto start_item = [&](const BwdItem& it, int n_steps) {
+      cur.first(p, it.col, it.c0);
       fut = cur;
-      ok = fetch(fut, lv, dv);
-      if (ok) {
-        write_aug(0, lv, dv);
-        mbar_arrive_warp(&s.aug0_ready);
-        if (n_steps > 1) {
-          fut.next(p, col, c0);
-          ok = fetch(fut, lv, dv);
-        }
+      ok = fetch(it, fut, lv, dv);
+      if (!ok) return;
+      write_aug(i & 1, lv, dv);
+      mbar_arrive_warp(&s.aug0_ready);
+      if (n_steps > 1) {
+        fut.next(p, it.col, it.c0);
+        ok = fetch(it, fut, lv, dv);
       }
-    }
-    for (int i = 0; i < n_steps && ok; ++i) {
+    };
+    int n_steps = bwd_steps(p, s.item[0]);
+    if (n_steps > 0) start_item(s.item[0], n_steps);
+    for (uint32_t n = 0;; ++n) {
+    const BwdItem& it = s.item[n & 1];
+    const int c0 = it.c0;
+    const int key_c = c0 + key_t;                    // key inside the block column
+    const bool key_ok = key_c < it.col.kv_len;
+    if (n > 0) trace_stamp(p.trace, it.linear, 0);
+    trace_stamp(p.trace, it.linear, 1);
+    trace_ident(p.trace, it.linear, it.col_idx);
+    for (int k = 0; k < n_steps && ok; ++k, ++i) {
       const uint32_t ph = i & 1;
       const AttnSeg& sg = cur.sg;
       const bool prof = i == BWD_PROF_STEP && quad == 0 && lane == 0;
@@ -581,7 +664,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       BWD_PROF(prof, pslot + 0);
       // row terms of step i+1 into the operand tile (its previous user, step i-1, is complete: this
       // thread has consumed dP^T(i-1)); the arrival on p_ready below publishes them
-      if (i + 1 < n_steps) write_aug((i + 1) & 1, lv, dv);
+      if (k + 1 < n_steps) write_aug((i + 1) & 1, lv, dv);
       BWD_PROF(prof, pslot + 7);
       // visible iff key_c <= r + diag  <=>  r >= key_c - diag   (r relative to this half)
       const int r_half = cur.t * BWD_QT + wg * 64;
@@ -589,9 +672,9 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       // ... and key_c >= r + lo  <=>  r <= key_c - lo
       const int r_last = (sg.causal & SEG_LOWER) ? key_c - sg.lo - r_half : 63;
       // the row terms of step i+2 travel while this step computes
-      if (i + 2 < n_steps) {
-        fut.next(p, col, c0);
-        if (!fetch(fut, lv, dv)) { ok = false; break; }
+      if (k + 2 < n_steps) {
+        fut.next(p, it.col, c0);
+        if (!fetch(it, fut, lv, dv)) { ok = false; break; }
       }
 
       // ---- phase A: P^T = exp2((S^T - lse / scale) * scale) -> TMEM (packed bf16) ------------
@@ -647,15 +730,29 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       tc_fence_before_sync();
       mbar_arrive_warp(&s.ds_ready);
       BWD_PROF(prof, pslot + 6);
-      if (i + 1 < n_steps) cur.next(p, col, c0);
+      if (k + 1 < n_steps) cur.next(p, it.col, c0);
+    }
+    // the next item's first row terms go out before this one's results, so that its scores can start
+    int more = 0;
+    if (ok) {
+      if (lane == 0) more = item_ready(n + 1) ? 1 : 0;
+      more = __shfl_sync(0xFFFFFFFFu, more, 0);
+    }
+    const int n_done = n_steps;
+    if (more) {
+      n_steps = bwd_steps(p, s.item[(n + 1) & 1]);
+      if (n_steps > 0) start_item(s.item[(n + 1) & 1], n_steps);
     }
     // ---------------------------------- dK / dV epilogue ------------------------------------
-    if (n_steps > 0 && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.dkv_full, 0, wc, 310));
+    if (n_done > 0 && ok) {
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.dkv_full, live & 1, wc, 310));
+      ++live;
+    }
     tc_fence_after_sync();
-    const int slot = col.g_slot;
-    const long grow = static_cast<long>(col.g_start + key_c);
-    const long goff = batch * p.dkv_batch_stride[slot] + grow * p.dkv_row_stride[slot] +
-                      static_cast<long>(kv_head) * ATTN_D;
+    const int slot = it.col.g_slot;
+    const long grow = static_cast<long>(it.col.g_start + key_c);
+    const long goff = it.batch * p.dkv_batch_stride[slot] + grow * p.dkv_row_stride[slot] +
+                      static_cast<long>(it.kv_head) * ATTN_D;
 #pragma unroll 1
     for (int which = wg; which <= wg; ++which) {      // warpgroup 0 stores dK, warpgroup 1 dV
       const uint32_t t_acc = tmem_base + lane_base + which * 128;
@@ -664,7 +761,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         uint32_t av[32];
-        if (n_steps > 0) {
+        if (n_done > 0) {
           tmem_ld_x32(t_acc + c * 32, av);
           tmem_wait_ld();
         } else {
@@ -673,7 +770,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         }
         if (!key_ok) continue;
         if (p.dkv_add_f32[slot]) {
-          if (n_steps == 0) continue;
+          if (n_done == 0) continue;
           float* dst = static_cast<float*>(base) + goff + c * 32;
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
@@ -699,9 +796,15 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         }
       }
     }
+    trace_stamp(p.trace, it.linear, 2);
+    tc_fence_before_sync();                  // dK / dV have been read; published by the next p_ready
+    __syncwarp();
+    if (lane == 0 && p.persist) mbar_arrive(&s.item_empty[n & 1]);
+    if (!more || !ok) break;
+    }
   } else {
     // =============================== dQ drain warpgroup =====================================
-    reg_alloc<160>();        // holds a whole 128-query dQ^T slice in registers
+    reg_alloc<BWD_REGS_DRAIN>();        // holds a whole 128-query dQ^T slice in registers
     const int quad = warp & 3;                       // TMEM lanes quad*32.. = head-dim slice
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t t_dq = tmem_base + lane_base + 384;
@@ -709,16 +812,15 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     bool ok = true;
     uint32_t i = 0;
     uint32_t n_chunk = 0;
+    for (uint32_t n = 0;; ++n) {
+    const BwdItem& it = s.item[n & 1];
+    const int c0 = it.c0;
     for (int g = 0; g < p.kv_group && ok; ++g) {
-      const int head = kv_head * p.kv_group + g;
-      for (int e = col.seg_begin; e < col.seg_end && ok; ++e) {
+      const int head = it.kv_head * p.kv_group + g;
+      for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
         const AttnSeg sg = bwd_seg(p, e);
         const int nq = seg_num_qt(sg, c0);
         const CUtensorMap* tdq = &p.tmdQ[sg.src];
-        const long rs = p.dq_row_stride[sg.src];
-        float* dq_col = p.dq_ptr[sg.src] + batch * p.dq_batch_stride[sg.src] +
-                        static_cast<long>(head) * ATTN_D + quad * 32 + lane;
-        const int tokens = p.q_tokens[sg.src];
         for (int t = seg_first_qt(sg, c0); t < nq; ++t, ++i) {
           BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 48);
           if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.dq_full, i & 1, wc, 400))) { ok = false; break; }
@@ -733,28 +835,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
           tc_fence_before_sync();
           mbar_arrive_warp(&s.dq_free);
           BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 50);
-          if (BWD_DQ_DIRECT) {
-            // lane = head-dim element, register = query: the 32 lanes of one instruction cover 128
-            // contiguous bytes of one query row
-            float* dst = dq_col + static_cast<long>(qrow) * rs;
-            const int n_valid = min(BWD_QT, tokens - qrow);      // rows that exist in the accumulator
-            if (n_valid == BWD_QT) {
-#pragma unroll
-              for (int h = 0; h < 4; ++h)
-#pragma unroll
-                for (int c = 0; c < 32; ++c)
-                  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + (h * 32 + c) * rs),
-                               "f"(__uint_as_float(dv[h][c]) * p.scale) : "memory");
-            } else {
-#pragma unroll
-              for (int h = 0; h < 4; ++h)
-#pragma unroll
-                for (int c = 0; c < 32; ++c)
-                  if (h * 32 + c < n_valid)
-                    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + (h * 32 + c) * rs),
-                                 "f"(__uint_as_float(dv[h][c]) * p.scale) : "memory");
-            }
-          } else {
+          {
 #pragma unroll
             for (int h = 0; h < 8; ++h) {              // 16 queries at a time, three staging tiles in turn
               // The four warps fill one [16 queries][128 head-dim] tile (a 32-wide slice each) and one
@@ -771,7 +852,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
               asm volatile("bar.sync 1, 128;" ::: "memory");
               BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 53 + (h >> 1) * 3);
               if (quad == 0 && lane == 0) {
-                tma_reduce_add_4d(tdq, tile, 0, head, qrow + h * 16, batch);
+                tma_reduce_add_4d(tdq, tile, 0, head, qrow + h * 16, it.batch);
                 tma_store_commit();
               }
               BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 54 + (h >> 1) * 3);
@@ -782,13 +863,20 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         }
       }
     }
+    __syncwarp();
+    int more = 0;
+    if (lane == 0) {
+      if (p.persist) mbar_arrive(&s.item_empty[n & 1]);
+      more = ok && item_ready(n + 1) ? 1 : 0;
+    }
+    if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
+    }
     if (lane == 0) tma_store_wait_all();
     __syncwarp();
   }
 
   tc_fence_before_sync();
   __syncthreads();
-  trace_stamp(p.trace, cta_linear, 2);
   if (warp == BWD_MMA_WARP) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
@@ -880,9 +968,6 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
                          static_cast<uint64_t>(bstr) * 4};
       uint32_t box[4] = {128, 1, 16, 1};
       if (make_tmap_f32(&p.tmdQ[i], q_side[i].dq, 4, dims, str, box)) return -1;
-      p.dq_ptr[i] = q_side[i].dq;
-      p.dq_row_stride[i] = q_side[i].dq_row_stride;
-      p.dq_batch_stride[i] = bstr;
     }
   }
   for (int i = 0; i < n_kv; ++i) {
@@ -920,6 +1005,7 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
     const long grid_ctas = static_cast<long>(n_tiles) * n_kv_heads * batch;
     p.stage.n_copy_ctas = static_cast<int>(n_copy_ctas < grid_ctas ? n_copy_ctas : grid_ctas);
   }
+  p.persist = stage_flags == nullptr;
   p.stage.flags = stage_flags;
   p.stage.epoch = stage_epoch;
   p.stage.ticket = stage_ticket;
@@ -1050,9 +1136,6 @@ extern "C" int ua_attn_bwd_dense_noalloc(const void* q, const void* k, const voi
                        static_cast<uint64_t>(n_dq) * 4};
     uint32_t box[4] = {128, 1, 16, 1};
     if (make_tmap_f32(&p.tmdQ[0], dq32, 4, dims, str, box)) return -1;
-    p.dq_ptr[0] = dq32;
-    p.dq_row_stride[0] = static_cast<long>(n_heads) * ATTN_D;
-    p.dq_batch_stride[0] = n_dq;
   }
   p.lse_ptr[0] = lse;
   p.dvec_ptr[0] = dvec;
@@ -1076,6 +1159,7 @@ extern "C" int ua_attn_bwd_dense_noalloc(const void* q, const void* k, const voi
   p.stage.tasks = nullptr;
   p.stage.n_tasks = 0;
   p.stage.n_copy_ctas = 0;
+  p.persist = 1;
   p.stage.flags = nullptr;
   p.stage.epoch = 1;
   p.stage.ticket = nullptr;
