@@ -106,6 +106,7 @@ struct BwdParams {
   // dense launches (cols == nullptr): one column, one query segment, no tables
   BwdCol dense_col;
   AttnSeg dense_seg;
+  int tail_heads;                   // see item_index
   int persist;                      // CTAs take over further items (0: one item per CTA)
   StageParams stage;                // optional in-kernel staging of remote blocks
   KernelTrace trace;                // optional per-CTA time stamps
@@ -188,12 +189,13 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdParams& p, int bx, int by) 
   // (dense: the first key tiles are seen by the most queries under a causal mask, so the natural order
   // is heaviest first)
   const bool dense = p.cols == nullptr;
-  const int i = bx % p.n_tiles;
+  const ItemIndex ix = item_index(bx, p.n_tiles, gridDim.x / p.n_tiles, p.tail_heads);
+  const int i = ix.tile;
   const int2 tl = dense ? make_int2(0, i) : p.tiles[i];
   it.col = dense ? p.dense_col : p.cols[tl.x];
   it.col_idx = tl.x;
   it.c0 = tl.y * ATTN_TILE;
-  it.kv_head = bx / p.n_tiles;
+  it.kv_head = ix.head;
   it.batch = by;
   it.linear = by * gridDim.x + bx;
   it.exists = 1;
@@ -1006,6 +1008,7 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
     p.stage.n_copy_ctas = static_cast<int>(n_copy_ctas < grid_ctas ? n_copy_ctas : grid_ctas);
   }
   p.persist = stage_flags == nullptr;
+  p.tail_heads = stage_flags == nullptr && dense != 1 ? tail_heads(n_tiles, n_kv_heads, sm_count()) : 1;
   p.stage.flags = stage_flags;
   p.stage.epoch = stage_epoch;
   p.stage.ticket = stage_ticket;
@@ -1160,6 +1163,7 @@ extern "C" int ua_attn_bwd_dense_noalloc(const void* q, const void* k, const voi
   p.stage.n_tasks = 0;
   p.stage.n_copy_ctas = 0;
   p.persist = 1;
+  p.tail_heads = causal ? tail_heads(n_tiles, n_kv_heads, sm_count()) : 1;
   p.stage.flags = nullptr;
   p.stage.epoch = 1;
   p.stage.ticket = nullptr;

@@ -66,6 +66,27 @@ struct KernelTrace {
   int cap;                 // CTAs that fit
 };
 
+// Order of the work items of a launch over `heads` x `n_tiles` (tiles heaviest first). Head by head, the
+// tiles of a head run side by side and its key/value (or query) blocks are read into L2 once for all
+// of them. But then the last head's heaviest tiles start when everything else is nearly done, and the
+// launch waits for them. So the last `tail` heads run tile by tile instead: their heaviest tiles first,
+// their lightest last. TAIL_WAVES x SMs items are enough for that: under a causal mask the heaviest
+// tile is about twice the average, so those items keep every SM busy for twice the heaviest one.
+// Measured (us), head by head -> this: 8k causal tokens forward, 32 heads, 574 -> 518, backward 1350 -> 1302,
+// with 32 / 8 heads 1545 -> 1266; 12 documents in 16k tokens, 32 / 8 heads, forward 536 -> 497, backward
+// 1236 -> 1088. Launches whose items are all alike (dense, not causal) stay head by head.
+struct ItemIndex { int head, tile; };
+__host__ __device__ __forceinline__ ItemIndex item_index(int bx, int n_tiles, int heads, int tail) {
+  const int lead = (heads - tail) * n_tiles;
+  if (bx < lead) return ItemIndex{bx / n_tiles, bx % n_tiles};
+  return ItemIndex{heads - tail + (bx - lead) % tail, (bx - lead) / tail};
+}
+constexpr int TAIL_WAVES = 4;
+inline int tail_heads(int n_tiles, int heads, int sms) {
+  const int t = (TAIL_WAVES * sms + n_tiles - 1) / n_tiles;
+  return t < heads ? t : heads;
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ void trace_stamp(const KernelTrace& kt, int cta_linear, int slot) {
   if (kt.buf != nullptr && cta_linear < kt.cap && threadIdx.x == 0) {

@@ -93,6 +93,7 @@ struct FwdParams {
   float* part_o;       // not null: fp32 partial results [batch, parts, tokens, heads, 128] ...
   float* part_lse;     // ... and [batch, parts, tokens, heads]; parts = n_split (x 2 if FEW)
   int n_parts;
+  int tail_heads;      // see item_index
   int persist;         // CTAs take over further items (0: one item per CTA)
   StageParams stage;   // optional in-kernel staging of remote K/V (and Q) blocks
   KernelTrace trace;   // optional per-CTA time stamps
@@ -172,8 +173,8 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdParams& p, int bx, int by) 
   constexpr int CTA_ROWS = FEW ? ATTN_TILE : 2 * ATTN_TILE;
   const bool dense = p.rows == nullptr;
   // (packed launches: `head` is the key/value head and stands for all its query heads)
-  const int head = bx / p.n_tiles;
-  const int i = bx % p.n_tiles;
+  const ItemIndex ix = item_index(bx, p.n_tiles, gridDim.x / p.n_tiles, p.tail_heads);
+  const int head = ix.head, i = ix.tile;
   // dense tiles run from the last rows to the first: under a causal mask the heaviest ones come first
   const int2 tl = dense ? make_int2(0, (p.n_tiles - 1 - i) / p.n_split) : p.tiles[i];
   it.split = dense ? (p.n_tiles - 1 - i) % p.n_split : 0;
@@ -901,6 +902,7 @@ extern "C" int ua_attn_fwd(const UaTensorSrc* q_src, int n_q, const UaTensorSrc*
   }
   p.n_split = 1;
   p.persist = stage_flags == nullptr;
+  p.tail_heads = stage_flags == nullptr ? tail_heads(n_tiles, n_heads, sm_count()) : 1;
   return launch_fwd<false>(p, n_heads, batch, stream);
 }
 
@@ -991,17 +993,6 @@ static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_he
   return d;
 }
 
-static int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-  if (dev < 64 && cached[dev] > 0) return cached[dev];
-  int n = 148;
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  if (dev < 64) cached[dev] = n;
-  return n;
-}
-
 }  // namespace ua
 
 // Partial results per (batch, token, head) that ua_attn_fwd_dense needs room for: the caller's
@@ -1047,6 +1038,7 @@ extern "C" int ua_attn_fwd_dense(const UaTensorSrc* q, const UaTensorSrc* k, con
   p.status = status;
   p.stage.epoch = 1;
   p.persist = 1;
+  p.tail_heads = causal ? tail_heads(p.n_tiles, d.heads, sm_count()) : 1;
   const long n_rows = static_cast<long>(batch) * sq * n_heads;
   if (d.n_parts > 0) {
     p.n_parts = d.n_parts;
