@@ -88,3 +88,28 @@ def test_dense_backward_equals_the_table_launch(B, Sq, Skv, H, Hk, causal):
     A.check_status()
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
     assert (res[0][2] - res[1][2]).norm() <= 1e-6 * res[1][2].norm()
+
+
+@pytest.mark.parametrize("B,S,H,Hk,kind", [(1, 130, 2, 1, "causal"), (2, 257, 4, 2, "full"), (3, 64, 2, 2, "causal"), (1, 256, 4, 4, "blocks")])
+def test_backward_in_one_call_equals_its_parts(B, S, H, Hk, kind):
+    """attn_bwd_local against rowdot / fill, table launch and cast made one by one; K / V as views of one buffer."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    from ultraattn_b200 import api, patterns as P
+    from ultraattn_b200.ops import elementwise as E
+    g = torch.Generator(device="cuda").manual_seed(S)
+    mk = lambda s, h: torch.randn(B, s, h, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, d_o, kv = mk(S, H), mk(S, H), mk(S, 2 * Hk)
+    k, v = kv[:, :, :Hk], kv[:, :, Hk:]
+    pat = {"causal": P.causal(1), "full": P.full(1), "blocks": P.causal(2)}[kind]
+    fplan, bplan = api.local_plans(pat, S, q.device)
+    o, lse = torch.empty_like(q), torch.empty(B, H, S, device="cuda")
+    A.attn_fwd([q], [k], [v], [(o, lse)], fplan)
+    dense = {"causal": 2, "full": 1, "blocks": 0}[kind]
+    got = api.local_backward(q, k, v, o, lse, d_o, bplan, None, dense)
+    dvec, dq32 = E.bwd_prepare(o, d_o)
+    out = A.BwdKvOut(torch.empty_like(k.contiguous()), torch.empty_like(v.contiguous()))
+    A.attn_bwd([A.BwdQSide(q, d_o, lse, dvec, dq32)], [k], [v], [out], bplan)
+    A.check_status()
+    assert torch.equal(got[1], out.dk) and torch.equal(got[2], out.dv)
+    assert (got[0].float() - dq32).norm() <= 2 ** -8 * dq32.norm()

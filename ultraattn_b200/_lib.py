@@ -48,8 +48,8 @@ def _declare(lib):
         "ua_attn_fwd": [POINTER(UaTensorSrc), i, POINTER(UaTensorSrc), POINTER(UaTensorSrc), i,
                         POINTER(UaOutDst), i, vp, vp, vp, i, i, i, i, f, vp, vp, i, i, vp, i, vp, vp],
         "ua_attn_fwd_dense_parts": [i, i, i, i, i, i, i],
-        "ua_attn_fwd_dense": [POINTER(UaTensorSrc), POINTER(UaTensorSrc), POINTER(UaTensorSrc), POINTER(UaOutDst), i, f,
-                              i, vp, vp, vp],
+        "ua_attn_fwd_dense": [c_char_p, i, f, i, vp, vp, vp],        # a packed block: see ops/attention.py
+        "ua_attn_bwd_local": [c_char_p, f, vp, vp],
         "ua_attn_bwd": [POINTER(UaTensorSrc), POINTER(UaTensorSrc), POINTER(UaBwdQSide), i,
                         POINTER(UaTensorSrc), POINTER(UaTensorSrc), i, POINTER(UaBwdKvOut), i,
                         vp, vp, vp, i, i, i, i, i, f, vp, vp, i, i, vp, i, vp, vp],
@@ -109,8 +109,15 @@ def load():
     return _lib
 
 
-def check(rc: int, what: str) -> None:
-    LAUNCHES[0] += 1
+def stream_of(t) -> int:
+    """The current CUDA stream of the tensor's device, as the C calls take it. (torch.cuda.current_stream
+    builds a Stream object first, several microseconds a call.)"""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
+def check(rc: int, what: str, launches: int = 1) -> None:
+    LAUNCHES[0] += launches
     if rc != 0:
         msg = load().ua_last_error().decode(errors="replace")
         raise RuntimeError(f"{what} failed: {msg}")

@@ -66,22 +66,15 @@ class _LocalAttention(torch.autograd.Function):
 def local_backward(q, k, v, o, lse, d_o, bplan, softmax_scale=None, dense: int = 0):
     """dQ, dK, dV of the single-device operator (bf16 on CUDA, input dtype on CPU). ``dense`` = 1 / 2:
     full / causal attention over all tokens; ``bplan`` is not read."""
-    dvec, dq32 = E.bwd_prepare(o, d_o)
     if q.is_cuda:
-        dk = torch.empty_like(k)
-        dv = torch.empty_like(v)
-    else:
-        dk = torch.zeros(k.shape, dtype=torch.float32, device=q.device)
-        dv = torch.zeros(v.shape, dtype=torch.float32, device=q.device)
-    side, kv_out = A.BwdQSide(q, d_o, lse, dvec, dq32), A.BwdKvOut(dk, dv)
-    if dense:
-        A.attn_bwd_dense(side, k, v, kv_out, dense == 2, softmax_scale)
-    else:
-        A.attn_bwd([side], [k], [v], [kv_out], bplan, softmax_scale)
-    if q.is_cuda:
-        dq = torch.empty_like(q)
-        E.cast_scale(dq32, dq)
+        dq, dk, dv = torch.empty(q.shape, dtype=q.dtype, device=q.device), torch.empty_like(k), torch.empty_like(v)
+        A.attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, bplan, dense, softmax_scale)
         return dq, dk, dv
+    dvec, dq32 = E.bwd_prepare(o, d_o)
+    dk = torch.zeros(k.shape, dtype=torch.float32, device=q.device)
+    dv = torch.zeros(v.shape, dtype=torch.float32, device=q.device)
+    side, kv_out = A.BwdQSide(q, d_o, lse, dvec, dq32), A.BwdKvOut(dk, dv)
+    A.attn_bwd([side], [k], [v], [kv_out], bplan, softmax_scale)
     return dq32.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype)
 
 

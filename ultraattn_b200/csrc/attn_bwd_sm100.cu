@@ -1055,6 +1055,52 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
   return 0;
 }
 
+// The whole backward of attention on one device: D = rowdot(O, dO) and the zeroing of the dQ accumulator,
+// the kernel above, the cast of dQ to bf16. One call, so that a short sequence is not bound by the host.
+extern "C" int ua_bwd_prepare(const void* o, const void* d_o, float* dvec, float* dq, long o_bstride, long o_stride,
+                              long do_bstride, long do_stride, int batch, int tokens, int heads, cudaStream_t stream);
+extern "C" int ua_cast_scale(const float* src, void* dst, long n, float scale, int accumulate, cudaStream_t stream);
+
+struct UaLocalBwd {
+  UaTensorSrc q, k, v, d_o;
+  const void* o;
+  long o_row_stride, o_batch_stride;
+  const float* lse;              // [batch, heads, tokens], contiguous; dvec alike
+  float* dvec;
+  float* dq32;                   // [batch, tokens, heads, 128] workspace
+  void* dq;                      // bf16, contiguous
+  void* dk;                      // bf16
+  void* dv;
+  long dkv_row_stride, dkv_batch_stride;
+  const void* cols;              // tables as in ua_attn_bwd, not read if dense
+  const void* segs;
+  const void* tiles;
+  long n_tiles, dense;
+};
+
+extern "C" int ua_attn_bwd_local(const UaLocalBwd* t, float softmax_scale, int* status, cudaStream_t stream) {
+  const long batch = t->q.batch, tokens = t->q.tokens, heads = t->q.heads;
+  if (ua_bwd_prepare(t->o, t->d_o.ptr, t->dvec, t->dq32, t->o_batch_stride, t->o_row_stride, t->d_o.batch_stride,
+                     t->d_o.token_stride, static_cast<int>(batch), static_cast<int>(tokens), static_cast<int>(heads), stream))
+    return -1;
+  UaBwdQSide side;
+  memset(&side, 0, sizeof(side));
+  side.lse = t->lse;
+  side.dvec = t->dvec;
+  side.lse_head_stride = tokens;
+  side.lse_batch_stride = tokens * heads;
+  side.dq = t->dq32;
+  side.dq_row_stride = heads * ATTN_D;
+  side.dq_batch_stride = tokens * heads * ATTN_D;
+  const UaBwdKvOut out = {t->dk, t->dv, t->dkv_row_stride, t->dkv_batch_stride, 0, 0};
+  if (ua_attn_bwd(&t->q, &t->d_o, &side, 1, &t->k, &t->v, 1, &out, 1, t->cols, t->segs, t->tiles,
+                  static_cast<int>(t->n_tiles), static_cast<int>(t->dense), static_cast<int>(heads),
+                  static_cast<int>(t->k.heads), static_cast<int>(batch), softmax_scale, status, nullptr, 0, 0, nullptr, 1,
+                  nullptr, stream))
+    return -1;
+  return ua_cast_scale(t->dq32, t->dq, batch * tokens * heads * ATTN_D, 1.0f, 0, stream);
+}
+
 // =================================================================================================
 // Allocation-free dense backward (declared in ultraattn_noalloc.h)
 // =================================================================================================

@@ -1002,11 +1002,18 @@ extern "C" int ua_attn_fwd_dense_parts(int batch, int sq, int skv, int n_heads, 
   return plan_dense(batch, sq, skv, n_heads, n_kv_heads, causal, n_split, sm_count()).n_parts;
 }
 
+// The tensors of a dense launch in one block, so that a caller marshals one argument.
+struct UaDenseFwd {
+  UaTensorSrc q, k, v;
+  UaOutDst out;
+};
+
 // All queries of `q` against all keys: O and lse of softmax(scale Q K^T) V; causal: key c is visible
 // to query r iff c <= r + skv - sq.
-extern "C" int ua_attn_fwd_dense(const UaTensorSrc* q, const UaTensorSrc* k, const UaTensorSrc* v, const UaOutDst* out,
-                                 int causal, float softmax_scale, int n_split, float* workspace, int* status,
-                                 cudaStream_t stream) {
+extern "C" int ua_attn_fwd_dense(const UaDenseFwd* t, int causal, float softmax_scale, int n_split, float* workspace,
+                                 int* status, cudaStream_t stream) {
+  const UaTensorSrc *q = &t->q, *k = &t->k, *v = &t->v;
+  const UaOutDst* out = &t->out;
   const int batch = static_cast<int>(q->batch), sq = static_cast<int>(q->tokens), skv = static_cast<int>(k->tokens);
   const int n_heads = static_cast<int>(q->heads), n_kv_heads = static_cast<int>(k->heads);
   if (sq <= 0 || batch <= 0) return 0;

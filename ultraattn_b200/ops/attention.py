@@ -17,6 +17,7 @@ input of the backward (orchestrated_attn/utils.py:148-188).
 from __future__ import annotations
 
 import math
+import struct
 from dataclasses import dataclass
 from typing import Sequence
 
@@ -311,11 +312,22 @@ def tensor_map_cache_stats() -> tuple[int, int]:
     return int(h.value), int(m.value)
 
 
-def _src_struct(t: torch.Tensor) -> _lib.UaTensorSrc:
-    assert t.dim() == 4 and t.dtype == torch.bfloat16 and t.stride(3) == 1 and t.shape[3] == 128, \
+# Argument blocks of 64-bit fields (struct UaDenseFwd, UaLocalBwd of csrc/): one packed block costs the
+# host a few microseconds less than the ctypes structures of the table launches.
+_DENSE_FWD = struct.Struct("=27q")
+_LOCAL_BWD = struct.Struct("=44q")
+
+
+def _src_fields(t: torch.Tensor) -> tuple:
+    """struct UaTensorSrc: pointer, tokens, heads, batch, strides of token, head, batch."""
+    shape, st = t.shape, t.stride()
+    assert len(shape) == 4 and t.dtype == torch.bfloat16 and st[3] == 1 and shape[3] == 128, \
         "attention sources must be bf16 [batch, tokens, heads, 128] with contiguous head dim"
-    return _lib.UaTensorSrc(t.data_ptr(), t.shape[1], t.shape[2], t.shape[0], t.stride(1),
-                            t.stride(2), t.stride(0))
+    return t.data_ptr(), shape[1], shape[2], shape[0], st[1], st[2], st[0]
+
+
+def _src_struct(t: torch.Tensor) -> _lib.UaTensorSrc:
+    return _lib.UaTensorSrc(*_src_fields(t))
 
 
 def attn_fwd_cuda(q_srcs: Sequence[torch.Tensor], k_srcs: Sequence[torch.Tensor],
@@ -345,7 +357,7 @@ def attn_fwd_cuda(q_srcs: Sequence[torch.Tensor], k_srcs: Sequence[torch.Tensor]
                          plan.rows_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(),
                          plan.n_tiles, n_heads, n_kv_heads, q0.shape[0], scale, st.data_ptr(),
                          *_stage_args(stage),
-                         torch.cuda.current_stream(q0.device).cuda_stream)
+                         _lib.stream_of(q0))
     _lib.check(rc, "ua_attn_fwd")
 
 
@@ -365,16 +377,16 @@ def attn_fwd_dense(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tuple
             return attn_fwd_reference([q], [k], [v], [out], rows, softmax_scale)
     lib = _lib.load()
     o, lse = out
-    assert o.dtype == torch.bfloat16 and lse.dtype == torch.float32 and o.stride(3) == 1
-    assert o.stride(2) == 128 and lse.stride(2) == 1
+    so, sl = o.stride(), lse.stride()
+    assert o.dtype == torch.bfloat16 and lse.dtype == torch.float32 and so[3] == 1 and so[2] == 128 and sl[2] == 1
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     parts = lib.ua_attn_fwd_dense_parts(B, sq, skv, H, k.shape[2], int(causal), n_split)
     ws = torch.empty(parts * B * sq * H * 129, dtype=torch.float32, device=q.device) if parts else None
-    dst = _lib.UaOutDst(o.data_ptr(), lse.data_ptr(), o.stride(1), o.stride(0), lse.stride(1), lse.stride(0))
-    rc = lib.ua_attn_fwd_dense(_src_struct(q), _src_struct(k), _src_struct(v), dst, int(causal), scale, n_split,
-                               ws.data_ptr() if parts else None, status_buffer(q.device).data_ptr(),
-                               torch.cuda.current_stream(q.device).cuda_stream)
-    _lib.check(rc, "ua_attn_fwd_dense")
+    block = _DENSE_FWD.pack(*_src_fields(q), *_src_fields(k), *_src_fields(v), o.data_ptr(), lse.data_ptr(), so[1], so[0],
+                            sl[1], sl[0])
+    rc = lib.ua_attn_fwd_dense(block, int(causal), scale, n_split, ws.data_ptr() if parts else None,
+                               status_buffer(q.device).data_ptr(), _lib.stream_of(q))
+    _lib.check(rc, "ua_attn_fwd_dense", 2 if parts else 1)
 
 
 def _stage_args(stage):
@@ -586,7 +598,7 @@ def attn_bwd_cuda(q_sides: Sequence[BwdQSide], k_srcs, v_srcs, kv_outs: Sequence
                                                   plan.tiles_t.data_ptr(), plan.n_tiles)
     rc = lib.ua_attn_bwd(qs, dos, sides, nq, ks, vs, len(k_srcs), kos, len(ko), *tables, dense, n_heads, n_kv_heads, q0.shape[0], scale, st.data_ptr(),
                          *_stage_args(stage),
-                         torch.cuda.current_stream(q0.device).cuda_stream)
+                         _lib.stream_of(q0))
     _lib.check(rc, "ua_attn_bwd")
 
 
@@ -654,6 +666,31 @@ def attn_bwd_dense(q_side: BwdQSide, k, v, kv_out: BwdKvOut, causal: bool, softm
         if not q_side.q.is_cuda:
             return attn_bwd_reference([q_side], [k], [v], [kv_out], cols, softmax_scale)
     attn_bwd_cuda([q_side], [k], [v], [kv_out], None, softmax_scale, None, 2 if causal else 1)
+
+
+def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense: int = 0, softmax_scale=None) -> torch.Tensor:
+    """The whole backward on one CUDA device in one call of the library: D = rowdot(O, dO) (returned, ``[B,
+    H, S]``), the kernel under ``plan`` (or ``dense`` = 1 / 2: all queries against all keys, without a mask /
+    causal), dQ cast into ``dq``; ``dk`` and ``dv`` are written by the kernel."""
+    B, S, H, D = q.shape
+    assert lse.dtype == torch.float32 and lse.is_contiguous() and dq.is_contiguous()
+    assert o.shape == q.shape == d_o.shape == dq.shape and o.dtype == dq.dtype == dk.dtype == dv.dtype == torch.bfloat16
+    so, sd, sk = o.stride(), d_o.stride(), dk.stride()
+    assert so[3] == 1 and so[2] == 128 and sd[2] == 128 and sk[3] == 1 and sk[2] == 128 and sk == dv.stride()
+    if debug_bounds_enabled():
+        cols = plan.cols if not dense else [Col(0, 0, k.shape[1], (Seg(0, 0, S, dense == 2, k.shape[1] - S),), 0, 0)]
+        _raise_if_bad("backward", check_bwd_tables(cols, [BwdQSide(q, d_o, lse, lse, q)], [k], [v], [BwdKvOut(dk, dv)]))
+    n = B * S * H
+    ws = torch.empty(n * (D + 1), dtype=torch.float32, device=q.device)      # dQ accumulator, then D
+    w = ws.data_ptr()
+    tables = (0, 0, 0, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(), plan.n_tiles)
+    block = _LOCAL_BWD.pack(*_src_fields(q), *_src_fields(k), *_src_fields(v), *_src_fields(d_o), o.data_ptr(), so[1], so[0],
+                            lse.data_ptr(), w + 4 * n * D, w, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), sk[1], sk[0],
+                            *tables, dense)
+    scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
+    rc = _lib.load().ua_attn_bwd_local(block, scale, status_buffer(q.device).data_ptr(), _lib.stream_of(q))
+    _lib.check(rc, "ua_attn_bwd_local", 3)
+    return ws[n * D:].view(B, H, S)
 
 
 def cols_from_block_table(table: np.ndarray, block: int, kv_block: int | None = None) -> list[Col]:

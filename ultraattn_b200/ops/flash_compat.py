@@ -59,6 +59,10 @@ def _forward(q, k, v, rows, out, softmax_scale):
 def _backward(dout, q, k, v, out, lse, dq, dk, dv, cols, softmax_scale, softmax_d, causal=False):
     """``cols``: the work items of a packed batch, or None: all queries against all keys (``causal``)."""
     B, S, H, D = q.shape
+    if q.is_cuda and softmax_d is None and lse.is_contiguous() and dq.is_contiguous():
+        return A.attn_bwd_local(q, k, v, out, lse, dout.contiguous(), dq, dk, dv,
+                                None if cols is None else A.BwdPlan(cols, q.device),
+                                0 if cols is not None else (2 if causal else 1), softmax_scale)
     if softmax_d is None:
         softmax_d, dq32 = E.bwd_prepare(out, dout)
     else:
