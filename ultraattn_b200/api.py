@@ -127,8 +127,12 @@ class _VarlenAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cu_seqlens, causal, softmax_scale):
         fplan, bplan = varlen_plans(cu_seqlens, causal, q.device)
-        o = torch.zeros_like(q)
-        lse = torch.full((q.shape[0], q.shape[2], q.shape[1]), float("-inf"), dtype=torch.float32, device=q.device)
+        # the kernel writes every token of every sequence; only tokens outside all of them need a fill
+        full = cu_seqlens[0] == 0 and cu_seqlens[-1] == q.shape[1] and all(a <= b for a, b in zip(cu_seqlens, cu_seqlens[1:]))
+        o = (torch.empty_like if full else torch.zeros_like)(q)
+        lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
+        if not full:
+            lse.fill_(float("-inf"))
         A.attn_fwd([q], [k], [v], [(o, lse)], fplan, softmax_scale)
         ctx.save_for_backward(q, k, v, o, lse)
         ctx.bplan, ctx.scale = bplan, softmax_scale
