@@ -82,6 +82,35 @@ class _Linear(torch.autograd.Function):
         return dx, dw
 
 
+class _LinearBackwardOnly(torch.autograd.Function):
+    """The gradients of :class:`_Linear` without its product: stands for the last linear layer of a
+    recomputed segment, whose value nothing reads (the output has its shape and no storage of its own).
+    One of the recomputed products of a layer, [tokens, ffn] x [ffn, hidden], is saved that way."""
+
+    @staticmethod
+    def forward(ctx, x, w):
+        ctx.save_for_backward(x, w)
+        return x.new_zeros(()).expand(x.shape[0], w.shape[0])
+
+    backward = staticmethod(_Linear.backward)
+
+
+class _Embedding(torch.autograd.Function):
+    """Rows of ``w`` [vocab, hidden]; the backward sums the gradient rows of equal ids in fp32, in token
+    order, in one pass over the result (csrc/elementwise.cu)."""
+
+    @staticmethod
+    def forward(ctx, ids, w):
+        ctx.save_for_backward(ids)
+        ctx.vocab = w.shape[0]
+        return F.embedding(ids, w)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (ids,) = ctx.saved_tensors
+        return None, E.embedding_bwd(ids, dy.contiguous(), ctx.vocab)
+
+
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps):
@@ -230,8 +259,8 @@ class _Layer(torch.autograd.Function):
                     a = ul.recompute_out(o, wo)                              # projection only, attention is NOT recomputed
                 a2 = a.requires_grad_()
                 x2 = x.detach().requires_grad_()
-                y = model._seg_ffn(x2, li, a2)
-                torch.autograd.backward([y], [dy])
+                xs, y = model._seg_ffn_grad(x2, li, a2)
+                torch.autograd.backward([xs, y], [dy, dy])
                 with torch.no_grad():
                     dh, dwqkv, dwo = ul.backward(a2.grad, h.detach(), wqkv, wo, o, lse, cos, sin, attn_in_place=True)
                     wqkv.grad.add_(dwqkv)
@@ -243,8 +272,8 @@ class _Layer(torch.autograd.Function):
             q, k, v = model._seg_qkv(x1, li)                    # recomputed (cheap)
             x2 = x.detach().requires_grad_()
             o2 = o.detach().requires_grad_()
-            y = model._seg_out(x2, o2, li)                      # recomputed, attention is NOT
-            torch.autograd.backward([y], [dy])
+            xs, y = model._seg_ffn_grad(x2, li, model._seg_attn_out(x2, o2, li))     # recomputed, attention is NOT
+            torch.autograd.backward([xs, y], [dy, dy])          # the layer's output is xs + y
             dq, dk, dv = model._attn_bwd(o2.grad, q.detach(), k.detach(), v.detach(), o, lse)
             torch.autograd.backward([q, k, v], [dq, dk, dv])
         return x1.grad + x2.grad, None, None
@@ -403,21 +432,33 @@ class LlamaModel:
         k = _rope_any(k.contiguous(), cos, sin, self._pos, c.head_dim)
         return q.unsqueeze(0), k.unsqueeze(0), v.contiguous().unsqueeze(0)
 
-    def _seg_out(self, x, o, li):
+    def _seg_attn_out(self, x, o, li):
         c, p = self.cfg, self.p
-        a = _Linear.apply(o.reshape(x.shape[0], c.n_heads * c.head_dim), p[f"l{li}.wo"])
-        return self._seg_ffn(x, li, a)
+        return _Linear.apply(o.reshape(x.shape[0], c.n_heads * c.head_dim), p[f"l{li}.wo"])
+
+    def _seg_out(self, x, o, li):
+        return self._seg_ffn(x, li, self._seg_attn_out(x, o, li))
 
     def _seg_ffn(self, x, li, a=None):
         """Second half of a layer on x (+ a, the attention block's output, added inside the norm
         kernel): x' + W_down(SwiGLU(W_gate,up(RMSNorm(x')))) with x' = x + a."""
+        x, z = self._seg_ffn_hidden(x, li, a)
+        return x + _Linear.apply(z, self.p[f"l{li}.wdown"])
+
+    def _seg_ffn_grad(self, x, li, a):
+        """The two terms of :meth:`_seg_ffn`'s sum, for a backward through them: x' and a stand-in for the
+        product with W_down that is never computed."""
+        x, z = self._seg_ffn_hidden(x, li, a)
+        return x, _LinearBackwardOnly.apply(z, self.p[f"l{li}.wdown"])
+
+    def _seg_ffn_hidden(self, x, li, a=None):
+        """(x', SwiGLU(W_gate,up(RMSNorm(x'))))"""
         c, p = self.cfg, self.p
         if a is not None:
             x, h = _AddRMSNorm.apply(x, a, p[f"l{li}.norm2"], c.eps)
         else:
             h = _RMSNorm.apply(x, p[f"l{li}.norm2"], c.eps)
-        gu = _Linear.apply(h, p[f"l{li}.wgu"])
-        return x + _Linear.apply(_Swiglu.apply(gu), p[f"l{li}.wdown"])
+        return x, _Swiglu.apply(_Linear.apply(h, p[f"l{li}.wgu"]))
 
     def _window(self):
         w = self.cfg.sliding_window
@@ -465,7 +506,7 @@ class LlamaModel:
         T = ids.shape[0]
         self._pos = (pos if pos is not None else torch.arange(T, device=ids.device)).to(torch.int32)
         self._n_pos = int(self._pos.max().item()) + 1 if pos is not None else T
-        x = F.embedding(ids, self.p["embed"])
+        x = _Embedding.apply(ids, self.p["embed"])
         for li in range(self.cfg.n_layers):
             x = _Layer.apply(x, self, li)
         return _RMSNorm.apply(x, self.p["norm_f"], self.cfg.eps)
@@ -477,7 +518,8 @@ class LlamaModel:
         n_total = n_total_tokens or ids.shape[0] * self.world
         total = h.new_zeros((), dtype=torch.float32)
         for a in range(0, h.shape[0], chunk):
-            total = total + _ChunkLoss.apply(h[a:a + chunk], self.p["lm_head"], targets[a:a + chunk])
+            last = a + chunk >= h.shape[0]
+            total = total + _ChunkLoss.apply(h[a:a + chunk], self.p["lm_head"], targets[a:a + chunk], last)
         return total / n_total
 
     # ------------------------------- optimizer --------------------------------------------------
@@ -518,21 +560,26 @@ class LlamaModel:
 
 
 class _ChunkLoss(torch.autograd.Function):
-    """Sum of token cross-entropies of one chunk; logits live only inside this function."""
+    """Sum of token cross-entropies of one chunk. The logits of a chunk are computed again in its
+    backward; those of the last chunk (``keep``), whose backward is the first to run, are kept for it:
+    one chunk of logits exists at a time either way."""
 
     @staticmethod
-    def forward(ctx, h, w, targets):
-        lse, rows = E.xent_fwd(G.gemm(h, w), targets)        # one pass over the bf16 logits
+    def forward(ctx, h, w, targets, keep=False):
+        logits = G.gemm(h, w)
+        lse, rows = E.xent_fwd(logits, targets)              # one pass over the bf16 logits
         ctx.save_for_backward(h, w, targets, lse)
+        ctx.logits = logits if keep and any(ctx.needs_input_grad) else None
         return rows.sum()
 
     @staticmethod
     def backward(ctx, g):
         h, w, targets, lse = ctx.saved_tensors
-        dl = E.xent_bwd_(G.gemm(h, w), targets, lse, g)     # logits again, turned into their gradient in place
+        logits, ctx.logits = ctx.logits, None                # turned into their gradient in place: good for one use
+        dl = E.xent_bwd_(G.gemm(h, w) if logits is None else logits, targets, lse, g)
         dh = G.gemm(dl, w, b_is_kn=True)
         dw = G.gemm(dl, h, a_is_km=True, b_is_kn=True)
-        return dh, dw, None
+        return dh, dw, None, None
 
 
 def estimate_memory(cfg: LlamaConfig, seq_len: int, cp: int = 1, offload_checkpoints: bool = False,

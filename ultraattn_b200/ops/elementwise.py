@@ -264,6 +264,20 @@ def xent_bwd_(logits: torch.Tensor, targets: torch.Tensor, lse: torch.Tensor, g:
     return logits
 
 
+def embedding_bwd(ids: torch.Tensor, dy: torch.Tensor, vocab: int) -> torch.Tensor:
+    """Gradient [vocab, H] of an embedding lookup: row v = sum of ``dy`` [T, H] over the tokens with id
+    v, in fp32 and token order; rows of ids that do not occur are zero."""
+    T, H = dy.shape
+    if not (dy.is_cuda and dy.dtype == torch.bfloat16 and H % 8 == 0 and T > 0):
+        return torch.zeros(vocab, H, dtype=dy.dtype, device=dy.device).index_add_(0, ids.reshape(-1), dy)
+    sorted_ids, order = torch.sort(ids.reshape(-1).long(), stable=True)
+    out = torch.empty(vocab, H, dtype=dy.dtype, device=dy.device)
+    rc = _lib.load().ua_embedding_bwd(sorted_ids.data_ptr(), order.data_ptr(), dy.data_ptr(), out.data_ptr(), T, H, vocab,
+                                      _stream(dy))
+    _lib.check(rc, "ua_embedding_bwd")
+    return out
+
+
 def peer_add_(dst: torch.Tensor, src: torch.Tensor, zero_src: bool = False) -> None:
     """dst += src for contiguous fp32 tensors; ``dst`` may be a view of a peer GPU's memory
     (this framework's own kernel does the adds — library kernels never touch peer memory)."""
