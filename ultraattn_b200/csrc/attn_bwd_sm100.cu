@@ -112,6 +112,14 @@ struct BwdParams {
   KernelTrace trace;                // optional per-CTA time stamps
 };
 
+// Where dK / dV go, copied into shared memory at the start (kernel parameters indexed by a run-time slot
+// cost several hundred clocks a miss in the constant cache).
+struct BwdGradOut {
+  uint8_t* dk;
+  uint8_t* dv;
+  long row_stride, batch_stride;      // elements
+};
+
 struct __align__(1024) BwdSmem {
   uint8_t k[BWD_TILE_BYTES];
   uint8_t v[BWD_TILE_BYTES];
@@ -150,6 +158,9 @@ struct __align__(1024) BwdSmem {
   BwdItem item[2];       // item number n in slot n & 1
   uint64_t item_full[2];
   uint64_t item_empty[2];
+  BwdGradOut grads[ATTN_MAX_SRC];
+  uint32_t add_f32;      // bit i: gradient slot i is added to in fp32
+  float scale;
   uint32_t tmem_base;
   int abort_flag;
   int stage_slot;
@@ -277,6 +288,78 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, boo
   }
 }
 
+// dK / dV of one item (`any`: it had steps; without, zeros are stored and nothing is added). Warpgroup 0
+// stores dK, warpgroup 1 dV. A thread owns a row; the warps turn 32 x 128-byte blocks around in their
+// part of the dS tile, which no product reads any more and which the same warp writes next, so that an
+// instruction covers four whole rows of a block instead of 16 bytes of each of 32. Storing from
+// registers -> this (us): 512 tokens, 8 heads 61 -> 59, 4 x 2000 tokens 362 -> 351, window 512 in 16k
+// tokens, 32 heads 700 -> 610. Called, not inlined: the step loop needs the registers.
+__device__ __noinline__ void bwd_store_grads(BwdSmem& s, uint32_t item_slot, uint32_t tmem_base, bool any) {
+  const BwdItem& it = s.item[item_slot];
+  const int slot = it.col.g_slot;
+  const bool add_f32 = ((s.add_f32 >> slot) & 1u) != 0;
+  if (!any && add_f32) return;
+  const BwdGradOut& go = s.grads[slot];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wg = warp >> 2, quad = warp & 3;
+  const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + wg * 128;
+  const float mul = wg == 0 ? s.scale : 1.0f;
+  uint8_t* blk = s.ds + warp * 4096;
+  const int sub = lane >> 3, ch = lane & 7;                      // row of four, 16-byte chunk
+  const int esz = add_f32 ? 4 : 2;
+  const long row_bytes = go.row_stride * esz;
+  const int key0 = it.c0 + quad * 32 + sub;                      // this lane's first key inside the column
+  const int kv_len = it.col.kv_len;
+  uint8_t* base = (wg == 0 ? go.dk : go.dv) + (it.batch * go.batch_stride + static_cast<long>(it.kv_head) * ATTN_D) * esz +
+                  (it.col.g_start + static_cast<long>(key0)) * row_bytes + ch * 16;
+#pragma unroll 1
+  for (int c = 0; c < esz; ++c) {                                // 128-byte column blocks of a row
+    if (add_f32) {
+      uint32_t av[32];
+      tmem_ld_x32(t_acc + c * 32, av);
+      tmem_wait_ld();
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(blk + sw128_offset(lane, q)) =
+            make_float4(__uint_as_float(av[q * 4 + 0]) * mul, __uint_as_float(av[q * 4 + 1]) * mul,
+                        __uint_as_float(av[q * 4 + 2]) * mul, __uint_as_float(av[q * 4 + 3]) * mul);
+    } else {
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t av[32];
+        tmem_ld_x32(t_acc + c * 64 + hf * 32, av);
+        tmem_wait_ld();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint4 o = make_uint4(0u, 0u, 0u, 0u);
+          if (any) {
+            o.x = pack_bf16x2(__uint_as_float(av[q * 8 + 0]) * mul, __uint_as_float(av[q * 8 + 1]) * mul);
+            o.y = pack_bf16x2(__uint_as_float(av[q * 8 + 2]) * mul, __uint_as_float(av[q * 8 + 3]) * mul);
+            o.z = pack_bf16x2(__uint_as_float(av[q * 8 + 4]) * mul, __uint_as_float(av[q * 8 + 5]) * mul);
+            o.w = pack_bf16x2(__uint_as_float(av[q * 8 + 6]) * mul, __uint_as_float(av[q * 8 + 7]) * mul);
+          }
+          *reinterpret_cast<uint4*>(blk + sw128_offset(lane, hf * 4 + q)) = o;
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const uint4 val = *reinterpret_cast<const uint4*>(blk + sw128_offset(r * 4 + sub, ch));
+      if (key0 + r * 4 < kv_len) {
+        uint8_t* dst = base + r * 4 * row_bytes + c * 128;
+        if (add_f32)
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(val.x)),
+                       "f"(__uint_as_float(val.y)), "f"(__uint_as_float(val.z)), "f"(__uint_as_float(val.w))
+                       : "memory");
+        else
+          *reinterpret_cast<uint4*>(dst) = val;
+      }
+    }
+    __syncwarp();
+  }
+}
+
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -327,6 +410,16 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     s.item[0] = item0;
     s.abort_flag = 0;
     fence_mbar_init();
+  }
+  if (warp == 1) {
+    if (lane < ATTN_MAX_SRC)
+      s.grads[lane] = BwdGradOut{static_cast<uint8_t*>(p.dk_ptr[lane]), static_cast<uint8_t*>(p.dv_ptr[lane]),
+                                 p.dkv_row_stride[lane], p.dkv_batch_stride[lane]};
+    const uint32_t add = __ballot_sync(0xFFFFFFFFu, lane < ATTN_MAX_SRC && p.dkv_add_f32[lane < ATTN_MAX_SRC ? lane : 0] != 0);
+    if (lane == 0) {
+      s.add_f32 = add;
+      s.scale = p.scale;
+    }
   }
   if (warp == BWD_MMA_WARP) {
     tmem_alloc(&s.tmem_base, 512);
@@ -751,71 +844,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       ++live;
     }
     tc_fence_after_sync();
-    const int slot = it.col.g_slot;
-    const bool add_f32 = p.dkv_add_f32[slot] != 0;
-    if (n_done > 0 || !add_f32) {
-      // warpgroup 0 stores dK, warpgroup 1 dV. A thread owns a row; the warps turn 32 x 128-byte blocks
-      // around in their part of the dS tile, which no product reads any more and which the same warp
-      // writes next, so that an instruction covers four whole rows of a block instead of 16 bytes of
-      // each of 32. Storing from registers -> this (us): 512 tokens, 8 heads 61 -> 59, 4 x 2000 tokens
-      // 362 -> 351, window 512 in 16k tokens, 32 heads 700 -> 610.
-      const uint32_t t_acc = tmem_base + lane_base + wg * 128;
-      const float mul = wg == 0 ? p.scale : 1.0f;
-      uint8_t* base = static_cast<uint8_t*>(wg == 0 ? p.dk_ptr[slot] : p.dv_ptr[slot]);
-      uint8_t* blk = s.ds + warp * 4096;
-      const int sub = lane >> 3, ch = lane & 7;                      // row of four, 16-byte chunk
-      const int esz = add_f32 ? 4 : 2;
-#pragma unroll 1
-      for (int c = 0; c < esz; ++c) {                                // 128-byte column blocks of a row
-        if (add_f32) {
-          uint32_t av[32];
-          tmem_ld_x32(t_acc + c * 32, av);
-          tmem_wait_ld();
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            *reinterpret_cast<float4*>(blk + sw128_offset(lane, q)) =
-                make_float4(__uint_as_float(av[q * 4 + 0]) * mul, __uint_as_float(av[q * 4 + 1]) * mul,
-                            __uint_as_float(av[q * 4 + 2]) * mul, __uint_as_float(av[q * 4 + 3]) * mul);
-        } else {
-#pragma unroll 1
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t av[32];
-            tmem_ld_x32(t_acc + c * 64 + hf * 32, av);
-            tmem_wait_ld();
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 o = make_uint4(0u, 0u, 0u, 0u);
-              if (n_done > 0) {
-                o.x = pack_bf16x2(__uint_as_float(av[q * 8 + 0]) * mul, __uint_as_float(av[q * 8 + 1]) * mul);
-                o.y = pack_bf16x2(__uint_as_float(av[q * 8 + 2]) * mul, __uint_as_float(av[q * 8 + 3]) * mul);
-                o.z = pack_bf16x2(__uint_as_float(av[q * 8 + 4]) * mul, __uint_as_float(av[q * 8 + 5]) * mul);
-                o.w = pack_bf16x2(__uint_as_float(av[q * 8 + 6]) * mul, __uint_as_float(av[q * 8 + 7]) * mul);
-              }
-              *reinterpret_cast<uint4*>(blk + sw128_offset(lane, hf * 4 + q)) = o;
-            }
-          }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const int rr = r * 4 + sub;                                // row inside the warp's 32
-          const int key = c0 + quad * 32 + rr;
-          const uint4 val = *reinterpret_cast<const uint4*>(blk + sw128_offset(rr, ch));
-          if (key < it.col.kv_len) {
-            uint8_t* dst = base + (it.batch * p.dkv_batch_stride[slot] +
-                                   static_cast<long>(it.col.g_start + key) * p.dkv_row_stride[slot] +
-                                   static_cast<long>(it.kv_head) * ATTN_D) * esz + c * 128 + ch * 16;
-            if (add_f32)
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(val.x)),
-                           "f"(__uint_as_float(val.y)), "f"(__uint_as_float(val.z)), "f"(__uint_as_float(val.w))
-                           : "memory");
-            else
-              *reinterpret_cast<uint4*>(dst) = val;
-          }
-        }
-        __syncwarp();
-      }
-    }
+    bwd_store_grads(s, n & 1, tmem_base, n_done > 0);
     trace_stamp(p.trace, it.linear, 2);
     tc_fence_before_sync();                  // dK / dV have been read; published by the next p_ready
     __syncwarp();
