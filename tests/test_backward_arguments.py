@@ -1,0 +1,104 @@
+"""What the one-call backward accepts and refuses before anything is launched (CPU, the library replaced by a
+recorder), and packed batches with tokens outside every sequence (GPU, against float64)."""
+import math
+
+import pytest
+import torch
+
+from ultraattn_b200 import _lib
+from ultraattn_b200.ops import attention as A
+from ultraattn_b200.ops import flash_compat as F
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """Calls of the one-call backward as (fields of the argument block, scale); nothing is launched."""
+    got = []
+
+    class Library:
+        def ua_attn_bwd_local(self, block, scale, status, stream):
+            got.append((A._LOCAL_BWD.unpack(block), scale))
+            return 0
+
+    monkeypatch.setattr(_lib, "load", lambda: Library())
+    monkeypatch.setattr(_lib, "stream_of", lambda t: 0)
+    monkeypatch.setattr(A, "status_buffer", lambda device: torch.zeros(4, dtype=torch.int32))
+    return got
+
+
+def _bf16(*shape):
+    return torch.zeros(*shape, dtype=torch.bfloat16)
+
+
+def _local(B=1, S=64, H=4, Hk=2, **other):
+    t = dict(q=_bf16(B, S, H, 128), k=_bf16(B, S, Hk, 128), v=_bf16(B, S, Hk, 128), o=_bf16(B, S, H, 128),
+             lse=torch.zeros(B, H, S), d_o=_bf16(B, S, H, 128), dq=_bf16(B, S, H, 128), dk=_bf16(B, S, Hk, 128),
+             dv=_bf16(B, S, Hk, 128))
+    t.update(other)
+    return A.attn_bwd_local(plan=None, dense=2, **t)
+
+
+def test_one_call_backward_refuses_other_shapes(calls):
+    _local()
+    assert len(calls) == 1
+    for bad in (dict(lse=torch.zeros(1, 4, 63)), dict(lse=torch.zeros(1, 4, 65)), dict(lse=torch.zeros(1, 64, 4)),
+                dict(lse=torch.zeros(1, 1, 64)), dict(dk=_bf16(1, 63, 2, 128)), dict(dv=_bf16(1, 64, 1, 128))):
+        with pytest.raises(AssertionError):
+            _local(**bad)
+    assert len(calls) == 1
+
+
+def test_packed_lse_covers_the_whole_buffer():
+    cu, H, total = [0, 5, 5, 12], 3, 16
+    lse = torch.randn(H, total)
+    packed = F._packed_lse(F._pad_lse(lse, cu, 7), cu, total)
+    assert packed.shape == (H, total) and packed.is_contiguous()
+    assert torch.equal(packed[:, :12], lse[:, :12]) and (packed[:, 12:] == -math.inf).all()
+
+
+def _documents(q, k, v, cu, causal):
+    """float64 attention of the documents ``cu``; zeros elsewhere. ``[tokens, heads, 128]``."""
+    o = torch.zeros_like(q)
+    for a, b in zip(cu[:-1], cu[1:]):
+        G = q.shape[1] // k.shape[1]
+        s = torch.einsum("qhd,khd->hqk", q[a:b], k[a:b].repeat_interleave(G, 1)) / math.sqrt(128)
+        if causal:
+            s = s.masked_fill(torch.ones(b - a, b - a, dtype=torch.bool, device=q.device).triu(1), float("-inf"))
+        o[a:b] = torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v[a:b].repeat_interleave(G, 1))
+    return o
+
+
+def _close(got, want):
+    # P, dS and every result are rounded to bf16 (2^-9 each, independent errors); 8 of them is far outside
+    return (got.double() - want).norm() <= 8 * 2 ** -9 * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window", [(-1, -1), (60, 0)])
+def test_packed_batch_with_a_tail_outside_the_sequences(window):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    T, H, Hk, cu = 512, 4, 2, [0, 100, 421]
+    g = torch.Generator(device="cuda").manual_seed(0)
+    mk = lambda h: torch.randn(T, h, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, k, v, d_o = mk(H), mk(Hk), mk(Hk), mk(H)
+    d_o[cu[-1]:] = 0
+    args = (cu, cu, 321, 321, 0.0, None, True, window)
+    o, *_, lse, _, _ = F._flash_attn_varlen_forward(q, k, v, *args)
+    dq, dk, dv = (torch.full_like(t, float("nan")) for t in (q, k, v))
+    F._flash_attn_varlen_backward(d_o, q, k, v, o, lse, dq, dk, dv, *args)
+    A.check_status()
+    qd, kd, vd = (t.double().requires_grad_() for t in (q, k, v))
+    if window == (-1, -1):
+        ref = _documents(qd, kd, vd, cu, True)
+    else:
+        s = torch.einsum("qhd,khd->hqk", qd, kd.repeat_interleave(2, 1)) / math.sqrt(128)
+        r, c = torch.arange(T, device="cuda")[:, None], torch.arange(T, device="cuda")[None]
+        doc = torch.bucketize(torch.arange(T, device="cuda"), torch.tensor(cu, device="cuda"), right=True)
+        seen = (c <= r) & (c >= r - window[0]) & (doc[:, None] == doc[None]) & (r < cu[-1])
+        p = torch.softmax(s.masked_fill(~seen, -1e30), -1) * seen
+        ref = torch.einsum("hqk,khd->qhd", p, vd.repeat_interleave(2, 1))
+    ref.backward(d_o.double())
+    assert _close(o, ref.detach())
+    for got, want in ((dq, qd.grad), (dk, kd.grad), (dv, vd.grad)):
+        assert _close(got, want) and (got[cu[-1]:] == 0).all()

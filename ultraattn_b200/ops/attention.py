@@ -674,6 +674,9 @@ def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense
     causal), dQ cast into ``dq``; ``dk`` and ``dv`` are written by the kernel."""
     B, S, H, D = q.shape
     assert lse.dtype == torch.float32 and lse.is_contiguous() and dq.is_contiguous()
+    # (the library takes the strides of lse, and how far dK / dV are written, from the shapes of q and k)
+    assert lse.shape == (B, H, S), f"lse must be [batch, heads, tokens] of the queries {(B, H, S)}, not {tuple(lse.shape)}"
+    assert all(n >= m for g in (dk, dv) for n, m in zip(g.shape, k.shape)), "dK / dV have no room for every key"
     assert o.shape == q.shape == d_o.shape == dq.shape and o.dtype == dq.dtype == dk.dtype == dv.dtype == torch.bfloat16
     so, sd, sk = o.stride(), d_o.stride(), dk.stride()
     assert so[3] == 1 and so[2] == 128 and sd[2] == 128 and sk[3] == 1 and sk[2] == 128 and sk == dv.stride()

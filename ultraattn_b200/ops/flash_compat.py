@@ -134,6 +134,15 @@ def _pad_lse(lse_packed, cu_q, max_seqlen_q):
     return out
 
 
+def _packed_lse(softmax_lse, cu_q, total: int):
+    """The inverse of :func:`_pad_lse`: padded [n_seq, H, max_seqlen] -> [H, total]; tokens outside every
+    sequence attend to nothing (-inf)."""
+    out = torch.full((softmax_lse.shape[1], total), float("-inf"), dtype=softmax_lse.dtype, device=softmax_lse.device)
+    for i, (a, b) in enumerate(_bounds(cu_q)):
+        out[:, a:b] = softmax_lse[i, :, :b - a]
+    return out
+
+
 def _flash_attn_varlen_forward(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, dropout_p,
                                softmax_scale, causal, window_size=(-1, -1), alibi_slopes=None,
                                return_softmax=False, block_table=None, out: Optional[torch.Tensor] = None):
@@ -167,10 +176,7 @@ def _flash_attn_varlen_backward(dout, q, k, v, out, softmax_lse, dq, dk, dv, cu_
     ``[H, Tq]``. Writes ``dq``, ``dk``, ``dv`` (packed) in place."""
     _check(dropout_p, window_size, alibi_slopes, windows_ok=True)
     bq, bk = _bounds(cu_seqlens_q), _bounds(cu_seqlens_k)
-    if softmax_lse.dim() == 3:
-        lse = torch.cat([softmax_lse[i, :, :b - a] for i, (a, b) in enumerate(bq)], dim=1)
-    else:
-        lse = softmax_lse
+    lse = _packed_lse(softmax_lse, cu_seqlens_q, q.shape[0]) if softmax_lse.dim() == 3 else softmax_lse
     if _windowed(window_size):
         assert bq == bk, "sliding windows need equal query and key lengths"
         if softmax_d is None:
