@@ -48,6 +48,33 @@ def test_one_call_backward_refuses_other_shapes(calls):
     assert len(calls) == 1
 
 
+def _one_head(S, pad=0):
+    """[2, S, 1, 128] whose head axis has the stride of all tokens."""
+    t = _bf16(2, 1, S + pad, 128)[:, :, :S].transpose(1, 2)
+    assert t.stride(2) == (S + pad) * 128
+    return t
+
+
+def test_one_call_backward_takes_any_stride_of_an_axis_of_one(calls):
+    S = 64
+    t = {n: _one_head(S) for n in ("o", "d_o", "dk", "dv")}
+    _local(B=2, S=S, H=1, Hk=1, **t)
+    _local(B=2, S=S, H=1, Hk=1, dk=_one_head(S), dv=_bf16(2, S, 1, 128))             # the same addresses
+    # one token: its stride means nothing either
+    one = _bf16(2, 4, 1, 128).transpose(1, 2)
+    _local(B=2, S=1, H=4, Hk=4, o=one, d_o=one, dk=one, dv=_bf16(2, 1, 4, 128))
+    assert len(calls) == 3
+    f = calls[0][0]
+    assert f[21:28] == (t["d_o"].data_ptr(), S, 1, 2, 128, S * 128, S * 128)         # q, k, v: seven fields each
+    assert f[28:31] == (t["o"].data_ptr(), 128, S * 128)
+    assert f[35:39] == (t["dk"].data_ptr(), t["dv"].data_ptr(), 128, S * 128)
+    heads_apart = _bf16(2, 4, S, 128).transpose(1, 2)                                # more than one: they must lie side by side
+    for bad in (dict(o=heads_apart), dict(d_o=heads_apart), dict(H=2, Hk=1, dk=_one_head(S), dv=_one_head(S, 3))):
+        with pytest.raises(AssertionError):
+            _local(**{"B": 2, "S": S, **bad})
+    assert len(calls) == 3
+
+
 def test_packed_lse_covers_the_whole_buffer():
     cu, H, total = [0, 5, 5, 12], 3, 16
     lse = torch.randn(H, total)
@@ -102,3 +129,42 @@ def test_packed_batch_with_a_tail_outside_the_sequences(window):
     assert _close(o, ref.detach())
     for got, want in ((dq, qd.grad), (dk, kd.grad), (dv, vd.grad)):
         assert _close(got, want) and (got[cu[-1]:] == 0).all()
+
+
+def _attend(kind, q, k, v):
+    from ultraattn_b200 import api, attention, patterns as P
+    if kind == "dense":
+        return attention(q, k, v, P.causal(1))
+    if kind == "blocks":
+        return attention(q, k, v, P.causal(2))
+    if kind == "flash":
+        return F.flash_attn_func(q, k, v, causal=True)
+    if kind == "varlen":
+        return api.varlen_attention(q, k, v, [0, q.shape[1]])
+    from ultraattn_b200.ops.window import sliding_window_attention
+    return sliding_window_attention(q, k, v, (k.shape[1] - 1 if kind == "wide window" else 70, 0), causal=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["dense", "blocks", "flash", "varlen"])
+def test_one_head_through_transposes(kind):
+    """The output's gradient, and a single key / value head, come in as views of [B, 1, S, 128]."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    B, S = (1 if kind == "varlen" else 2), 300
+    g = torch.Generator(device="cuda").manual_seed(1)
+    mk = lambda *s: torch.randn(*s, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    for H in (1, 4):
+        q, d_o, k, v = mk(B, S, H), mk(B, H, S), mk(B, 1, S).transpose(1, 2), mk(B, 1, S).transpose(1, 2)
+        q, k, v = (t.requires_grad_() for t in (q, k, v))
+        o = _attend(kind, q, k, v)
+        got = torch.autograd.grad(o.transpose(1, 2), (q, k, v), d_o)
+        A.check_status()
+        qd, kd, vd = (t.detach().double().requires_grad_() for t in (q, k, v))
+        s = torch.einsum("bqhd,bkd->bhqk", qd, kd[:, :, 0]) / math.sqrt(128)
+        r, c = torch.arange(S, device="cuda")[:, None], torch.arange(S, device="cuda")[None]
+        s = s.masked_fill((c > r) | ((c < r - 70) & (kind == "window")), float("-inf"))
+        ref = torch.einsum("bhqk,bkd->bhqd", torch.softmax(s, -1), vd[:, :, 0])
+        want = torch.autograd.grad(ref, (qd, kd, vd), d_o.double())
+        assert _close(o.transpose(1, 2).detach(), ref.detach())
+        assert all(_close(a, b) for a, b in zip(got, want))

@@ -668,6 +668,14 @@ def attn_bwd_dense(q_side: BwdQSide, k, v, kv_out: BwdKvOut, causal: bool, softm
     attn_bwd_cuda([q_side], [k], [v], [kv_out], None, softmax_scale, None, 2 if causal else 1)
 
 
+def _row_strides(t: torch.Tensor) -> tuple[int, int]:
+    """(token, batch) strides of ``[batch, tokens, heads, 128]`` whose heads lie side by side. What stride an
+    axis of size 1 has means nothing: one head seen through a transpose has that of the tokens."""
+    st = t.stride()
+    assert st[3] == 1 and (st[2] == 128 or t.shape[2] == 1), "the heads of a token must be contiguous"
+    return st[1], st[0]
+
+
 def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense: int = 0, softmax_scale=None) -> torch.Tensor:
     """The whole backward on one CUDA device in one call of the library: D = rowdot(O, dO) (returned, ``[B,
     H, S]``), the kernel under ``plan`` (or ``dense`` = 1 / 2: all queries against all keys, without a mask /
@@ -678,8 +686,9 @@ def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense
     assert lse.shape == (B, H, S), f"lse must be [batch, heads, tokens] of the queries {(B, H, S)}, not {tuple(lse.shape)}"
     assert all(n >= m for g in (dk, dv) for n, m in zip(g.shape, k.shape)), "dK / dV have no room for every key"
     assert o.shape == q.shape == d_o.shape == dq.shape and o.dtype == dq.dtype == dk.dtype == dv.dtype == torch.bfloat16
-    so, sd, sk = o.stride(), d_o.stride(), dk.stride()
-    assert so[3] == 1 and so[2] == 128 and sd[2] == 128 and sk[3] == 1 and sk[2] == 128 and sk == dv.stride()
+    so, sk, sv = _row_strides(o), _row_strides(dk), _row_strides(dv)
+    _row_strides(d_o)
+    assert all(x == y for x, y, n in zip(sk, sv, (k.shape[1], B)) if n > 1), "dK and dV must be laid out alike"
     if debug_bounds_enabled():
         cols = plan.cols if not dense else [Col(0, 0, k.shape[1], (Seg(0, 0, S, dense == 2, k.shape[1] - S),), 0, 0)]
         _raise_if_bad("backward", check_bwd_tables(cols, [BwdQSide(q, d_o, lse, lse, q)], [k], [v], [BwdKvOut(dk, dv)]))
@@ -687,8 +696,8 @@ def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense
     ws = torch.empty(n * (D + 1), dtype=torch.float32, device=q.device)      # dQ accumulator, then D
     w = ws.data_ptr()
     tables = (0, 0, 0, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(), plan.n_tiles)
-    block = _LOCAL_BWD.pack(*_src_fields(q), *_src_fields(k), *_src_fields(v), *_src_fields(d_o), o.data_ptr(), so[1], so[0],
-                            lse.data_ptr(), w + 4 * n * D, w, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), sk[1], sk[0],
+    block = _LOCAL_BWD.pack(*_src_fields(q), *_src_fields(k), *_src_fields(v), *_src_fields(d_o), o.data_ptr(), *so,
+                            lse.data_ptr(), w + 4 * n * D, w, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *sk,
                             *tables, dense)
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     rc = _lib.load().ua_attn_bwd_local(block, scale, status_buffer(q.device).data_ptr(), _lib.stream_of(q))
