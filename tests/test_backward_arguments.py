@@ -75,6 +75,20 @@ def test_one_call_backward_takes_any_stride_of_an_axis_of_one(calls):
     assert len(calls) == 3
 
 
+@pytest.mark.parametrize("full", [True, False])
+def test_window_gradients_of_one_head_are_laid_out_for_the_kernel(monkeypatch, full):
+    from ultraattn_b200.ops import window as W
+    outs = []
+    monkeypatch.setattr(A, "attn_bwd", lambda sides, k, v, kv, plan, scale: outs.extend(kv))
+    S, k, v = 64, _one_head(64), _one_head(64)
+    q = _bf16(2, S, 4, 128)
+    z = torch.zeros(2, 4, S)
+    dq, dk, dv = W._cuda_backward(q, q, k, v, z, z, torch.zeros(2, S, 4, 128), None, None, full, 1.0)
+    assert dk.shape == k.shape and dv.shape == v.shape
+    for t in (outs[0].dk, outs[0].dv):
+        assert t.stride() == (S * 128, 128, 128, 1)
+
+
 def test_packed_lse_covers_the_whole_buffer():
     cu, H, total = [0, 5, 5, 12], 3, 16
     lse = torch.randn(H, total)
@@ -146,7 +160,7 @@ def _attend(kind, q, k, v):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kind", ["dense", "blocks", "flash", "varlen"])
+@pytest.mark.parametrize("kind", ["dense", "blocks", "flash", "varlen", "window", "wide window"])
 def test_one_head_through_transposes(kind):
     """The output's gradient, and a single key / value head, come in as views of [B, 1, S, 128]."""
     if not torch.cuda.is_available():

@@ -270,8 +270,9 @@ def _cuda_forward(q, k, v, out, fplan, full: bool, scale):
 def _cuda_backward(d_o, q, k, v, lse, softmax_d, dq32, bplan, sink_idx, full: bool, scale):
     """One launch: fp32 dQ accumulator (zeroed ``dq32``), dK / dV written in the inputs' type by their only producer (the
     sink keys', which have several, go through a small fp32 buffer)."""
-    new = torch.empty_like if full else torch.zeros_like
-    dk, dv = new(k), new(v)
+    # (from the shapes: empty_like would keep the strides that one key/value head has through a transpose)
+    new = torch.empty if full else torch.zeros
+    dk, dv = (new(t.shape, dtype=t.dtype, device=t.device) for t in (k, v))
     outs = [A.BwdKvOut(dk, dv)]
     if sink_idx is not None:
         shape = (k.shape[0], sink_idx.numel(), k.shape[2], k.shape[3])
