@@ -182,3 +182,36 @@ def test_one_head_through_transposes(kind):
         want = torch.autograd.grad(ref, (qd, kd, vd), d_o.double())
         assert _close(o.transpose(1, 2).detach(), ref.detach())
         assert all(_close(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("packed", [False, True])
+def test_fp32_key_gradients_are_added_into(packed):
+    """dK / dV in fp32: the same gradients with and without D given, on top of what the buffers hold (the packed
+    form clears them first)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    B, S, H, Hk = 1, 300, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(2)
+    mk = lambda h: torch.randn(B, S, h, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, k, v, d_o = mk(H), mk(Hk), mk(Hk), mk(H)
+    cu = [0, 120, 300]
+    if packed:
+        q, k, v, d_o = (t[0] for t in (q, k, v, d_o))
+        o, *_, lse, _, _ = F._flash_attn_varlen_forward(q, k, v, cu, cu, 180, 180, 0.0, None, True)
+        back = lambda dq, dk, dv, d: F._flash_attn_varlen_backward(d_o, q, k, v, o, lse, dq, dk, dv, cu, cu, 180, 180, 0.0, None,
+                                                                   True, softmax_d=d)[3]
+    else:
+        o, *_, lse, _, _ = F._flash_attn_forward(q, k, v, 0.0, None, True)
+        back = lambda dq, dk, dv, d: F._flash_attn_backward(d_o, q, k, v, o, lse, dq, dk, dv, 0.0, None, True, softmax_d=d)[3]
+    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+    d = back(dq, dk, dv, None)                                     # bf16: written
+    start = 0.0 if packed else 3.0
+    for given in (None, d):
+        dq2, dk2, dv2 = torch.empty_like(q), torch.full_like(k, 3.0, dtype=torch.float32), torch.full_like(v, 3.0, dtype=torch.float32)
+        d2 = back(dq2, dk2, dv2, given)
+        A.check_status()
+        assert torch.equal(d2, d)
+        assert (dq2.float() - dq.float()).norm() <= 2 ** -8 * dq.float().norm()      # (summed in arrival order, then rounded)
+        for a, b in ((dk2, dk), (dv2, dv)):
+            assert (a - start - b.float()).norm() <= 2 ** -8 * b.float().norm()

@@ -58,7 +58,9 @@ def _forward(q, k, v, rows, out, softmax_scale):
 def _backward(dout, q, k, v, out, lse, dq, dk, dv, cols, softmax_scale, softmax_d, causal=False):
     """``cols``: the work items of a packed batch, or None: all queries against all keys (``causal``)."""
     B, S, H, D = q.shape
-    if q.is_cuda and softmax_d is None and lse.is_contiguous() and dq.is_contiguous():
+    # (fp32 dK / dV, which the kernel adds into, take the way of separate calls)
+    if (q.is_cuda and softmax_d is None and lse.is_contiguous() and dq.is_contiguous()
+            and dk.dtype == dv.dtype == torch.bfloat16):
         return A.attn_bwd_local(q, k, v, out, lse, dout.contiguous(), dq, dk, dv,
                                 None if cols is None else A.BwdPlan(cols, q.device),
                                 0 if cols is not None else (2 if causal else 1), softmax_scale)
