@@ -215,3 +215,30 @@ def test_fp32_key_gradients_are_added_into(packed):
         assert (dq2.float() - dq.float()).norm() <= 2 ** -8 * dq.float().norm()      # (summed in arrival order, then rounded)
         for a, b in ((dk2, dk), (dv2, dv)):
             assert (a - start - b.float()).norm() <= 2 ** -8 * b.float().norm()
+
+
+def test_preparation_refuses_misaligned_tensors_before_the_launch():
+    """Argument checks at the C entry: no launch happens (and no GPU is needed)."""
+    lib = _lib.load()
+    n = 4 * 2 * 128
+    ok = dict(o=1 << 20, d_o=2 << 20, dvec=3 << 20, dq=4 << 20, o_b=n, o_t=256, d_b=n, d_t=256, batch=2, tokens=4, heads=2)
+    for bad in (dict(o=(1 << 20) + 2), dict(d_o=(2 << 20) + 8), dict(dq=(4 << 20) + 4), dict(o_t=257), dict(d_t=260),
+                dict(o_b=n + 1), dict(d_b=n + 4)):
+        a = {**ok, **bad}
+        assert lib.ua_bwd_prepare(*a.values(), None) != 0
+        assert b"16 bytes" in lib.ua_last_error()
+
+
+@pytest.mark.gpu
+def test_preparation_reads_heads_that_lie_apart():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    from ultraattn_b200.ops import elementwise as E
+    B, S, H = 2, 70, 3
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mk = lambda *s: torch.randn(*s, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    plain, apart, one = mk(B, S, H), mk(B, H, S).transpose(1, 2), mk(B, 1, S).transpose(1, 2)
+    for o, d_o in ((plain, apart), (apart, plain), (one, one * 2)):
+        d, zero = E.bwd_prepare(o, d_o)
+        assert (zero == 0).all()
+        assert (d - (o.double() * d_o.double()).sum(-1).transpose(1, 2)).abs().max() < 1e-3

@@ -810,6 +810,10 @@ extern "C" int ua_bwd_prepare(const void* o, const void* d_o, float* dvec, float
                               long do_bstride, long do_stride, int batch, int tokens, int heads, cudaStream_t stream) {
   const long threads = static_cast<long>(batch) * tokens * heads * 16;
   if (threads == 0) return 0;
+  // the kernel reads and writes 16 bytes at a time (o and d_o may be views of a caller's buffers)
+  const long odd = (tokens > 1 ? o_stride | do_stride : 0) | (batch > 1 ? o_bstride | do_bstride : 0);
+  const auto at = reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o) | reinterpret_cast<uintptr_t>(dq);
+  if (odd % 8 != 0 || at % 16 != 0) UA_FAIL("ua_bwd_prepare: O and dO must start, and step, in multiples of 16 bytes");
   bwd_prepare_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), dvec, dq, o_bstride, o_stride,
       do_bstride, do_stride, batch, tokens, heads);

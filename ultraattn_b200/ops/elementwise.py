@@ -75,6 +75,8 @@ def bwd_prepare(o: torch.Tensor, d_o: torch.Tensor) -> tuple[torch.Tensor, torch
             rowdot(o[b], d_o[b], dvec[b])
         return dvec, torch.zeros(B, S, H, D, dtype=torch.float32, device=o.device)
     dq = torch.empty(B, S, H, D, dtype=torch.float32, device=o.device)
+    # the kernel finds a token's heads side by side
+    o, d_o = (t if t.stride(3) == 1 and (t.stride(2) == D or H == 1) else t.contiguous() for t in (o, d_o))
     rc = _lib.load().ua_bwd_prepare(o.data_ptr(), d_o.data_ptr(), dvec.data_ptr(), dq.data_ptr(), o.stride(0),
                                     o.stride(1), d_o.stride(0), d_o.stride(1), B, S, H, _stream(o))
     _lib.check(rc, "ua_bwd_prepare")
