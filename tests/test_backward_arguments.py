@@ -48,6 +48,11 @@ def test_one_call_backward_refuses_other_shapes(calls):
     assert len(calls) == 1
 
 
+def test_returned_row_products_do_not_keep_the_workspace(calls):
+    d = _local()
+    assert d.shape == (1, 4, 64) and d.untyped_storage().nbytes() == 4 * d.numel()
+
+
 def _one_head(S, pad=0):
     """[2, S, 1, 128] whose head axis has the stride of all tokens."""
     t = _bf16(2, 1, S + pad, 128)[:, :, :S].transpose(1, 2)

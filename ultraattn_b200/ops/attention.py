@@ -692,17 +692,17 @@ def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense
     if debug_bounds_enabled():
         cols = plan.cols if not dense else [Col(0, 0, k.shape[1], (Seg(0, 0, S, dense == 2, k.shape[1] - S),), 0, 0)]
         _raise_if_bad("backward", check_bwd_tables(cols, [BwdQSide(q, d_o, lse, lse, q)], [k], [v], [BwdKvOut(dk, dv)]))
-    n = B * S * H
-    ws = torch.empty(n * (D + 1), dtype=torch.float32, device=q.device)      # dQ accumulator, then D
-    w = ws.data_ptr()
+    # (two tensors: a caller who keeps D must not keep the dQ accumulator, 128 times its size, alive with it)
+    dvec = torch.empty(B, H, S, dtype=torch.float32, device=q.device)
+    dq32 = torch.empty(B * S * H * D, dtype=torch.float32, device=q.device)
     tables = (0, 0, 0, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(), plan.n_tiles)
     block = _LOCAL_BWD.pack(*_src_fields(q), *_src_fields(k), *_src_fields(v), *_src_fields(d_o), o.data_ptr(), *so,
-                            lse.data_ptr(), w + 4 * n * D, w, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *sk,
+                            lse.data_ptr(), dvec.data_ptr(), dq32.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *sk,
                             *tables, dense)
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     rc = _lib.load().ua_attn_bwd_local(block, scale, status_buffer(q.device).data_ptr(), _lib.stream_of(q))
     _lib.check(rc, "ua_attn_bwd_local", 3)
-    return ws[n * D:].view(B, H, S)
+    return dvec
 
 
 def cols_from_block_table(table: np.ndarray, block: int, kv_block: int | None = None) -> list[Col]:
