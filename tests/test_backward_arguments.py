@@ -247,3 +247,35 @@ def test_preparation_reads_heads_that_lie_apart():
         d, zero = E.bwd_prepare(o, d_o)
         assert (zero == 0).all()
         assert (d - (o.double() * d_o.double()).sum(-1).transpose(1, 2)).abs().max() < 1e-3
+
+
+def test_plans_know_how_many_gradient_rows_they_write():
+    from ultraattn_b200 import api, patterns as P
+    tokens = lambda plans: plans[1].kv_tokens
+    assert tokens(api.varlen_plans([0, 5, 5, 12], True, "cpu")) == 12
+    assert tokens(api.prefix_lm_plans(16, 3, "cpu", [0, 2, 9])) == 9
+    for pattern in (P.causal(4), P.star(4, 1), P.streaming(4, 1, 2)):       # (empty blocks are columns too: zeros)
+        assert tokens(api.local_plans(pattern, 64, "cpu")) == 64
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prefix", [None, 30])
+def test_gradients_of_tokens_outside_every_sequence_are_zero(prefix):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    from ultraattn_b200 import api
+    T, H, Hk, cu = 512, 4, 2, [0, 100, 421]
+    g = torch.Generator(device="cuda").manual_seed(4)
+    mk = lambda h: torch.randn(T, h, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, k, v, d_o = mk(H).requires_grad_(), mk(Hk).requires_grad_(), mk(Hk).requires_grad_(), mk(H)
+    o = (api.varlen_attention(q, k, v, cu) if prefix is None else
+         api.prefix_lm_attention(q, k, v, prefix, cu_seqlens=cu))
+    junk = [torch.full_like(t, float("nan")) for t in (q, k, v, k, v)]      # what the allocator hands out next holds NaN
+    del junk
+    got = torch.autograd.grad(o, (q, k, v), d_o)
+    A.check_status()
+    assert (o[cu[-1]:] == 0).all() and all((t[cu[-1]:] == 0).all() for t in got)
+    if prefix is None:
+        ref = [t.detach().double().requires_grad_() for t in (q, k, v)]
+        _documents(*ref, cu, True).backward(d_o.double())
+        assert all(_close(a, b.grad) for a, b in zip(got, ref))

@@ -67,7 +67,10 @@ def local_backward(q, k, v, o, lse, d_o, bplan, softmax_scale=None, dense: int =
     """dQ, dK, dV of the single-device operator (bf16 on CUDA, input dtype on CPU). ``dense`` = 1 / 2:
     full / causal attention over all tokens; ``bplan`` is not read."""
     if q.is_cuda:
-        dq, dk, dv = torch.empty(q.shape, dtype=q.dtype, device=q.device), torch.empty_like(k), torch.empty_like(v)
+        # the kernel writes the gradients of every key in a column of the plan; only keys outside all of them
+        # (tokens of a packed buffer that belong to no sequence) need a fill
+        new = torch.empty_like if dense or bplan.kv_tokens == k.shape[1] else torch.zeros_like
+        dq, dk, dv = torch.empty(q.shape, dtype=q.dtype, device=q.device), new(k), new(v)
         A.attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, bplan, dense, softmax_scale)
         return dq, dk, dv
     dvec, dq32 = E.bwd_prepare(o, d_o)

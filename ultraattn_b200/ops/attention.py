@@ -533,6 +533,7 @@ class BwdPlan:
                 tiles.append((_col_steps(c, t * TILE), ci, t))
         tiles = _launch_order(tiles)
         self.n_tiles = len(tiles)
+        self.kv_tokens = sum(c.kv_len for c in self.cols)      # gradient rows that the columns write
         self.total_steps = sum(c for c, _, _ in tiles)
         seg_arr = np.array(segs, dtype=np.int32).reshape(-1, 8) if segs else np.zeros((1, 8), np.int32)
         tile_arr = (np.array([(ci, t) for _, ci, t in tiles], dtype=np.int32).reshape(-1, 2)
