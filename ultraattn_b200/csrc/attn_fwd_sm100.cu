@@ -142,7 +142,7 @@ struct __align__(1024) FwdSmem {
   uint64_t p_full[2];
   uint64_t p_part[2];    // the first P_PART keys of P are there
   uint64_t q_empty;
-  uint64_t o_full;
+  uint64_t o_full[2];    // FEW: of each sub-tile that had a key tile; else [0] for both
   uint4 clc;             // response of a cancellation request
   uint64_t clc_full;
   FwdItem item[2];       // item number n in slot n & 1
@@ -432,6 +432,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       mbar_init(&s.s_full[i], 1);
       mbar_init(&s.p_full[i], act_warps);   // one arrival per softmax warp
       mbar_init(&s.p_part[i], act_warps);
+      mbar_init(&s.o_full[i], 1);
       mbar_init(&s.item_full[i], 1);
       mbar_init(&s.item_empty[i], 1 + 2 * act_warps);   // MMA warp and softmax warps
     }
@@ -443,7 +444,6 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     }
     mbar_init(&s.q_empty, 1);
     mbar_init(&s.clc_full, 1);
-    mbar_init(&s.o_full, 1);
     s.item[0] = item0;
     s.abort_flag = 0;
     fence_mbar_init();
@@ -662,7 +662,11 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
             }
           }
           if (!ok) break;
-          tc_commit(&s.o_full);
+          // A sub-tile's next completion must not come before its warps have seen this one. They have when
+          // they arrive on p_full of the next item, which only a sub-tile with a key tile there is
+          // waited for: with one barrier for both, two items in a row could complete it unseen.
+          tc_commit(&s.o_full[0]);
+          if (FEW && n_total > 1) tc_commit(&s.o_full[1]);
           kv += n_total;
           ++live;
         }
@@ -683,7 +687,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     const uint32_t tO = tmem_base + lane_base + 256 + w * 128;
     const float NEG_INF = -INFINITY;
     uint32_t cnt = 0;                        // score tiles of this sub-tile so far
-    uint32_t live = 0;
+    uint32_t live = 0;                       // items with a key tile for this sub-tile so far
     for (uint32_t n = 0;; ++n) {
     const FwdItem& it = s.item[n & 1];       // (stays in shared memory: the score loop needs the registers)
     const int r_blk = (it.r0 + r_cta) >> psh;               // query token inside the query block
@@ -805,13 +809,13 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       }
     }
     // ---------------------------------- epilogue --------------------------------------------
-    const uint32_t n_total = j;
-    if (n_total > 0 && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full, live & 1, wc, 310 + w));
+    const bool any = j > (FEW ? static_cast<uint32_t>(w) : 0u);
+    if (any && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full[FEW ? w : 0], live & 1, wc, 310 + w));
     tc_fence_after_sync();
-    if constexpr (FEW) fwd_epilogue<true>(s, n & 1, tO, l, m_use, n_total > static_cast<uint32_t>(w));
-    else fwd_epilogue_call(s, n & 1, tO, l, m_use, n_total > 0);
+    if constexpr (FEW) fwd_epilogue<true>(s, n & 1, tO, l, m_use, any);
+    else fwd_epilogue_call(s, n & 1, tO, l, m_use, any);
     trace_stamp(p.trace, it.linear, 2);
-    if (n_total > 0) ++live;
+    if (any) ++live;
     if (!ok) break;
     __syncwarp();                            // every lane is done reading the item
     int more = 0;
