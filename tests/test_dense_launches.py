@@ -113,3 +113,32 @@ def test_backward_in_one_call_equals_its_parts(B, S, H, Hk, kind):
     A.check_status()
     assert torch.equal(got[1], out.dk) and torch.equal(got[2], out.dv)
     assert (got[0].float() - dq32).norm() <= 2 ** -8 * dq32.norm()
+
+
+@pytest.mark.parametrize("Sq", [1, 300])
+@pytest.mark.parametrize("n_split", [1, 4])
+def test_values_that_are_not_finite_do_not_depend_on_the_split(Sq, n_split):
+    """A NaN or infinite score: the row has O = 0 and lse = -inf. A NaN in V: NaN in that column of O."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    Skv, H = 1400, 2
+    g = torch.Generator(device="cuda").manual_seed(5)
+    mk = lambda s: torch.randn(1, s, H, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, k, v = mk(Sq), mk(Skv), mk(Skv)
+    for value in (float("nan"), float("inf")):
+        k2 = k.clone()
+        k2[0, 700, 0, 5] = value
+        q2 = q.clone()
+        q2[:, :, 0, 5] = 1.0
+        o, lse = torch.full_like(q, 7.0), torch.full((1, H, Sq), 7.0, device="cuda")
+        A.attn_fwd_dense(q2, k2, v, (o, lse), False, None, n_split)
+        assert (o[:, :, 0] == 0).all() and (lse[:, 0] == -math.inf).all()
+        assert torch.isfinite(lse[:, 1]).all() and (o[:, :, 1] != 0).any(-1).all()
+    v2 = v.clone()
+    v2[0, 900, 1, 3] = float("nan")
+    k2 = k * 30                                     # parts whose weight is exactly zero, too
+    o, lse = torch.full_like(q, 7.0), torch.full((1, H, Sq), 7.0, device="cuda")
+    A.attn_fwd_dense(q, k2, v2, (o, lse), False, None, n_split)
+    A.check_status()
+    bad = torch.isnan(o[0])
+    assert bad[:, 1, 3].all() and bad.sum() == Sq and torch.isfinite(lse).all()

@@ -273,7 +273,10 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
   // fp32 part of a split launch: rows of 128 floats, [batch, parts, tokens, heads]
   const bool f32 = s.hot.part_o != nullptr;
   const long part0 = f32 ? (static_cast<long>(it.batch) * s.hot.n_parts + (FEW ? 2 * it.split + w : it.split)) * it.row.q_len : 0;
-  if (f32) lptr = s.hot.part_lse + (part0 + r_blk) * s.hot.n_heads + qh;
+  if (f32) {
+    lptr = s.hot.part_lse + (part0 + r_blk) * s.hot.n_heads + qh;
+    if (any && l != l) lse = l;          // a NaN score makes the whole row one without keys (combine_kernel), not this part
+  }
   if (valid_row) *lptr = lse;
   if (!FEW && !it.row.accumulate) {
     // A thread owns a row, so storing from registers would scatter 16 bytes to each of 32 rows per
@@ -847,9 +850,15 @@ combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_
   const long batch = r / per_part, in = r % per_part;           // in = token * heads + head
   const long first = batch * n_parts * per_part + in;
   float mx = -INFINITY;
-  for (int i = lane; i < n_parts; i += 32) mx = fmaxf(mx, part_lse[first + i * per_part]);
+  bool bad = false;                    // a NaN score: the row comes out as in a launch without parts, O = 0 and lse = -inf
+  for (int i = lane; i < n_parts; i += 32) {
+    const float x = part_lse[first + i * per_part];
+    bad |= x != x;
+    mx = fmaxf(mx, x);
+  }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, d));
+  if (__any_sync(0xFFFFFFFFu, bad)) mx = -INFINITY;
   float tot = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (mx > -INFINITY) {
@@ -857,13 +866,11 @@ combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_
     for (int i = 0; i < n_parts; ++i) {
       const float w = __expf(part_lse[first + i * per_part] - mx);
       const float4 v = *reinterpret_cast<const float4*>(part_o + (first + i * per_part) * ATTN_D + lane * 4);
-      tot += w;
-      if (w != 0.f) {
-        acc.x += w * v.x;
-        acc.y += w * v.y;
-        acc.z += w * v.z;
-        acc.w += w * v.w;
-      }
+      tot += w;                          // (w = 0 also times what is not finite, as P V does with P = 0)
+      acc.x += w * v.x;
+      acc.y += w * v.y;
+      acc.z += w * v.z;
+      acc.w += w * v.w;
     }
   }
   const float inv = tot > 0.f ? 1.f / tot : 0.f;
