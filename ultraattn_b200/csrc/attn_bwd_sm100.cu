@@ -832,6 +832,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     if (ok) {
       if (lane == 0) more = item_ready(n + 1) ? 1 : 0;
       more = __shfl_sync(0xFFFFFFFFu, more, 0);
+      __syncwarp();                          // lane 0 has seen the item; this makes it visible to the others (a shuffle does not)
     }
     const int n_done = n_steps;
     if (more) {
@@ -919,6 +920,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       more = ok && item_ready(n + 1) ? 1 : 0;
     }
     if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
+    __syncwarp();
     }
     if (lane == 0) tma_store_wait_all();
     __syncwarp();

@@ -824,6 +824,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     int more = 0;
     if (lane == 0) more = next_item(n) ? 1 : 0;
     if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
+    __syncwarp();                            // lane 0 has seen the item; this makes it visible to the others (a shuffle does not)
     }
   }
   }
