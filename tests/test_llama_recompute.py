@@ -45,3 +45,28 @@ def test_embedding_gradient_on_the_kernel(T, H, V, kind):
     ref = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
     # one rounding to bf16 of an fp32 sum
     assert ((got.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-5).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,H,kind", [(33, 8, "runs"), (2000, 64, "runs"), (3001, 2056, "runs"), (6000, 128, "one id"),
+                                      (6000, 128, "a third"), (20000, 256, "runs")])
+def test_embedding_gradient_of_frequent_ids(T, H, kind):
+    """Runs around the length from which on an id's rows are summed in pieces, at every place in a piece."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    V, c = 400, E._embedding_chunk(T)
+    g = torch.Generator().manual_seed(T)
+    if kind == "runs":
+        lengths = torch.tensor([c, c + 1, 1, c - 1, 2 * c + 1, 3, 2 * c, 5 * c + 2, c + 1]).repeat(T)
+        ids = torch.repeat_interleave(torch.arange(len(lengths)) * 2 % V, lengths)[:T].sort().values     # (odd ids do not occur)
+    else:
+        ids = torch.randint(0, V, (T,), generator=g)
+        ids[torch.rand(T, generator=g) < (1.0 if kind == "one id" else 0.3)] = V - 1
+    ids = ids[torch.randperm(T, generator=g)].cuda()
+    dy = torch.randn(T, H, generator=g).to("cuda", torch.bfloat16)
+    got = E.embedding_bwd(ids, dy, V)
+    zero = torch.zeros(V, H, device="cuda", dtype=torch.float64)
+    ref, size = zero.index_add(0, ids, dy.double()), zero.index_add(0, ids, dy.double().abs())
+    # additions in a row: along a piece, then along the pieces; each rounds to 2^-24 of what has been summed; bf16 once
+    assert ((got.double() - ref).abs() <= 2 ** -8 * ref.abs() + (c + T // c + 2) * 2 ** -24 * size).all()
+    assert torch.equal(got, E.embedding_bwd(ids, dy, V))

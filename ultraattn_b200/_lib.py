@@ -65,7 +65,7 @@ def _declare(lib):
                          vp],
         "ua_rowdot": [vp, vp, vp, l, l, l, i, i, vp],
         "ua_bwd_prepare": [vp, vp, vp, vp, l, l, l, l, i, i, i, vp],
-        "ua_embedding_bwd": [vp, vp, vp, vp, i, i, i, vp],
+        "ua_embedding_bwd": [vp, vp, vp, vp, vp, vp, i, i, i, i, vp],
         "ua_cast_scale": [vp, vp, l, f, i, vp],
         "ua_rmsnorm_fwd": [vp, vp, vp, vp, i, i, f, vp],
         "ua_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, i, i, vp],

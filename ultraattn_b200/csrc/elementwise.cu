@@ -152,36 +152,95 @@ bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __r
   if (valid && sub == 0) dvec[(b * heads + head) * tokens + tok] = acc;
 }
 
-// Gradient of an embedding lookup. One block per vocabulary row: it finds its run in the sorted ids by
-// binary search, sums those rows of dy in fp32 (in token order: the sort is stable) and writes the row,
-// zeros if the run is empty. One pass: T * H * 2 bytes in, vocab * H * 2 out. 8192 tokens, 32000 x 4096:
-// 0.10 ms (0.05 at the memory rate) against 0.73 for the library's two kernels and fill.
-__global__ void __launch_bounds__(256)
-embedding_bwd_kernel(const long* __restrict__ sorted_ids, const long* __restrict__ order,
-                     const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ out, int tokens, int hidden) {
-  __shared__ int run[2];
-  const long v = blockIdx.x;
-  if (threadIdx.x < 2) {                 // first position with an id >= v (thread 0), > v (thread 1)
-    const long key = v + threadIdx.x;
-    int lo = 0, hi = tokens;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (sorted_ids[mid] < key) lo = mid + 1; else hi = mid;
-    }
-    run[threadIdx.x] = lo;
+// Gradient of an embedding lookup, from the sorted ids: the rows of equal ids are a run, and the gradient of a
+// vocabulary row is the sum of its run's rows of dy, in fp32 and token order (the sort is stable).
+//   embedding_bwd_kernel: one block per vocabulary row sums its run and writes the row (zeros if the run is
+//     empty). One pass: T * H * 2 bytes in, vocab * H * 2 out.
+//   embedding_runs_kernel, in front of it, finds where the runs start (a binary search per vocabulary row: in the
+//     blocks above it would be a dozen dependent loads before each row), and sums the long ones in pieces: a run
+//     longer than `chunk` (padding, a separator, the frequent words of a text) would be a serial walk of one block.
+//     A block takes `chunk` positions of the sorted ids and sums what they hold of such runs; being longer
+//     than the chunk, a run covers its first or its last position, so two partial rows per chunk are
+//     enough. The vocabulary row then adds its partials. chunk is about sqrt(T): neither the walk
+//     along a chunk nor the one along the partials is long.
+// Rows of 4096, 32000 vocabulary rows, with the sort, us; library's kernels / one block per run, searching for
+// itself / this:
+//   1024 tokens, uniform ids 130 / 103 / 97; one id in a third of them 130 / 321 / 103
+//   8192 tokens, uniform 766 / 202 / 179; a third 671 / 2134 / 204; one id only 442 / 6962 / 202; Zipf 566 / 773 / 243
+//   65536 tokens, uniform 2567 / 306 / 278; a third 2426 / 15877 / 314; one id only 1546 / 56422 / 382
+constexpr int EMB_THREADS = 256;
+constexpr int EMB_COLS = EMB_THREADS * 8;      // columns of a block's pass
+
+// first position of the ascending ids that is >= key
+__device__ __forceinline__ int first_at_least(const long* __restrict__ ids, int n, long key) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ids[mid] < key) lo = mid + 1; else hi = mid;
   }
-  __syncthreads();
-  const int begin = run[0], end = run[1];
-  for (int c = threadIdx.x * 8; c < hidden; c += 256 * 8) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8                          // independent loads: an id that fills the sequence is one block's work
-    for (int i = begin; i < end; ++i) {
-      const uint4 x = *reinterpret_cast<const uint4*>(dy + order[i] * hidden + c);
-      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+  return lo;
+}
+__device__ __forceinline__ void add_row(float (&acc)[8], const uint4& x) {
+  const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        acc[2 * q] += bf_lo(w[q]);
-        acc[2 * q + 1] += bf_hi(w[q]);
+  for (int q = 0; q < 4; ++q) {
+    acc[2 * q] += bf_lo(w[q]);
+    acc[2 * q + 1] += bf_hi(w[q]);
+  }
+}
+
+// start: [vocab + 1] first positions; part: [chunks][2][hidden]. The first `part_blocks` blocks (chunks x column
+// passes) sum, the others search.
+__global__ void __launch_bounds__(EMB_THREADS)
+embedding_runs_kernel(const long* __restrict__ sorted_ids, const long* __restrict__ order, const __nv_bfloat16* __restrict__ dy,
+                      float* __restrict__ part, int* __restrict__ start, int tokens, int hidden, int vocab, int chunk,
+                      int part_blocks) {
+  if (static_cast<int>(blockIdx.x) >= part_blocks) {
+    const int v = (blockIdx.x - part_blocks) * EMB_THREADS + threadIdx.x;
+    if (v <= vocab) start[v] = first_at_least(sorted_ids, tokens, v);
+    return;
+  }
+  __shared__ int run[4];                 // [begin, end) of the runs at the chunk's first and at its last position
+  const int passes = (hidden + EMB_COLS - 1) / EMB_COLS;
+  const int k = blockIdx.x / passes;
+  const int a = k * chunk, b = min(tokens, a + chunk);
+  if (threadIdx.x < 4)
+    run[threadIdx.x] = first_at_least(sorted_ids, tokens, sorted_ids[threadIdx.x < 2 ? a : b - 1] + (threadIdx.x & 1));
+  __syncthreads();
+  const int c = (blockIdx.x % passes) * EMB_COLS + threadIdx.x * 8;
+  if (c >= hidden) return;
+#pragma unroll 1
+  for (int e = 0; e < 2; ++e) {
+    const int begin = run[2 * e], end = run[2 * e + 1];
+    if (end - begin <= chunk || (e == 1 && begin <= a)) continue;        // short, or the first position's run again
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const int last = min(end, b);
+#pragma unroll 8
+    for (int i = max(begin, a); i < last; ++i) add_row(acc, *reinterpret_cast<const uint4*>(dy + order[i] * hidden + c));
+    float4* d = reinterpret_cast<float4*>(part + (static_cast<long>(k) * 2 + e) * hidden + c);
+    d[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    d[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  }
+}
+
+__global__ void __launch_bounds__(EMB_THREADS)
+embedding_bwd_kernel(const long* __restrict__ order, const __nv_bfloat16* __restrict__ dy, const float* __restrict__ part,
+                     const int* __restrict__ start, __nv_bfloat16* __restrict__ out, int hidden, int chunk) {
+  const long v = blockIdx.x;
+  const int begin = start[v], end = start[v + 1];
+  for (int c = threadIdx.x * 8; c < hidden; c += EMB_COLS) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (end - begin <= chunk) {
+#pragma unroll 4
+      for (int i = begin; i < end; ++i) add_row(acc, *reinterpret_cast<const uint4*>(dy + order[i] * hidden + c));
+    } else {
+#pragma unroll 4
+      for (int k = begin / chunk; k <= (end - 1) / chunk; ++k) {
+        const int e = begin <= k * chunk ? 0 : 1;
+        const float4* p = reinterpret_cast<const float4*>(part + (static_cast<long>(k) * 2 + e) * hidden + c);
+        const float4 x = p[0], y = p[1];
+        acc[0] += x.x; acc[1] += x.y; acc[2] += x.z; acc[3] += x.w;
+        acc[4] += y.x; acc[5] += y.y; acc[6] += y.z; acc[7] += y.w;
       }
     }
     uint4 o;
@@ -821,12 +880,21 @@ extern "C" int ua_bwd_prepare(const void* o, const void* d_o, float* dvec, float
   return 0;
 }
 
-extern "C" int ua_embedding_bwd(const long* sorted_ids, const long* order, const void* dy, void* out, int tokens, int hidden,
-                                int vocab, cudaStream_t stream) {
+// part: 2 * ceil(tokens / chunk) rows of `hidden` floats; start: vocab + 1 ints.
+extern "C" int ua_embedding_bwd(const long* sorted_ids, const long* order, const void* dy, float* part, int* start, void* out,
+                                int tokens, int hidden, int vocab, int chunk, cudaStream_t stream) {
   if (hidden % 8 != 0) UA_FAIL("ua_embedding_bwd: hidden must be a multiple of 8");
+  if (chunk <= 0) UA_FAIL("ua_embedding_bwd: chunk must be positive");
   if (vocab <= 0 || hidden <= 0) return 0;
-  embedding_bwd_kernel<<<static_cast<unsigned>(vocab), 256, 0, stream>>>(
-      sorted_ids, order, static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(out), tokens, hidden);
+  const auto d = static_cast<const __nv_bfloat16*>(dy);
+  // (no run is longer than the chunk if there is only one chunk)
+  const int chunks = tokens > chunk ? (tokens + chunk - 1) / chunk : 0;
+  const int part_blocks = chunks * ((hidden + EMB_COLS - 1) / EMB_COLS);
+  embedding_runs_kernel<<<part_blocks + vocab / EMB_THREADS + 1, EMB_THREADS, 0, stream>>>(sorted_ids, order, d, part, start, tokens,
+                                                                                       hidden, vocab, chunk, part_blocks);
+  UA_CUDA(cudaGetLastError());
+  embedding_bwd_kernel<<<static_cast<unsigned>(vocab), EMB_THREADS, 0, stream>>>(order, d, part, start,
+                                                                                 static_cast<__nv_bfloat16*>(out), hidden, chunk);
   UA_CUDA(cudaGetLastError());
   return 0;
 }

@@ -266,17 +266,26 @@ def xent_bwd_(logits: torch.Tensor, targets: torch.Tensor, lse: torch.Tensor, g:
     return logits
 
 
+def _embedding_chunk(tokens: int) -> int:
+    """Positions of the sorted ids that one block sums: the power of two next to sqrt(tokens), 32 at least."""
+    return 1 << max(5, ((tokens - 1).bit_length() + 1) // 2)
+
+
 def embedding_bwd(ids: torch.Tensor, dy: torch.Tensor, vocab: int) -> torch.Tensor:
     """Gradient [vocab, H] of an embedding lookup: row v = sum of ``dy`` [T, H] over the tokens with id
-    v, in fp32 and token order; rows of ids that do not occur are zero."""
+    v, in fp32 and token order (long runs of an id in pieces of :func:`_embedding_chunk`); rows of ids that do
+    not occur are zero."""
     T, H = dy.shape
     if not (dy.is_cuda and dy.dtype == torch.bfloat16 and H % 8 == 0 and T > 0):
         return torch.zeros(vocab, H, dtype=dy.dtype, device=dy.device).index_add_(0, ids.reshape(-1), dy)
     sorted_ids, order = torch.sort(ids.reshape(-1).long(), stable=True)
     out = torch.empty(vocab, H, dtype=dy.dtype, device=dy.device)
-    rc = _lib.load().ua_embedding_bwd(sorted_ids.data_ptr(), order.data_ptr(), dy.data_ptr(), out.data_ptr(), T, H, vocab,
-                                      _stream(dy))
-    _lib.check(rc, "ua_embedding_bwd")
+    chunk = _embedding_chunk(T)
+    part = torch.empty(2 * -(-T // chunk), H, dtype=torch.float32, device=dy.device)
+    start = torch.empty(vocab + 1, dtype=torch.int32, device=dy.device)
+    rc = _lib.load().ua_embedding_bwd(sorted_ids.data_ptr(), order.data_ptr(), dy.data_ptr(), part.data_ptr(), start.data_ptr(),
+                                      out.data_ptr(), T, H, vocab, chunk, _stream(dy))
+    _lib.check(rc, "ua_embedding_bwd", 2)
     return out
 
 
