@@ -461,203 +461,203 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     // last warpgroup (TMA, MMA, two idle warps): the drain warpgroup takes most of its registers.
     // The instruction sits inside this branch so that the other roles keep their full budget.
     reg_dealloc<BWD_REGS_LOAD>();
-  if (warp == BWD_TMA_WARP) {
-    // =============================== TMA producer ===========================================
-    if (lane == 0) {
-      bool ok = true;
-      BwdItem it = item0;
-      uint32_t i = 0;          // steps loaded so far
-      uint32_t live = 0;       // items with steps so far
-      for (uint32_t n = 0; ok; ++n) {
-        bool first = true;
-        for (int g = 0; g < p.kv_group && ok; ++g) {
-          const int head = it.kv_head * p.kv_group + g;
-          for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
-            const AttnSeg sg = bwd_seg(p, e);
-            const int nq = seg_num_qt(sg, it.c0);
-            if (seg_first_qt(sg, it.c0) < nq &&
-                !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
-              report_error(wc, UA_ERR_FLAG_TIMEOUT, 121, sg.wait_flag);
-              ok = false;
-              break;
-            }
-            for (int t = seg_first_qt(sg, it.c0); t < nq; ++t, ++i) {
-              const int st = i & 1;
-              const int qrow = sg.start + t * BWD_QT;
-              if (!mbar_wait(&s.q_empty[st], ((i >> 1) & 1) ^ 1, wc, 100)) { ok = false; break; }
-              mbar_arrive_expect_tx(&s.q_full[st], BWD_TILE_BYTES);
-              tma_load_4d(s.q[st], &p.tmQ[sg.src], &s.q_full[st], 0, head, qrow, it.batch);
-              tma_load_4d(s.q[st] + 16384, &p.tmQ[sg.src], &s.q_full[st], 64, head, qrow, it.batch);
-              if (first) {
-                first = false;
-                // the previous item's products have read its K and V
-                if (live > 0 && !mbar_wait(&s.kv_empty, (live - 1) & 1, wc, 102)) { ok = false; break; }
-                if (!wait_staged(p.stage.flags, it.col.kv_wait_flag, it.col.kv_wait_count * p.stage.epoch,
-                                 wc.budget_ns)) {
-                  report_error(wc, UA_ERR_FLAG_TIMEOUT, 120, it.col.kv_wait_flag);
-                  ok = false;
-                  break;
-                }
-                const int krow = it.col.kv_start + it.c0;
-                mbar_arrive_expect_tx(&s.kv_full, 2 * BWD_TILE_BYTES);
-                tma_load_4d(s.k, &p.tmK[it.col.kv_src], &s.kv_full, 0, it.kv_head, krow, it.batch);
-                tma_load_4d(s.k + 16384, &p.tmK[it.col.kv_src], &s.kv_full, 64, it.kv_head, krow, it.batch);
-                tma_load_4d(s.v, &p.tmV[it.col.kv_src], &s.kv_full, 0, it.kv_head, krow, it.batch);
-                tma_load_4d(s.v + 16384, &p.tmV[it.col.kv_src], &s.kv_full, 64, it.kv_head, krow, it.batch);
-                ++live;
+    if (warp == BWD_TMA_WARP) {
+      // =============================== TMA producer ===========================================
+      if (lane == 0) {
+        bool ok = true;
+        BwdItem it = item0;
+        uint32_t i = 0;          // steps loaded so far
+        uint32_t live = 0;       // items with steps so far
+        for (uint32_t n = 0; ok; ++n) {
+          bool first = true;
+          for (int g = 0; g < p.kv_group && ok; ++g) {
+            const int head = it.kv_head * p.kv_group + g;
+            for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
+              const AttnSeg sg = bwd_seg(p, e);
+              const int nq = seg_num_qt(sg, it.c0);
+              if (seg_first_qt(sg, it.c0) < nq &&
+                  !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
+                report_error(wc, UA_ERR_FLAG_TIMEOUT, 121, sg.wait_flag);
+                ok = false;
+                break;
               }
-              if (!mbar_wait(&s.do_empty, (i & 1) ^ 1, wc, 101)) { ok = false; break; }
-              mbar_arrive_expect_tx(&s.do_full, BWD_TILE_BYTES);
-              tma_load_4d(s.d_o, &p.tmdO[sg.src], &s.do_full, 0, head, qrow, it.batch);
-              tma_load_4d(s.d_o + 16384, &p.tmdO[sg.src], &s.do_full, 64, head, qrow, it.batch);
+              for (int t = seg_first_qt(sg, it.c0); t < nq; ++t, ++i) {
+                const int st = i & 1;
+                const int qrow = sg.start + t * BWD_QT;
+                if (!mbar_wait(&s.q_empty[st], ((i >> 1) & 1) ^ 1, wc, 100)) { ok = false; break; }
+                mbar_arrive_expect_tx(&s.q_full[st], BWD_TILE_BYTES);
+                tma_load_4d(s.q[st], &p.tmQ[sg.src], &s.q_full[st], 0, head, qrow, it.batch);
+                tma_load_4d(s.q[st] + 16384, &p.tmQ[sg.src], &s.q_full[st], 64, head, qrow, it.batch);
+                if (first) {
+                  first = false;
+                  // the previous item's products have read its K and V
+                  if (live > 0 && !mbar_wait(&s.kv_empty, (live - 1) & 1, wc, 102)) { ok = false; break; }
+                  if (!wait_staged(p.stage.flags, it.col.kv_wait_flag, it.col.kv_wait_count * p.stage.epoch,
+                                   wc.budget_ns)) {
+                    report_error(wc, UA_ERR_FLAG_TIMEOUT, 120, it.col.kv_wait_flag);
+                    ok = false;
+                    break;
+                  }
+                  const int krow = it.col.kv_start + it.c0;
+                  mbar_arrive_expect_tx(&s.kv_full, 2 * BWD_TILE_BYTES);
+                  tma_load_4d(s.k, &p.tmK[it.col.kv_src], &s.kv_full, 0, it.kv_head, krow, it.batch);
+                  tma_load_4d(s.k + 16384, &p.tmK[it.col.kv_src], &s.kv_full, 64, it.kv_head, krow, it.batch);
+                  tma_load_4d(s.v, &p.tmV[it.col.kv_src], &s.kv_full, 0, it.kv_head, krow, it.batch);
+                  tma_load_4d(s.v + 16384, &p.tmV[it.col.kv_src], &s.kv_full, 64, it.kv_head, krow, it.batch);
+                  ++live;
+                }
+                if (!mbar_wait(&s.do_empty, (i & 1) ^ 1, wc, 101)) { ok = false; break; }
+                mbar_arrive_expect_tx(&s.do_full, BWD_TILE_BYTES);
+                tma_load_4d(s.d_o, &p.tmdO[sg.src], &s.do_full, 0, head, qrow, it.batch);
+                tma_load_4d(s.d_o + 16384, &p.tmdO[sg.src], &s.do_full, 64, head, qrow, it.batch);
+              }
             }
           }
+          if (!ok || !p.persist) break;
+          // everything of this item is on its way: take over the next one
+          mbar_arrive_expect_tx(&s.clc_full, 16);
+          clc_try_cancel(&s.clc, &s.clc_full);
+          if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
+          int bx, by;
+          const bool got = clc_read(&s.clc, bx, by);
+          fence_proxy_async_smem();               // read before the next response may overwrite it
+          if (got) it = bwd_item(p, bx, by);
+          else it.exists = 0;
+          // the slot's previous item (n - 1) is done with
+          const uint32_t slot = (n + 1) & 1;
+          if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
+          s.item[slot] = it;
+          mbar_arrive(&s.item_full[slot]);
+          if (!got) break;
         }
-        if (!ok || !p.persist) break;
-        // everything of this item is on its way: take over the next one
-        mbar_arrive_expect_tx(&s.clc_full, 16);
-        clc_try_cancel(&s.clc, &s.clc_full);
-        if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
-        int bx, by;
-        const bool got = clc_read(&s.clc, bx, by);
-        fence_proxy_async_smem();               // read before the next response may overwrite it
-        if (got) it = bwd_item(p, bx, by);
-        else it.exists = 0;
-        // the slot's previous item (n - 1) is done with
-        const uint32_t slot = (n + 1) & 1;
-        if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
-        s.item[slot] = it;
-        mbar_arrive(&s.item_full[slot]);
-        if (!got) break;
       }
-    }
-  } else if (warp == BWD_MMA_WARP) {
-    // =============================== MMA issuer =============================================
-    if (lane == 0) {
-      const uint32_t idesc_kk = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T: both K-major
-      const uint32_t idesc_kn = make_idesc_bf16(128, 128, 0, 1);   // dV, dK: B N-major
-      const uint32_t idesc_nn = make_idesc_bf16(128, 128, 1, 1);   // dQ^T: A, B MN-major
-      const uint32_t t_dk = tmem_base + 0;
-      const uint32_t t_dv = tmem_base + 128;
-      const uint32_t t_st = tmem_base + 256;     // S^T, later P^T (packed) at columns 0-31, 64-95
-      const uint32_t t_dp = tmem_base + 384;     // dP^T, later dQ^T
-      // one base descriptor per operand view; every instruction adds its (16-byte unit) offset to
-      // the address field, which cannot carry out of it for addresses inside shared memory
-      const uint64_t k_kmaj = make_smem_desc_sw128(smem_u32(s.k), 16, 1024);        // A of S^T
-      const uint64_t k_mmaj = make_smem_desc_sw128(smem_u32(s.k), 16384, 1024);     // A of dQ^T
-      const uint64_t v_kmaj = make_smem_desc_sw128(smem_u32(s.v), 16, 1024);        // A of dP^T
-      const uint64_t do_kmaj = make_smem_desc_sw128(smem_u32(s.d_o), 16, 1024);     // B of dP^T
-      const uint64_t do_nmaj = make_smem_desc_sw128(smem_u32(s.d_o), 16384, 1024);  // B of dV
-      const uint64_t ds_kmaj = make_smem_desc_sw128(smem_u32(s.ds), 16, 1024);      // A of dK
-      const uint64_t ds_nmaj = make_smem_desc_sw128(smem_u32(s.ds), 16384, 1024);   // B of dQ^T
-      const uint64_t q_kmaj0 = make_smem_desc_sw128(smem_u32(s.q[0]), 16, 1024);    // B of S^T
-      const uint64_t q_nmaj0 = make_smem_desc_sw128(smem_u32(s.q[0]), 16384, 1024); // B of dK
-      const uint64_t ones_lse_d = make_smem_desc_noswz(smem_u32(s.ones_lse), 2048, 128);
-      const uint64_t ones_d_d = make_smem_desc_noswz(smem_u32(s.ones_d), 2048, 128);
-      // stage 0: chunks at aug[0] and aug_zero (4096 apart); stage 1: at aug[1] and aug_zero (2048 apart)
-      const uint64_t aug_desc[2] = {make_smem_desc_noswz(smem_u32(s.aug[0]), 4096, 128),
-                                    make_smem_desc_noswz(smem_u32(s.aug[1]), 2048, 128)};
-      constexpr uint64_t Q_STAGE = BWD_TILE_BYTES >> 4;
-      // K-major operands: 16 elements of the reduction = 32 B, the two 64-element halves 16384 B apart
-      auto koff = [](int kk) -> uint64_t { return static_cast<uint64_t>(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4); };
-      // MN-major operands: 16 rows of the reduction = 2048 B
-      auto noff = [](int kk) -> uint64_t { return static_cast<uint64_t>((kk * 2048) >> 4); };
-      auto issue_st = [&](int st) {
-        const uint64_t qd = q_kmaj0 + st * Q_STAGE;
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_ss(t_st, k_kmaj + koff(kk), qd + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
-        umma_ss(t_st, ones_lse_d, aug_desc[st], idesc_kk, 1u);     // - lse / scale
-      };
-      auto issue_dp = [&](int st) {
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_ss(t_dp, v_kmaj + koff(kk), do_kmaj + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
-        umma_ss(t_dp, ones_d_d, aug_desc[st], idesc_kk, 1u);       // - D
-      };
-      bool ok = true;
-      uint32_t i = 0;                   // steps so far
-      uint32_t live = 0;
-      for (uint32_t n = 0; ok; ++n) {
-        const int n_steps = bwd_steps(p, s.item[n & 1]);
-        if (n_steps > 0) {
-        if (!mbar_wait(&s.kv_full, live & 1, wc, 200)) break;
-        if (!mbar_wait(&s.q_full[i & 1], (i >> 1) & 1, wc, 201)) break;
-        if (!mbar_wait(&s.aug0_ready, live & 1, wc, 208)) break;
-        tc_fence_after_sync();
-        issue_st(i & 1);
-        tc_commit(&s.s_full);
-        if (!mbar_wait(&s.do_full, i & 1, wc, 202)) break;
-        // dP^T lands where the previous item's last dQ^T was. (That dK / dV of that item have been read
-        // out before they are started anew is implied by p_ready: the warps arrive after their epilogue.)
-        if (i > 0 && !mbar_wait(&s.dq_free, (i - 1) & 1, wc, 209)) break;
-        tc_fence_after_sync();
-        issue_dp(i & 1);
-        tc_commit(&s.dp_full);
-        for (int k = 0; k < n_steps; ++k, ++i) {
-          const int st = i & 1;
-          const uint32_t ph = i & 1;
-          const uint64_t qn = q_nmaj0 + st * Q_STAGE;
-          const bool more = k + 1 < n_steps;
-          // dV += P^T dO : A = P^T in TMEM (queries 0-63 packed at columns 0-31, 64-127 at 64-95),
-          // B = dO as an N-major operand (16 query rows = 2048 B, d-halves 16384 B apart)
-          BWD_PROF(i == BWD_PROF_STEP, 0);
-          if (!mbar_wait(&s.p_ready, ph, wc, 203)) { ok = false; break; }
-          BWD_PROF(i == BWD_PROF_STEP, 1);
-          tc_fence_after_sync();
+    } else if (warp == BWD_MMA_WARP) {
+      // =============================== MMA issuer =============================================
+      if (lane == 0) {
+        const uint32_t idesc_kk = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T: both K-major
+        const uint32_t idesc_kn = make_idesc_bf16(128, 128, 0, 1);   // dV, dK: B N-major
+        const uint32_t idesc_nn = make_idesc_bf16(128, 128, 1, 1);   // dQ^T: A, B MN-major
+        const uint32_t t_dk = tmem_base + 0;
+        const uint32_t t_dv = tmem_base + 128;
+        const uint32_t t_st = tmem_base + 256;     // S^T, later P^T (packed) at columns 0-31, 64-95
+        const uint32_t t_dp = tmem_base + 384;     // dP^T, later dQ^T
+        // one base descriptor per operand view; every instruction adds its (16-byte unit) offset to
+        // the address field, which cannot carry out of it for addresses inside shared memory
+        const uint64_t k_kmaj = make_smem_desc_sw128(smem_u32(s.k), 16, 1024);        // A of S^T
+        const uint64_t k_mmaj = make_smem_desc_sw128(smem_u32(s.k), 16384, 1024);     // A of dQ^T
+        const uint64_t v_kmaj = make_smem_desc_sw128(smem_u32(s.v), 16, 1024);        // A of dP^T
+        const uint64_t do_kmaj = make_smem_desc_sw128(smem_u32(s.d_o), 16, 1024);     // B of dP^T
+        const uint64_t do_nmaj = make_smem_desc_sw128(smem_u32(s.d_o), 16384, 1024);  // B of dV
+        const uint64_t ds_kmaj = make_smem_desc_sw128(smem_u32(s.ds), 16, 1024);      // A of dK
+        const uint64_t ds_nmaj = make_smem_desc_sw128(smem_u32(s.ds), 16384, 1024);   // B of dQ^T
+        const uint64_t q_kmaj0 = make_smem_desc_sw128(smem_u32(s.q[0]), 16, 1024);    // B of S^T
+        const uint64_t q_nmaj0 = make_smem_desc_sw128(smem_u32(s.q[0]), 16384, 1024); // B of dK
+        const uint64_t ones_lse_d = make_smem_desc_noswz(smem_u32(s.ones_lse), 2048, 128);
+        const uint64_t ones_d_d = make_smem_desc_noswz(smem_u32(s.ones_d), 2048, 128);
+        // stage 0: chunks at aug[0] and aug_zero (4096 apart); stage 1: at aug[1] and aug_zero (2048 apart)
+        const uint64_t aug_desc[2] = {make_smem_desc_noswz(smem_u32(s.aug[0]), 4096, 128),
+                                      make_smem_desc_noswz(smem_u32(s.aug[1]), 2048, 128)};
+        constexpr uint64_t Q_STAGE = BWD_TILE_BYTES >> 4;
+        // K-major operands: 16 elements of the reduction = 32 B, the two 64-element halves 16384 B apart
+        auto koff = [](int kk) -> uint64_t { return static_cast<uint64_t>(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4); };
+        // MN-major operands: 16 rows of the reduction = 2048 B
+        auto noff = [](int kk) -> uint64_t { return static_cast<uint64_t>((kk * 2048) >> 4); };
+        auto issue_st = [&](int st) {
+          const uint64_t qd = q_kmaj0 + st * Q_STAGE;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            umma_ts(t_dv, t_st + (kk >> 2) * 64 + (kk & 3) * 8, do_nmaj + noff(kk), idesc_kn,
-                    (k > 0 || kk > 0) ? 1u : 0u);
-          tc_commit(&s.do_empty);
-          // S^T of the next step right behind it: it overwrites P^T(i), which dV(i) reads first
-          // because the tensor pipe executes in issue order
-          if (more) {
-            if (!mbar_wait(&s.q_full[st ^ 1], ((i + 1) >> 1) & 1, wc, 205)) { ok = false; break; }
+            umma_ss(t_st, k_kmaj + koff(kk), qd + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
+          umma_ss(t_st, ones_lse_d, aug_desc[st], idesc_kk, 1u);     // - lse / scale
+        };
+        auto issue_dp = [&](int st) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            umma_ss(t_dp, v_kmaj + koff(kk), do_kmaj + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
+          umma_ss(t_dp, ones_d_d, aug_desc[st], idesc_kk, 1u);       // - D
+        };
+        bool ok = true;
+        uint32_t i = 0;                   // steps so far
+        uint32_t live = 0;
+        for (uint32_t n = 0; ok; ++n) {
+          const int n_steps = bwd_steps(p, s.item[n & 1]);
+          if (n_steps > 0) {
+            if (!mbar_wait(&s.kv_full, live & 1, wc, 200)) break;
+            if (!mbar_wait(&s.q_full[i & 1], (i >> 1) & 1, wc, 201)) break;
+            if (!mbar_wait(&s.aug0_ready, live & 1, wc, 208)) break;
             tc_fence_after_sync();
-            BWD_PROF(i == BWD_PROF_STEP, 2);
-            issue_st(st ^ 1);
+            issue_st(i & 1);
             tc_commit(&s.s_full);
-          }
-          BWD_PROF(i == BWD_PROF_STEP, 3);
-          // dQ^T = K^T dS^T : A = K as an M-major operand, B = dS^T as an N-major operand (two
-          // 64-query panels 16384 B apart); lands where dP^T was
-          if (!mbar_wait(&s.ds_ready, ph, wc, 204)) { ok = false; break; }
-          BWD_PROF(i == BWD_PROF_STEP, 4);
-          tc_fence_after_sync();
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_ss(t_dp, k_mmaj + noff(kk), ds_nmaj + noff(kk), idesc_nn, kk > 0 ? 1u : 0u);
-          tc_commit(&s.dq_full);
-          // dK += dS^T Q : A = dS^T in shared memory (K-major over queries: panel kk/4, 32 B per
-          // step), B = Q as an N-major operand; runs while the drain warpgroup reads dQ^T
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_ss(t_dk, ds_kmaj + koff(kk), qn + noff(kk), idesc_kn, (k > 0 || kk > 0) ? 1u : 0u);
-          tc_commit(&s.q_empty[st]);
-          BWD_PROF(i == BWD_PROF_STEP, 5);
-          if (more) {
-            if (!mbar_wait(&s.do_full, (i + 1) & 1, wc, 206)) { ok = false; break; }
-            BWD_PROF(i == BWD_PROF_STEP, 6);
-            // dP^T(i+1) lands where dQ^T(i) is: wait until the drain warpgroup has read it
-            if (!mbar_wait(&s.dq_free, ph, wc, 207)) { ok = false; break; }
-            BWD_PROF(i == BWD_PROF_STEP, 7);
+            if (!mbar_wait(&s.do_full, i & 1, wc, 202)) break;
+            // dP^T lands where the previous item's last dQ^T was. (That dK / dV of that item have been read
+            // out before they are started anew is implied by p_ready: the warps arrive after their epilogue.)
+            if (i > 0 && !mbar_wait(&s.dq_free, (i - 1) & 1, wc, 209)) break;
             tc_fence_after_sync();
-            issue_dp(st ^ 1);
+            issue_dp(i & 1);
             tc_commit(&s.dp_full);
-            BWD_PROF(i == BWD_PROF_STEP, 8);
+            for (int k = 0; k < n_steps; ++k, ++i) {
+              const int st = i & 1;
+              const uint32_t ph = i & 1;
+              const uint64_t qn = q_nmaj0 + st * Q_STAGE;
+              const bool more = k + 1 < n_steps;
+              // dV += P^T dO : A = P^T in TMEM (queries 0-63 packed at columns 0-31, 64-127 at 64-95),
+              // B = dO as an N-major operand (16 query rows = 2048 B, d-halves 16384 B apart)
+              BWD_PROF(i == BWD_PROF_STEP, 0);
+              if (!mbar_wait(&s.p_ready, ph, wc, 203)) { ok = false; break; }
+              BWD_PROF(i == BWD_PROF_STEP, 1);
+              tc_fence_after_sync();
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                umma_ts(t_dv, t_st + (kk >> 2) * 64 + (kk & 3) * 8, do_nmaj + noff(kk), idesc_kn,
+                        (k > 0 || kk > 0) ? 1u : 0u);
+              tc_commit(&s.do_empty);
+              // S^T of the next step right behind it: it overwrites P^T(i), which dV(i) reads first
+              // because the tensor pipe executes in issue order
+              if (more) {
+                if (!mbar_wait(&s.q_full[st ^ 1], ((i + 1) >> 1) & 1, wc, 205)) { ok = false; break; }
+                tc_fence_after_sync();
+                BWD_PROF(i == BWD_PROF_STEP, 2);
+                issue_st(st ^ 1);
+                tc_commit(&s.s_full);
+              }
+              BWD_PROF(i == BWD_PROF_STEP, 3);
+              // dQ^T = K^T dS^T : A = K as an M-major operand, B = dS^T as an N-major operand (two
+              // 64-query panels 16384 B apart); lands where dP^T was
+              if (!mbar_wait(&s.ds_ready, ph, wc, 204)) { ok = false; break; }
+              BWD_PROF(i == BWD_PROF_STEP, 4);
+              tc_fence_after_sync();
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                umma_ss(t_dp, k_mmaj + noff(kk), ds_nmaj + noff(kk), idesc_nn, kk > 0 ? 1u : 0u);
+              tc_commit(&s.dq_full);
+              // dK += dS^T Q : A = dS^T in shared memory (K-major over queries: panel kk/4, 32 B per
+              // step), B = Q as an N-major operand; runs while the drain warpgroup reads dQ^T
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                umma_ss(t_dk, ds_kmaj + koff(kk), qn + noff(kk), idesc_kn, (k > 0 || kk > 0) ? 1u : 0u);
+              tc_commit(&s.q_empty[st]);
+              BWD_PROF(i == BWD_PROF_STEP, 5);
+              if (more) {
+                if (!mbar_wait(&s.do_full, (i + 1) & 1, wc, 206)) { ok = false; break; }
+                BWD_PROF(i == BWD_PROF_STEP, 6);
+                // dP^T(i+1) lands where dQ^T(i) is: wait until the drain warpgroup has read it
+                if (!mbar_wait(&s.dq_free, ph, wc, 207)) { ok = false; break; }
+                BWD_PROF(i == BWD_PROF_STEP, 7);
+                tc_fence_after_sync();
+                issue_dp(st ^ 1);
+                tc_commit(&s.dp_full);
+                BWD_PROF(i == BWD_PROF_STEP, 8);
+              }
+            }
+            if (!ok) break;
+            tc_commit(&s.kv_empty);
+            tc_commit(&s.dkv_full);
+            ++live;
           }
+          if (p.persist) mbar_arrive(&s.item_empty[n & 1]);
+          if (!item_ready(n + 1)) break;
         }
-        if (!ok) break;
-        tc_commit(&s.kv_empty);
-        tc_commit(&s.dkv_full);
-        ++live;
-        }
-        if (p.persist) mbar_arrive(&s.item_empty[n & 1]);
-        if (!item_ready(n + 1)) break;
       }
     }
-  }
   } else if (warp < 8) {
     // =============================== softmax warpgroups =====================================
     const int wg = warp >> 2;                        // which half of the 128 query columns
@@ -743,114 +743,114 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     int n_steps = bwd_steps(p, s.item[0]);
     if (n_steps > 0) start_item(s.item[0], n_steps);
     for (uint32_t n = 0;; ++n) {
-    const BwdItem& it = s.item[n & 1];
-    const int c0 = it.c0;
-    const int key_c = c0 + key_t;                    // key inside the block column
-    const bool key_ok = key_c < it.col.kv_len;
-    if (n > 0) trace_stamp(p.trace, it.linear, 0);
-    trace_stamp(p.trace, it.linear, 1);
-    trace_ident(p.trace, it.linear, it.col_idx);
-    for (int k = 0; k < n_steps && ok; ++k, ++i) {
-      const uint32_t ph = i & 1;
-      const AttnSeg& sg = cur.sg;
-      const bool prof = i == BWD_PROF_STEP && quad == 0 && lane == 0;
-      const int pslot = 16 + wg * 16;
-      (void)prof; (void)pslot;
-      BWD_PROF(prof, pslot + 0);
-      // row terms of step i+1 into the operand tile (its previous user, step i-1, is complete: this
-      // thread has consumed dP^T(i-1)); the arrival on p_ready below publishes them
-      if (k + 1 < n_steps) write_aug((i + 1) & 1, lv, dv);
-      BWD_PROF(prof, pslot + 7);
-      // visible iff key_c <= r + diag  <=>  r >= key_c - diag   (r relative to this half)
-      const int r_half = cur.t * BWD_QT + wg * 64;
-      const int r_first = (sg.causal & SEG_UPPER) ? key_c - sg.diag - r_half : 0;
-      // ... and key_c >= r + lo  <=>  r <= key_c - lo
-      const int r_last = (sg.causal & SEG_LOWER) ? key_c - sg.lo - r_half : 63;
-      // the row terms of step i+2 travel while this step computes
-      if (k + 2 < n_steps) {
-        fut.next(p, it.col, c0);
-        if (!fetch(it, fut, lv, dv)) { ok = false; break; }
-      }
+      const BwdItem& it = s.item[n & 1];
+      const int c0 = it.c0;
+      const int key_c = c0 + key_t;                    // key inside the block column
+      const bool key_ok = key_c < it.col.kv_len;
+      if (n > 0) trace_stamp(p.trace, it.linear, 0);
+      trace_stamp(p.trace, it.linear, 1);
+      trace_ident(p.trace, it.linear, it.col_idx);
+      for (int k = 0; k < n_steps && ok; ++k, ++i) {
+        const uint32_t ph = i & 1;
+        const AttnSeg& sg = cur.sg;
+        const bool prof = i == BWD_PROF_STEP && quad == 0 && lane == 0;
+        const int pslot = 16 + wg * 16;
+        (void)prof; (void)pslot;
+        BWD_PROF(prof, pslot + 0);
+        // row terms of step i+1 into the operand tile (its previous user, step i-1, is complete: this
+        // thread has consumed dP^T(i-1)); the arrival on p_ready below publishes them
+        if (k + 1 < n_steps) write_aug((i + 1) & 1, lv, dv);
+        BWD_PROF(prof, pslot + 7);
+        // visible iff key_c <= r + diag  <=>  r >= key_c - diag   (r relative to this half)
+        const int r_half = cur.t * BWD_QT + wg * 64;
+        const int r_first = (sg.causal & SEG_UPPER) ? key_c - sg.diag - r_half : 0;
+        // ... and key_c >= r + lo  <=>  r <= key_c - lo
+        const int r_last = (sg.causal & SEG_LOWER) ? key_c - sg.lo - r_half : 63;
+        // the row terms of step i+2 travel while this step computes
+        if (k + 2 < n_steps) {
+          fut.next(p, it.col, c0);
+          if (!fetch(it, fut, lv, dv)) { ok = false; break; }
+        }
 
-      // ---- phase A: P^T = exp2((S^T - lse / scale) * scale) -> TMEM (packed bf16) ------------
-      BWD_PROF(prof, pslot + 1);
-      if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full, ph, wc, 300))) { ok = false; break; }
-      BWD_PROF(prof, pslot + 2);
-      tc_fence_after_sync();
-      uint32_t pk[32];                 // this thread's 64 probabilities, packed; kept for phase B
-      if (__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63))
-        bwd_phase_a<false>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
-      else
-        bwd_phase_a<true>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
-      // packed P^T of this half goes to the first 32 columns of this half's own S^T columns
-      // (the other warpgroup may still be reading its fp32 half)
-      BWD_PROF(prof, pslot + 3);
-      tmem_st_x32(t_st, pk);
-      tmem_wait_st();
-      tc_fence_before_sync();
-      mbar_arrive_warp(&s.p_ready);
-      BWD_PROF(prof, pslot + 4);
+        // ---- phase A: P^T = exp2((S^T - lse / scale) * scale) -> TMEM (packed bf16) ------------
+        BWD_PROF(prof, pslot + 1);
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full, ph, wc, 300))) { ok = false; break; }
+        BWD_PROF(prof, pslot + 2);
+        tc_fence_after_sync();
+        uint32_t pk[32];                 // this thread's 64 probabilities, packed; kept for phase B
+        if (__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63))
+          bwd_phase_a<false>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
+        else
+          bwd_phase_a<true>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
+        // packed P^T of this half goes to the first 32 columns of this half's own S^T columns
+        // (the other warpgroup may still be reading its fp32 half)
+        BWD_PROF(prof, pslot + 3);
+        tmem_st_x32(t_st, pk);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive_warp(&s.p_ready);
+        BWD_PROF(prof, pslot + 4);
 
-      // ---- phase B: dS^T = P^T * (dP^T - D) -> shared memory ------------------------------
-      if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.dp_full, ph, wc, 301))) { ok = false; break; }
-      BWD_PROF(prof, pslot + 5);
-      tc_fence_after_sync();
-      uint8_t* ds_panel = s.ds + wg * 16384;     // this half's 64-query panel
-      {
-        uint32_t dp[2][32];
-        tmem_ld_x32(t_dp, dp[0]);
-        tmem_ld_x32(t_dp + 32, dp[1]);
-        tmem_wait_ld();
-        BWD_PROF(prof, pslot + 8);
+        // ---- phase B: dS^T = P^T * (dP^T - D) -> shared memory ------------------------------
+        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.dp_full, ph, wc, 301))) { ok = false; break; }
+        BWD_PROF(prof, pslot + 5);
+        tc_fence_after_sync();
+        uint8_t* ds_panel = s.ds + wg * 16384;     // this half's 64-query panel
+        {
+          uint32_t dp[2][32];
+          tmem_ld_x32(t_dp, dp[0]);
+          tmem_ld_x32(t_dp + 32, dp[1]);
+          tmem_wait_ld();
+          BWD_PROF(prof, pslot + 8);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+          for (int h = 0; h < 2; ++h) {
 #pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {          // 8 queries = one 16-byte chunk
-            uint32_t w4[4];
+            for (int ch = 0; ch < 4; ++ch) {          // 8 queries = one 16-byte chunk
+              uint32_t w4[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              // (dP - D), as it comes out of the tensor core, rounded to bf16 pairs, times the bf16
-              // probabilities (masked ones are 0)
-              const uint32_t x = pack_bf16x2(__uint_as_float(dp[h][ch * 8 + 2 * c]),
-                                             __uint_as_float(dp[h][ch * 8 + 2 * c + 1]));
-              w4[c] = mul_bf16x2(pk[h * 16 + ch * 4 + c], x);
+              for (int c = 0; c < 4; ++c) {
+                // (dP - D), as it comes out of the tensor core, rounded to bf16 pairs, times the bf16
+                // probabilities (masked ones are 0)
+                const uint32_t x = pack_bf16x2(__uint_as_float(dp[h][ch * 8 + 2 * c]),
+                                               __uint_as_float(dp[h][ch * 8 + 2 * c + 1]));
+                w4[c] = mul_bf16x2(pk[h * 16 + ch * 4 + c], x);
+              }
+              *reinterpret_cast<uint4*>(ds_panel + sw128_offset(key_t, h * 4 + ch)) =
+                  make_uint4(w4[0], w4[1], w4[2], w4[3]);
             }
-            *reinterpret_cast<uint4*>(ds_panel + sw128_offset(key_t, h * 4 + ch)) =
-                make_uint4(w4[0], w4[1], w4[2], w4[3]);
           }
         }
+        BWD_PROF(prof, pslot + 9);
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
+        mbar_arrive_warp(&s.ds_ready);
+        BWD_PROF(prof, pslot + 6);
+        if (k + 1 < n_steps) cur.next(p, it.col, c0);
       }
-      BWD_PROF(prof, pslot + 9);
-      fence_proxy_async_smem();
-      tc_fence_before_sync();
-      mbar_arrive_warp(&s.ds_ready);
-      BWD_PROF(prof, pslot + 6);
-      if (k + 1 < n_steps) cur.next(p, it.col, c0);
-    }
-    // the next item's first row terms go out before this one's results, so that its scores can start
-    int more = 0;
-    if (ok) {
-      if (lane == 0) more = item_ready(n + 1) ? 1 : 0;
-      more = __shfl_sync(0xFFFFFFFFu, more, 0);
-      __syncwarp();                          // lane 0 has seen the item; this makes it visible to the others (a shuffle does not)
-    }
-    const int n_done = n_steps;
-    if (more) {
-      n_steps = bwd_steps(p, s.item[(n + 1) & 1]);
-      if (n_steps > 0) start_item(s.item[(n + 1) & 1], n_steps);
-    }
-    // ---------------------------------- dK / dV epilogue ------------------------------------
-    if (n_done > 0 && ok) {
-      ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.dkv_full, live & 1, wc, 310));
-      ++live;
-    }
-    tc_fence_after_sync();
-    bwd_store_grads(s, n & 1, tmem_base, n_done > 0);
-    trace_stamp(p.trace, it.linear, 2);
-    tc_fence_before_sync();                  // dK / dV have been read; published by the next p_ready
-    __syncwarp();
-    if (lane == 0 && p.persist) mbar_arrive(&s.item_empty[n & 1]);
-    if (!more || !ok) break;
+      // the next item's first row terms go out before this one's results, so that its scores can start
+      int more = 0;
+      if (ok) {
+        if (lane == 0) more = item_ready(n + 1) ? 1 : 0;
+        more = __shfl_sync(0xFFFFFFFFu, more, 0);
+        __syncwarp();                          // lane 0 has seen the item; this makes it visible to the others (a shuffle does not)
+      }
+      const int n_done = n_steps;
+      if (more) {
+        n_steps = bwd_steps(p, s.item[(n + 1) & 1]);
+        if (n_steps > 0) start_item(s.item[(n + 1) & 1], n_steps);
+      }
+      // ---------------------------------- dK / dV epilogue ------------------------------------
+      if (n_done > 0 && ok) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.dkv_full, live & 1, wc, 310));
+        ++live;
+      }
+      tc_fence_after_sync();
+      bwd_store_grads(s, n & 1, tmem_base, n_done > 0);
+      trace_stamp(p.trace, it.linear, 2);
+      tc_fence_before_sync();                  // dK / dV have been read; published by the next p_ready
+      __syncwarp();
+      if (lane == 0 && p.persist) mbar_arrive(&s.item_empty[n & 1]);
+      if (!more || !ok) break;
     }
   } else {
     // =============================== dQ drain warpgroup =====================================
@@ -863,64 +863,64 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     uint32_t i = 0;
     uint32_t n_chunk = 0;
     for (uint32_t n = 0;; ++n) {
-    const BwdItem& it = s.item[n & 1];
-    const int c0 = it.c0;
-    for (int g = 0; g < p.kv_group && ok; ++g) {
-      const int head = it.kv_head * p.kv_group + g;
-      for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
-        const AttnSeg sg = bwd_seg(p, e);
-        const int nq = seg_num_qt(sg, c0);
-        const CUtensorMap* tdq = &p.tmdQ[sg.src];
-        for (int t = seg_first_qt(sg, c0); t < nq; ++t, ++i) {
-          BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 48);
-          if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.dq_full, i & 1, wc, 400))) { ok = false; break; }
-          BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 49);
-          tc_fence_after_sync();
-          const int qrow = sg.start + t * BWD_QT;
-          // read the whole slice and hand TMEM back at once: dP^T of the next step is waiting for it
-          uint32_t dv[4][32];
+      const BwdItem& it = s.item[n & 1];
+      const int c0 = it.c0;
+      for (int g = 0; g < p.kv_group && ok; ++g) {
+        const int head = it.kv_head * p.kv_group + g;
+        for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
+          const AttnSeg sg = bwd_seg(p, e);
+          const int nq = seg_num_qt(sg, c0);
+          const CUtensorMap* tdq = &p.tmdQ[sg.src];
+          for (int t = seg_first_qt(sg, c0); t < nq; ++t, ++i) {
+            BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 48);
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.dq_full, i & 1, wc, 400))) { ok = false; break; }
+            BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 49);
+            tc_fence_after_sync();
+            const int qrow = sg.start + t * BWD_QT;
+            // read the whole slice and hand TMEM back at once: dP^T of the next step is waiting for it
+            uint32_t dv[4][32];
 #pragma unroll
-          for (int h = 0; h < 4; ++h) tmem_ld_x32(t_dq + h * 32, dv[h]);
-          tmem_wait_ld();
-          tc_fence_before_sync();
-          mbar_arrive_warp(&s.dq_free);
-          BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 50);
-          {
+            for (int h = 0; h < 4; ++h) tmem_ld_x32(t_dq + h * 32, dv[h]);
+            tmem_wait_ld();
+            tc_fence_before_sync();
+            mbar_arrive_warp(&s.dq_free);
+            BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 50);
+            {
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {              // 16 queries at a time, three staging tiles in turn
-              // The four warps fill one [16 queries][128 head-dim] tile (a 32-wide slice each) and one
-              // thread issues a single reduce with 512-byte rows. The reduce issued three chunks
-              // ago (same tile) must have finished reading it; the last two may still be in flight.
-              if (quad == 0 && lane == 0) tma_store_wait_read_all_but<2>();
-              asm volatile("bar.sync 1, 128;" ::: "memory");
-              BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 52 + (h >> 1) * 3);
-              float* tile = stage + ((n_chunk + h) % 3) * 2048;
+              for (int h = 0; h < 8; ++h) {              // 16 queries at a time, three staging tiles in turn
+                // The four warps fill one [16 queries][128 head-dim] tile (a 32-wide slice each) and one
+                // thread issues a single reduce with 512-byte rows. The reduce issued three chunks
+                // ago (same tile) must have finished reading it; the last two may still be in flight.
+                if (quad == 0 && lane == 0) tma_store_wait_read_all_but<2>();
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 52 + (h >> 1) * 3);
+                float* tile = stage + ((n_chunk + h) % 3) * 2048;
 #pragma unroll
-              for (int c = 0; c < 16; ++c)
-                tile[c * 128 + quad * 32 + lane] = __uint_as_float(dv[h >> 1][(h & 1) * 16 + c]) * p.scale;
-              fence_proxy_async_smem();
-              asm volatile("bar.sync 1, 128;" ::: "memory");
-              BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 53 + (h >> 1) * 3);
-              if (quad == 0 && lane == 0) {
-                tma_reduce_add_4d(tdq, tile, 0, head, qrow + h * 16, it.batch);
-                tma_store_commit();
+                for (int c = 0; c < 16; ++c)
+                  tile[c * 128 + quad * 32 + lane] = __uint_as_float(dv[h >> 1][(h & 1) * 16 + c]) * p.scale;
+                fence_proxy_async_smem();
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 53 + (h >> 1) * 3);
+                if (quad == 0 && lane == 0) {
+                  tma_reduce_add_4d(tdq, tile, 0, head, qrow + h * 16, it.batch);
+                  tma_store_commit();
+                }
+                BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 54 + (h >> 1) * 3);
               }
-              BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 54 + (h >> 1) * 3);
             }
+            n_chunk += 8;
+            BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 51);
           }
-          n_chunk += 8;
-          BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 51);
         }
       }
-    }
-    __syncwarp();
-    int more = 0;
-    if (lane == 0) {
-      if (p.persist) mbar_arrive(&s.item_empty[n & 1]);
-      more = ok && item_ready(n + 1) ? 1 : 0;
-    }
-    if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
-    __syncwarp();
+      __syncwarp();
+      int more = 0;
+      if (lane == 0) {
+        if (p.persist) mbar_arrive(&s.item_empty[n & 1]);
+        more = ok && item_ready(n + 1) ? 1 : 0;
+      }
+      if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
+      __syncwarp();
     }
     if (lane == 0) tma_store_wait_all();
     __syncwarp();

@@ -342,51 +342,51 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
   __nv_bfloat16* optr = od.o + it.batch * od.o_batch_stride + orow * od.o_row_stride + static_cast<long>(qh) * ATTN_D;
   float* pptr = f32 ? s.hot.part_o + ((part0 + r_blk) * s.hot.n_heads + qh) * ATTN_D : nullptr;
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-      uint32_t ov[32];
-      if (any) {
-        tmem_ld_x32(tO + c * 32, ov);
-        tmem_wait_ld();
-      } else {
+  for (int c = 0; c < 4; ++c) {
+    uint32_t ov[32];
+    if (any) {
+      tmem_ld_x32(tO + c * 32, ov);
+      tmem_wait_ld();
+    } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) ov[i] = 0u;
+      for (int i = 0; i < 32; ++i) ov[i] = 0u;
+    }
+    if (valid_row && pptr != nullptr) {
+      float4* d4 = reinterpret_cast<float4*>(pptr + c * 32);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        float f[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 4 + i]) * fnew;
+        d4[q] = make_float4(f[0], f[1], f[2], f[3]);
       }
-      if (valid_row && pptr != nullptr) {
-        float4* d4 = reinterpret_cast<float4*>(pptr + c * 32);
+    } else if (valid_row) {
+      uint4* d4 = reinterpret_cast<uint4*>(optr + c * 32);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          float f[4];
+      for (int q = 0; q < 4; ++q) {
+        float f[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 4 + i]) * fnew;
-          d4[q] = make_float4(f[0], f[1], f[2], f[3]);
-        }
-      } else if (valid_row) {
-        uint4* d4 = reinterpret_cast<uint4*>(optr + c * 32);
+        for (int i = 0; i < 8; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 8 + i]) * fnew;
+        if (it.row.accumulate) {
+          const uint4 old = d4[q];
+          const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float f[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 8 + i]) * fnew;
-          if (it.row.accumulate) {
-            const uint4 old = d4[q];
-            const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float lo = __uint_as_float(ow[i] << 16);
-              const float hi = __uint_as_float(ow[i] & 0xFFFF0000u);
-              f[2 * i] += w_old * lo;
-              f[2 * i + 1] += w_old * hi;
-            }
+          for (int i = 0; i < 4; ++i) {
+            const float lo = __uint_as_float(ow[i] << 16);
+            const float hi = __uint_as_float(ow[i] & 0xFFFF0000u);
+            f[2 * i] += w_old * lo;
+            f[2 * i + 1] += w_old * hi;
           }
-          uint4 o;
-          o.x = pack_bf16x2(f[0], f[1]);
-          o.y = pack_bf16x2(f[2], f[3]);
-          o.z = pack_bf16x2(f[4], f[5]);
-          o.w = pack_bf16x2(f[6], f[7]);
-          d4[q] = o;
         }
+        uint4 o;
+        o.x = pack_bf16x2(f[0], f[1]);
+        o.y = pack_bf16x2(f[2], f[3]);
+        o.z = pack_bf16x2(f[4], f[5]);
+        o.w = pack_bf16x2(f[6], f[7]);
+        d4[q] = o;
       }
     }
+  }
 }
 
 // Called, not inlined, by the two-tile form: inlined, its addresses compete with the score loop for
@@ -484,349 +484,349 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
   };
 
   if (warp >= FWD_SOFTMAX_WARPS) {
-  reg_dealloc<FWD_REGS_LOAD>();
-  if (warp == FWD_TMA_WARP) {
-    // =============================== TMA producer and scheduler ==============================
-    if (lane == 0) {
-      bool ok = true;
-      FwdItem it = item0;
-      uint32_t j = 0;          // K / V tiles loaded so far
-      uint32_t live = 0;       // items with keys so far
-      for (uint32_t n = 0; ok; ++n) {
-        if (fwd_total(p, it) > 0) {
-          const CUtensorMap* tq = &p.tmQ[it.row.q_src];
-          tma_prefetch_desc(tq);
-          if (!wait_staged(p.stage.flags, it.row.q_wait_flag, it.row.q_wait_count * p.stage.epoch, wc.budget_ns)) {
-            report_error(wc, UA_ERR_FLAG_TIMEOUT, 110, it.row.q_wait_flag);
-            ok = false;
-          }
-          // the previous item's last scores have been computed
-          if (ok && live > 0 && !mbar_wait(&s.q_empty, (live - 1) & 1, wc, 102)) ok = false;
-          for (int w = 0; w < (FEW ? 1 : 2) && ok; ++w) {
-            mbar_arrive_expect_tx(&s.q_full[w], FWD_TILE_BYTES);
-            const int qrow = it.row.q_start + it.tok0 + ((w * ATTN_TILE) >> psh);
-            tma_load_4d(s.q[w], tq, &s.q_full[w], 0, it.q_head, qrow, it.batch);
-            tma_load_4d(s.q[w] + 16384, tq, &s.q_full[w], 64, it.q_head, qrow, it.batch);
-          }
-          ++live;
-          for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
-            const AttnSeg sg = fwd_seg(p, e);
-            const TileRange tr = fwd_tiles(p, it, sg);
-            const CUtensorMap* tk = &p.tmK[sg.src];
-            const CUtensorMap* tv = &p.tmV[sg.src];
-            if (tr.first < tr.end &&
-                !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
-              report_error(wc, UA_ERR_FLAG_TIMEOUT, 111, sg.wait_flag);
+    reg_dealloc<FWD_REGS_LOAD>();
+    if (warp == FWD_TMA_WARP) {
+      // =============================== TMA producer and scheduler ==============================
+      if (lane == 0) {
+        bool ok = true;
+        FwdItem it = item0;
+        uint32_t j = 0;          // K / V tiles loaded so far
+        uint32_t live = 0;       // items with keys so far
+        for (uint32_t n = 0; ok; ++n) {
+          if (fwd_total(p, it) > 0) {
+            const CUtensorMap* tq = &p.tmQ[it.row.q_src];
+            tma_prefetch_desc(tq);
+            if (!wait_staged(p.stage.flags, it.row.q_wait_flag, it.row.q_wait_count * p.stage.epoch, wc.budget_ns)) {
+              report_error(wc, UA_ERR_FLAG_TIMEOUT, 110, it.row.q_wait_flag);
               ok = false;
-              break;
             }
-            for (int t = tr.first; t < tr.end; ++t, ++j) {
-              const int st = j % STAGES;
-              const uint32_t ph = (j / STAGES) & 1;
-              const int krow = sg.start + t * ATTN_TILE;
-              if (!mbar_wait(&s.k_empty[st], ph ^ 1, wc, 100)) { ok = false; break; }
-              mbar_arrive_expect_tx(&s.k_full[st], FWD_TILE_BYTES);
-              tma_load_4d(s.k[st], tk, &s.k_full[st], 0, it.kv_head, krow, it.batch);
-              tma_load_4d(s.k[st] + 16384, tk, &s.k_full[st], 64, it.kv_head, krow, it.batch);
-              if (!mbar_wait(&s.v_empty[st], ph ^ 1, wc, 101)) { ok = false; break; }
-              mbar_arrive_expect_tx(&s.v_full[st], FWD_TILE_BYTES);
-              tma_load_4d(s.v[st], tv, &s.v_full[st], 0, it.kv_head, krow, it.batch);
-              tma_load_4d(s.v[st] + 16384, tv, &s.v_full[st], 64, it.kv_head, krow, it.batch);
+            // the previous item's last scores have been computed
+            if (ok && live > 0 && !mbar_wait(&s.q_empty, (live - 1) & 1, wc, 102)) ok = false;
+            for (int w = 0; w < (FEW ? 1 : 2) && ok; ++w) {
+              mbar_arrive_expect_tx(&s.q_full[w], FWD_TILE_BYTES);
+              const int qrow = it.row.q_start + it.tok0 + ((w * ATTN_TILE) >> psh);
+              tma_load_4d(s.q[w], tq, &s.q_full[w], 0, it.q_head, qrow, it.batch);
+              tma_load_4d(s.q[w] + 16384, tq, &s.q_full[w], 64, it.q_head, qrow, it.batch);
+            }
+            ++live;
+            for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
+              const AttnSeg sg = fwd_seg(p, e);
+              const TileRange tr = fwd_tiles(p, it, sg);
+              const CUtensorMap* tk = &p.tmK[sg.src];
+              const CUtensorMap* tv = &p.tmV[sg.src];
+              if (tr.first < tr.end &&
+                  !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
+                report_error(wc, UA_ERR_FLAG_TIMEOUT, 111, sg.wait_flag);
+                ok = false;
+                break;
+              }
+              for (int t = tr.first; t < tr.end; ++t, ++j) {
+                const int st = j % STAGES;
+                const uint32_t ph = (j / STAGES) & 1;
+                const int krow = sg.start + t * ATTN_TILE;
+                if (!mbar_wait(&s.k_empty[st], ph ^ 1, wc, 100)) { ok = false; break; }
+                mbar_arrive_expect_tx(&s.k_full[st], FWD_TILE_BYTES);
+                tma_load_4d(s.k[st], tk, &s.k_full[st], 0, it.kv_head, krow, it.batch);
+                tma_load_4d(s.k[st] + 16384, tk, &s.k_full[st], 64, it.kv_head, krow, it.batch);
+                if (!mbar_wait(&s.v_empty[st], ph ^ 1, wc, 101)) { ok = false; break; }
+                mbar_arrive_expect_tx(&s.v_full[st], FWD_TILE_BYTES);
+                tma_load_4d(s.v[st], tv, &s.v_full[st], 0, it.kv_head, krow, it.batch);
+                tma_load_4d(s.v[st] + 16384, tv, &s.v_full[st], 64, it.kv_head, krow, it.batch);
+              }
             }
           }
+          if (!ok || !p.persist) break;
+          // everything of this item is on its way: take over the next one
+          mbar_arrive_expect_tx(&s.clc_full, 16);
+          clc_try_cancel(&s.clc, &s.clc_full);
+          if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
+          int bx, by;
+          const bool got = clc_read(&s.clc, bx, by);
+          fence_proxy_async_smem();               // read before the next response may overwrite it
+          if (got) it = fwd_item<FEW>(p, bx, by);
+          else it.exists = 0;
+          // the slot's previous item (n - 1) is done with
+          const uint32_t slot = (n + 1) & 1;
+          if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
+          s.item[slot] = it;
+          mbar_arrive(&s.item_full[slot]);
+          if (!got) break;
         }
-        if (!ok || !p.persist) break;
-        // everything of this item is on its way: take over the next one
-        mbar_arrive_expect_tx(&s.clc_full, 16);
-        clc_try_cancel(&s.clc, &s.clc_full);
-        if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
-        int bx, by;
-        const bool got = clc_read(&s.clc, bx, by);
-        fence_proxy_async_smem();               // read before the next response may overwrite it
-        if (got) it = fwd_item<FEW>(p, bx, by);
-        else it.exists = 0;
-        // the slot's previous item (n - 1) is done with
-        const uint32_t slot = (n + 1) & 1;
-        if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
-        s.item[slot] = it;
-        mbar_arrive(&s.item_full[slot]);
-        if (!got) break;
       }
-    }
-  } else if (warp == FWD_MMA_WARP) {
-    // =============================== MMA issuer =============================================
-    if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S = Q K^T, both K-major
-      const uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);   // O += P V, V is N-major
-      const uint32_t tS[2] = {tmem_base + 0, tmem_base + 128};
-      const uint32_t tO[2] = {tmem_base + 256, tmem_base + 384};
-      auto issue_s = [&](int w, int st) {
-        const uint32_t qa = smem_u32(s.q[FEW ? 0 : w]);
-        const uint32_t ka = smem_u32(s.k[st]);
+    } else if (warp == FWD_MMA_WARP) {
+      // =============================== MMA issuer =============================================
+      if (lane == 0) {
+        const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S = Q K^T, both K-major
+        const uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);   // O += P V, V is N-major
+        const uint32_t tS[2] = {tmem_base + 0, tmem_base + 128};
+        const uint32_t tO[2] = {tmem_base + 256, tmem_base + 384};
+        auto issue_s = [&](int w, int st) {
+          const uint32_t qa = smem_u32(s.q[FEW ? 0 : w]);
+          const uint32_t ka = smem_u32(s.k[st]);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_ss(tS[w], make_smem_desc_sw128(qa + off, 16, 1024),
-                  make_smem_desc_sw128(ka + off, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
-        }
-      };
-      auto issue_pv = [&](int w, int st, bool acc, int k0, int k1) {
-        const uint32_t va = smem_u32(s.v[st]);
+          for (int kk = 0; kk < 8; ++kk) {
+            const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
+            umma_ss(tS[w], make_smem_desc_sw128(qa + off, 16, 1024),
+                    make_smem_desc_sw128(ka + off, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
+          }
+        };
+        auto issue_pv = [&](int w, int st, bool acc, int k0, int k1) {
+          const uint32_t va = smem_u32(s.v[st]);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          if (kk < k0 || kk >= k1) continue;
-          // A: 16 keys = 8 packed columns of P; B: 16 key rows = 2048 B, d-halves 16384 B apart
-          umma_ts(tO[w], tS[w] + kk * 8, make_smem_desc_sw128(va + kk * 2048, 16384, 1024),
-                  idesc_o, (acc || kk > 0) ? 1u : 0u);
-        }
-      };
-      bool ok = true;
-      uint32_t kv = 0;                  // K / V tiles of the items before this one
-      uint32_t live = 0;
-      uint32_t p_cnt[2] = {0, 0};       // FEW: tiles of each sub-tile so far
-      for (uint32_t n = 0; ok; ++n) {
-        const int n_total = fwd_total(p, s.item[n & 1]);
-        if (n_total > 0) {
-          // (that O of the previous item has been read out is implied by p_full of this one's first tile:
-          // the same warps arrive there after their epilogue)
-          if (!mbar_wait(&s.q_full[0], live & 1, wc, 200)) break;
-          if constexpr (FEW) {
-            // key tile j belongs to sub-tile j & 1; its scores are issued two tiles ahead
-            auto next_s = [&](int j) -> bool {
-              const uint32_t g = kv + j;
-              if (!mbar_wait(&s.k_full[g % STAGES], (g / STAGES) & 1, wc, 201)) return false;
-              tc_fence_after_sync();
-              issue_s(j & 1, g % STAGES);
-              tc_commit(&s.s_full[j & 1]);
-              tc_commit(&s.k_empty[g % STAGES]);
-              if (j + 1 == n_total) tc_commit(&s.q_empty);
-              return true;
-            };
-            ok = next_s(0) && (n_total < 2 || next_s(1));
-            for (int j = 0; j < n_total && ok; ++j) {
-              const int w = j & 1, st = (kv + j) % STAGES;
-              if (!mbar_wait(&s.v_full[st], ((kv + j) / STAGES) & 1, wc, 203)) { ok = false; break; }
-              if (!mbar_wait(&s.p_full[w], p_cnt[w] & 1, wc, 204)) { ok = false; break; }
-              ++p_cnt[w];
-              tc_fence_after_sync();
-              issue_pv(w, st, j >= 2, 0, 8);
-              tc_commit(&s.v_empty[st]);
-              if (j + 2 < n_total) ok = next_s(j + 2);
-            }
-          } else {
-            if (!mbar_wait(&s.k_full[kv % STAGES], (kv / STAGES) & 1, wc, 201)) break;
-            tc_fence_after_sync();
-            issue_s(0, kv % STAGES);
-            tc_commit(&s.s_full[0]);
-            if (!mbar_wait(&s.q_full[1], live & 1, wc, 202)) break;
-            tc_fence_after_sync();
-            issue_s(1, kv % STAGES);
-            tc_commit(&s.s_full[1]);
-            tc_commit(&s.k_empty[kv % STAGES]);
-            if (n_total == 1) tc_commit(&s.q_empty);
-            for (int j = 0; j < n_total; ++j) {
-              const uint32_t g = kv + j;
-              const int st = g % STAGES;
-              const uint32_t ph = (g / STAGES) & 1;
-              const int stn = (g + 1) % STAGES;
-              const uint32_t phn = ((g + 1) / STAGES) & 1;
-              const bool more = (j + 1 < n_total);
-              FWD_PROF(g == FWD_PROF_TILE, 0);
-              if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
-              if (!mbar_wait(&s.p_part[0], g & 1, wc, 204)) { ok = false; break; }
-              FWD_PROF(g == FWD_PROF_TILE, 1);
-              tc_fence_after_sync();
-              issue_pv(0, st, j > 0, 0, P_PART / 16);
-              if (!mbar_wait(&s.p_full[0], g & 1, wc, 207)) { ok = false; break; }
-              tc_fence_after_sync();
-              issue_pv(0, st, j > 0, P_PART / 16, 8);
-              if (more) {
-                if (!mbar_wait(&s.k_full[stn], phn, wc, 205)) { ok = false; break; }
+          for (int kk = 0; kk < 8; ++kk) {
+            if (kk < k0 || kk >= k1) continue;
+            // A: 16 keys = 8 packed columns of P; B: 16 key rows = 2048 B, d-halves 16384 B apart
+            umma_ts(tO[w], tS[w] + kk * 8, make_smem_desc_sw128(va + kk * 2048, 16384, 1024),
+                    idesc_o, (acc || kk > 0) ? 1u : 0u);
+          }
+        };
+        bool ok = true;
+        uint32_t kv = 0;                  // K / V tiles of the items before this one
+        uint32_t live = 0;
+        uint32_t p_cnt[2] = {0, 0};       // FEW: tiles of each sub-tile so far
+        for (uint32_t n = 0; ok; ++n) {
+          const int n_total = fwd_total(p, s.item[n & 1]);
+          if (n_total > 0) {
+            // (that O of the previous item has been read out is implied by p_full of this one's first tile:
+            // the same warps arrive there after their epilogue)
+            if (!mbar_wait(&s.q_full[0], live & 1, wc, 200)) break;
+            if constexpr (FEW) {
+              // key tile j belongs to sub-tile j & 1; its scores are issued two tiles ahead
+              auto next_s = [&](int j) -> bool {
+                const uint32_t g = kv + j;
+                if (!mbar_wait(&s.k_full[g % STAGES], (g / STAGES) & 1, wc, 201)) return false;
                 tc_fence_after_sync();
-                issue_s(0, stn);
-                tc_commit(&s.s_full[0]);
+                issue_s(j & 1, g % STAGES);
+                tc_commit(&s.s_full[j & 1]);
+                tc_commit(&s.k_empty[g % STAGES]);
+                if (j + 1 == n_total) tc_commit(&s.q_empty);
+                return true;
+              };
+              ok = next_s(0) && (n_total < 2 || next_s(1));
+              for (int j = 0; j < n_total && ok; ++j) {
+                const int w = j & 1, st = (kv + j) % STAGES;
+                if (!mbar_wait(&s.v_full[st], ((kv + j) / STAGES) & 1, wc, 203)) { ok = false; break; }
+                if (!mbar_wait(&s.p_full[w], p_cnt[w] & 1, wc, 204)) { ok = false; break; }
+                ++p_cnt[w];
+                tc_fence_after_sync();
+                issue_pv(w, st, j >= 2, 0, 8);
+                tc_commit(&s.v_empty[st]);
+                if (j + 2 < n_total) ok = next_s(j + 2);
               }
-              FWD_PROF(g == FWD_PROF_TILE, 2);
-              if (!mbar_wait(&s.p_part[1], g & 1, wc, 206)) { ok = false; break; }
-              FWD_PROF(g == FWD_PROF_TILE, 3);
+            } else {
+              if (!mbar_wait(&s.k_full[kv % STAGES], (kv / STAGES) & 1, wc, 201)) break;
               tc_fence_after_sync();
-              issue_pv(1, st, j > 0, 0, P_PART / 16);
-              if (!mbar_wait(&s.p_full[1], g & 1, wc, 208)) { ok = false; break; }
+              issue_s(0, kv % STAGES);
+              tc_commit(&s.s_full[0]);
+              if (!mbar_wait(&s.q_full[1], live & 1, wc, 202)) break;
               tc_fence_after_sync();
-              issue_pv(1, st, j > 0, P_PART / 16, 8);
-              tc_commit(&s.v_empty[st]);
-              if (more) {
-                issue_s(1, stn);
-                tc_commit(&s.s_full[1]);
-                tc_commit(&s.k_empty[stn]);
-                if (j + 2 == n_total) tc_commit(&s.q_empty);
+              issue_s(1, kv % STAGES);
+              tc_commit(&s.s_full[1]);
+              tc_commit(&s.k_empty[kv % STAGES]);
+              if (n_total == 1) tc_commit(&s.q_empty);
+              for (int j = 0; j < n_total; ++j) {
+                const uint32_t g = kv + j;
+                const int st = g % STAGES;
+                const uint32_t ph = (g / STAGES) & 1;
+                const int stn = (g + 1) % STAGES;
+                const uint32_t phn = ((g + 1) / STAGES) & 1;
+                const bool more = (j + 1 < n_total);
+                FWD_PROF(g == FWD_PROF_TILE, 0);
+                if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
+                if (!mbar_wait(&s.p_part[0], g & 1, wc, 204)) { ok = false; break; }
+                FWD_PROF(g == FWD_PROF_TILE, 1);
+                tc_fence_after_sync();
+                issue_pv(0, st, j > 0, 0, P_PART / 16);
+                if (!mbar_wait(&s.p_full[0], g & 1, wc, 207)) { ok = false; break; }
+                tc_fence_after_sync();
+                issue_pv(0, st, j > 0, P_PART / 16, 8);
+                if (more) {
+                  if (!mbar_wait(&s.k_full[stn], phn, wc, 205)) { ok = false; break; }
+                  tc_fence_after_sync();
+                  issue_s(0, stn);
+                  tc_commit(&s.s_full[0]);
+                }
+                FWD_PROF(g == FWD_PROF_TILE, 2);
+                if (!mbar_wait(&s.p_part[1], g & 1, wc, 206)) { ok = false; break; }
+                FWD_PROF(g == FWD_PROF_TILE, 3);
+                tc_fence_after_sync();
+                issue_pv(1, st, j > 0, 0, P_PART / 16);
+                if (!mbar_wait(&s.p_full[1], g & 1, wc, 208)) { ok = false; break; }
+                tc_fence_after_sync();
+                issue_pv(1, st, j > 0, P_PART / 16, 8);
+                tc_commit(&s.v_empty[st]);
+                if (more) {
+                  issue_s(1, stn);
+                  tc_commit(&s.s_full[1]);
+                  tc_commit(&s.k_empty[stn]);
+                  if (j + 2 == n_total) tc_commit(&s.q_empty);
+                }
+                FWD_PROF(g == FWD_PROF_TILE, 4);
               }
-              FWD_PROF(g == FWD_PROF_TILE, 4);
             }
+            if (!ok) break;
+            // A sub-tile's next completion must not come before its warps have seen this one. They have when
+            // they arrive on p_full of the next item, which only a sub-tile with a key tile there is
+            // waited for: with one barrier for both, two items in a row could complete it unseen.
+            tc_commit(&s.o_full[0]);
+            if (FEW && n_total > 1) tc_commit(&s.o_full[1]);
+            kv += n_total;
+            ++live;
           }
-          if (!ok) break;
-          // A sub-tile's next completion must not come before its warps have seen this one. They have when
-          // they arrive on p_full of the next item, which only a sub-tile with a key tile there is
-          // waited for: with one barrier for both, two items in a row could complete it unseen.
-          tc_commit(&s.o_full[0]);
-          if (FEW && n_total > 1) tc_commit(&s.o_full[1]);
-          kv += n_total;
-          ++live;
+          if (!next_item(n)) break;
         }
-        if (!next_item(n)) break;
       }
     }
-  }
   } else {
-  reg_alloc<FWD_REGS_SOFTMAX>();
-  if ((warp & 3) < act_warps) {
-    // =============================== softmax + epilogue =====================================
-    const int w = warp >> 2;                 // sub-tile
-    const int quad = warp & 3;               // TMEM lane quadrant of this warp
-    const int r_tile = quad * 32 + lane;     // row inside the 128-row sub-tile
-    const int r_cta = (FEW ? 0 : w * ATTN_TILE) + r_tile;   // row inside the CTA's tile
-    const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tS = tmem_base + lane_base + w * 128;
-    const uint32_t tO = tmem_base + lane_base + 256 + w * 128;
-    const float NEG_INF = -INFINITY;
-    uint32_t cnt = 0;                        // score tiles of this sub-tile so far
-    uint32_t live = 0;                       // items with a key tile for this sub-tile so far
-    for (uint32_t n = 0;; ++n) {
-    const FwdItem& it = s.item[n & 1];       // (stays in shared memory: the score loop needs the registers)
-    const int r_blk = (it.r0 + r_cta) >> psh;               // query token inside the query block
-    if (n > 0) trace_stamp(p.trace, it.linear, 0);
-    trace_stamp(p.trace, it.linear, 1);
-    trace_ident(p.trace, it.linear, it.row_idx);
-    float m_use = NEG_INF;   // running reference max, log2 units (already scaled)
-    float l = 0.f;           // row sum
-    bool ok = true;
-    uint32_t j = 0;
-    for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
-      const AttnSeg sg = fwd_seg(p, e);
-      const TileRange tr = fwd_tiles(p, it, sg);
-      for (int t = tr.first; t < tr.end; ++t, ++j) {
-        if (FEW && (j & 1) != static_cast<uint32_t>(w)) continue;
-        const bool prof = (n == 0) && (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0;
-        const int pslot = 8 + w * 24 + (static_cast<int>(j) - FWD_PROF_TILE) * 8;
-        (void)prof; (void)pslot;
-        FWD_PROF(prof, pslot + 0);
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full[w], cnt & 1, wc, 300 + w))) { ok = false; break; }
-        FWD_PROF(prof, pslot + 1);
-        ++cnt;
-        tc_fence_after_sync();
-        float sv[ATTN_TILE];
-        {
-          uint32_t(&raw)[ATTN_TILE] = reinterpret_cast<uint32_t(&)[ATTN_TILE]>(sv);
+    reg_alloc<FWD_REGS_SOFTMAX>();
+    if ((warp & 3) < act_warps) {
+      // =============================== softmax + epilogue =====================================
+      const int w = warp >> 2;                 // sub-tile
+      const int quad = warp & 3;               // TMEM lane quadrant of this warp
+      const int r_tile = quad * 32 + lane;     // row inside the 128-row sub-tile
+      const int r_cta = (FEW ? 0 : w * ATTN_TILE) + r_tile;   // row inside the CTA's tile
+      const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+      const uint32_t tS = tmem_base + lane_base + w * 128;
+      const uint32_t tO = tmem_base + lane_base + 256 + w * 128;
+      const float NEG_INF = -INFINITY;
+      uint32_t cnt = 0;                        // score tiles of this sub-tile so far
+      uint32_t live = 0;                       // items with a key tile for this sub-tile so far
+      for (uint32_t n = 0;; ++n) {
+        const FwdItem& it = s.item[n & 1];       // (stays in shared memory: the score loop needs the registers)
+        const int r_blk = (it.r0 + r_cta) >> psh;               // query token inside the query block
+        if (n > 0) trace_stamp(p.trace, it.linear, 0);
+        trace_stamp(p.trace, it.linear, 1);
+        trace_ident(p.trace, it.linear, it.row_idx);
+        float m_use = NEG_INF;   // running reference max, log2 units (already scaled)
+        float l = 0.f;           // row sum
+        bool ok = true;
+        uint32_t j = 0;
+        for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
+          const AttnSeg sg = fwd_seg(p, e);
+          const TileRange tr = fwd_tiles(p, it, sg);
+          for (int t = tr.first; t < tr.end; ++t, ++j) {
+            if (FEW && (j & 1) != static_cast<uint32_t>(w)) continue;
+            const bool prof = (n == 0) && (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0;
+            const int pslot = 8 + w * 24 + (static_cast<int>(j) - FWD_PROF_TILE) * 8;
+            (void)prof; (void)pslot;
+            FWD_PROF(prof, pslot + 0);
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full[w], cnt & 1, wc, 300 + w))) { ok = false; break; }
+            FWD_PROF(prof, pslot + 1);
+            ++cnt;
+            tc_fence_after_sync();
+            float sv[ATTN_TILE];
+            {
+              uint32_t(&raw)[ATTN_TILE] = reinterpret_cast<uint32_t(&)[ATTN_TILE]>(sv);
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            tmem_ld_x32(tS + c * 32, reinterpret_cast<uint32_t(&)[32]>(raw[c * 32]));
-          tmem_wait_ld();
-        }
-        FWD_PROF(prof, pslot + 2);
-        // masking: key index c (segment-relative) allowed iff c < len, c <= r + diag and c >= r + lo
-        const int c0 = t * ATTN_TILE;
-        int limit = sg.len - c0;                               // columns < limit are in range
-        if (sg.causal & SEG_UPPER) limit = min(limit, r_blk + sg.diag - c0 + 1);
-        if (limit < ATTN_TILE) {
+              for (int c = 0; c < 4; ++c)
+                tmem_ld_x32(tS + c * 32, reinterpret_cast<uint32_t(&)[32]>(raw[c * 32]));
+              tmem_wait_ld();
+            }
+            FWD_PROF(prof, pslot + 2);
+            // masking: key index c (segment-relative) allowed iff c < len, c <= r + diag and c >= r + lo
+            const int c0 = t * ATTN_TILE;
+            int limit = sg.len - c0;                               // columns < limit are in range
+            if (sg.causal & SEG_UPPER) limit = min(limit, r_blk + sg.diag - c0 + 1);
+            if (limit < ATTN_TILE) {
 #pragma unroll
-          for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i < limit) ? sv[i] : NEG_INF;
-        }
-        if (sg.causal & SEG_LOWER) {
-          const int first = r_blk + sg.lo - c0;                // columns >= first are in range
-          if (first > 0) {
+              for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i < limit) ? sv[i] : NEG_INF;
+            }
+            if (sg.causal & SEG_LOWER) {
+              const int first = r_blk + sg.lo - c0;                // columns >= first are in range
+              if (first > 0) {
 #pragma unroll
-            for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i >= first) ? sv[i] : NEG_INF;
-          }
-        }
-        // eight independent running maxima, two new values per instruction: one dependent chain of
-        // compares would cost more than the exponentials
-        float mx8[8];
+                for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i >= first) ? sv[i] : NEG_INF;
+              }
+            }
+            // eight independent running maxima, two new values per instruction: one dependent chain of
+            // compares would cost more than the exponentials
+            float mx8[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(sv[i], sv[8 + i]);
+            for (int i = 0; i < 8; ++i) mx8[i] = fmaxf(sv[i], sv[8 + i]);
 #pragma unroll
-        for (int i = 16; i < ATTN_TILE; i += 16)
+            for (int i = 16; i < ATTN_TILE; i += 16)
 #pragma unroll
-          for (int k = 0; k < 8; ++k) mx8[k] = fmax3(mx8[k], sv[i + k], sv[i + 8 + k]);
-        float mx = fmaxf(fmax3(mx8[0], mx8[1], mx8[2]), fmax3(mx8[3], mx8[4], mx8[5]));
-        mx = fmax3(mx, mx8[6], mx8[7]);
-        mx *= p.scale_log2;
-        const float m_new = fmaxf(m_use, mx);
-        // lazy rescale: only when the running max grew by more than 2^8 (warp-uniform branch,
-        // because the TMEM accesses below are warp-collective)
-        const bool need = (m_new - m_use > 8.0f) || (m_use == NEG_INF && m_new > NEG_INF);
-        if (j < (FEW ? 2u : 1u)) {
-          m_use = m_new;
-        } else if (__any_sync(0xFFFFFFFFu, need)) {
-          const float alpha = need ? fast_exp2(m_use - m_new) : 1.0f;
-          if (need) m_use = m_new;
-          l *= alpha;
+              for (int k = 0; k < 8; ++k) mx8[k] = fmax3(mx8[k], sv[i + k], sv[i + 8 + k]);
+            float mx = fmaxf(fmax3(mx8[0], mx8[1], mx8[2]), fmax3(mx8[3], mx8[4], mx8[5]));
+            mx = fmax3(mx, mx8[6], mx8[7]);
+            mx *= p.scale_log2;
+            const float m_new = fmaxf(m_use, mx);
+            // lazy rescale: only when the running max grew by more than 2^8 (warp-uniform branch,
+            // because the TMEM accesses below are warp-collective)
+            const bool need = (m_new - m_use > 8.0f) || (m_use == NEG_INF && m_new > NEG_INF);
+            if (j < (FEW ? 2u : 1u)) {
+              m_use = m_new;
+            } else if (__any_sync(0xFFFFFFFFu, need)) {
+              const float alpha = need ? fast_exp2(m_use - m_new) : 1.0f;
+              if (need) m_use = m_new;
+              l *= alpha;
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t ov[32];
-            tmem_ld_x32(tO + c * 32, ov);
-            tmem_wait_ld();
+              for (int c = 0; c < 4; ++c) {
+                uint32_t ov[32];
+                tmem_ld_x32(tO + c * 32, ov);
+                tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-            tmem_st_x32(tO + c * 32, ov);
-          }
-        }
-        FWD_PROF(prof, pslot + 3);
-        const float m_eff = (m_use == NEG_INF) ? 0.f : m_use;
-        // multiply-add and row sum on packed pairs; four independent partial sums
-        const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
-        const uint64_t nm2 = f2_pack(-m_eff, -m_eff);
-        uint64_t ls2[4];
+                for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+                tmem_st_x32(tO + c * 32, ov);
+              }
+            }
+            FWD_PROF(prof, pslot + 3);
+            const float m_eff = (m_use == NEG_INF) ? 0.f : m_use;
+            // multiply-add and row sum on packed pairs; four independent partial sums
+            const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
+            const uint64_t nm2 = f2_pack(-m_eff, -m_eff);
+            uint64_t ls2[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) ls2[k] = f2_pack(0.f, 0.f);
+            for (int k = 0; k < 4; ++k) ls2[k] = f2_pack(0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t pk[16];
+            for (int c = 0; c < 4; ++c) {
+              uint32_t pk[16];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            float x0, x1;
-            f2_unpack(f2_fma(f2_pack(sv[c * 32 + 2 * i], sv[c * 32 + 2 * i + 1]), sc2, nm2), x0, x1);
-            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-            ls2[i & 3] = f2_add(ls2[i & 3], f2_pack(p0, p1));
-            pk[i] = pack_bf16x2(p0, p1);
-          }
-          tmem_st_x16(tS + c * 16, pk);
-          if (!FEW && c == P_PART / 32 - 1) {      // (FEW is bound by memory, not by this chain)
+              for (int i = 0; i < 16; ++i) {
+                float x0, x1;
+                f2_unpack(f2_fma(f2_pack(sv[c * 32 + 2 * i], sv[c * 32 + 2 * i + 1]), sc2, nm2), x0, x1);
+                const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+                ls2[i & 3] = f2_add(ls2[i & 3], f2_pack(p0, p1));
+                pk[i] = pack_bf16x2(p0, p1);
+              }
+              tmem_st_x16(tS + c * 16, pk);
+              if (!FEW && c == P_PART / 32 - 1) {      // (FEW is bound by memory, not by this chain)
+                tmem_wait_st();
+                tc_fence_before_sync();
+                mbar_arrive_warp(&s.p_part[w]);
+              }
+            }
+            float ls4[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              float a, b;
+              f2_unpack(ls2[k], a, b);
+              ls4[k] = a + b;
+            }
+            l += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
+            FWD_PROF(prof, pslot + 4);
             tmem_wait_st();
             tc_fence_before_sync();
-            mbar_arrive_warp(&s.p_part[w]);
+            mbar_arrive_warp(&s.p_full[w]);
+            FWD_PROF(prof, pslot + 5);
           }
         }
-        float ls4[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float a, b;
-          f2_unpack(ls2[k], a, b);
-          ls4[k] = a + b;
-        }
-        l += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
-        FWD_PROF(prof, pslot + 4);
-        tmem_wait_st();
-        tc_fence_before_sync();
-        mbar_arrive_warp(&s.p_full[w]);
-        FWD_PROF(prof, pslot + 5);
+        // ---------------------------------- epilogue --------------------------------------------
+        const bool any = j > (FEW ? static_cast<uint32_t>(w) : 0u);
+        if (any && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full[FEW ? w : 0], live & 1, wc, 310 + w));
+        tc_fence_after_sync();
+        if constexpr (FEW) fwd_epilogue<true>(s, n & 1, tO, l, m_use, any);
+        else fwd_epilogue_call(s, n & 1, tO, l, m_use, any);
+        trace_stamp(p.trace, it.linear, 2);
+        if (any) ++live;
+        if (!ok) break;
+        __syncwarp();                            // every lane is done reading the item
+        int more = 0;
+        if (lane == 0) more = next_item(n) ? 1 : 0;
+        if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
+        __syncwarp();                            // lane 0 has seen the item; this makes it visible to the others (a shuffle does not)
       }
     }
-    // ---------------------------------- epilogue --------------------------------------------
-    const bool any = j > (FEW ? static_cast<uint32_t>(w) : 0u);
-    if (any && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full[FEW ? w : 0], live & 1, wc, 310 + w));
-    tc_fence_after_sync();
-    if constexpr (FEW) fwd_epilogue<true>(s, n & 1, tO, l, m_use, any);
-    else fwd_epilogue_call(s, n & 1, tO, l, m_use, any);
-    trace_stamp(p.trace, it.linear, 2);
-    if (any) ++live;
-    if (!ok) break;
-    __syncwarp();                            // every lane is done reading the item
-    int more = 0;
-    if (lane == 0) more = next_item(n) ? 1 : 0;
-    if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
-    __syncwarp();                            // lane 0 has seen the item; this makes it visible to the others (a shuffle does not)
-    }
-  }
   }
 
   tc_fence_before_sync();
