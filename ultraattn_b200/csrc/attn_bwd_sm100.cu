@@ -192,6 +192,7 @@ __device__ long long g_bwd_prof[64];
 #define BWD_PROF(cond, slot) do { } while (0)
 #endif
 constexpr int BWD_PROF_STEP = 8;
+constexpr int BWD_PROF_SPAN = 32;      // steps between the stamps 0 and 9 of the MMA warp
 
 // Walks the (query head of the group, query segment, 128-query tile) steps of one key tile in the
 // order every role of the CTA uses.
@@ -602,6 +603,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
               // dV += P^T dO : A = P^T in TMEM (queries 0-63 packed at columns 0-31, 64-127 at 64-95),
               // B = dO as an N-major operand (16 query rows = 2048 B, d-halves 16384 B apart)
               BWD_PROF(i == BWD_PROF_STEP, 0);
+              BWD_PROF(i == BWD_PROF_STEP + BWD_PROF_SPAN, 9);
               if (!mbar_wait(&s.p_ready, ph, wc, 203)) { ok = false; break; }
               BWD_PROF(i == BWD_PROF_STEP, 1);
               tc_fence_after_sync();

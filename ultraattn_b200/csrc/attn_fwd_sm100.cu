@@ -39,18 +39,22 @@ constexpr int FWD_SOFTMAX_WARPS = 8;
 constexpr int FWD_TMA_WARP = 8;
 constexpr int FWD_MMA_WARP = 9;
 // three warpgroups (the last one: TMA, MMA and two idle warps), so that the register file can be
-// re-balanced by warpgroup: a softmax thread holds its row's 128 scores besides everything else and
-// spills at the 168 registers an even split leaves; 2 x 200 + 104 <= 3 x 168
+// re-balanced by warpgroup: a softmax thread holds its row's 128 scores besides everything else;
+// 2 x 200 + 104 <= 3 x 168. The compiler allocates for the 168 of the launch: in the two-tile form three words
+// that do not change in the score loop stay outside them and are read back once per tile (ncu: 3.1 local loads
+// per warp and tile, 12 stores per CTA in all); the FEW form has none.
 constexpr int FWD_THREADS = 384;
 constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 104, FWD_REGS_SOFTMAX = 200;
 static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
-// The MMA warp starts P V on the first 96 keys of a tile while the softmax warps compute the last 32. A
-// tile pair is bound by two chains of the same length, 3350 clocks: the 32 MMAs, which take 89 clocks each
-// with TMA writes and operand reads on one shared-memory port, and one sub-tile's softmax (1950) plus
-// its own 16 MMAs. Measured (us) without -> with: 4 x 2000 tokens 184 -> 180, causal 8k tokens, 32 heads
-// 592 -> 576, full 16k 3630 -> 3560; 32 or 64 keys in front of the hand-over are within 0.5 %. With 128
-// keys' maxima found beside the exponentials of the tile (against the running maximum) the softmax
-// is 100 clocks shorter and nothing faster.
+// The MMA warp starts P V on the first 96 keys of a tile while the softmax warps compute the last 32. A pair of
+// tiles takes 3320 clocks (full attention, 16k tokens), and what it follows is one sub-tile's own cycle, because P
+// overwrites S: with clock stamps, which make it 3500, the softmax takes 1915 from seeing the scores to
+// handing over P, and its next scores are there 1590 later (its own 16 MMAs, 90 clocks each with TMA writes
+// and operand reads on the same shared memory, and the hand-overs). The MMA warp issues during 2 x 1450 of
+// the 3500 and waits for P in the rest. Measured (us) without -> with: 4 x 2000 tokens 184 -> 180, causal 8k
+// tokens, 32 heads 592 -> 576, full 16k 3630 -> 3560; 32 or 64 keys in front of the hand-over are within 0.5 %. With
+// 128 keys' maxima found beside the exponentials of the tile (against the running maximum) the softmax is 100
+// clocks shorter and nothing faster.
 constexpr int P_PART = 96;
 constexpr int FWD_TILE_BYTES = ATTN_TILE * ATTN_D * 2;  // 32 KB: [2 d-halves][128 rows][128 B]
 
@@ -182,6 +186,7 @@ __device__ long long g_fwd_prof[64];
 #define FWD_PROF(cond, slot) do { } while (0)
 #endif
 constexpr int FWD_PROF_TILE = 8;
+constexpr int FWD_PROF_SPAN = 32;      // tiles between the stamps 0 and 5 of the MMA warp
 
 
 template <bool FEW>
@@ -390,8 +395,8 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
 }
 
 // Called, not inlined, by the two-tile form: inlined, its addresses compete with the score loop for
-// registers, which costs the loop spills and 2 % of its rate. (The FEW form has registers to spare, and a
-// call costs its short items 4 %.)
+// registers, which costs the loop further spills (20 to 236 bytes, where the call has 12) and 2 % of its
+// rate. (The FEW form has registers to spare, and a call costs its short items 4 %.)
 __device__ __noinline__ void fwd_epilogue_call(FwdSmem<false>& s, uint32_t slot, uint32_t tO, float l, float m_use, bool any) {
   fwd_epilogue<false>(s, slot, tO, l, m_use, any);
 }
@@ -632,6 +637,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
                 const uint32_t phn = ((g + 1) / STAGES) & 1;
                 const bool more = (j + 1 < n_total);
                 FWD_PROF(g == FWD_PROF_TILE, 0);
+              FWD_PROF(g == FWD_PROF_TILE + FWD_PROF_SPAN, 5);
                 if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
                 if (!mbar_wait(&s.p_part[0], g & 1, wc, 204)) { ok = false; break; }
                 FWD_PROF(g == FWD_PROF_TILE, 1);

@@ -597,9 +597,8 @@ def attn_bwd_cuda(q_sides: Sequence[BwdQSide], k_srcs, v_srcs, kv_outs: Sequence
     st = status_buffer(q0.device)
     tables = (None, None, None, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(),
                                                   plan.tiles_t.data_ptr(), plan.n_tiles)
-    rc = lib.ua_attn_bwd(qs, dos, sides, nq, ks, vs, len(k_srcs), kos, len(ko), *tables, dense, n_heads, n_kv_heads, q0.shape[0], scale, st.data_ptr(),
-                         *_stage_args(stage),
-                         _lib.stream_of(q0))
+    rc = lib.ua_attn_bwd(qs, dos, sides, nq, ks, vs, len(k_srcs), kos, len(ko), *tables, dense, n_heads, n_kv_heads,
+                         q0.shape[0], scale, st.data_ptr(), *_stage_args(stage), _lib.stream_of(q0))
     _lib.check(rc, "ua_attn_bwd")
 
 
