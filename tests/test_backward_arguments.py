@@ -279,3 +279,11 @@ def test_gradients_of_tokens_outside_every_sequence_are_zero(prefix):
         ref = [t.detach().double().requires_grad_() for t in (q, k, v)]
         _documents(*ref, cu, True).backward(d_o.double())
         assert all(_close(a, b.grad) for a, b in zip(got, ref))
+
+
+def test_plans_know_whether_a_few_tiles_hold_most_of_the_work():
+    from ultraattn_b200 import api, patterns as P
+    skewed = lambda pattern: api.local_plans(pattern, 4096, "cpu")[1].skewed
+    assert not any(skewed(p) for p in (P.causal(1), P.full(1), P.strided(32, 4, 2)))
+    assert all(skewed(p) for p in (P.global_local(32, 1, 2), P.star(32, 1), P.streaming(32, 1, 2)))
+    assert not A.BwdPlan([]).skewed

@@ -119,3 +119,20 @@ def test_dense(B, Sq, Skv, H, Hk, causal):
     grads = local_backward(q, k, v, o, lse, d_o, None, None, 2 if causal else 1)
     r, c = torch.arange(Sq, device="cuda")[:, None], torch.arange(Skv, device="cuda")[None]
     _check(o, lse, grads, q, k, v, d_o, (c <= r + Skv - Sq) if causal else torch.ones(Sq, Skv, dtype=torch.bool, device="cuda"))
+
+
+def test_backward_with_a_limited_number_of_interleaved_heads():
+    """12288 tokens, groups of four: five of the six heads end the launch together, one runs in front. Every
+    head's dK and dV as in a launch of its own, bit for bit; dQ is summed in arrival order."""
+    from ultraattn_b200.api import local_backward
+    S, H, Hk = 12288, 24, 6
+    q, k, v, d_o = _rand(5, (1, S, H), (1, S, Hk), (1, S, Hk), (1, S, H))
+    o, lse = torch.empty_like(q), torch.empty(1, H, S, device="cuda")
+    A.attn_fwd_dense(q, k, v, (o, lse), True)
+    dq, dk, dv = local_backward(q, k, v, o, lse, d_o, None, None, 2)
+    for h in range(Hk):
+        qs, ks = slice(4 * h, 4 * h + 4), slice(h, h + 1)
+        part = local_backward(q[:, :, qs], k[:, :, ks], v[:, :, ks], o[:, :, qs], lse[:, qs].contiguous(), d_o[:, :, qs], None, None, 2)
+        assert torch.equal(dk[:, :, ks], part[1]) and torch.equal(dv[:, :, ks], part[2])
+        assert (dq[:, :, qs].float() - part[0].float()).norm() <= 2 ** -8 * part[0].float().norm()
+    A.check_status()

@@ -52,7 +52,7 @@ def _declare(lib):
         "ua_attn_bwd_local": [c_char_p, f, vp, vp],
         "ua_attn_bwd": [POINTER(UaTensorSrc), POINTER(UaTensorSrc), POINTER(UaBwdQSide), i,
                         POINTER(UaTensorSrc), POINTER(UaTensorSrc), i, POINTER(UaBwdKvOut), i,
-                        vp, vp, vp, i, i, i, i, i, f, vp, vp, i, i, vp, i, vp, vp],
+                        vp, vp, vp, i, i, i, i, i, i, f, vp, vp, i, i, vp, i, vp, vp],
         "ua_barrier": [POINTER(vp), i, i, i, ctypes.c_uint, ctypes.c_double, vp, vp],
         "ua_xent_fwd": [vp, vp, vp, vp, l, l, i, vp],
         "ua_xent_bwd": [vp, vp, vp, vp, l, l, i, vp],

@@ -988,12 +988,13 @@ static int encode_src_box(CUtensorMap* tm, const UaTensorSrc& t, uint32_t rows) 
 static int g_bwd_smem_set[64] = {0};
 
 // dense = 0: tables; 1 / 2: all queries of source 0 against all its keys, without a mask / causal (key c is
-// visible to query r iff c <= r + skv - sq); the table arguments are then not read.
+// visible to query r iff c <= r + skv - sq); the table arguments are then not read. skewed: the plan's heaviest tile
+// has far more work than the average one.
 extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
                            const UaBwdQSide* q_side, int n_q, const UaTensorSrc* k_src,
                            const UaTensorSrc* v_src, int n_kv, const UaBwdKvOut* kv_out, int n_out,
                            const void* cols_dev, const void* segs_dev, const void* tiles_dev,
-                           int n_tiles, int dense, int n_heads, int n_kv_heads, int batch,
+                           int n_tiles, int dense, int skewed, int n_heads, int n_kv_heads, int batch,
                            float softmax_scale, int* status, const void* copy_tasks_dev,
                            int n_copy_tasks, int n_copy_ctas, unsigned int* stage_flags,
                            int stage_epoch, unsigned int* stage_ticket, cudaStream_t stream) {
@@ -1059,7 +1060,12 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
     p.stage.n_copy_ctas = static_cast<int>(n_copy_ctas < grid_ctas ? n_copy_ctas : grid_ctas);
   }
   p.persist = stage_flags == nullptr;
-  p.tail_heads = stage_flags == nullptr && dense != 1 ? tail_heads(n_tiles, n_kv_heads, sm_count()) : 1;
+  // What the items of a key/value head walk on the query side, for the limit of tail_heads. Plans with a few tiles
+  // that are far heavier than the others have no limit: their end is worth more than their traffic (global +
+  // local blocks, 32 / 8 heads, 32768 tokens 5001 us with 3 heads interleaved, 5420 with 2, 6049 head by head).
+  long head_bytes = 0;
+  for (int i = 0; i < n_q && !skewed; ++i) head_bytes += q_src[i].tokens * (n_heads / n_kv_heads) * (ATTN_D * 8L);
+  p.tail_heads = stage_flags == nullptr && dense != 1 ? tail_heads(n_tiles, n_kv_heads, sm_count(), head_bytes) : 1;
   p.stage.flags = stage_flags;
   p.stage.epoch = stage_epoch;
   p.stage.ticket = stage_ticket;
@@ -1108,7 +1114,7 @@ struct UaLocalBwd {
   const void* cols;              // tables as in ua_attn_bwd, not read if dense
   const void* segs;
   const void* tiles;
-  long n_tiles, dense;
+  long n_tiles, dense, skewed;
 };
 
 extern "C" int ua_attn_bwd_local(const UaLocalBwd* t, float softmax_scale, int* status, cudaStream_t stream) {
@@ -1127,7 +1133,7 @@ extern "C" int ua_attn_bwd_local(const UaLocalBwd* t, float softmax_scale, int* 
   side.dq_batch_stride = tokens * heads * ATTN_D;
   const UaBwdKvOut out = {t->dk, t->dv, t->dkv_row_stride, t->dkv_batch_stride, 0, 0};
   if (ua_attn_bwd(&t->q, &t->d_o, &side, 1, &t->k, &t->v, 1, &out, 1, t->cols, t->segs, t->tiles,
-                  static_cast<int>(t->n_tiles), static_cast<int>(t->dense), static_cast<int>(heads),
+                  static_cast<int>(t->n_tiles), static_cast<int>(t->dense), static_cast<int>(t->skewed), static_cast<int>(heads),
                   static_cast<int>(t->k.heads), static_cast<int>(batch), softmax_scale, status, nullptr, 0, 0, nullptr, 1,
                   nullptr, stream))
     return -1;
@@ -1260,7 +1266,7 @@ extern "C" int ua_attn_bwd_dense_noalloc(const void* q, const void* k, const voi
   p.stage.n_tasks = 0;
   p.stage.n_copy_ctas = 0;
   p.persist = 1;
-  p.tail_heads = causal ? tail_heads(n_tiles, n_kv_heads, sm_count()) : 1;
+  p.tail_heads = causal ? tail_heads(n_tiles, n_kv_heads, sm_count(), tokens * p.kv_group * (ATTN_D * 8L)) : 1;
   p.stage.flags = nullptr;
   p.stage.epoch = 1;
   p.stage.ticket = nullptr;

@@ -82,8 +82,17 @@ __host__ __device__ __forceinline__ ItemIndex item_index(int bx, int n_tiles, in
   return ItemIndex{heads - tail + (bx - lead) % tail, (bx - lead) / tail};
 }
 constexpr int TAIL_WAVES = 4;
-inline int tail_heads(int n_tiles, int heads, int sms) {
-  const int t = (TAIL_WAVES * sms + n_tiles - 1) / n_tiles;
+// Interleaved heads are in flight together, each at all its places at once: when they do not fit L2 any more, that
+// costs more than the launch's end gains. `head_bytes` (0: no limit) is what the items of one head walk;
+// together the interleaved ones may have twice the size of L2. Backward (a token of a query head: Q and
+// dO in bf16, dQ in fp32, 1 KB), causal, us, with the heads that the waves alone ask for / limited / head by head:
+// 32 / 8 heads, 12288 tokens 3243 (7 heads) / 2797 (5) / 2955; 16384 tokens 5440 (5) / 4716 (4) / 4865, with 16.5 GB of
+// DRAM traffic at 5 heads, 3.9 at 3 and 0.9 head by head; 24576 tokens 10585 (4) / 10468 (2) / 10637; 64 / 16
+// heads, 16384 tokens 9940 (5) / 9363 (4) / 9560. 8192 tokens, 32 / 8 heads stay under it: 1264 (8) / 1491 head by head.
+constexpr long TAIL_BYTES = 256L << 20;
+inline int tail_heads(int n_tiles, int heads, int sms, long head_bytes = 0) {
+  int t = (TAIL_WAVES * sms + n_tiles - 1) / n_tiles;
+  if (head_bytes > 0 && t * head_bytes > TAIL_BYTES) t = head_bytes < TAIL_BYTES ? static_cast<int>(TAIL_BYTES / head_bytes) : 1;
   return t < heads ? t : heads;
 }
 

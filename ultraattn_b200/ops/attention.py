@@ -315,7 +315,7 @@ def tensor_map_cache_stats() -> tuple[int, int]:
 # Argument blocks of 64-bit fields (struct UaDenseFwd, UaLocalBwd of csrc/): one packed block costs the
 # host a few microseconds less than the ctypes structures of the table launches.
 _DENSE_FWD = struct.Struct("=27q")
-_LOCAL_BWD = struct.Struct("=44q")
+_LOCAL_BWD = struct.Struct("=45q")
 
 
 def _src_fields(t: torch.Tensor) -> tuple:
@@ -534,6 +534,8 @@ class BwdPlan:
         tiles = _launch_order(tiles)
         self.n_tiles = len(tiles)
         self.kv_tokens = sum(c.kv_len for c in self.cols)      # gradient rows that the columns write
+        # (causal blocks: heaviest tile twice the average, strided ones 1.8; global + local 9, star and streaming 12 to 20)
+        self.skewed = bool(tiles) and max(t[0] for t in tiles) * len(tiles) > 3 * sum(t[0] for t in tiles)
         self.total_steps = sum(c for c, _, _ in tiles)
         seg_arr = np.array(segs, dtype=np.int32).reshape(-1, 8) if segs else np.zeros((1, 8), np.int32)
         tile_arr = (np.array([(ci, t) for _, ci, t in tiles], dtype=np.int32).reshape(-1, 2)
@@ -597,7 +599,8 @@ def attn_bwd_cuda(q_sides: Sequence[BwdQSide], k_srcs, v_srcs, kv_outs: Sequence
     st = status_buffer(q0.device)
     tables = (None, None, None, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(),
                                                   plan.tiles_t.data_ptr(), plan.n_tiles)
-    rc = lib.ua_attn_bwd(qs, dos, sides, nq, ks, vs, len(k_srcs), kos, len(ko), *tables, dense, n_heads, n_kv_heads,
+    skewed = 0 if dense else int(plan.skewed)
+    rc = lib.ua_attn_bwd(qs, dos, sides, nq, ks, vs, len(k_srcs), kos, len(ko), *tables, dense, skewed, n_heads, n_kv_heads,
                          q0.shape[0], scale, st.data_ptr(), *_stage_args(stage), _lib.stream_of(q0))
     _lib.check(rc, "ua_attn_bwd")
 
@@ -698,7 +701,7 @@ def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense
     tables = (0, 0, 0, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(), plan.n_tiles)
     block = _LOCAL_BWD.pack(*_src_fields(q), *_src_fields(k), *_src_fields(v), *_src_fields(d_o), o.data_ptr(), *so,
                             lse.data_ptr(), dvec.data_ptr(), dq32.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *sk,
-                            *tables, dense)
+                            *tables, dense, 0 if dense else int(plan.skewed))
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     rc = _lib.load().ua_attn_bwd_local(block, scale, status_buffer(q.device).data_ptr(), _lib.stream_of(q))
     _lib.check(rc, "ua_attn_bwd_local", 3)
