@@ -12,14 +12,18 @@
 //
 // CTA: warps 0-3 softmax / correction / epilogue of sub-tile 0 (one thread per query
 // row, 128 score columns each), warps 4-7 the same for sub-tile 1, then one TMA producer warp and
-// one tcgen05.mma issuer warp (one elected thread; it also owns the TMEM allocation). The two
+// the tcgen05.mma issuer warps (one elected thread each; the first owns the TMEM allocation). The two
 // sub-tiles run ping-pong, so that the tensor core works on one while the softmax warps work on
 // the other:
 //   FEW = false: 256 query rows, 128 per sub-tile; both sub-tiles visit every key tile
 //   FEW = true:  up to 128 query rows, the same ones in both sub-tiles, which take the key tiles in
 //                turn (decoding: a handful of rows behind a long cache)
-// TMEM (512 columns): S0 | S1 | O0 | O1, 128 fp32 columns each; P (bf16) overwrites the first
-// 64 columns of its S region and is consumed from TMEM as the A operand of the PV product.
+// TMEM (512 columns):
+//   FEW = false: S 128 | P0 64 | P1 64 | O0 128 | O1 128. The score tile is shared: a softmax thread has its row's
+//                128 scores in registers 300 clocks after they are there, and from then on the other sub-tile's
+//                next scores may be computed. Q K^T and P V then have an issuing warp each.
+//   FEW = true:  S0 | S1 | O0 | O1, P (bf16) overwrites the first 64 columns of its S; one issuing warp.
+// P is consumed from TMEM as the A operand of the PV product.
 //
 // Two kinds of launches use the kernel. Table launches (ua_attn_fwd) read rows, segments and tiles
 // from device tables. Dense launches (ua_attn_fwd_dense: all queries against all keys, causal or
@@ -37,25 +41,28 @@ namespace ua {
 
 constexpr int FWD_SOFTMAX_WARPS = 8;
 constexpr int FWD_TMA_WARP = 8;
-constexpr int FWD_MMA_WARP = 9;
-// three warpgroups (the last one: TMA, MMA and two idle warps), so that the register file can be
-// re-balanced by warpgroup: a softmax thread holds its row's 128 scores besides everything else;
-// 2 x 200 + 104 <= 3 x 168. The compiler allocates for the 168 of the launch: in the two-tile form three words
-// that do not change in the score loop stay outside them and are read back once per tile (ncu: 3.1 local loads
-// per warp and tile, 12 stores per CTA in all); the FEW form has none.
+constexpr int FWD_QK_WARP = 9;         // issues S = Q K^T; owns the TMEM allocation
+constexpr int FWD_PV_WARP = 10;        // issues O += P V
+// three warpgroups (the last one: TMA, MMA and an idle warp), so that the register file can be
+// re-balanced by warpgroup: a softmax thread holds its row's 128 scores besides everything else (the assembler
+// allocates for the new number behind setmaxnreg); 2 x 216 + 72 <= 3 x 168.
 constexpr int FWD_THREADS = 384;
-constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 104, FWD_REGS_SOFTMAX = 200;
+constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 72, FWD_REGS_SOFTMAX = 216;
 static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
-// The MMA warp starts P V on the first 96 keys of a tile while the softmax warps compute the last 32. A pair of
-// tiles takes 3320 clocks (full attention, 16k tokens), and what it follows is one sub-tile's own cycle, because P
-// overwrites S: with clock stamps, which make it 3500, the softmax takes 1915 from seeing the scores to
-// handing over P, and its next scores are there 1590 later (its own 16 MMAs, 90 clocks each with TMA writes
-// and operand reads on the same shared memory, and the hand-overs). The MMA warp issues during 2 x 1450 of
-// the 3500 and waits for P in the rest. Measured (us) without -> with: 4 x 2000 tokens 184 -> 180, causal 8k
-// tokens, 32 heads 592 -> 576, full 16k 3630 -> 3560; 32 or 64 keys in front of the hand-over are within 0.5 %. With
-// 128 keys' maxima found beside the exponentials of the tile (against the running maximum) the softmax is 100
-// clocks shorter and nothing faster.
-constexpr int P_PART = 96;
+// What a pair of 128 x 128 tiles (one of each sub-tile) takes. The tensor core needs 2048 clocks for its 32 products,
+// the special-function units the same for the exponentials. Before, one thread issued all products and P overwrote S:
+// 3320 clocks a pair. With the softmax left out (P handed on as it came) the same products took 2980, because the
+// tensor core accepts an instruction only when the one before has started, so that every wait (70 clocks even if
+// the phase is complete) and commit (30) of the issuing thread leaves it idle, ten of them a pair: two issuing
+// warps 2210. And a sub-tile's cycle was its softmax plus its own products; with a shared score tile Q K^T of the next
+// tile no longer waits for P V. What is left of it follows the score tile: loaded into registers (290 clocks), seen by the
+// issuing warp (230), Q K^T (512 - 630), seen by the softmax warps (290), twice a pair: 2850.
+// The tile loop's instructions are kept few and close together (masks in a rolled loop over tensor memory, one
+// vote for all that is rare, errors reported by a call): the instruction cache missed 99 times a pair before, 25
+// now, and every miss stops all four warps of a sub-tile. B200, us, before -> now: 8192 causal tokens, 32 heads 510 ->
+// 477; 16384 tokens, 8 heads 995 -> 910, 32 heads 3500 -> 3260 (1250 -> 1345 TFLOP/s); 512 queries behind 32768 keys, 32 / 8
+// heads 282 -> 252. Part of the exponentials as a polynomial of degree 5 on the FMA pipe (1/8, 1/4, 3/8 of them): 914 ->
+// 924, 956, 1048 us. P handed over in two parts (96 + 32 keys): 2 % slower in this form.
 constexpr int FWD_TILE_BYTES = ATTN_TILE * ATTN_D * 2;  // 32 KB: [2 d-halves][128 rows][128 B]
 
 struct FwdRow {
@@ -144,9 +151,9 @@ struct __align__(1024) FwdSmem {
   uint64_t v_empty[STAGES];
   uint64_t s_full[2];
   uint64_t p_full[2];
-  uint64_t p_part[2];    // the first P_PART keys of P are there
   uint64_t q_empty;
-  uint64_t o_full[2];    // FEW: of each sub-tile that had a key tile; else [0] for both
+  uint64_t s_free;       // the scores have been read into registers
+  uint64_t pv_done[2];   // O += P V of a tile is complete: P may be overwritten, O read
   uint4 clc;             // response of a cancellation request
   uint64_t clc_full;
   FwdItem item[2];       // item number n in slot n & 1
@@ -394,13 +401,6 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
   }
 }
 
-// Called, not inlined, by the two-tile form: inlined, its addresses compete with the score loop for
-// registers, which costs the loop further spills (20 to 236 bytes, where the call has 12) and 2 % of its
-// rate. (The FEW form has registers to spare, and a call costs its short items 4 %.)
-__device__ __noinline__ void fwd_epilogue_call(FwdSmem<false>& s, uint32_t slot, uint32_t tO, float l, float m_use, bool any) {
-  fwd_epilogue<false>(s, slot, tO, l, m_use, any);
-}
-
 // Persistent CTAs: the grid has one CTA per work item, and a CTA that is done with an item cancels one
 // that has not started yet and takes its place (cluster launch control), so that the hardware's own
 // dispatch order stays the schedule. The TMA warp runs ahead: it takes over the next item as soon as
@@ -411,6 +411,29 @@ __device__ __noinline__ void fwd_epilogue_call(FwdSmem<false>& s, uint32_t slot,
 // 4096 in 16k tokens 1140 -> 1090; 4 x 2000 tokens 192 -> 182; causal 8k 609 -> 588, 16k 2010 -> 1978.
 // Launches that stage peers' blocks run one item per CTA (p.persist = 0): their CTAs must be able to
 // wait for each other's copies.
+// Columns outside [low, lim) of a score tile (of this thread's row) become -inf, in tensor memory and before the
+// scores are read: few tiles need it, and 128 compares in the tile loop push its other instructions out of the
+// instruction cache.
+__device__ __forceinline__ void fwd_mask(uint32_t tS, int low, int lim) {
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c, low -= 32, lim -= 32, tS += 32) {
+    if (__all_sync(0xFFFFFFFFu, low <= 0 && lim >= 32)) continue;
+    uint32_t v[32];
+    if (__any_sync(0xFFFFFFFFu, low < 32 && lim > 0)) {
+      tmem_ld_x32(tS, v);
+      tmem_wait_ld();
+    }
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = (i >= low && i < lim) ? v[i] : 0xFF800000u;
+    tmem_st_x32(tS, v);
+  }
+  tmem_wait_st();
+}
+// A branch that is never taken (a CTA's 2^32nd score tile). The assembler moves arithmetic over everything that is not a
+// branch, and put the maxima in front of the arrival on s_free, which the other sub-tile's scores wait for
+// (16k tokens, 8 heads: 1038 us without, 917 with).
+#define PIN if (__builtin_expect(cnt == 0xFFFFFFFFu, 0)) break;
+
 template <bool FEW>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ FwdParams p) {
@@ -439,10 +462,9 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.s_full[i], 1);
       mbar_init(&s.p_full[i], act_warps);   // one arrival per softmax warp
-      mbar_init(&s.p_part[i], act_warps);
-      mbar_init(&s.o_full[i], 1);
+      mbar_init(&s.pv_done[i], 1);
       mbar_init(&s.item_full[i], 1);
-      mbar_init(&s.item_empty[i], 1 + 2 * act_warps);   // MMA warp and softmax warps
+      mbar_init(&s.item_empty[i], (FEW ? 1 : 2) + 2 * act_warps);   // MMA and softmax warps
     }
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&s.k_full[i], 1);
@@ -451,6 +473,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       mbar_init(&s.v_empty[i], 1);
     }
     mbar_init(&s.q_empty, 1);
+    mbar_init(&s.s_free, act_warps);
     mbar_init(&s.clc_full, 1);
     s.item[0] = item0;
     s.abort_flag = 0;
@@ -468,7 +491,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       s.hot.pack_shift = p.pack_shift;
     }
   }
-  if (warp == FWD_MMA_WARP) {
+  if (warp == FWD_QK_WARP) {
     tmem_alloc(&s.tmem_base, 512);
     tmem_relinquish();
   }
@@ -477,6 +500,11 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
   tc_fence_after_sync();
   const uint32_t tmem_base = s.tmem_base;
   WaitCtx wc{&s.abort_flag, p.status, 4000000000ull};
+  auto wait = [&](uint64_t* bar, uint32_t parity, int where) -> bool {
+    if (mbar_wait_quiet(bar, parity, wc)) return true;
+    report_error_call(wc.abort_flag, wc.status, UA_ERR_MBAR_TIMEOUT, where, static_cast<int>(parity));
+    return false;
+  };
 
   // Consumers: done with item n; true once item n + 1 is in its slot (false: there is none, or a wait
   // gave up). One thread calls it.
@@ -484,7 +512,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     if (!p.persist) return false;
     mbar_arrive(&s.item_empty[n & 1]);
     const uint32_t m = n + 1;
-    if (!mbar_wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, wc, 120)) return false;
+    if (!wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, 120)) return false;
     return s.item[m & 1].exists != 0;
   };
 
@@ -502,11 +530,11 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
             const CUtensorMap* tq = &p.tmQ[it.row.q_src];
             tma_prefetch_desc(tq);
             if (!wait_staged(p.stage.flags, it.row.q_wait_flag, it.row.q_wait_count * p.stage.epoch, wc.budget_ns)) {
-              report_error(wc, UA_ERR_FLAG_TIMEOUT, 110, it.row.q_wait_flag);
+              report_error_call(wc.abort_flag, wc.status, UA_ERR_FLAG_TIMEOUT, 110, it.row.q_wait_flag);
               ok = false;
             }
             // the previous item's last scores have been computed
-            if (ok && live > 0 && !mbar_wait(&s.q_empty, (live - 1) & 1, wc, 102)) ok = false;
+            if (ok && live > 0 && !wait(&s.q_empty, (live - 1) & 1, 102)) ok = false;
             for (int w = 0; w < (FEW ? 1 : 2) && ok; ++w) {
               mbar_arrive_expect_tx(&s.q_full[w], FWD_TILE_BYTES);
               const int qrow = it.row.q_start + it.tok0 + ((w * ATTN_TILE) >> psh);
@@ -521,7 +549,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               const CUtensorMap* tv = &p.tmV[sg.src];
               if (tr.first < tr.end &&
                   !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
-                report_error(wc, UA_ERR_FLAG_TIMEOUT, 111, sg.wait_flag);
+                report_error_call(wc.abort_flag, wc.status, UA_ERR_FLAG_TIMEOUT, 111, sg.wait_flag);
                 ok = false;
                 break;
               }
@@ -529,11 +557,11 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
                 const int st = j % STAGES;
                 const uint32_t ph = (j / STAGES) & 1;
                 const int krow = sg.start + t * ATTN_TILE;
-                if (!mbar_wait(&s.k_empty[st], ph ^ 1, wc, 100)) { ok = false; break; }
+                if (!wait(&s.k_empty[st], ph ^ 1, 100)) { ok = false; break; }
                 mbar_arrive_expect_tx(&s.k_full[st], FWD_TILE_BYTES);
                 tma_load_4d(s.k[st], tk, &s.k_full[st], 0, it.kv_head, krow, it.batch);
                 tma_load_4d(s.k[st] + 16384, tk, &s.k_full[st], 64, it.kv_head, krow, it.batch);
-                if (!mbar_wait(&s.v_empty[st], ph ^ 1, wc, 101)) { ok = false; break; }
+                if (!wait(&s.v_empty[st], ph ^ 1, 101)) { ok = false; break; }
                 mbar_arrive_expect_tx(&s.v_full[st], FWD_TILE_BYTES);
                 tma_load_4d(s.v[st], tv, &s.v_full[st], 0, it.kv_head, krow, it.batch);
                 tma_load_4d(s.v[st] + 16384, tv, &s.v_full[st], 64, it.kv_head, krow, it.batch);
@@ -544,7 +572,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           // everything of this item is on its way: take over the next one
           mbar_arrive_expect_tx(&s.clc_full, 16);
           clc_try_cancel(&s.clc, &s.clc_full);
-          if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
+          if (!wait(&s.clc_full, n & 1, 104)) break;
           int bx, by;
           const bool got = clc_read(&s.clc, bx, by);
           fence_proxy_async_smem();               // read before the next response may overwrite it
@@ -552,54 +580,51 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           else it.exists = 0;
           // the slot's previous item (n - 1) is done with
           const uint32_t slot = (n + 1) & 1;
-          if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
+          if (n >= 1 && !wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, 103)) break;
           s.item[slot] = it;
           mbar_arrive(&s.item_full[slot]);
           if (!got) break;
         }
       }
-    } else if (warp == FWD_MMA_WARP) {
-      // =============================== MMA issuer =============================================
+    } else if (warp == FWD_QK_WARP || (!FEW && warp == FWD_PV_WARP)) {
+      // =============================== MMA issuers ============================================
       if (lane == 0) {
         const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S = Q K^T, both K-major
         const uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);   // O += P V, V is N-major
-        const uint32_t tS[2] = {tmem_base + 0, tmem_base + 128};
-        const uint32_t tO[2] = {tmem_base + 256, tmem_base + 384};
         auto issue_s = [&](int w, int st) {
           const uint32_t qa = smem_u32(s.q[FEW ? 0 : w]);
           const uint32_t ka = smem_u32(s.k[st]);
+          const uint32_t tS = tmem_base + (FEW ? w * 128 : 0);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-            umma_ss(tS[w], make_smem_desc_sw128(qa + off, 16, 1024),
-                    make_smem_desc_sw128(ka + off, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
+            umma_ss(tS, make_smem_desc_sw128(qa + off, 16, 1024), make_smem_desc_sw128(ka + off, 16, 1024), idesc_s,
+                    kk > 0 ? 1u : 0u);
           }
         };
-        auto issue_pv = [&](int w, int st, bool acc, int k0, int k1) {
+        auto issue_pv = [&](int w, int st, bool acc) {
           const uint32_t va = smem_u32(s.v[st]);
+          const uint32_t tP = tmem_base + (FEW ? w * 128 : 128 + w * 64), tO = tmem_base + 256 + w * 128;
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            if (kk < k0 || kk >= k1) continue;
+          for (int kk = 0; kk < 8; ++kk)
             // A: 16 keys = 8 packed columns of P; B: 16 key rows = 2048 B, d-halves 16384 B apart
-            umma_ts(tO[w], tS[w] + kk * 8, make_smem_desc_sw128(va + kk * 2048, 16384, 1024),
-                    idesc_o, (acc || kk > 0) ? 1u : 0u);
-          }
+            umma_ts(tO, tP + kk * 8, make_smem_desc_sw128(va + kk * 2048, 16384, 1024), idesc_o, (acc || kk > 0) ? 1u : 0u);
         };
         bool ok = true;
-        uint32_t kv = 0;                  // K / V tiles of the items before this one
+        uint32_t kv = 0;                  // K / V tiles so far
         uint32_t live = 0;
-        uint32_t p_cnt[2] = {0, 0};       // FEW: tiles of each sub-tile so far
-        for (uint32_t n = 0; ok; ++n) {
-          const int n_total = fwd_total(p, s.item[n & 1]);
-          if (n_total > 0) {
-            // (that O of the previous item has been read out is implied by p_full of this one's first tile:
-            // the same warps arrive there after their epilogue)
-            if (!mbar_wait(&s.q_full[0], live & 1, wc, 200)) break;
-            if constexpr (FEW) {
+        // (that O of the previous item has been read out is implied by P of an item's first tile: the same warps
+        // write it after their epilogue)
+        if constexpr (FEW) {
+          uint32_t phase = 0;             // bit w: parity of sub-tile w's next P
+          for (uint32_t n = 0; ok; ++n) {
+            const int n_total = fwd_total(p, s.item[n & 1]);
+            if (n_total > 0) {
+              if (!wait(&s.q_full[0], live & 1, 200)) break;
               // key tile j belongs to sub-tile j & 1; its scores are issued two tiles ahead
               auto next_s = [&](int j) -> bool {
                 const uint32_t g = kv + j;
-                if (!mbar_wait(&s.k_full[g % STAGES], (g / STAGES) & 1, wc, 201)) return false;
+                if (!wait(&s.k_full[g % STAGES], (g / STAGES) & 1, 201)) return false;
                 tc_fence_after_sync();
                 issue_s(j & 1, g % STAGES);
                 tc_commit(&s.s_full[j & 1]);
@@ -610,76 +635,66 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               ok = next_s(0) && (n_total < 2 || next_s(1));
               for (int j = 0; j < n_total && ok; ++j) {
                 const int w = j & 1, st = (kv + j) % STAGES;
-                if (!mbar_wait(&s.v_full[st], ((kv + j) / STAGES) & 1, wc, 203)) { ok = false; break; }
-                if (!mbar_wait(&s.p_full[w], p_cnt[w] & 1, wc, 204)) { ok = false; break; }
-                ++p_cnt[w];
+                if (!wait(&s.v_full[st], ((kv + j) / STAGES) & 1, 203)) { ok = false; break; }
+                if (!wait(&s.p_full[w], (phase >> w) & 1, 204)) { ok = false; break; }
+                phase ^= 1u << w;
                 tc_fence_after_sync();
-                issue_pv(w, st, j >= 2, 0, 8);
+                issue_pv(w, st, j >= 2);
+                tc_commit(&s.pv_done[w]);
                 tc_commit(&s.v_empty[st]);
                 if (j + 2 < n_total) ok = next_s(j + 2);
               }
-            } else {
-              if (!mbar_wait(&s.k_full[kv % STAGES], (kv / STAGES) & 1, wc, 201)) break;
-              tc_fence_after_sync();
-              issue_s(0, kv % STAGES);
-              tc_commit(&s.s_full[0]);
-              if (!mbar_wait(&s.q_full[1], live & 1, wc, 202)) break;
-              tc_fence_after_sync();
-              issue_s(1, kv % STAGES);
-              tc_commit(&s.s_full[1]);
-              tc_commit(&s.k_empty[kv % STAGES]);
-              if (n_total == 1) tc_commit(&s.q_empty);
-              for (int j = 0; j < n_total; ++j) {
-                const uint32_t g = kv + j;
-                const int st = g % STAGES;
-                const uint32_t ph = (g / STAGES) & 1;
-                const int stn = (g + 1) % STAGES;
-                const uint32_t phn = ((g + 1) / STAGES) & 1;
-                const bool more = (j + 1 < n_total);
-                FWD_PROF(g == FWD_PROF_TILE, 0);
-              FWD_PROF(g == FWD_PROF_TILE + FWD_PROF_SPAN, 5);
-                if (!mbar_wait(&s.v_full[st], ph, wc, 203)) { ok = false; break; }
-                if (!mbar_wait(&s.p_part[0], g & 1, wc, 204)) { ok = false; break; }
-                FWD_PROF(g == FWD_PROF_TILE, 1);
-                tc_fence_after_sync();
-                issue_pv(0, st, j > 0, 0, P_PART / 16);
-                if (!mbar_wait(&s.p_full[0], g & 1, wc, 207)) { ok = false; break; }
-                tc_fence_after_sync();
-                issue_pv(0, st, j > 0, P_PART / 16, 8);
-                if (more) {
-                  if (!mbar_wait(&s.k_full[stn], phn, wc, 205)) { ok = false; break; }
-                  tc_fence_after_sync();
-                  issue_s(0, stn);
-                  tc_commit(&s.s_full[0]);
-                }
-                FWD_PROF(g == FWD_PROF_TILE, 2);
-                if (!mbar_wait(&s.p_part[1], g & 1, wc, 206)) { ok = false; break; }
-                FWD_PROF(g == FWD_PROF_TILE, 3);
-                tc_fence_after_sync();
-                issue_pv(1, st, j > 0, 0, P_PART / 16);
-                if (!mbar_wait(&s.p_full[1], g & 1, wc, 208)) { ok = false; break; }
-                tc_fence_after_sync();
-                issue_pv(1, st, j > 0, P_PART / 16, 8);
-                tc_commit(&s.v_empty[st]);
-                if (more) {
-                  issue_s(1, stn);
-                  tc_commit(&s.s_full[1]);
-                  tc_commit(&s.k_empty[stn]);
-                  if (j + 2 == n_total) tc_commit(&s.q_empty);
-                }
-                FWD_PROF(g == FWD_PROF_TILE, 4);
-              }
+              if (!ok) break;
+              kv += n_total;
+              ++live;
             }
-            if (!ok) break;
-            // A sub-tile's next completion must not come before its warps have seen this one. They have when
-            // they arrive on p_full of the next item, which only a sub-tile with a key tile there is
-            // waited for: with one barrier for both, two items in a row could complete it unseen.
-            tc_commit(&s.o_full[0]);
-            if (FEW && n_total > 1) tc_commit(&s.o_full[1]);
-            kv += n_total;
-            ++live;
+            if (!next_item(n)) break;
           }
-          if (!next_item(n)) break;
+        } else if (warp == FWD_QK_WARP) {
+          uint32_t use = 0;               // score tiles so far (of both sub-tiles)
+          auto scores = [&](int w, int st) -> bool {
+            if (use > 0 && !wait(&s.s_free, (use - 1) & 1, 206)) return false;
+            ++use;
+            tc_fence_after_sync();
+            issue_s(w, st);
+            tc_commit(&s.s_full[w]);
+            return true;
+          };
+          for (uint32_t n = 0; ok; ++n) {
+            const int n_total = fwd_total(p, s.item[n & 1]);
+            if (n_total > 0) {
+              if (!wait(&s.q_full[0], live & 1, 200)) break;
+              if (!wait(&s.q_full[1], live & 1, 202)) break;
+              for (int j = 0; j < n_total && ok; ++j, ++kv) {
+                const int st = kv % STAGES;
+                FWD_PROF(kv == FWD_PROF_TILE, 0);
+                FWD_PROF(kv == FWD_PROF_TILE + FWD_PROF_SPAN, 5);
+                ok = wait(&s.k_full[st], (kv / STAGES) & 1, 201) && scores(0, st) && scores(1, st);
+                if (ok) tc_commit(&s.k_empty[st]);
+              }
+              if (!ok) break;
+              tc_commit(&s.q_empty);
+              ++live;
+            }
+            if (!next_item(n)) break;
+          }
+        } else {
+          auto product = [&](int w, int st, bool acc) -> bool {
+            if (!wait(&s.p_full[w], kv & 1, 204 + w)) return false;
+            tc_fence_after_sync();
+            issue_pv(w, st, acc);
+            tc_commit(&s.pv_done[w]);
+            return true;
+          };
+          for (uint32_t n = 0; ok; ++n) {
+            const int n_total = fwd_total(p, s.item[n & 1]);
+            for (int j = 0; j < n_total && ok; ++j, ++kv) {
+              const int st = kv % STAGES;
+              ok = wait(&s.v_full[st], (kv / STAGES) & 1, 203) && product(0, st, j > 0) && product(1, st, j > 0);
+              if (ok) tc_commit(&s.v_empty[st]);
+            }
+            if (!ok || !next_item(n)) break;
+          }
         }
       }
     }
@@ -692,14 +707,15 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       const int r_tile = quad * 32 + lane;     // row inside the 128-row sub-tile
       const int r_cta = (FEW ? 0 : w * ATTN_TILE) + r_tile;   // row inside the CTA's tile
       const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-      const uint32_t tS = tmem_base + lane_base + w * 128;
+      const uint32_t tS = tmem_base + lane_base + (FEW ? w * 128 : 0);
+      const uint32_t tP = FEW ? tS : tmem_base + lane_base + 128 + w * 64;
       const uint32_t tO = tmem_base + lane_base + 256 + w * 128;
       const float NEG_INF = -INFINITY;
       uint32_t cnt = 0;                        // score tiles of this sub-tile so far
-      uint32_t live = 0;                       // items with a key tile for this sub-tile so far
       for (uint32_t n = 0;; ++n) {
         const FwdItem& it = s.item[n & 1];       // (stays in shared memory: the score loop needs the registers)
         const int r_blk = (it.r0 + r_cta) >> psh;               // query token inside the query block
+        const int r_warp = (it.r0 + r_cta - lane) >> psh, r_warp_last = (it.r0 + r_cta - lane + 31) >> psh;
         if (n > 0) trace_stamp(p.trace, it.linear, 0);
         trace_stamp(p.trace, it.linear, 1);
         trace_ident(p.trace, it.linear, it.row_idx);
@@ -710,16 +726,43 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
           const AttnSeg sg = fwd_seg(p, e);
           const TileRange tr = fwd_tiles(p, it, sg);
+          // this row sees the columns [low, lim) of the segment; every row of the warp sees all of the
+          // tiles [clear_first, clear_end), and no row anything outside [some_first, some_end)
+          const bool up = (sg.causal & SEG_UPPER) != 0, down = (sg.causal & SEG_LOWER) != 0;
+          auto end_of = [&](int r) { return up ? min(sg.len, r + sg.diag + 1) : sg.len; };
+          auto first_of = [&](int r) { return down ? max(0, r + sg.lo) : 0; };
+          const int lim = end_of(r_blk), low = first_of(r_blk);
+          const int clear_end = end_of(r_warp) >> 7, some_end = (end_of(r_warp_last) + ATTN_TILE - 1) >> 7;
+          const int some_first = first_of(r_warp) >> 7, clear_first = (first_of(r_warp_last) + ATTN_TILE - 1) >> 7;
           for (int t = tr.first; t < tr.end; ++t, ++j) {
             if (FEW && (j & 1) != static_cast<uint32_t>(w)) continue;
             const bool prof = (n == 0) && (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0;
             const int pslot = 8 + w * 24 + (static_cast<int>(j) - FWD_PROF_TILE) * 8;
             (void)prof; (void)pslot;
             FWD_PROF(prof, pslot + 0);
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full[w], cnt & 1, wc, 300 + w))) { ok = false; break; }
+            ok = mbar_wait_quiet(&s.s_full[w], cnt & 1, wc);             // (looked at below)
             FWD_PROF(prof, pslot + 1);
             ++cnt;
             tc_fence_after_sync();
+            if (t < some_first || t >= some_end) {
+              // Nothing to see here for these 32 rows (a tile that only the other sub-tile, or another warp, needs): P = 0,
+              // and neither the maximum nor the sum changes.
+              if (!FEW) mbar_arrive_warp(&s.s_free);
+              if (j >= (FEW ? 2u : 1u)) ok = mbar_wait_quiet(&s.pv_done[w], cnt & 1, wc) && ok;
+              ok = __all_sync(0xFFFFFFFFu, ok);
+              if (!ok) break;
+              tc_fence_after_sync();
+              uint32_t zero[32];
+#pragma unroll
+              for (int i = 0; i < 32; ++i) zero[i] = 0u;
+              tmem_st_x32(tP, zero);
+              tmem_st_x32(tP + 32, zero);
+              tmem_wait_st();
+              tc_fence_before_sync();
+              mbar_arrive_warp(&s.p_full[w]);
+              continue;
+            }
+            if (t < clear_first || t >= clear_end) fwd_mask(tS, low - t * ATTN_TILE, lim - t * ATTN_TILE);
             float sv[ATTN_TILE];
             {
               uint32_t(&raw)[ATTN_TILE] = reinterpret_cast<uint32_t(&)[ATTN_TILE]>(sv);
@@ -728,22 +771,12 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
                 tmem_ld_x32(tS + c * 32, reinterpret_cast<uint32_t(&)[32]>(raw[c * 32]));
               tmem_wait_ld();
             }
+            if (!FEW) {
+              tc_fence_before_sync();
+              mbar_arrive_warp(&s.s_free);
+              PIN
+            }
             FWD_PROF(prof, pslot + 2);
-            // masking: key index c (segment-relative) allowed iff c < len, c <= r + diag and c >= r + lo
-            const int c0 = t * ATTN_TILE;
-            int limit = sg.len - c0;                               // columns < limit are in range
-            if (sg.causal & SEG_UPPER) limit = min(limit, r_blk + sg.diag - c0 + 1);
-            if (limit < ATTN_TILE) {
-#pragma unroll
-              for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i < limit) ? sv[i] : NEG_INF;
-            }
-            if (sg.causal & SEG_LOWER) {
-              const int first = r_blk + sg.lo - c0;                // columns >= first are in range
-              if (first > 0) {
-#pragma unroll
-                for (int i = 0; i < ATTN_TILE; ++i) sv[i] = (i >= first) ? sv[i] : NEG_INF;
-              }
-            }
             // eight independent running maxima, two new values per instruction: one dependent chain of
             // compares would cost more than the exponentials
             float mx8[8];
@@ -755,25 +788,35 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               for (int k = 0; k < 8; ++k) mx8[k] = fmax3(mx8[k], sv[i + k], sv[i + 8 + k]);
             float mx = fmaxf(fmax3(mx8[0], mx8[1], mx8[2]), fmax3(mx8[3], mx8[4], mx8[5]));
             mx = fmax3(mx, mx8[6], mx8[7]);
+            PIN
             mx *= p.scale_log2;
             const float m_new = fmaxf(m_use, mx);
-            // lazy rescale: only when the running max grew by more than 2^8 (warp-uniform branch,
-            // because the TMEM accesses below are warp-collective)
-            const bool need = (m_new - m_use > 8.0f) || (m_use == NEG_INF && m_new > NEG_INF);
+            FWD_PROF(prof, pslot + 6);
+            // P V of the tile before is complete: P may be overwritten, and O rescaled
+            bool need = false;
             if (j < (FEW ? 2u : 1u)) {
               m_use = m_new;
-            } else if (__any_sync(0xFFFFFFFFu, need)) {
+            } else {
+              ok = mbar_wait_quiet(&s.pv_done[w], cnt & 1, wc) && ok;
+              tc_fence_after_sync();
+              // lazy rescale: only when the running max grew by more than 2^8
+              need = (m_new - m_use > 8.0f) || (m_use == NEG_INF && m_new > NEG_INF);
+            }
+            // (one vote for all that is rare; warp-uniform, because accesses to tensor memory are warp-collective)
+            if (__any_sync(0xFFFFFFFFu, need || !ok)) {
+              ok = __all_sync(0xFFFFFFFFu, ok);
+              if (!ok) break;
               const float alpha = need ? fast_exp2(m_use - m_new) : 1.0f;
               if (need) m_use = m_new;
               l *= alpha;
 #pragma unroll 1
-              for (int c = 0; c < 4; ++c) {
-                uint32_t ov[32];
-                tmem_ld_x32(tO + c * 32, ov);
+              for (int c = 0; c < 8; ++c) {
+                uint32_t ov[16];
+                tmem_ld_x16(tO + c * 16, ov);
                 tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-                tmem_st_x32(tO + c * 32, ov);
+                for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+                tmem_st_x16(tO + c * 16, ov);
               }
             }
             FWD_PROF(prof, pslot + 3);
@@ -795,13 +838,13 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
                 ls2[i & 3] = f2_add(ls2[i & 3], f2_pack(p0, p1));
                 pk[i] = pack_bf16x2(p0, p1);
               }
-              tmem_st_x16(tS + c * 16, pk);
-              if (!FEW && c == P_PART / 32 - 1) {      // (FEW is bound by memory, not by this chain)
-                tmem_wait_st();
-                tc_fence_before_sync();
-                mbar_arrive_warp(&s.p_part[w]);
-              }
+              tmem_st_x16(tP + c * 16, pk);
             }
+            tmem_wait_st();
+            tc_fence_before_sync();
+            mbar_arrive_warp(&s.p_full[w]);
+            PIN
+            FWD_PROF(prof, pslot + 4);
             float ls4[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -810,21 +853,16 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               ls4[k] = a + b;
             }
             l += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
-            FWD_PROF(prof, pslot + 4);
-            tmem_wait_st();
-            tc_fence_before_sync();
-            mbar_arrive_warp(&s.p_full[w]);
             FWD_PROF(prof, pslot + 5);
           }
         }
         // ---------------------------------- epilogue --------------------------------------------
         const bool any = j > (FEW ? static_cast<uint32_t>(w) : 0u);
-        if (any && ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.o_full[FEW ? w : 0], live & 1, wc, 310 + w));
+        if (any && ok) ok = __all_sync(0xFFFFFFFFu, wait(&s.pv_done[w], (cnt & 1) ^ 1, 310 + w));
         tc_fence_after_sync();
-        if constexpr (FEW) fwd_epilogue<true>(s, n & 1, tO, l, m_use, any);
-        else fwd_epilogue_call(s, n & 1, tO, l, m_use, any);
+        if (!ok) report_error_call(wc.abort_flag, wc.status, UA_ERR_MBAR_TIMEOUT, 300 + w, static_cast<int>(j));
+        fwd_epilogue<FEW>(s, n & 1, tO, l, m_use, any);
         trace_stamp(p.trace, it.linear, 2);
-        if (any) ++live;
         if (!ok) break;
         __syncwarp();                            // every lane is done reading the item
         int more = 0;
@@ -837,7 +875,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == FWD_MMA_WARP) {
+  if (warp == FWD_QK_WARP) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }

@@ -141,6 +141,36 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+// The same in few instructions, for loops whose instructions should stay close together: one that gives up says so
+// to its caller, who reports it (report_error_call) where nothing is in the way.
+__device__ __forceinline__ bool mbar_wait_quiet(uint64_t* bar, uint32_t parity, const WaitCtx& w) {
+  const uint32_t addr = smem_u32(bar);
+  uint32_t t0 = 0;
+  for (uint32_t it = 1;; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P1;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((it & 0x3FF) == 0) {
+      uint32_t now;
+      asm volatile("mov.u32 %0, %globaltimer_lo;" : "=r"(now));
+      if (it == 0x400) t0 = now;
+      if (*w.abort_flag || now - t0 > static_cast<uint32_t>(w.budget_ns)) return false;
+    }
+  }
+}
+static __device__ __noinline__ void report_error_call(volatile int* abort_flag, int* status, int code, int where, int extra) {
+  if (*abort_flag) return;              // (somebody else gave up first)
+  report_error(WaitCtx{abort_flag, status, 0}, code, where, extra);
+}
+
 // ----------------------------------------------------------------------------------------------
 // Cluster launch control: take over a CTA of the grid that has not started
 // ----------------------------------------------------------------------------------------------
