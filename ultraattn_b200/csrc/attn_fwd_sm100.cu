@@ -57,11 +57,13 @@ static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setm
 // warps 2210. And a sub-tile's cycle was its softmax plus its own products; with a shared score tile Q K^T of the next
 // tile no longer waits for P V. What is left of it follows the score tile: loaded into registers (290 clocks), seen by the
 // issuing warp (230), Q K^T (512 - 630), seen by the softmax warps (290), twice a pair: 2850.
-// The tile loop's instructions are kept few and close together (masks in a rolled loop over tensor memory, one
-// vote for all that is rare, errors reported by a call): the instruction cache missed 99 times a pair before, 25
-// now, and every miss stops all four warps of a sub-tile. B200, us, before -> now: 8192 causal tokens, 32 heads 510 ->
-// 477; 16384 tokens, 8 heads 995 -> 910, 32 heads 3500 -> 3260 (1250 -> 1345 TFLOP/s); 512 queries behind 32768 keys, 32 / 8
-// heads 282 -> 252. Part of the exponentials as a polynomial of degree 5 on the FMA pipe (1/8, 1/4, 3/8 of them): 914 ->
+// The instructions of all roles are kept few and close together (masks in a rolled loop over tensor memory, one
+// vote for all that is rare, errors reported by a call, loops over segments not unrolled, 32-bit divisions, operand
+// descriptors by addition): the instruction cache missed 99 times a pair before, 17 now, and every miss stops all four
+// warps of a sub-tile; builds that differ in nothing but that (15 and 53 misses a pair) took 918 and 968 us for 16384
+// tokens, 8 heads. B200, us, before -> now: 8192 causal tokens, 32 heads 510 -> 453; 16384 tokens, 8 heads 995 -> 876, 32
+// heads 3450 -> 3140 (1275 -> 1400 TFLOP/s); 512 queries behind 32768 keys, 32 / 8 heads 260 -> 222; 1000 causal tokens, 32 / 8
+// heads 26.6 -> 24.0. Part of the exponentials as a polynomial of degree 5 on the FMA pipe (1/8, 1/4, 3/8 of them): 914 ->
 // 924, 956, 1048 us. P handed over in two parts (96 + 32 keys): 2 % slower in this form.
 constexpr int FWD_TILE_BYTES = ATTN_TILE * ATTN_D * 2;  // 32 KB: [2 d-halves][128 rows][128 B]
 
@@ -121,6 +123,13 @@ struct FwdItem {
   int linear;                // index in the grid (time stamps)
   int exists;                // 0: there is no further item
 };
+// What the producer hands to the other roles: the item, the key tiles it visits and its first segments, which would
+// otherwise be a global-memory latency at the beginning of every item and segment of every role.
+constexpr int FWD_SEG_CACHE = 4;
+struct FwdWork : FwdItem {
+  int total;
+  AttnSeg seg[FWD_SEG_CACHE];
+};
 
 // Where results go, copied into shared memory at the start: kernel parameters that are indexed by a
 // run-time slot, or have not been touched for a while, come through the constant cache with several
@@ -156,7 +165,7 @@ struct __align__(1024) FwdSmem {
   uint64_t pv_done[2];   // O += P V of a tile is complete: P may be overwritten, O read
   uint4 clc;             // response of a cancellation request
   uint64_t clc_full;
-  FwdItem item[2];       // item number n in slot n & 1
+  FwdWork item[2];       // item number n in slot n & 1
   uint64_t item_full[2];
   uint64_t item_empty[2];
   FwdHot hot;
@@ -228,25 +237,32 @@ __device__ __forceinline__ TileRange fwd_tiles(const FwdParams& p, const FwdItem
   TileRange tr = seg_tiles(sg, it.tok0, it.tok_last);
   if (p.n_split > 1) {
     const int n = tr.end - tr.first, base = tr.first;
-    tr.first = base + static_cast<int>(static_cast<long>(n) * it.split / p.n_split);
-    tr.end = base + static_cast<int>(static_cast<long>(n) * (it.split + 1) / p.n_split);
+    // (n < 2^24 tiles; in 32 bits: a 64-bit division is a hundred instructions)
+    const unsigned q = static_cast<unsigned>(n) / p.n_split, r = static_cast<unsigned>(n) % p.n_split;
+    tr.first = base + static_cast<int>(q * it.split + r * it.split / p.n_split);
+    tr.end = base + static_cast<int>(q * (it.split + 1) + r * (it.split + 1) / p.n_split);
   }
   return tr;
 }
-__device__ __forceinline__ int fwd_total(const FwdParams& p, const FwdItem& it) {
+__device__ __forceinline__ void fwd_publish(const FwdParams& p, const FwdItem& it, FwdWork& dst) {
+  static_cast<FwdItem&>(dst) = it;
   int n = 0;
+#pragma unroll 1
   for (int e = it.row.seg_begin; e < it.row.seg_end; ++e) {
-    const TileRange tr = fwd_tiles(p, it, fwd_seg(p, e));
+    const AttnSeg sg = fwd_seg(p, e);
+    const TileRange tr = fwd_tiles(p, it, sg);
     n += tr.end - tr.first;
+    if (e - it.row.seg_begin < FWD_SEG_CACHE) dst.seg[e - it.row.seg_begin] = sg;
   }
-  return n;
+  dst.total = n;
 }
 
 // The output of one item: this thread's row (l: row sum, m_use: reference maximum, `any`: its sub-tile has
 // seen a key tile) normalised, merged with what is there (row.accumulate) or written as a fp32 part
 // of a split launch.
-template <bool FEW>
-__device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uint32_t tO, float l, float m_use, bool any) {
+// `ready` waits until the last product is complete; what does not depend on it comes first.
+template <bool FEW, typename Ready>
+__device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uint32_t tO, float l, float m_use, bool any, Ready ready) {
   const FwdItem& it = s.item[slot];
   const float NEG_INF = -INFINITY;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -309,6 +325,10 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
                                                      (it.row.o_start + static_cast<long>(it.tok0)) * od.o_row_stride +
                                                      static_cast<long>(it.q_head) * ATTN_D);
     base += ch * 16;
+    uint8_t* dst[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dst[i] = base + ((rc0 + i * 4) >> psh) * row_bytes + ((rc0 + i * 4) & hmask) * head_bytes;
+    ready();
 #pragma unroll 1
     for (int c = 0; c * 128 < head_bytes; ++c) {
       if (f32) {
@@ -323,34 +343,37 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
           *reinterpret_cast<float4*>(blk + sw128_offset(lane, q)) = make_float4(f[0], f[1], f[2], f[3]);
         }
       } else {
+        uint32_t ov[2][32];
+        tmem_ld_x32(tO + c * 64, ov[0]);
+        tmem_ld_x32(tO + c * 64 + 32, ov[1]);
+        tmem_wait_ld();
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-          uint32_t ov[32];
-          tmem_ld_x32(tO + c * 64 + hf * 32, ov);
-          tmem_wait_ld();
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             float f[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 8 + i]) * fnew;
+            for (int i = 0; i < 8; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[hf][q * 8 + i]) * fnew;
             *reinterpret_cast<uint4*>(blk + sw128_offset(lane, hf * 4 + q)) =
                 make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
           }
         }
       }
       __syncwarp();
+      uint4 val[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) val[i] = *reinterpret_cast<const uint4*>(blk + sw128_offset(i * 4 + sub, ch));
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int rc = rc0 + i * 4;
-        const uint4 val = *reinterpret_cast<const uint4*>(blk + sw128_offset(i * 4 + sub, ch));
-        if (rc < rows_here)
-          *reinterpret_cast<uint4*>(base + (rc >> psh) * row_bytes + (rc & hmask) * head_bytes + c * 128) = val;
+        if (rc0 + i * 4 < rows_here) *reinterpret_cast<uint4*>(dst[i]) = val[i];
+        dst[i] += 128;
       }
       __syncwarp();
     }
     return;
   }
   // few rows, or a merge with what is there: straight from registers
+  ready();
   __nv_bfloat16* optr = od.o + it.batch * od.o_batch_stride + orow * od.o_row_stride + static_cast<long>(qh) * ATTN_D;
   float* pptr = f32 ? s.hot.part_o + ((part0 + r_blk) * s.hot.n_heads + qh) * ATTN_D : nullptr;
 #pragma unroll 1
@@ -406,26 +429,39 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
 // dispatch order stays the schedule. The TMA warp runs ahead: it takes over the next item as soon as
 // the loads of this one are issued, its Q and first K / V tiles arrive while the softmax warps write
 // this item's output, and the MMA warp issues its first scores. TMEM, barriers and descriptors are
-// set up once. One item per CTA -> this (B200, us): 64
+// set up once. The producer hands an item over with what the others need of it (number of tiles, first segments), and
+// issues a CTA's first loads while tensor memory is being allocated: 512 causal tokens, 8 heads 21.3 -> 14.8 us,
+// 12 documents in 16k tokens 406 -> 365. One item per CTA -> this (B200, us): 64
 // sequences of 512 keys, one query, 32 heads 184 -> 143; 12 documents in 16k tokens 599 -> 546; window
 // 4096 in 16k tokens 1140 -> 1090; 4 x 2000 tokens 192 -> 182; causal 8k 609 -> 588, 16k 2010 -> 1978.
 // Launches that stage peers' blocks run one item per CTA (p.persist = 0): their CTAs must be able to
 // wait for each other's copies.
+// The columns of a segment that query r sees are [seg_first_of, seg_end_of); both grow with r.
+__device__ __forceinline__ int seg_end_of(const AttnSeg& sg, int r) {
+  return (sg.causal & SEG_UPPER) ? min(sg.len, r + sg.diag + 1) : sg.len;
+}
+__device__ __forceinline__ int seg_first_of(const AttnSeg& sg, int r) {
+  return (sg.causal & SEG_LOWER) ? max(0, r + sg.lo) : 0;
+}
 // Columns outside [low, lim) of a score tile (of this thread's row) become -inf, in tensor memory and before the
 // scores are read: few tiles need it, and 128 compares in the tile loop push its other instructions out of the
-// instruction cache.
-__device__ __forceinline__ void fwd_mask(uint32_t tS, int low, int lim) {
+// instruction cache. Blocks of 32 columns that all rows of the warp see ([clear_lo, clear_hi)) stay as they are.
+// `r`: this thread's query token, r_first and r_last those of the warp's first and last row; c0: the tile's first column.
+__device__ __forceinline__ void fwd_mask(uint32_t tS, const AttnSeg& sg, int r, int r_first, int r_last, int c0) {
+  const int low = seg_first_of(sg, r) - c0, lim = seg_end_of(sg, r) - c0;
+  const int some_lo = seg_first_of(sg, r_first) - c0, clear_lo = seg_first_of(sg, r_last) - c0;
+  const int clear_hi = seg_end_of(sg, r_first) - c0, some_hi = seg_end_of(sg, r_last) - c0;
 #pragma unroll 1
-  for (int c = 0; c < 4; ++c, low -= 32, lim -= 32, tS += 32) {
-    if (__all_sync(0xFFFFFFFFu, low <= 0 && lim >= 32)) continue;
+  for (int c = 0; c < ATTN_TILE; c += 32) {
+    if (c >= clear_lo && c + 32 <= clear_hi) continue;
     uint32_t v[32];
-    if (__any_sync(0xFFFFFFFFu, low < 32 && lim > 0)) {
-      tmem_ld_x32(tS, v);
+    if (c < some_hi && c + 32 > some_lo) {
+      tmem_ld_x32(tS + c, v);
       tmem_wait_ld();
     }
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = (i >= low && i < lim) ? v[i] : 0xFF800000u;
-    tmem_st_x32(tS, v);
+    for (int i = 0; i < 32; ++i) v[i] = (c + i >= low && c + i < lim) ? v[i] : 0xFF800000u;
+    tmem_st_x32(tS + c, v);
   }
   tmem_wait_st();
 }
@@ -445,19 +481,24 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
   const int lane = threadIdx.x & 31;
   const int psh = p.pack_shift;
 
-  const FwdItem item0 = fwd_item<FEW>(p, blockIdx.x, blockIdx.y);
-  trace_stamp(p.trace, item0.linear, 0);
-  {
+  if (p.stage.flags != nullptr) {
     // does this CTA read a staged block? then it first helps to empty the copy queue
-    bool waits = item0.row.q_wait_flag != 0;
-    for (int e = item0.row.seg_begin; e < item0.row.seg_end && !waits; ++e) waits = fwd_seg(p, e).wait_flag != 0;
-    drain_stage_queue(p.stage, waits, item0.linear, &s.stage_slot);
+    const FwdItem it = fwd_item<FEW>(p, blockIdx.x, blockIdx.y);
+    trace_stamp(p.trace, it.linear, 0);
+    bool waits = it.row.q_wait_flag != 0;
+    for (int e = it.row.seg_begin; e < it.row.seg_end && !waits; ++e) waits = fwd_seg(p, e).wait_flag != 0;
+    drain_stage_queue(p.stage, waits, it.linear, &s.stage_slot);
+  } else {
+    trace_stamp(p.trace, blockIdx.y * gridDim.x + blockIdx.x, 0);
   }
   // FEW: warps without a valid row have nothing to do (their scores are never read back). The
   // launch has one row tile, so the number is the same for all its items.
-  const int act_warps = FEW ? (item0.rows_here + 31) / 32 : 4;
+  const int act_warps = FEW ? (min(ATTN_TILE, p.dense_row.q_len << psh) + 31) / 32 : 4;
 
-  if (threadIdx.x == 0) {
+  // The producer sets the barriers up, looks up its first item and goes on to load it; the others meet at
+  // a named barrier once tensor memory is there as well.
+  FwdItem item0;
+  if (warp == FWD_TMA_WARP && lane == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.s_full[i], 1);
@@ -475,9 +516,10 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     mbar_init(&s.q_empty, 1);
     mbar_init(&s.s_free, act_warps);
     mbar_init(&s.clc_full, 1);
-    s.item[0] = item0;
     s.abort_flag = 0;
     fence_mbar_init();
+    item0 = fwd_item<FEW>(p, blockIdx.x, blockIdx.y);
+    fwd_publish(p, item0, s.item[0]);
   }
   if (warp == 1) {
     if (lane < ATTN_MAX_SRC)
@@ -495,10 +537,16 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     tmem_alloc(&s.tmem_base, 512);
     tmem_relinquish();
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = s.tmem_base;
+  uint32_t tmem_base = 0;
+  if (warp == FWD_TMA_WARP) {
+    __syncwarp();
+    named_barrier_arrive(1, FWD_THREADS);
+  } else {
+    tc_fence_before_sync();
+    named_barrier_sync(1, FWD_THREADS);
+    tc_fence_after_sync();
+    tmem_base = s.tmem_base;
+  }
   WaitCtx wc{&s.abort_flag, p.status, 4000000000ull};
   auto wait = [&](uint64_t* bar, uint32_t parity, int where) -> bool {
     if (mbar_wait_quiet(bar, parity, wc)) return true;
@@ -506,14 +554,16 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     return false;
   };
 
-  // Consumers: done with item n; true once item n + 1 is in its slot (false: there is none, or a wait
-  // gave up). One thread calls it.
+  // Consumers: true once item n + 1 is in its slot (false: there is none, or a wait gave up). They hand
+  // item n back by an arrival on item_empty when they have read what they need of it.
   auto next_item = [&](uint32_t n) -> bool {
-    if (!p.persist) return false;
-    mbar_arrive(&s.item_empty[n & 1]);
     const uint32_t m = n + 1;
-    if (!wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, 120)) return false;
-    return s.item[m & 1].exists != 0;
+    return p.persist && wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, 120) && s.item[m & 1].exists != 0;
+  };
+  auto take_total = [&](uint32_t n) -> int {         // (the MMA issuers need nothing else of an item)
+    const int total = s.item[n & 1].total;
+    if (p.persist) mbar_arrive(&s.item_empty[n & 1]);
+    return total;
   };
 
   if (warp >= FWD_SOFTMAX_WARPS) {
@@ -526,7 +576,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         uint32_t j = 0;          // K / V tiles loaded so far
         uint32_t live = 0;       // items with keys so far
         for (uint32_t n = 0; ok; ++n) {
-          if (fwd_total(p, it) > 0) {
+          if (s.item[n & 1].total > 0) {
             const CUtensorMap* tq = &p.tmQ[it.row.q_src];
             tma_prefetch_desc(tq);
             if (!wait_staged(p.stage.flags, it.row.q_wait_flag, it.row.q_wait_count * p.stage.epoch, wc.budget_ns)) {
@@ -542,6 +592,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               tma_load_4d(s.q[w] + 16384, tq, &s.q_full[w], 64, it.q_head, qrow, it.batch);
             }
             ++live;
+#pragma unroll 1
             for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
               const AttnSeg sg = fwd_seg(p, e);
               const TileRange tr = fwd_tiles(p, it, sg);
@@ -553,6 +604,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
                 ok = false;
                 break;
               }
+#pragma unroll 1
               for (int t = tr.first; t < tr.end; ++t, ++j) {
                 const int st = j % STAGES;
                 const uint32_t ph = (j / STAGES) & 1;
@@ -577,11 +629,11 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           const bool got = clc_read(&s.clc, bx, by);
           fence_proxy_async_smem();               // read before the next response may overwrite it
           if (got) it = fwd_item<FEW>(p, bx, by);
-          else it.exists = 0;
           // the slot's previous item (n - 1) is done with
           const uint32_t slot = (n + 1) & 1;
           if (n >= 1 && !wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, 103)) break;
-          s.item[slot] = it;
+          if (got) fwd_publish(p, it, s.item[slot]);
+          else s.item[slot].exists = 0;
           mbar_arrive(&s.item_full[slot]);
           if (!got) break;
         }
@@ -591,24 +643,27 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       if (lane == 0) {
         const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S = Q K^T, both K-major
         const uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);   // O += P V, V is N-major
+        // one base descriptor per operand; a tile and an instruction add their offset (in 16-byte units) to the
+        // address field, which cannot carry out of it for addresses inside shared memory
+        const uint64_t q_desc = make_smem_desc_sw128(smem_u32(s.q[0]), 16, 1024), k_desc = make_smem_desc_sw128(smem_u32(s.k[0]), 16, 1024);
+        const uint64_t v_desc = make_smem_desc_sw128(smem_u32(s.v[0]), 16384, 1024);
+        constexpr uint32_t TILE16 = FWD_TILE_BYTES >> 4;
         auto issue_s = [&](int w, int st) {
-          const uint32_t qa = smem_u32(s.q[FEW ? 0 : w]);
-          const uint32_t ka = smem_u32(s.k[st]);
+          const uint64_t qa = q_desc + (FEW ? 0 : w) * TILE16, ka = k_desc + st * TILE16;
           const uint32_t tS = tmem_base + (FEW ? w * 128 : 0);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-            umma_ss(tS, make_smem_desc_sw128(qa + off, 16, 1024), make_smem_desc_sw128(ka + off, 16, 1024), idesc_s,
-                    kk > 0 ? 1u : 0u);
+            const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
+            umma_ss(tS, qa + off, ka + off, idesc_s, kk > 0 ? 1u : 0u);
           }
         };
         auto issue_pv = [&](int w, int st, bool acc) {
-          const uint32_t va = smem_u32(s.v[st]);
+          const uint64_t va = v_desc + st * TILE16;
           const uint32_t tP = tmem_base + (FEW ? w * 128 : 128 + w * 64), tO = tmem_base + 256 + w * 128;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
             // A: 16 keys = 8 packed columns of P; B: 16 key rows = 2048 B, d-halves 16384 B apart
-            umma_ts(tO, tP + kk * 8, make_smem_desc_sw128(va + kk * 2048, 16384, 1024), idesc_o, (acc || kk > 0) ? 1u : 0u);
+            umma_ts(tO, tP + kk * 8, va + ((kk * 2048) >> 4), idesc_o, (acc || kk > 0) ? 1u : 0u);
         };
         bool ok = true;
         uint32_t kv = 0;                  // K / V tiles so far
@@ -618,7 +673,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         if constexpr (FEW) {
           uint32_t phase = 0;             // bit w: parity of sub-tile w's next P
           for (uint32_t n = 0; ok; ++n) {
-            const int n_total = fwd_total(p, s.item[n & 1]);
+            const int n_total = take_total(n);
             if (n_total > 0) {
               if (!wait(&s.q_full[0], live & 1, 200)) break;
               // key tile j belongs to sub-tile j & 1; its scores are issued two tiles ahead
@@ -661,7 +716,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
             return true;
           };
           for (uint32_t n = 0; ok; ++n) {
-            const int n_total = fwd_total(p, s.item[n & 1]);
+            const int n_total = take_total(n);
             if (n_total > 0) {
               if (!wait(&s.q_full[0], live & 1, 200)) break;
               if (!wait(&s.q_full[1], live & 1, 202)) break;
@@ -687,7 +742,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
             return true;
           };
           for (uint32_t n = 0; ok; ++n) {
-            const int n_total = fwd_total(p, s.item[n & 1]);
+            const int n_total = take_total(n);
             for (int j = 0; j < n_total && ok; ++j, ++kv) {
               const int st = kv % STAGES;
               ok = wait(&s.v_full[st], (kv / STAGES) & 1, 203) && product(0, st, j > 0) && product(1, st, j > 0);
@@ -713,9 +768,11 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       const float NEG_INF = -INFINITY;
       uint32_t cnt = 0;                        // score tiles of this sub-tile so far
       for (uint32_t n = 0;; ++n) {
-        const FwdItem& it = s.item[n & 1];       // (stays in shared memory: the score loop needs the registers)
-        const int r_blk = (it.r0 + r_cta) >> psh;               // query token inside the query block
-        const int r_warp = (it.r0 + r_cta - lane) >> psh, r_warp_last = (it.r0 + r_cta - lane + 31) >> psh;
+        const FwdWork& it = s.item[n & 1];       // (stays in shared memory: the score loop needs the registers)
+        auto seg_of = [&](int e) -> AttnSeg {
+          const int k = e - it.row.seg_begin;
+          return k < FWD_SEG_CACHE ? it.seg[k] : fwd_seg(p, e);
+        };
         if (n > 0) trace_stamp(p.trace, it.linear, 0);
         trace_stamp(p.trace, it.linear, 1);
         trace_ident(p.trace, it.linear, it.row_idx);
@@ -723,18 +780,25 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         float l = 0.f;           // row sum
         bool ok = true;
         uint32_t j = 0;
+#pragma unroll 1
         for (int e = it.row.seg_begin; e < it.row.seg_end && ok; ++e) {
-          const AttnSeg sg = fwd_seg(p, e);
-          const TileRange tr = fwd_tiles(p, it, sg);
-          // this row sees the columns [low, lim) of the segment; every row of the warp sees all of the
-          // tiles [clear_first, clear_end), and no row anything outside [some_first, some_end)
-          const bool up = (sg.causal & SEG_UPPER) != 0, down = (sg.causal & SEG_LOWER) != 0;
-          auto end_of = [&](int r) { return up ? min(sg.len, r + sg.diag + 1) : sg.len; };
-          auto first_of = [&](int r) { return down ? max(0, r + sg.lo) : 0; };
-          const int lim = end_of(r_blk), low = first_of(r_blk);
-          const int clear_end = end_of(r_warp) >> 7, some_end = (end_of(r_warp_last) + ATTN_TILE - 1) >> 7;
-          const int some_first = first_of(r_warp) >> 7, clear_first = (first_of(r_warp_last) + ATTN_TILE - 1) >> 7;
-          for (int t = tr.first; t < tr.end; ++t, ++j) {
+          // Every row of the warp sees all of the tiles [clear_first, clear_end), and no row anything outside
+          // [some_first, some_end).
+          int t, t_end, clear_first, clear_end, some_first, some_end;
+          {
+            const AttnSeg sg = seg_of(e);
+            const TileRange tr = fwd_tiles(p, it, sg);
+            t = tr.first;
+            t_end = tr.end;
+            const int r_first = (it.r0 + r_cta - lane) >> psh, r_last = (it.r0 + r_cta - lane + 31) >> psh;
+            clear_end = seg_end_of(sg, r_first) >> 7;
+            some_end = (seg_end_of(sg, r_last) + ATTN_TILE - 1) >> 7;
+            some_first = seg_first_of(sg, r_first) >> 7;
+            clear_first = (seg_first_of(sg, r_last) + ATTN_TILE - 1) >> 7;
+            if (r_cta - lane >= it.rows_here) some_end = 0;              // (rows behind the last one)
+          }
+#pragma unroll 1
+          for (; t < t_end; ++t, ++j) {
             if (FEW && (j & 1) != static_cast<uint32_t>(w)) continue;
             const bool prof = (n == 0) && (j == FWD_PROF_TILE || j == FWD_PROF_TILE + 1) && quad == 0 && lane == 0;
             const int pslot = 8 + w * 24 + (static_cast<int>(j) - FWD_PROF_TILE) * 8;
@@ -762,7 +826,9 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               mbar_arrive_warp(&s.p_full[w]);
               continue;
             }
-            if (t < clear_first || t >= clear_end) fwd_mask(tS, low - t * ATTN_TILE, lim - t * ATTN_TILE);
+            if (t < clear_first || t >= clear_end) {
+              fwd_mask(tS, seg_of(e), (it.r0 + r_cta) >> psh, (it.r0 + r_cta - lane) >> psh, (it.r0 + r_cta - lane + 31) >> psh, t * ATTN_TILE);
+            }
             float sv[ATTN_TILE];
             {
               uint32_t(&raw)[ATTN_TILE] = reinterpret_cast<uint32_t(&)[ATTN_TILE]>(sv);
@@ -858,17 +924,15 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         }
         // ---------------------------------- epilogue --------------------------------------------
         const bool any = j > (FEW ? static_cast<uint32_t>(w) : 0u);
-        if (any && ok) ok = __all_sync(0xFFFFFFFFu, wait(&s.pv_done[w], (cnt & 1) ^ 1, 310 + w));
-        tc_fence_after_sync();
+        fwd_epilogue<FEW>(s, n & 1, tO, l, m_use, any, [&]() {
+          if (any && ok) ok = mbar_wait_quiet(&s.pv_done[w], (cnt & 1) ^ 1, wc);
+          tc_fence_after_sync();
+        });
         if (!ok) report_error_call(wc.abort_flag, wc.status, UA_ERR_MBAR_TIMEOUT, 300 + w, static_cast<int>(j));
-        fwd_epilogue<FEW>(s, n & 1, tO, l, m_use, any);
         trace_stamp(p.trace, it.linear, 2);
-        if (!ok) break;
         __syncwarp();                            // every lane is done reading the item
-        int more = 0;
-        if (lane == 0) more = next_item(n) ? 1 : 0;
-        if (!__shfl_sync(0xFFFFFFFFu, more, 0)) break;
-        __syncwarp();                            // lane 0 has seen the item; this makes it visible to the others (a shuffle does not)
+        if (lane == 0 && p.persist) mbar_arrive(&s.item_empty[n & 1]);
+        if (!__all_sync(0xFFFFFFFFu, ok && next_item(n))) break;
       }
     }
   }

@@ -44,6 +44,14 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// A hardware barrier of `threads` threads, some of which only arrive.
+__device__ __forceinline__ void named_barrier_sync(int id, int threads) {
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_barrier_arrive(int id, int threads) {
+  asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // ----------------------------------------------------------------------------------------------
 // mbarrier
 // ----------------------------------------------------------------------------------------------
