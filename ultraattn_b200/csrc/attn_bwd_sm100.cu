@@ -37,6 +37,12 @@
 //               into the dQ accumulator; two reduces are in flight while the next tile is staged
 //   warp  12  : TMA producer (K, V once; Q double-buffered; dO single-buffered)
 //   warp  13  : tcgen05.mma issuer, TMEM allocation
+// The five roles' loops are about 30 KB of instructions a step, more than the instruction cache holds (103 misses a step in
+// a build of 115 KB). So they are kept short: descriptors in 32-bit words, one elected thread instead of lane 0 (the
+// assembler then knows that operands are uniform), loops over segments not unrolled, masks in a rolled loop over
+// tensor memory, errors reported by a call: 92 KB. Backward, us, before -> after: 8192 causal tokens, 32 heads 1263 ->
+// 1220, 4 x 2048 tokens full 209 -> 206, 16384 full unchanged (power and shared memory bound it). Two issuing warps, as in
+// the forward, are 5 % slower here: the order dV, S^T, dQ^T, dK, dP^T is what keeps the softmax warps fed.
 // dK/dV leave the CTA either as bf16 stores (the CTA is their only producer) or as fp32
 // red.add into an accumulator that may live in a peer GPU's memory (partial gradients of a
 // key/value block computed away from its owner).
@@ -247,6 +253,7 @@ struct BwdStepIter {
 // number of (head, segment, query tile) steps of an item; identical in every role
 __device__ __forceinline__ int bwd_steps(const BwdParams& p, const BwdItem& it) {
   int per_head = 0;
+#pragma unroll 1
   for (int e = it.col.seg_begin; e < it.col.seg_end; ++e) {
     const AttnSeg sg = bwd_seg(p, e);
     const int n = seg_num_qt(sg, it.c0) - seg_first_qt(sg, it.c0);
@@ -261,12 +268,24 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   return d;
 }
 
+// Scores of one thread's 64 queries outside [r_first, r_last] become -inf, in tensor memory and before they are read
+// (tiles at a bound only; a second form of the exponentials with 128 compares would cost every step its place in the
+// instruction cache).
+__device__ __forceinline__ void bwd_mask(uint32_t t_st, int r_first, int r_last) {
+#pragma unroll 1
+  for (int h = 0; h < 64; h += 32) {
+    uint32_t v[32];
+    tmem_ld_x32(t_st + h, v);
+    tmem_wait_ld();
+#pragma unroll
+    for (int c = 0; c < 32; ++c) v[c] = (h + c >= r_first && h + c <= r_last) ? v[c] : 0xFF800000u;
+    tmem_st_x32(t_st + h, v);
+  }
+  tmem_wait_st();
+}
 // P^T of one thread's 64 queries: exp2(x * scale_log2) with x = S^T - lse / scale as it comes out
-// of the tensor core, packed to bf16 pairs. MASK applies the causal / key-tail mask (tiles that
-// need none skip the compares).
-template <bool MASK>
-__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, bool key_ok, int r_first, int r_last,
-                                            uint32_t (&pk)[32]) {
+// of the tensor core, packed to bf16 pairs.
+__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, uint32_t (&pk)[32]) {
   float sv[2][32];
   tmem_ld_x32(t_st, reinterpret_cast<uint32_t(&)[32]>(sv[0]));
   tmem_ld_x32(t_st + 32, reinterpret_cast<uint32_t(&)[32]>(sv[1]));
@@ -280,12 +299,8 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, boo
       f2_unpack(f2_mul(f2_pack(sv[h][c], sv[h][c + 1]), sc2), x0, x1);     // two products per instruction
       // (some of them as a polynomial on the FMA pipe is slower: the phase is bound by instruction
       // issue, not by the special-function unit)
-      const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-      sv[h][c] = (!MASK || (key_ok && (h * 32 + c) >= r_first && (h * 32 + c) <= r_last)) ? p0 : 0.f;
-      sv[h][c + 1] = (!MASK || (key_ok && (h * 32 + c + 1) >= r_first && (h * 32 + c + 1) <= r_last)) ? p1 : 0.f;
+      pk[h * 16 + c / 2] = pack_bf16x2(fast_exp2(x0), fast_exp2(x1));
     }
-#pragma unroll
-    for (int c = 0; c < 16; ++c) pk[h * 16 + c] = pack_bf16x2(sv[h][2 * c], sv[h][2 * c + 1]);
   }
 }
 
@@ -445,6 +460,11 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   tc_fence_after_sync();
   const uint32_t tmem_base = s.tmem_base;
   WaitCtx wc{&s.abort_flag, p.status, 4000000000ull};
+  auto wait = [&](uint64_t* bar, uint32_t parity, int where) -> bool {
+    if (mbar_wait_quiet(bar, parity, wc)) return true;
+    report_error_call(wc.abort_flag, wc.status, UA_ERR_MBAR_TIMEOUT, where, static_cast<int>(parity));
+    return false;
+  };
 
   // Persistent CTAs (see the forward kernel): a CTA that is done with an item takes over one whose CTA
   // has not started. Its Q and dO arrive early, K and V as soon as the last product has read the old
@@ -454,7 +474,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   // Consumers wait for item m (m >= 1) with item_ready and hand their slot back with item_done.
   auto item_ready = [&](uint32_t m) -> bool {
     if (!p.persist) return false;
-    if (!mbar_wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, wc, 130)) return false;
+    if (!wait(&s.item_full[m & 1], ((m >> 1) - ((m & 1) ^ 1)) & 1, 130)) return false;
     return s.item[m & 1].exists != 0;
   };
 
@@ -471,31 +491,34 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         uint32_t live = 0;       // items with steps so far
         for (uint32_t n = 0; ok; ++n) {
           bool first = true;
+#pragma unroll 1
           for (int g = 0; g < p.kv_group && ok; ++g) {
             const int head = it.kv_head * p.kv_group + g;
+#pragma unroll 1
             for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
               const AttnSeg sg = bwd_seg(p, e);
               const int nq = seg_num_qt(sg, it.c0);
               if (seg_first_qt(sg, it.c0) < nq &&
                   !wait_staged(p.stage.flags, sg.wait_flag, sg.wait_count * p.stage.epoch, wc.budget_ns)) {
-                report_error(wc, UA_ERR_FLAG_TIMEOUT, 121, sg.wait_flag);
+                report_error_call(wc.abort_flag, wc.status, UA_ERR_FLAG_TIMEOUT, 121, sg.wait_flag);
                 ok = false;
                 break;
               }
+#pragma unroll 1
               for (int t = seg_first_qt(sg, it.c0); t < nq; ++t, ++i) {
                 const int st = i & 1;
                 const int qrow = sg.start + t * BWD_QT;
-                if (!mbar_wait(&s.q_empty[st], ((i >> 1) & 1) ^ 1, wc, 100)) { ok = false; break; }
+                if (!wait(&s.q_empty[st], ((i >> 1) & 1) ^ 1, 100)) { ok = false; break; }
                 mbar_arrive_expect_tx(&s.q_full[st], BWD_TILE_BYTES);
                 tma_load_4d(s.q[st], &p.tmQ[sg.src], &s.q_full[st], 0, head, qrow, it.batch);
                 tma_load_4d(s.q[st] + 16384, &p.tmQ[sg.src], &s.q_full[st], 64, head, qrow, it.batch);
                 if (first) {
                   first = false;
                   // the previous item's products have read its K and V
-                  if (live > 0 && !mbar_wait(&s.kv_empty, (live - 1) & 1, wc, 102)) { ok = false; break; }
+                  if (live > 0 && !wait(&s.kv_empty, (live - 1) & 1, 102)) { ok = false; break; }
                   if (!wait_staged(p.stage.flags, it.col.kv_wait_flag, it.col.kv_wait_count * p.stage.epoch,
                                    wc.budget_ns)) {
-                    report_error(wc, UA_ERR_FLAG_TIMEOUT, 120, it.col.kv_wait_flag);
+                    report_error_call(wc.abort_flag, wc.status, UA_ERR_FLAG_TIMEOUT, 120, it.col.kv_wait_flag);
                     ok = false;
                     break;
                   }
@@ -507,7 +530,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
                   tma_load_4d(s.v + 16384, &p.tmV[it.col.kv_src], &s.kv_full, 64, it.kv_head, krow, it.batch);
                   ++live;
                 }
-                if (!mbar_wait(&s.do_empty, (i & 1) ^ 1, wc, 101)) { ok = false; break; }
+                if (!wait(&s.do_empty, (i & 1) ^ 1, 101)) { ok = false; break; }
                 mbar_arrive_expect_tx(&s.do_full, BWD_TILE_BYTES);
                 tma_load_4d(s.d_o, &p.tmdO[sg.src], &s.do_full, 0, head, qrow, it.batch);
                 tma_load_4d(s.d_o + 16384, &p.tmdO[sg.src], &s.do_full, 64, head, qrow, it.batch);
@@ -518,7 +541,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
           // everything of this item is on its way: take over the next one
           mbar_arrive_expect_tx(&s.clc_full, 16);
           clc_try_cancel(&s.clc, &s.clc_full);
-          if (!mbar_wait(&s.clc_full, n & 1, wc, 104)) break;
+          if (!wait(&s.clc_full, n & 1, 104)) break;
           int bx, by;
           const bool got = clc_read(&s.clc, bx, by);
           fence_proxy_async_smem();               // read before the next response may overwrite it
@@ -526,7 +549,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
           else it.exists = 0;
           // the slot's previous item (n - 1) is done with
           const uint32_t slot = (n + 1) & 1;
-          if (n >= 1 && !mbar_wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, wc, 103)) break;
+          if (n >= 1 && !wait(&s.item_empty[slot], ((n - 1) >> 1) & 1, 103)) break;
           s.item[slot] = it;
           mbar_arrive(&s.item_full[slot]);
           if (!got) break;
@@ -534,7 +557,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       }
     } else if (warp == BWD_MMA_WARP) {
       // =============================== MMA issuer =============================================
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t idesc_kk = make_idesc_bf16(128, 128, 0, 0);   // S^T, dP^T: both K-major
         const uint32_t idesc_kn = make_idesc_bf16(128, 128, 0, 1);   // dV, dK: B N-major
         const uint32_t idesc_nn = make_idesc_bf16(128, 128, 1, 1);   // dQ^T: A, B MN-major
@@ -544,37 +567,37 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         const uint32_t t_dp = tmem_base + 384;     // dP^T, later dQ^T
         // one base descriptor per operand view; every instruction adds its (16-byte unit) offset to
         // the address field, which cannot carry out of it for addresses inside shared memory
-        const uint64_t k_kmaj = make_smem_desc_sw128(smem_u32(s.k), 16, 1024);        // A of S^T
-        const uint64_t k_mmaj = make_smem_desc_sw128(smem_u32(s.k), 16384, 1024);     // A of dQ^T
-        const uint64_t v_kmaj = make_smem_desc_sw128(smem_u32(s.v), 16, 1024);        // A of dP^T
-        const uint64_t do_kmaj = make_smem_desc_sw128(smem_u32(s.d_o), 16, 1024);     // B of dP^T
-        const uint64_t do_nmaj = make_smem_desc_sw128(smem_u32(s.d_o), 16384, 1024);  // B of dV
-        const uint64_t ds_kmaj = make_smem_desc_sw128(smem_u32(s.ds), 16, 1024);      // A of dK
-        const uint64_t ds_nmaj = make_smem_desc_sw128(smem_u32(s.ds), 16384, 1024);   // B of dQ^T
-        const uint64_t q_kmaj0 = make_smem_desc_sw128(smem_u32(s.q[0]), 16, 1024);    // B of S^T
-        const uint64_t q_nmaj0 = make_smem_desc_sw128(smem_u32(s.q[0]), 16384, 1024); // B of dK
-        const uint64_t ones_lse_d = make_smem_desc_noswz(smem_u32(s.ones_lse), 2048, 128);
-        const uint64_t ones_d_d = make_smem_desc_noswz(smem_u32(s.ones_d), 2048, 128);
+        const uint32_t k_kmaj = desc_lo(smem_u32(s.k), 16);         // A of S^T
+        const uint32_t k_mmaj = desc_lo(smem_u32(s.k), 16384);      // A of dQ^T
+        const uint32_t v_kmaj = desc_lo(smem_u32(s.v), 16);         // A of dP^T
+        const uint32_t do_kmaj = desc_lo(smem_u32(s.d_o), 16);      // B of dP^T
+        const uint32_t do_nmaj = desc_lo(smem_u32(s.d_o), 16384);   // B of dV
+        const uint32_t ds_kmaj = desc_lo(smem_u32(s.ds), 16);       // A of dK
+        const uint32_t ds_nmaj = desc_lo(smem_u32(s.ds), 16384);    // B of dQ^T
+        const uint32_t q_kmaj0 = desc_lo(smem_u32(s.q[0]), 16);     // B of S^T
+        const uint32_t q_nmaj0 = desc_lo(smem_u32(s.q[0]), 16384);  // B of dK
+        const uint32_t ones_lse_d = desc_lo(smem_u32(s.ones_lse), 2048);
+        const uint32_t ones_d_d = desc_lo(smem_u32(s.ones_d), 2048);
         // stage 0: chunks at aug[0] and aug_zero (4096 apart); stage 1: at aug[1] and aug_zero (2048 apart)
-        const uint64_t aug_desc[2] = {make_smem_desc_noswz(smem_u32(s.aug[0]), 4096, 128),
-                                      make_smem_desc_noswz(smem_u32(s.aug[1]), 2048, 128)};
-        constexpr uint64_t Q_STAGE = BWD_TILE_BYTES >> 4;
+        const uint32_t aug_desc0 = desc_lo(smem_u32(s.aug[0]), 4096), aug_desc1 = desc_lo(smem_u32(s.aug[1]), 2048);
+        constexpr uint32_t HI = desc_hi_sw128(1024), HI_AUG = desc_hi_noswz(128);
+        constexpr uint32_t Q_STAGE = BWD_TILE_BYTES >> 4;
         // K-major operands: 16 elements of the reduction = 32 B, the two 64-element halves 16384 B apart
-        auto koff = [](int kk) -> uint64_t { return static_cast<uint64_t>(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4); };
+        auto koff = [](int kk) -> uint32_t { return static_cast<uint32_t>(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4); };
         // MN-major operands: 16 rows of the reduction = 2048 B
-        auto noff = [](int kk) -> uint64_t { return static_cast<uint64_t>((kk * 2048) >> 4); };
+        auto noff = [](int kk) -> uint32_t { return static_cast<uint32_t>((kk * 2048) >> 4); };
         auto issue_st = [&](int st) {
-          const uint64_t qd = q_kmaj0 + st * Q_STAGE;
+          const uint32_t qd = q_kmaj0 + st * Q_STAGE;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            umma_ss(t_st, k_kmaj + koff(kk), qd + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
-          umma_ss(t_st, ones_lse_d, aug_desc[st], idesc_kk, 1u);     // - lse / scale
+            umma_ss_lo<HI, HI>(t_st, k_kmaj + koff(kk), qd + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
+          umma_ss_lo<HI_AUG, HI_AUG>(t_st, ones_lse_d, st ? aug_desc1 : aug_desc0, idesc_kk, 1u);     // - lse / scale
         };
         auto issue_dp = [&](int st) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            umma_ss(t_dp, v_kmaj + koff(kk), do_kmaj + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
-          umma_ss(t_dp, ones_d_d, aug_desc[st], idesc_kk, 1u);       // - D
+            umma_ss_lo<HI, HI>(t_dp, v_kmaj + koff(kk), do_kmaj + koff(kk), idesc_kk, kk > 0 ? 1u : 0u);
+          umma_ss_lo<HI_AUG, HI_AUG>(t_dp, ones_d_d, st ? aug_desc1 : aug_desc0, idesc_kk, 1u);       // - D
         };
         bool ok = true;
         uint32_t i = 0;                   // steps so far
@@ -582,40 +605,41 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         for (uint32_t n = 0; ok; ++n) {
           const int n_steps = bwd_steps(p, s.item[n & 1]);
           if (n_steps > 0) {
-            if (!mbar_wait(&s.kv_full, live & 1, wc, 200)) break;
-            if (!mbar_wait(&s.q_full[i & 1], (i >> 1) & 1, wc, 201)) break;
-            if (!mbar_wait(&s.aug0_ready, live & 1, wc, 208)) break;
+            if (!wait(&s.kv_full, live & 1, 200)) break;
+            if (!wait(&s.q_full[i & 1], (i >> 1) & 1, 201)) break;
+            if (!wait(&s.aug0_ready, live & 1, 208)) break;
             tc_fence_after_sync();
             issue_st(i & 1);
             tc_commit(&s.s_full);
-            if (!mbar_wait(&s.do_full, i & 1, wc, 202)) break;
+            if (!wait(&s.do_full, i & 1, 202)) break;
             // dP^T lands where the previous item's last dQ^T was. (That dK / dV of that item have been read
             // out before they are started anew is implied by p_ready: the warps arrive after their epilogue.)
-            if (i > 0 && !mbar_wait(&s.dq_free, (i - 1) & 1, wc, 209)) break;
+            if (i > 0 && !wait(&s.dq_free, (i - 1) & 1, 209)) break;
             tc_fence_after_sync();
             issue_dp(i & 1);
             tc_commit(&s.dp_full);
+#pragma unroll 1
             for (int k = 0; k < n_steps; ++k, ++i) {
               const int st = i & 1;
               const uint32_t ph = i & 1;
-              const uint64_t qn = q_nmaj0 + st * Q_STAGE;
+              const uint32_t qn = q_nmaj0 + st * Q_STAGE;
               const bool more = k + 1 < n_steps;
               // dV += P^T dO : A = P^T in TMEM (queries 0-63 packed at columns 0-31, 64-127 at 64-95),
               // B = dO as an N-major operand (16 query rows = 2048 B, d-halves 16384 B apart)
               BWD_PROF(i == BWD_PROF_STEP, 0);
               BWD_PROF(i == BWD_PROF_STEP + BWD_PROF_SPAN, 9);
-              if (!mbar_wait(&s.p_ready, ph, wc, 203)) { ok = false; break; }
+              if (!wait(&s.p_ready, ph, 203)) { ok = false; break; }
               BWD_PROF(i == BWD_PROF_STEP, 1);
               tc_fence_after_sync();
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
-                umma_ts(t_dv, t_st + (kk >> 2) * 64 + (kk & 3) * 8, do_nmaj + noff(kk), idesc_kn,
+                umma_ts_lo<HI>(t_dv, t_st + (kk >> 2) * 64 + (kk & 3) * 8, do_nmaj + noff(kk), idesc_kn,
                         (k > 0 || kk > 0) ? 1u : 0u);
               tc_commit(&s.do_empty);
               // S^T of the next step right behind it: it overwrites P^T(i), which dV(i) reads first
               // because the tensor pipe executes in issue order
               if (more) {
-                if (!mbar_wait(&s.q_full[st ^ 1], ((i + 1) >> 1) & 1, wc, 205)) { ok = false; break; }
+                if (!wait(&s.q_full[st ^ 1], ((i + 1) >> 1) & 1, 205)) { ok = false; break; }
                 tc_fence_after_sync();
                 BWD_PROF(i == BWD_PROF_STEP, 2);
                 issue_st(st ^ 1);
@@ -624,25 +648,25 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
               BWD_PROF(i == BWD_PROF_STEP, 3);
               // dQ^T = K^T dS^T : A = K as an M-major operand, B = dS^T as an N-major operand (two
               // 64-query panels 16384 B apart); lands where dP^T was
-              if (!mbar_wait(&s.ds_ready, ph, wc, 204)) { ok = false; break; }
+              if (!wait(&s.ds_ready, ph, 204)) { ok = false; break; }
               BWD_PROF(i == BWD_PROF_STEP, 4);
               tc_fence_after_sync();
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
-                umma_ss(t_dp, k_mmaj + noff(kk), ds_nmaj + noff(kk), idesc_nn, kk > 0 ? 1u : 0u);
+                umma_ss_lo<HI, HI>(t_dp, k_mmaj + noff(kk), ds_nmaj + noff(kk), idesc_nn, kk > 0 ? 1u : 0u);
               tc_commit(&s.dq_full);
               // dK += dS^T Q : A = dS^T in shared memory (K-major over queries: panel kk/4, 32 B per
               // step), B = Q as an N-major operand; runs while the drain warpgroup reads dQ^T
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
-                umma_ss(t_dk, ds_kmaj + koff(kk), qn + noff(kk), idesc_kn, (k > 0 || kk > 0) ? 1u : 0u);
+                umma_ss_lo<HI, HI>(t_dk, ds_kmaj + koff(kk), qn + noff(kk), idesc_kn, (k > 0 || kk > 0) ? 1u : 0u);
               tc_commit(&s.q_empty[st]);
               BWD_PROF(i == BWD_PROF_STEP, 5);
               if (more) {
-                if (!mbar_wait(&s.do_full, (i + 1) & 1, wc, 206)) { ok = false; break; }
+                if (!wait(&s.do_full, (i + 1) & 1, 206)) { ok = false; break; }
                 BWD_PROF(i == BWD_PROF_STEP, 6);
                 // dP^T(i+1) lands where dQ^T(i) is: wait until the drain warpgroup has read it
-                if (!mbar_wait(&s.dq_free, ph, wc, 207)) { ok = false; break; }
+                if (!wait(&s.dq_free, ph, 207)) { ok = false; break; }
                 BWD_PROF(i == BWD_PROF_STEP, 7);
                 tc_fence_after_sync();
                 issue_dp(st ^ 1);
@@ -752,6 +776,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       if (n > 0) trace_stamp(p.trace, it.linear, 0);
       trace_stamp(p.trace, it.linear, 1);
       trace_ident(p.trace, it.linear, it.col_idx);
+#pragma unroll 1
       for (int k = 0; k < n_steps && ok; ++k, ++i) {
         const uint32_t ph = i & 1;
         const AttnSeg& sg = cur.sg;
@@ -776,14 +801,12 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
 
         // ---- phase A: P^T = exp2((S^T - lse / scale) * scale) -> TMEM (packed bf16) ------------
         BWD_PROF(prof, pslot + 1);
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.s_full, ph, wc, 300))) { ok = false; break; }
+        if (!__all_sync(0xFFFFFFFFu, wait(&s.s_full, ph, 300))) { ok = false; break; }
         BWD_PROF(prof, pslot + 2);
         tc_fence_after_sync();
         uint32_t pk[32];                 // this thread's 64 probabilities, packed; kept for phase B
-        if (__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63))
-          bwd_phase_a<false>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
-        else
-          bwd_phase_a<true>(t_st, p.scale_log2, key_ok, r_first, r_last, pk);
+        if (!__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63)) bwd_mask(t_st, key_ok ? r_first : 64, r_last);
+        bwd_phase_a(t_st, p.scale_log2, pk);
         // packed P^T of this half goes to the first 32 columns of this half's own S^T columns
         // (the other warpgroup may still be reading its fp32 half)
         BWD_PROF(prof, pslot + 3);
@@ -794,7 +817,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         BWD_PROF(prof, pslot + 4);
 
         // ---- phase B: dS^T = P^T * (dP^T - D) -> shared memory ------------------------------
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.dp_full, ph, wc, 301))) { ok = false; break; }
+        if (!__all_sync(0xFFFFFFFFu, wait(&s.dp_full, ph, 301))) { ok = false; break; }
         BWD_PROF(prof, pslot + 5);
         tc_fence_after_sync();
         uint8_t* ds_panel = s.ds + wg * 16384;     // this half's 64-query panel
@@ -843,7 +866,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       }
       // ---------------------------------- dK / dV epilogue ------------------------------------
       if (n_done > 0 && ok) {
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s.dkv_full, live & 1, wc, 310));
+        ok = __all_sync(0xFFFFFFFFu, wait(&s.dkv_full, live & 1, 310));
         ++live;
       }
       tc_fence_after_sync();
@@ -863,19 +886,22 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     float* stage = s.dq_stage[0];
     bool ok = true;
     uint32_t i = 0;
-    uint32_t n_chunk = 0;
+    int slot = 0;                      // staging tile
     for (uint32_t n = 0;; ++n) {
       const BwdItem& it = s.item[n & 1];
       const int c0 = it.c0;
+#pragma unroll 1
       for (int g = 0; g < p.kv_group && ok; ++g) {
         const int head = it.kv_head * p.kv_group + g;
+#pragma unroll 1
         for (int e = it.col.seg_begin; e < it.col.seg_end && ok; ++e) {
           const AttnSeg sg = bwd_seg(p, e);
           const int nq = seg_num_qt(sg, c0);
           const CUtensorMap* tdq = &p.tmdQ[sg.src];
+#pragma unroll 1
           for (int t = seg_first_qt(sg, c0); t < nq; ++t, ++i) {
             BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 48);
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&s.dq_full, i & 1, wc, 400))) { ok = false; break; }
+            if (!__all_sync(0xFFFFFFFFu, wait(&s.dq_full, i & 1, 400))) { ok = false; break; }
             BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 49);
             tc_fence_after_sync();
             const int qrow = sg.start + t * BWD_QT;
@@ -896,7 +922,8 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
                 if (quad == 0 && lane == 0) tma_store_wait_read_all_but<2>();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 52 + (h >> 1) * 3);
-                float* tile = stage + ((n_chunk + h) % 3) * 2048;
+                float* tile = stage + slot * 2048;
+                slot = slot == 2 ? 0 : slot + 1;
 #pragma unroll
                 for (int c = 0; c < 16; ++c)
                   tile[c * 128 + quad * 32 + lane] = __uint_as_float(dv[h >> 1][(h & 1) * 16 + c]) * p.scale;
@@ -910,7 +937,6 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
                 BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0 && (h & 1) == 0, 54 + (h >> 1) * 3);
               }
             }
-            n_chunk += 8;
             BWD_PROF(i == BWD_PROF_STEP && quad == 0 && lane == 0, 51);
           }
         }

@@ -640,30 +640,31 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
       }
     } else if (warp == FWD_QK_WARP || (!FEW && warp == FWD_PV_WARP)) {
       // =============================== MMA issuers ============================================
-      if (lane == 0) {
+      if (elect_one()) {             // (not lane == 0: the assembler knows that one thread is left)
         const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S = Q K^T, both K-major
         const uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);   // O += P V, V is N-major
         // one base descriptor per operand; a tile and an instruction add their offset (in 16-byte units) to the
         // address field, which cannot carry out of it for addresses inside shared memory
-        const uint64_t q_desc = make_smem_desc_sw128(smem_u32(s.q[0]), 16, 1024), k_desc = make_smem_desc_sw128(smem_u32(s.k[0]), 16, 1024);
-        const uint64_t v_desc = make_smem_desc_sw128(smem_u32(s.v[0]), 16384, 1024);
+        const uint32_t q_desc = desc_lo(smem_u32(s.q[0]), 16), k_desc = desc_lo(smem_u32(s.k[0]), 16);
+        const uint32_t v_desc = desc_lo(smem_u32(s.v[0]), 16384);
+        constexpr uint32_t HI = desc_hi_sw128(1024);
         constexpr uint32_t TILE16 = FWD_TILE_BYTES >> 4;
         auto issue_s = [&](int w, int st) {
-          const uint64_t qa = q_desc + (FEW ? 0 : w) * TILE16, ka = k_desc + st * TILE16;
+          const uint32_t qa = q_desc + (FEW ? 0 : w) * TILE16, ka = k_desc + st * TILE16;
           const uint32_t tS = tmem_base + (FEW ? w * 128 : 0);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
-            umma_ss(tS, qa + off, ka + off, idesc_s, kk > 0 ? 1u : 0u);
+            umma_ss_lo<HI, HI>(tS, qa + off, ka + off, idesc_s, kk > 0 ? 1u : 0u);
           }
         };
         auto issue_pv = [&](int w, int st, bool acc) {
-          const uint64_t va = v_desc + st * TILE16;
+          const uint32_t va = v_desc + st * TILE16;
           const uint32_t tP = tmem_base + (FEW ? w * 128 : 128 + w * 64), tO = tmem_base + 256 + w * 128;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
             // A: 16 keys = 8 packed columns of P; B: 16 key rows = 2048 B, d-halves 16384 B apart
-            umma_ts(tO, tP + kk * 8, va + ((kk * 2048) >> 4), idesc_o, (acc || kk > 0) ? 1u : 0u);
+            umma_ts_lo<HI>(tO, tP + kk * 8, va + ((kk * 2048) >> 4), idesc_o, (acc || kk > 0) ? 1u : 0u);
         };
         bool ok = true;
         uint32_t kv = 0;                  // K / V tiles so far

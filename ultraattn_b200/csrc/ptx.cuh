@@ -464,6 +464,42 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
       : "memory");
 }
 
+// The same with descriptors in two words. All that changes between the products of a loop is the address in the low word;
+// the high one is a constant. (A 64-bit sum per operand and product makes an issuing loop twice as long.)
+template <uint32_t A_HI, uint32_t B_HI>
+__device__ __forceinline__ void umma_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 a, {%1, %5};\n\t"
+      "mov.b64 b, {%2, %6};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(A_HI), "n"(B_HI)
+      : "memory");
+}
+template <uint32_t B_HI>
+__device__ __forceinline__ void umma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 b;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(B_HI)
+      : "memory");
+}
+// words of make_smem_desc_sw128 / make_smem_desc_noswz
+constexpr uint32_t desc_hi_sw128(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
+constexpr uint32_t desc_hi_noswz(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14); }
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
+  return ((saddr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
+}
+
 // ----------------------------------------------------------------------------------------------
 // tcgen05: TMEM <-> registers. Shape 32x32b: thread t of the warp touches lane (warp%4)*32+t,
 // register i touches column base+i.
