@@ -13,6 +13,7 @@ from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_long, c_void_
 from . import build as _build
 
 _lib = None
+_host = None
 LAUNCHES = [0]      # kernels of this library launched so far (every wrapper reports here)
 
 
@@ -108,6 +109,25 @@ def load():
         raise ImportError(f"ultraattn_b200: kernel library is older than its sources and the rebuild failed: {e}") from e
     _lib = _declare(ctypes.CDLL(str(path)))
     return _lib
+
+
+def host():
+    """The native host part of single-device calls (csrc/host_ext.cpp), with the library's entry points."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+        import torch  # noqa: F401  (the extension's libraries)
+        lib = load()
+        path = str(_build.HOST_PATH)
+        loader = importlib.machinery.ExtensionFileLoader("ua_host", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ua_host", path, loader=loader))
+        loader.exec_module(mod)
+        address = lambda name: ctypes.cast(getattr(lib, name), c_void_p).value
+        mod.init(address("ua_attn_fwd_dense_parts"), address("ua_attn_fwd_dense"), address("ua_attn_bwd_local"),
+                 address("ua_last_error"))
+        _host = mod
+    return _host
 
 
 def stream_of(t) -> int:

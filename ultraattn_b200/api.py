@@ -43,13 +43,13 @@ def _dense_kind(pattern: BSA_Repr, q, k, v) -> int:
 class _LocalAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, pattern, softmax_scale):
-        o = torch.empty_like(q)
-        lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
         ctx.dense = _dense_kind(pattern, q, k, v)
         if ctx.dense:
             ctx.bplan = None
-            A.attn_fwd_dense(q, k, v, (o, lse), ctx.dense == 2, softmax_scale)
+            o, lse = A.dense_forward(q, k, v, ctx.dense == 2, softmax_scale)
         else:
+            o = torch.empty_like(q)
+            lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
             fplan, ctx.bplan = local_plans(pattern, q.shape[1], q.device)
             A.attn_fwd([q], [k], [v], [(o, lse)], fplan, softmax_scale)
         ctx.save_for_backward(q, k, v, o, lse)
@@ -69,7 +69,12 @@ def local_backward(q, k, v, o, lse, d_o, bplan, softmax_scale=None, dense: int =
     if q.is_cuda:
         # the kernel writes the gradients of every key in a column of the plan; only keys outside all of them
         # (tokens of a packed buffer that belong to no sequence) need a fill
-        new = torch.empty_like if dense or bplan.kv_tokens == k.shape[1] else torch.zeros_like
+        every_key = dense or bplan.kv_tokens == k.shape[1]
+        if every_key:
+            grads = A.local_backward(q, k, v, o, lse, d_o, bplan, dense, softmax_scale)
+            if grads is not None:
+                return grads
+        new = torch.empty_like if every_key else torch.zeros_like
         dq, dk, dv = torch.empty(q.shape, dtype=q.dtype, device=q.device), new(k), new(v)
         A.attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, bplan, dense, softmax_scale)
         return dq, dk, dv

@@ -4,6 +4,8 @@ Every ``csrc/*.cu`` file is compiled with ``-gencode arch=compute_100a,code=sm_1
 into ``ultraattn_b200/lib/libultraattn_sm100.so``. The library exposes a plain C ABI (loaded with
 ctypes by :mod:`ultraattn_b200._lib`), so no PyTorch headers are involved and a full rebuild
 takes well under a minute. nvcc cross-compiles, so this works on a machine without a GPU.
+``csrc/host_ext.cpp``, the native host part of single-device calls, is the one file that knows PyTorch:
+it becomes the Python extension ``lib/ua_host.so``.
 
 The reference ships no native code of its own (it builds NCCL and a flash-attention fork through
 ``scripts/Makefile:47-96``); this is the equivalent build step of this framework.
@@ -22,6 +24,7 @@ CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 LIB_PATH = LIB_DIR / "libultraattn_sm100.so"
 OBJ_DIR = LIB_DIR / "obj"
+HOST_PATH = LIB_DIR / "ua_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -50,12 +53,18 @@ def _newest_header_mtime() -> float:
 STAMP_PATH = LIB_DIR / "build_stamp.txt"
 
 
+def _torch_dir() -> Path:
+    import importlib.util
+    return Path(importlib.util.find_spec("torch").origin).parent          # (found, not imported)
+
+
 def source_digest() -> str:
     """Hash of everything the library is built from (sources, headers, compiler flags). File times
     do not survive every way of copying a tree to another machine; contents do."""
     import hashlib
     h = hashlib.sha256(" ".join(NVCC_FLAGS).encode())
-    for f in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))):
+    h.update((_torch_dir() / "version.py").read_bytes())          # (the extension is built for this PyTorch)
+    for f in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cpp"))):
         h.update(f.name.encode())
         h.update(f.read_bytes())
     return h.hexdigest()
@@ -63,7 +72,7 @@ def source_digest() -> str:
 
 def needs_build() -> bool:
     """True when the library is missing or was built from other sources than the present ones."""
-    if not LIB_PATH.exists() or not STAMP_PATH.exists():
+    if not LIB_PATH.exists() or not HOST_PATH.exists() or not STAMP_PATH.exists():
         return True
     return STAMP_PATH.read_text().strip() != source_digest()
 
@@ -108,7 +117,9 @@ def _build_locked(nvcc: str, force: bool, verbose: bool) -> Path:
         return obj
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
+        host = ex.submit(_build_host)
         objs = list(ex.map(compile_one, sources()))
+        host.result()
     tmp = LIB_PATH.with_suffix(".so.tmp")
     cmd = [nvcc, "-shared", "-o", str(tmp), *map(str, objs),
            "-gencode", "arch=compute_100a,code=sm_100a"]
@@ -118,6 +129,20 @@ def _build_locked(nvcc: str, force: bool, verbose: bool) -> Path:
     os.replace(tmp, LIB_PATH)          # a reader never sees a half-written library
     STAMP_PATH.write_text(source_digest() + "\n")
     return LIB_PATH
+
+
+def _build_host() -> None:
+    import sysconfig
+    torch_dir = _torch_dir()
+    tmp = HOST_PATH.with_suffix(".so.tmp")
+    cmd = [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{torch_dir / 'include'}",
+           f"-I{torch_dir / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
+           str(CSRC / "host_ext.cpp"), "-o", str(tmp), f"-L{torch_dir / 'lib'}", "-lc10", "-ltorch_cpu", "-ltorch_python",
+           f"-Wl,-rpath,{torch_dir / 'lib'}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for host_ext.cpp:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, HOST_PATH)
 
 
 if __name__ == "__main__":

@@ -389,6 +389,42 @@ def attn_fwd_dense(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: tuple
     _lib.check(rc, "ua_attn_fwd_dense", 2 if parts else 1)
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _native(*tensors) -> bool:
+    """Plain CUDA tensors, no debug mode: the native host part (csrc/host_ext.cpp) may be asked."""
+    return tensors[0].is_cuda and all(type(t) in _PLAIN for t in tensors) and not debug_bounds_enabled()
+
+
+def dense_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool, softmax_scale: float | None = None):
+    """(O, lse) of :func:`attn_fwd_dense`, in new tensors."""
+    if _native(q, k, v):
+        r = _lib.host().dense_forward(q, k, v, causal, softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(q.shape[3]),
+                                      status_buffer(q.device).data_ptr(), _lib.stream_of(q))
+        if r is not None:
+            _lib.LAUNCHES[0] += r[2]
+            return r[0], r[1]
+    o = torch.empty_like(q)
+    lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
+    attn_fwd_dense(q, k, v, (o, lse), causal, softmax_scale)
+    return o, lse
+
+
+def local_backward(q, k, v, o, lse, d_o, plan: "BwdPlan | None", dense: int = 0, softmax_scale=None):
+    """(dQ, dK, dV) of :func:`attn_bwd_local`, in new tensors; None: not for these (see there). A plan has to write
+    the gradient of every key."""
+    if not _native(q, k, v, o, lse, d_o):
+        return None
+    tables = (0, 0, 0, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(), plan.n_tiles)
+    r = _lib.host().local_backward(q, k, v, o, lse, d_o, *tables, dense, 0 if dense else int(plan.skewed),
+                                   softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(q.shape[3]),
+                                   status_buffer(q.device).data_ptr(), _lib.stream_of(q))
+    if r is not None:
+        _lib.LAUNCHES[0] += 3
+    return r
+
+
 def _stage_args(stage):
     if stage is None:
         return (None, 0, 0, None, 1, None)

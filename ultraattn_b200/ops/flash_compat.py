@@ -95,10 +95,12 @@ def _flash_attn_forward(q, k, v, dropout_p, softmax_scale, causal, window_size=(
     if _windowed(window_size):
         o, lse = W.window_forward(q, k, v, window_size, bool(causal), _scale(q, softmax_scale), out)
         return o, q, k, v, o, lse, None, None
-    o = out if out is not None else torch.empty_like(q)
+    if out is None:
+        o, lse = A.dense_forward(q, k, v, bool(causal), softmax_scale)
+        return o, q, k, v, o, lse, None, None
     lse = torch.empty(q.shape[0], q.shape[2], sq, dtype=torch.float32, device=q.device)
-    A.attn_fwd_dense(q, k, v, (o, lse), bool(causal), _scale(q, softmax_scale))
-    return o, q, k, v, o, lse, None, None
+    A.attn_fwd_dense(q, k, v, (out, lse), bool(causal), _scale(q, softmax_scale))
+    return out, q, k, v, out, lse, None, None
 
 
 def _flash_attn_backward(dout, q, k, v, out, softmax_lse, dq, dk, dv, dropout_p, softmax_scale, causal,
@@ -219,6 +221,10 @@ class _FlashFunc(torch.autograd.Function):
     def backward(ctx, d_o, _d_lse):
         q, k, v, o, lse = ctx.saved_tensors
         scale, causal, window = ctx.args
+        if q.is_cuda and not _windowed(window):
+            grads = A.local_backward(q, k, v, o, lse, d_o.contiguous(), None, 2 if causal else 1, scale)
+            if grads is not None:
+                return *grads, None, None, None
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         _flash_attn_backward(d_o.contiguous(), q, k, v, o, lse, dq, dk, dv, 0.0, scale, causal, window)
         return dq, dk, dv, None, None, None
