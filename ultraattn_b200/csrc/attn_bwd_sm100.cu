@@ -39,8 +39,8 @@
 //   warp  13  : tcgen05.mma issuer, TMEM allocation
 // The five roles' loops are about 30 KB of instructions a step, more than the instruction cache holds (103 misses a step in
 // a build of 115 KB). So they are kept short: descriptors in 32-bit words, one elected thread instead of lane 0 (the
-// assembler then knows that operands are uniform), loops over segments not unrolled, masks in a rolled loop over
-// tensor memory, errors reported by a call: 92 KB. Backward, us, before -> after: 8192 causal tokens, 32 heads 1263 ->
+// assembler then knows that operands are uniform), loops over segments not unrolled, one form of the
+// exponentials with and without a mask, errors reported by a call: 92 KB. Backward, us, before -> after: 8192 causal tokens, 32 heads 1263 ->
 // 1220, 4 x 2048 tokens full 209 -> 206, 16384 full unchanged (power and shared memory bound it). Two issuing warps, as in
 // the forward, are 5 % slower here: the order dV, S^T, dQ^T, dK, dP^T is what keeps the softmax warps fed.
 // dK/dV leave the CTA either as bf16 stores (the CTA is their only producer) or as fp32
@@ -268,28 +268,22 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   return d;
 }
 
-// Scores of one thread's 64 queries outside [r_first, r_last] become -inf, in tensor memory and before they are read
-// (tiles at a bound only; a second form of the exponentials with 128 compares would cost every step its place in the
-// instruction cache).
-__device__ __forceinline__ void bwd_mask(uint32_t t_st, int r_first, int r_last) {
-#pragma unroll 1
-  for (int h = 0; h < 64; h += 32) {
-    uint32_t v[32];
-    tmem_ld_x32(t_st + h, v);
-    tmem_wait_ld();
-#pragma unroll
-    for (int c = 0; c < 32; ++c) v[c] = (h + c >= r_first && h + c <= r_last) ? v[c] : 0xFF800000u;
-    tmem_st_x32(t_st + h, v);
-  }
-  tmem_wait_st();
-}
 // P^T of one thread's 64 queries: exp2(x * scale_log2) with x = S^T - lse / scale as it comes out
-// of the tensor core, packed to bf16 pairs.
-__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, uint32_t (&pk)[32]) {
+// of the tensor core, packed to bf16 pairs. `masked` (tiles at a bound): queries outside [r_first, r_last] get 0.
+__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, bool masked, int r_first, int r_last, uint32_t (&pk)[32]) {
   float sv[2][32];
   tmem_ld_x32(t_st, reinterpret_cast<uint32_t(&)[32]>(sv[0]));
   tmem_ld_x32(t_st + 32, reinterpret_cast<uint32_t(&)[32]>(sv[1]));
   tmem_wait_ld();
+  if (masked) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int a = min(max(r_first - h * 32, 0), 32), b = min(max(r_last + 1 - h * 32, 0), 32);
+      const uint32_t seen = (b > 0 ? 0xFFFFFFFFu >> (32 - b) : 0u) & (a < 32 ? 0xFFFFFFFFu << a : 0u);
+#pragma unroll
+      for (int c = 0; c < 32; ++c) sv[h][c] = (seen >> c) & 1u ? sv[h][c] : -INFINITY;
+    }
+  }
   const uint64_t sc2 = f2_pack(scale_log2, scale_log2);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -805,8 +799,8 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         BWD_PROF(prof, pslot + 2);
         tc_fence_after_sync();
         uint32_t pk[32];                 // this thread's 64 probabilities, packed; kept for phase B
-        if (!__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63)) bwd_mask(t_st, key_ok ? r_first : 64, r_last);
-        bwd_phase_a(t_st, p.scale_log2, pk);
+        const bool masked = !__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63);
+        bwd_phase_a(t_st, p.scale_log2, masked, key_ok ? r_first : 64, r_last, pk);
         // packed P^T of this half goes to the first 32 columns of this half's own S^T columns
         // (the other warpgroup may still be reading its fp32 half)
         BWD_PROF(prof, pslot + 3);

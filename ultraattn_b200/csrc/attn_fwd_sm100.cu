@@ -57,14 +57,14 @@ static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setm
 // warps 2210. And a sub-tile's cycle was its softmax plus its own products; with a shared score tile Q K^T of the next
 // tile no longer waits for P V. What is left of it follows the score tile: loaded into registers (290 clocks), seen by the
 // issuing warp (230), Q K^T (512 - 630), seen by the softmax warps (290), twice a pair: 2850.
-// The instructions of all roles are kept few and close together (masks in a rolled loop over tensor memory, one
-// vote for all that is rare, errors reported by a call, loops over segments not unrolled, 32-bit divisions, operand
-// descriptors by addition): the instruction cache missed 99 times a pair before, 17 now, and every miss stops all four
-// warps of a sub-tile; builds that differ in nothing but that (15 and 53 misses a pair) took 918 and 968 us for 16384
-// tokens, 8 heads. B200, us, before -> now: 8192 causal tokens, 32 heads 510 -> 453; 16384 tokens, 8 heads 995 -> 876, 32
-// heads 3450 -> 3140 (1275 -> 1400 TFLOP/s); 512 queries behind 32768 keys, 32 / 8 heads 260 -> 222; 1000 causal tokens, 32 / 8
-// heads 26.6 -> 24.0. Part of the exponentials as a polynomial of degree 5 on the FMA pipe (1/8, 1/4, 3/8 of them): 914 ->
-// 924, 956, 1048 us. P handed over in two parts (96 + 32 keys): 2 % slower in this form.
+// The instructions of all roles are kept few and close together (one vote for all that is rare, errors reported by a call,
+// loops over segments not unrolled, 32-bit divisions, operand descriptors by addition): the instruction cache missed 99
+// times a pair before, 17 now, and every miss stops all four warps of a sub-tile; builds that differ in nothing but that
+// (15 and 53 misses a pair) took 918 and 968 us for 16384 tokens, 8 heads. B200, us, before -> now: 8192 causal tokens, 32 heads
+// 510 -> 432; 16384 tokens, 8 heads 990 -> 847, 32 heads 3450 -> 3050 (1275 -> 1440 TFLOP/s); 512 queries behind 32768 keys, 32 / 8
+// heads 260 -> 222; 1000 causal tokens, 32 / 8 heads 26.6 -> 22.5. Part of the exponentials as a polynomial of degree 5 on the FMA
+// pipe (1/8, 1/4, 3/8 of them, at the 914 us of the time): 924, 956, 1048 us. P handed over in two parts (96 + 32 keys): 2 %
+// slower in this form.
 constexpr int FWD_TILE_BYTES = ATTN_TILE * ATTN_D * 2;  // 32 KB: [2 d-halves][128 rows][128 B]
 
 struct FwdRow {
@@ -443,28 +443,6 @@ __device__ __forceinline__ int seg_end_of(const AttnSeg& sg, int r) {
 __device__ __forceinline__ int seg_first_of(const AttnSeg& sg, int r) {
   return (sg.causal & SEG_LOWER) ? max(0, r + sg.lo) : 0;
 }
-// Columns outside [low, lim) of a score tile (of this thread's row) become -inf, in tensor memory and before the
-// scores are read: few tiles need it, and 128 compares in the tile loop push its other instructions out of the
-// instruction cache. Blocks of 32 columns that all rows of the warp see ([clear_lo, clear_hi)) stay as they are.
-// `r`: this thread's query token, r_first and r_last those of the warp's first and last row; c0: the tile's first column.
-__device__ __forceinline__ void fwd_mask(uint32_t tS, const AttnSeg& sg, int r, int r_first, int r_last, int c0) {
-  const int low = seg_first_of(sg, r) - c0, lim = seg_end_of(sg, r) - c0;
-  const int some_lo = seg_first_of(sg, r_first) - c0, clear_lo = seg_first_of(sg, r_last) - c0;
-  const int clear_hi = seg_end_of(sg, r_first) - c0, some_hi = seg_end_of(sg, r_last) - c0;
-#pragma unroll 1
-  for (int c = 0; c < ATTN_TILE; c += 32) {
-    if (c >= clear_lo && c + 32 <= clear_hi) continue;
-    uint32_t v[32];
-    if (c < some_hi && c + 32 > some_lo) {
-      tmem_ld_x32(tS + c, v);
-      tmem_wait_ld();
-    }
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = (c + i >= low && c + i < lim) ? v[i] : 0xFF800000u;
-    tmem_st_x32(tS + c, v);
-  }
-  tmem_wait_st();
-}
 // A branch that is never taken (a CTA's 2^32nd score tile). The assembler moves arithmetic over everything that is not a
 // branch, and put the maxima in front of the arrival on s_free, which the other sub-tile's scores wait for
 // (16k tokens, 8 heads: 1038 us without, 917 with).
@@ -827,9 +805,6 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               mbar_arrive_warp(&s.p_full[w]);
               continue;
             }
-            if (t < clear_first || t >= clear_end) {
-              fwd_mask(tS, seg_of(e), (it.r0 + r_cta) >> psh, (it.r0 + r_cta - lane) >> psh, (it.r0 + r_cta - lane + 31) >> psh, t * ATTN_TILE);
-            }
             float sv[ATTN_TILE];
             {
               uint32_t(&raw)[ATTN_TILE] = reinterpret_cast<uint32_t(&)[ATTN_TILE]>(sv);
@@ -844,6 +819,25 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
               PIN
             }
             FWD_PROF(prof, pslot + 2);
+            if (t < clear_first || t >= clear_end) {
+              // Columns outside [low, lim) become -inf, 32 at a time and only where some row needs it (two instructions a
+              // column with a mask in bits; in a loop over tensor memory, before the scores are read, a masked
+              // tile took 1000 clocks more: window of 1024 with sinks, 32k tokens, 350 -> 332 us).
+              const AttnSeg sg = seg_of(e);
+              const int r = (it.r0 + r_cta) >> psh, r_first = (it.r0 + r_cta - lane) >> psh, r_last = (it.r0 + r_cta - lane + 31) >> psh;
+              const int c0 = t * ATTN_TILE;
+              const int low = seg_first_of(sg, r) - c0, lim = seg_end_of(sg, r) - c0;
+              const int clear_lo = seg_first_of(sg, r_last) - c0, clear_hi = seg_end_of(sg, r_first) - c0;
+#pragma unroll
+              for (int c = 0; c < ATTN_TILE; c += 32) {
+                if (c >= clear_lo && c + 32 <= clear_hi) continue;
+                // bit i: column c + i is seen
+                const int a = min(max(low - c, 0), 32), b = min(max(lim - c, 0), 32);
+                const uint32_t seen = (b > 0 ? 0xFFFFFFFFu >> (32 - b) : 0u) & (a < 32 ? 0xFFFFFFFFu << a : 0u);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) sv[c + i] = (seen >> i) & 1u ? sv[c + i] : NEG_INF;
+              }
+            }
             // eight independent running maxima, two new values per instruction: one dependent chain of
             // compares would cost more than the exponentials
             float mx8[8];
