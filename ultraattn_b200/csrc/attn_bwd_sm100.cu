@@ -386,15 +386,6 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  const BwdItem item0 = bwd_item(p, blockIdx.x, blockIdx.y);
-  trace_stamp(p.trace, item0.linear, 0);
-  {
-    // does this CTA read a staged block? then it first helps to empty the copy queue
-    bool waits = item0.col.kv_wait_flag != 0;
-    for (int e = item0.col.seg_begin; e < item0.col.seg_end && !waits; ++e) waits = bwd_seg(p, e).wait_flag != 0;
-    drain_stage_queue(p.stage, waits, item0.linear, &s.stage_slot);
-  }
-
   if (threadIdx.x == 0) {
     mbar_init(&s.kv_full, 1);
     for (int i = 0; i < 2; ++i) {
@@ -417,7 +408,6 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       mbar_init(&s.item_full[i], 1);
       mbar_init(&s.item_empty[i], 13);        // MMA warp, eight softmax warps, four drain warps
     }
-    s.item[0] = item0;
     s.abort_flag = 0;
     fence_mbar_init();
   }
@@ -448,6 +438,17 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       *reinterpret_cast<uint4*>(s.aug[1] + row * 16) = zero;
     }
   }
+  grid_wait();
+  const BwdItem item0 = bwd_item(p, blockIdx.x, blockIdx.y);
+  trace_stamp(p.trace, item0.linear, 0);
+  {
+    // does this CTA read a staged block? then it first helps to empty the copy queue
+    bool waits = item0.col.kv_wait_flag != 0;
+    for (int e = item0.col.seg_begin; e < item0.col.seg_end && !waits; ++e) waits = bwd_seg(p, e).wait_flag != 0;
+    drain_stage_queue(p.stage, waits, item0.linear, &s.stage_slot);
+  }
+
+  if (threadIdx.x == 0) s.item[0] = item0;
   fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
@@ -538,6 +539,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
           if (!wait(&s.clc_full, n & 1, 104)) break;
           int bx, by;
           const bool got = clc_read(&s.clc, bx, by);
+          if (!got) grid_trigger();               // (not before: with the next kernel pending no CTA can be taken over)
           fence_proxy_async_smem();               // read before the next response may overwrite it
           if (got) it = bwd_item(p, bx, by);
           else it.exists = 0;
@@ -1109,8 +1111,7 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
     g_bwd_smem_set[dev] = 1;
   }
   dim3 grid(n_tiles * n_kv_heads, batch, 1);
-  attn_bwd_kernel<<<grid, BWD_THREADS, smem_bytes, stream>>>(p);
-  UA_CUDA(cudaGetLastError());
+  UA_CUDA(launch_kernel(attn_bwd_kernel, grid, BWD_THREADS, smem_bytes, stream, stage_flags == nullptr, p));
   return 0;
 }
 

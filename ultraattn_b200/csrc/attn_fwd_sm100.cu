@@ -460,14 +460,13 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
   const int psh = p.pack_shift;
 
   if (p.stage.flags != nullptr) {
+    grid_wait();
     // does this CTA read a staged block? then it first helps to empty the copy queue
     const FwdItem it = fwd_item<FEW>(p, blockIdx.x, blockIdx.y);
     trace_stamp(p.trace, it.linear, 0);
     bool waits = it.row.q_wait_flag != 0;
     for (int e = it.row.seg_begin; e < it.row.seg_end && !waits; ++e) waits = fwd_seg(p, e).wait_flag != 0;
     drain_stage_queue(p.stage, waits, it.linear, &s.stage_slot);
-  } else {
-    trace_stamp(p.trace, blockIdx.y * gridDim.x + blockIdx.x, 0);
   }
   // FEW: warps without a valid row have nothing to do (their scores are never read back). The
   // launch has one row tile, so the number is the same for all its items.
@@ -496,6 +495,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     mbar_init(&s.clc_full, 1);
     s.abort_flag = 0;
     fence_mbar_init();
+    grid_wait();
     item0 = fwd_item<FEW>(p, blockIdx.x, blockIdx.y);
     fwd_publish(p, item0, s.item[0]);
   }
@@ -516,6 +516,8 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     tmem_relinquish();
   }
   uint32_t tmem_base = 0;
+  grid_wait();
+  if (p.stage.flags == nullptr) trace_stamp(p.trace, blockIdx.y * gridDim.x + blockIdx.x, 0);
   if (warp == FWD_TMA_WARP) {
     __syncwarp();
     named_barrier_arrive(1, FWD_THREADS);
@@ -605,6 +607,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
           if (!wait(&s.clc_full, n & 1, 104)) break;
           int bx, by;
           const bool got = clc_read(&s.clc, bx, by);
+          if (!got) grid_trigger();               // (not before: with the next kernel pending no CTA can be taken over)
           fence_proxy_async_smem();               // read before the next response may overwrite it
           if (got) it = fwd_item<FEW>(p, bx, by);
           // the slot's previous item (n - 1) is done with
@@ -947,6 +950,8 @@ __global__ void __launch_bounds__(256)
 combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, int n_parts, int tokens, int heads,
                __nv_bfloat16* __restrict__ o, long o_row_stride, long o_batch_stride, float* __restrict__ lse,
                long lse_head_stride, long lse_batch_stride, long n_rows) {
+  grid_wait();
+  grid_trigger();
   const long r = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= n_rows) return;
@@ -1060,8 +1065,7 @@ static int launch_fwd(const FwdParams& p, int heads, int batch, cudaStream_t str
     if (dev < 64) smem_set[dev] = 1;
   }
   dim3 grid(p.n_tiles * heads, batch, 1);
-  attn_fwd_kernel<FEW><<<grid, FWD_THREADS, smem_bytes, stream>>>(p);
-  UA_CUDA(cudaGetLastError());
+  UA_CUDA(launch_kernel(attn_fwd_kernel<FEW>, grid, FWD_THREADS, smem_bytes, stream, p.stage.flags == nullptr, p));
   return 0;
 }
 
@@ -1279,10 +1283,9 @@ extern "C" int ua_attn_fwd_dense(const UaDenseFwd* t, int causal, float softmax_
   if (set_trace(p)) return -1;
   if (d.few ? launch_fwd<true>(p, d.heads, batch, stream) : launch_fwd<false>(p, d.heads, batch, stream)) return -1;
   if (d.n_parts > 0) {
-    combine_kernel<<<static_cast<unsigned>((n_rows + 7) / 8), 256, 0, stream>>>(
-        p.part_o, p.part_lse, d.n_parts, sq, n_heads, p.o_ptr[0], p.o_row_stride[0], p.o_batch_stride[0], p.lse_ptr[0],
-        p.lse_head_stride[0], p.lse_batch_stride[0], n_rows);
-    UA_CUDA(cudaGetLastError());
+    UA_CUDA(launch_kernel(combine_kernel, static_cast<unsigned>((n_rows + 7) / 8), 256, 0, stream, true, p.part_o, p.part_lse, d.n_parts,
+                          sq, n_heads, p.o_ptr[0], p.o_row_stride[0], p.o_batch_stride[0], p.lse_ptr[0], p.lse_head_stride[0],
+                          p.lse_batch_stride[0], n_rows));
   }
   return 0;
 }

@@ -126,6 +126,8 @@ __global__ void __launch_bounds__(256)
 bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ dvec,
                    float* __restrict__ dq, long o_bstride, long o_stride, long do_bstride, long do_stride, int batch,
                    int tokens, int heads) {
+  grid_wait();
+  grid_trigger();
   const int sub = threadIdx.x & 15;
   const long rid = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
   float acc = 0.f;
@@ -256,6 +258,8 @@ embedding_bwd_kernel(const long* __restrict__ order, const __nv_bfloat16* __rest
 __global__ void __launch_bounds__(256)
 cast_scale_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long n,
                   float scale, int accumulate) {
+  grid_wait();
+  grid_trigger();
   const long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i + 8 <= n) {
     const float4 a = *reinterpret_cast<const float4*>(src + i);
@@ -873,10 +877,9 @@ extern "C" int ua_bwd_prepare(const void* o, const void* d_o, float* dvec, float
   const long odd = (tokens > 1 ? o_stride | do_stride : 0) | (batch > 1 ? o_bstride | do_bstride : 0);
   const auto at = reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o) | reinterpret_cast<uintptr_t>(dq);
   if (odd % 8 != 0 || at % 16 != 0) UA_FAIL("ua_bwd_prepare: O and dO must start, and step, in multiples of 16 bytes");
-  bwd_prepare_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), dvec, dq, o_bstride, o_stride,
-      do_bstride, do_stride, batch, tokens, heads);
-  UA_CUDA(cudaGetLastError());
+  UA_CUDA(launch_kernel(bwd_prepare_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream, true,
+                        static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), dvec, dq, o_bstride, o_stride,
+                        do_bstride, do_stride, batch, tokens, heads));
   return 0;
 }
 
@@ -903,9 +906,8 @@ extern "C" int ua_cast_scale(const float* src, void* dst, long n, float scale, i
                              cudaStream_t stream) {
   if (n == 0) return 0;
   const long threads = (n + 7) / 8;
-  cast_scale_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
-      src, static_cast<__nv_bfloat16*>(dst), n, scale, accumulate);
-  UA_CUDA(cudaGetLastError());
+  UA_CUDA(launch_kernel(cast_scale_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream, true, src,
+                        static_cast<__nv_bfloat16*>(dst), n, scale, accumulate));
   return 0;
 }
 

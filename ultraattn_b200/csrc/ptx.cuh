@@ -44,6 +44,13 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Programmatic dependent launch (launch_kernel in host_common.cuh). `grid_wait`: the kernels before this one in the stream are
+// complete and their writes visible; a kernel touches global memory only behind it, and every thread passes it,
+// so that one kernel's end implies the ends of all before. `grid_trigger`: the next kernel may be set up as soon as all CTAs
+// of this one have started.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // A hardware barrier of `threads` threads, some of which only arrive.
 __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
