@@ -104,7 +104,7 @@ struct FwdParams {
   int pack_shift;      // log2 of the query heads packed into the rows of a tile (0 in table launches)
   int n_split;         // CTAs that share the keys of a tile
   float* part_o;       // not null: fp32 partial results [batch, parts, tokens, heads, 128] ...
-  float* part_lse;     // ... and [batch, parts, tokens, heads]; parts = n_split (x 2 if FEW)
+  float* part_lse;     // ... and [batch, parts, tokens, heads]; parts = n_split
   int n_parts;
   int tail_heads;      // see item_index
   int persist;         // CTAs take over further items (0: one item per CTA)
@@ -139,8 +139,9 @@ struct FwdOut {
   float* lse;
   long o_row_stride, o_batch_stride, lse_head_stride, lse_batch_stride;
 };
+template <bool FEW>
 struct FwdHot {
-  FwdOut out[ATTN_MAX_SRC];
+  FwdOut out[FEW ? 1 : ATTN_MAX_SRC];      // (FEW launches are dense: one slot)
   float* part_o;         // as in FwdParams
   float* part_lse;
   int n_parts, n_heads, pack_shift;
@@ -168,7 +169,10 @@ struct __align__(1024) FwdSmem {
   FwdWork item[2];       // item number n in slot n & 1
   uint64_t item_full[2];
   uint64_t item_empty[2];
-  FwdHot hot;
+  FwdHot<FEW> hot;
+  float2 stat[FEW ? ATTN_TILE : 1];     // sub-tile 1's reference maximum and sum per row, for sub-tile 0
+  uint64_t stat_full;    // ... and its O is complete
+  uint64_t merged;       // sub-tile 0 has read both
   uint32_t tmem_base;
   int abort_flag;
   int stage_slot;
@@ -261,14 +265,14 @@ __device__ __forceinline__ void fwd_publish(const FwdParams& p, const FwdItem& i
 // seen a key tile) normalised, merged with what is there (row.accumulate) or written as a fp32 part
 // of a split launch.
 // `ready` waits until the last product is complete; what does not depend on it comes first.
-template <bool FEW, typename Ready>
-__device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uint32_t tO, float l, float m_use, bool any, Ready ready) {
+template <typename Ready>
+__device__ __forceinline__ void fwd_epilogue(FwdSmem<false>& s, uint32_t slot, uint32_t tO, float l, float m_use, bool any, Ready ready) {
   const FwdItem& it = s.item[slot];
   const float NEG_INF = -INFINITY;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = warp >> 2, quad = warp & 3;
   const int psh = s.hot.pack_shift;
-  const int r_cta = (FEW ? 0 : w * ATTN_TILE) + quad * 32 + lane;
+  const int r_cta = w * ATTN_TILE + quad * 32 + lane;
   const int rows_here = it.rows_here;
   const bool valid_row = r_cta < rows_here;
   const int r_blk = (it.r0 + r_cta) >> psh;
@@ -300,13 +304,13 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
   const float fnew = inv * w_new;
   // fp32 part of a split launch: rows of 128 floats, [batch, parts, tokens, heads]
   const bool f32 = s.hot.part_o != nullptr;
-  const long part0 = f32 ? (static_cast<long>(it.batch) * s.hot.n_parts + (FEW ? 2 * it.split + w : it.split)) * it.row.q_len : 0;
+  const long part0 = f32 ? (static_cast<long>(it.batch) * s.hot.n_parts + it.split) * it.row.q_len : 0;
   if (f32) {
     lptr = s.hot.part_lse + (part0 + r_blk) * s.hot.n_heads + qh;
     if (any && l != l) lse = l;          // a NaN score makes the whole row one without keys (combine_kernel), not this part
   }
   if (valid_row) *lptr = lse;
-  if (!FEW && !it.row.accumulate) {
+  if (!it.row.accumulate) {
     // A thread owns a row, so storing from registers would scatter 16 bytes to each of 32 rows per
     // instruction. The warps turn their blocks of 32 rows x 128 bytes around in shared memory instead
     // (16-byte chunks swizzled by row: no bank conflicts either way) and store four whole rows of a block
@@ -314,7 +318,7 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
     // destinations in shared memory); forward (us): 512 queries behind 32768 keys 288 -> 281, 4 x 2000
     // tokens 168 -> 165, causal 8k tokens, 32 heads 508 -> 501.
     // (Without a key tile, `any` false, fnew is 0 and what tensor memory holds is not used.)
-    uint8_t* blk = s.o_stage[FEW ? 0 : warp];
+    uint8_t* blk = s.o_stage[warp];
     const int sub = lane >> 3, ch = lane & 7;                      // row of four, 16-byte chunk
     const long row_bytes = f32 ? static_cast<long>(s.hot.n_heads) * ATTN_D * 4 : od.o_row_stride * 2;
     const int head_bytes = f32 ? ATTN_D * 4 : ATTN_D * 2;
@@ -372,10 +376,9 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
     }
     return;
   }
-  // few rows, or a merge with what is there: straight from registers
+  // a merge with what is there: straight from registers
   ready();
   __nv_bfloat16* optr = od.o + it.batch * od.o_batch_stride + orow * od.o_row_stride + static_cast<long>(qh) * ATTN_D;
-  float* pptr = f32 ? s.hot.part_o + ((part0 + r_blk) * s.hot.n_heads + qh) * ATTN_D : nullptr;
 #pragma unroll 1
   for (int c = 0; c < 4; ++c) {
     uint32_t ov[32];
@@ -386,16 +389,7 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
 #pragma unroll
       for (int i = 0; i < 32; ++i) ov[i] = 0u;
     }
-    if (valid_row && pptr != nullptr) {
-      float4* d4 = reinterpret_cast<float4*>(pptr + c * 32);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float f[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 4 + i]) * fnew;
-        d4[q] = make_float4(f[0], f[1], f[2], f[3]);
-      }
-    } else if (valid_row) {
+    if (valid_row) {
       uint4* d4 = reinterpret_cast<uint4*>(optr + c * 32);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -436,6 +430,56 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<FEW>& s, uint32_t slot, uin
 // 4096 in 16k tokens 1140 -> 1090; 4 x 2000 tokens 192 -> 182; causal 8k 609 -> 588, 16k 2010 -> 1978.
 // Launches that stage peers' blocks run one item per CTA (p.persist = 0): their CTAs must be able to
 // wait for each other's copies.
+// FEW: the output of one item, of whose key tiles each sub-tile has seen half. The rows are the same, and so are their
+// lanes in tensor memory: sub-tile 0's warps take both sub-tiles' O from there, and sub-tile 1's maximum and sum
+// from shared memory, and write one result. Two fp32 parts per CTA and a launch that merged them -> this (B200, us, cold L2): 16
+// sequences of 8123 keys, one query, 32 / 8 heads 105.5 -> 103.4; 6 of 2449 keys, 16 heads 39.9 -> 36; 36 queries behind
+// 1913 keys, 8 heads 21.5 -> 19.5.
+__device__ __forceinline__ void few_epilogue(FwdSmem<true>& s, uint32_t slot, uint32_t tO, float l0, float m0) {
+  const FwdWork& it = s.item[slot];
+  const float NEG_INF = -INFINITY;
+  const int r = threadIdx.x;                                       // row = thread: warps 0-3
+  const float2 other = s.stat[r];
+  const float m = fmaxf(m0, other.x);
+  const float a0 = fast_exp2(m0 - m), a1 = fast_exp2(other.x - m);
+  const float l = (m0 > NEG_INF || l0 != l0 ? a0 * l0 : 0.f) + (other.x > NEG_INF || other.y != other.y ? a1 * other.y : 0.f);
+  const bool live = l > 0.f && m > NEG_INF, use0 = live && m0 > NEG_INF, use1 = live && other.x > NEG_INF;
+  const float lse0 = live ? (m + log2f(l)) * 0.6931471805599453f : NEG_INF;
+  const float f0 = a0 / l, f1 = a1 / l;
+  const int psh = s.hot.pack_shift;
+  const bool valid_row = r < it.rows_here, f32 = s.hot.part_o != nullptr;
+  const int tok = (it.r0 + r) >> psh, qh = it.q_head + (r & ((1 << psh) - 1));
+  const FwdOut& od = s.hot.out[0];
+  const long part = (static_cast<long>(it.batch) * s.hot.n_parts + it.split) * it.row.q_len + tok;
+  float* lptr = f32 ? s.hot.part_lse + part * s.hot.n_heads + qh : od.lse + it.batch * od.lse_batch_stride + qh * od.lse_head_stride + tok;
+  // (in a part, a NaN score is handed on: it makes the whole row one without keys, see combine_kernel)
+  if (valid_row) *lptr = f32 && l != l ? l : lse0;
+  __nv_bfloat16* optr = od.o + it.batch * od.o_batch_stride + tok * od.o_row_stride + static_cast<long>(qh) * ATTN_D;
+  float* pptr = s.hot.part_o + (part * s.hot.n_heads + qh) * ATTN_D;
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    uint32_t u[32], v[32];
+    tmem_ld_x32(tO + c * 32, u);
+    tmem_ld_x32(tO + 128 + c * 32, v);
+    tmem_wait_ld();
+    float f[32];
+    // (what tensor memory holds of a sub-tile without a key tile, or with all of its keys masked, is not used)
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      f[i] = (use0 ? __uint_as_float(u[i]) * f0 : 0.f) + (use1 ? __uint_as_float(v[i]) * f1 : 0.f);
+    if (!valid_row) continue;
+    if (f32) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        reinterpret_cast<float4*>(pptr + c * 32)[q] = make_float4(f[q * 4], f[q * 4 + 1], f[q * 4 + 2], f[q * 4 + 3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q)        // (8 bytes, as combine_kernel)
+        reinterpret_cast<uint2*>(optr + c * 32)[q] = make_uint2(pack_bf16x2(f[q * 4], f[q * 4 + 1]), pack_bf16x2(f[q * 4 + 2], f[q * 4 + 3]));
+    }
+  }
+}
+
 // The columns of a segment that query r sees are [seg_first_of, seg_end_of); both grow with r.
 __device__ __forceinline__ int seg_end_of(const AttnSeg& sg, int r) {
   return (sg.causal & SEG_UPPER) ? min(sg.len, r + sg.diag + 1) : sg.len;
@@ -492,6 +536,8 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     }
     mbar_init(&s.q_empty, 1);
     mbar_init(&s.s_free, act_warps);
+    mbar_init(&s.stat_full, act_warps);
+    mbar_init(&s.merged, act_warps);
     mbar_init(&s.clc_full, 1);
     s.abort_flag = 0;
     fence_mbar_init();
@@ -500,7 +546,7 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     fwd_publish(p, item0, s.item[0]);
   }
   if (warp == 1) {
-    if (lane < ATTN_MAX_SRC)
+    if (lane < (FEW ? 1 : ATTN_MAX_SRC))
       s.hot.out[lane] = FwdOut{p.o_ptr[lane], p.lse_ptr[lane], p.o_row_stride[lane], p.o_batch_stride[lane],
                                p.lse_head_stride[lane], p.lse_batch_stride[lane]};
     if (lane == 31) {
@@ -922,10 +968,27 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
         }
         // ---------------------------------- epilogue --------------------------------------------
         const bool any = j > (FEW ? static_cast<uint32_t>(w) : 0u);
-        fwd_epilogue<FEW>(s, n & 1, tO, l, m_use, any, [&]() {
+        auto ready = [&]() {
           if (any && ok) ok = mbar_wait_quiet(&s.pv_done[w], (cnt & 1) ^ 1, wc);
           tc_fence_after_sync();
-        });
+        };
+        if constexpr (FEW) {
+          ready();
+          if (w == 1) {
+            s.stat[r_tile] = make_float2(any ? m_use : NEG_INF, any ? l : 0.f);
+            tc_fence_before_sync();
+            mbar_arrive_warp(&s.stat_full);
+            ok = mbar_wait_quiet(&s.merged, n & 1, wc) && ok;      // (O is free for this sub-tile's next item)
+          } else {
+            ok = mbar_wait_quiet(&s.stat_full, n & 1, wc) && ok;
+            tc_fence_after_sync();
+            few_epilogue(s, n & 1, tO, any ? l : 0.f, any ? m_use : NEG_INF);
+            tc_fence_before_sync();
+            mbar_arrive_warp(&s.merged);
+          }
+        } else {
+          fwd_epilogue(s, n & 1, tO, l, m_use, any, ready);
+        }
         if (!ok) report_error_call(wc.abort_flag, wc.status, UA_ERR_MBAR_TIMEOUT, 300 + w, static_cast<int>(j));
         trace_stamp(p.trace, it.linear, 2);
         __syncwarp();                            // every lane is done reading the item
@@ -1208,7 +1271,7 @@ static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_he
     const double waves = static_cast<double>(static_cast<long>((ctas + sms - 1) / sms)) * heavy;
     const double filled = (ctas * CTA_US + total * tile_us) / sms + 0.5 * heavy;
     double us = ctas <= sms ? heavy : (waves < filled ? waves : filled);
-    const int parts = d.few ? 2 * z : (z > 1 ? z : 0);
+    const int parts = z > 1 ? z : 0;
     if (parts > 0)
       us += COMBINE_US + static_cast<double>(parts) * batch * sq * n_heads * (2.0 * ATTN_D * 4) / COMBINE_BYTES_PER_US;
     if (z == 1 || us < best) {
@@ -1217,7 +1280,7 @@ static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_he
     }
   }
   d.n_split = n_split > 0 ? (n_split < key_tiles ? n_split : key_tiles) : best_z;
-  d.n_parts = d.few ? 2 * d.n_split : (d.n_split > 1 ? d.n_split : 0);
+  d.n_parts = d.n_split > 1 ? d.n_split : 0;
   return d;
 }
 
