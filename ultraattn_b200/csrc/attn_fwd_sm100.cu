@@ -418,19 +418,19 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<false>& s, uint32_t slot, u
   }
 }
 
-// Persistent CTAs: the grid has one CTA per work item, and a CTA that is done with an item cancels one
-// that has not started yet and takes its place (cluster launch control), so that the hardware's own
-// dispatch order stays the schedule. The TMA warp runs ahead: it takes over the next item as soon as
-// the loads of this one are issued, its Q and first K / V tiles arrive while the softmax warps write
-// this item's output, and the MMA warp issues its first scores. TMEM, barriers and descriptors are
-// set up once. The producer hands an item over with what the others need of it (number of tiles, first segments), and
-// issues a CTA's first loads while tensor memory is being allocated: 512 causal tokens, 8 heads 21.3 -> 14.8 us,
-// 12 documents in 16k tokens 406 -> 365. One item per CTA -> this (B200, us): 64
-// sequences of 512 keys, one query, 32 heads 184 -> 143; 12 documents in 16k tokens 599 -> 546; window
-// 4096 in 16k tokens 1140 -> 1090; 4 x 2000 tokens 192 -> 182; causal 8k 609 -> 588, 16k 2010 -> 1978.
-// Launches that stage peers' blocks run one item per CTA (p.persist = 0): their CTAs must be able to
-// wait for each other's copies.
-// FEW: the output of one item, of whose key tiles each sub-tile has seen half. The rows are the same, and so are their
+// One step of a transpose of 16-byte pieces over lanes: of the pair (a, b), a lane with `odd` gives a for its partner's b.
+template <int XOR>
+__device__ __forceinline__ void swap_pieces(uint4& a, uint4& b, int odd) {
+  uint4 x = odd ? a : b;
+  x.x = __shfl_xor_sync(0xFFFFFFFFu, x.x, XOR);
+  x.y = __shfl_xor_sync(0xFFFFFFFFu, x.y, XOR);
+  x.z = __shfl_xor_sync(0xFFFFFFFFu, x.z, XOR);
+  x.w = __shfl_xor_sync(0xFFFFFFFFu, x.w, XOR);
+  if (odd) a = x;
+  else b = x;
+}
+
+// FEW: the output of one item of up to 128 rows, of whose key tiles each sub-tile has seen half. The rows are the same, and so are their
 // lanes in tensor memory: sub-tile 0's warps take both sub-tiles' O from there, and sub-tile 1's maximum and sum
 // from shared memory, and write one result. Two fp32 parts per CTA and a launch that merged them -> this (B200, us, cold L2): 16
 // sequences of 8123 keys, one query, 32 / 8 heads 105.5 -> 103.4; 6 of 2449 keys, 16 heads 39.9 -> 36; 36 queries behind
@@ -454,19 +454,55 @@ __device__ __forceinline__ void few_epilogue(FwdSmem<true>& s, uint32_t slot, ui
   float* lptr = f32 ? s.hot.part_lse + part * s.hot.n_heads + qh : od.lse + it.batch * od.lse_batch_stride + qh * od.lse_head_stride + tok;
   // (in a part, a NaN score is handed on: it makes the whole row one without keys, see combine_kernel)
   if (valid_row) *lptr = f32 && l != l ? l : lse0;
-  __nv_bfloat16* optr = od.o + it.batch * od.o_batch_stride + tok * od.o_row_stride + static_cast<long>(qh) * ATTN_D;
+  __nv_bfloat16* obase = od.o + it.batch * od.o_batch_stride;
+  __nv_bfloat16* optr = obase + tok * od.o_row_stride + static_cast<long>(qh) * ATTN_D;
   float* pptr = s.hot.part_o + (part * s.hot.n_heads + qh) * ATTN_D;
-#pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
+  // (what tensor memory holds of a sub-tile without a key tile, or with all of its keys masked, is not used)
+  const auto columns = [&](int c, float (&f)[32]) {
     uint32_t u[32], v[32];
     tmem_ld_x32(tO + c * 32, u);
     tmem_ld_x32(tO + 128 + c * 32, v);
     tmem_wait_ld();
-    float f[32];
-    // (what tensor memory holds of a sub-tile without a key tile, or with all of its keys masked, is not used)
 #pragma unroll
     for (int i = 0; i < 32; ++i)
       f[i] = (use0 ? __uint_as_float(u[i]) * f0 : 0.f) + (use1 ? __uint_as_float(v[i]) * f1 : 0.f);
+  };
+  // Many rows: four lanes exchange their rows' 16-byte pieces, so that a store covers 64 bytes of each of eight rows (8 of
+  // each of 32 otherwise, a quarter of a sector). Causal 1000 tokens, 8 heads 16.0 -> 15.2 us; with the 4 rows of a decode
+  // step it cost 0.3 to 1.4 us instead (2 x 600 keys 11.6 -> 12.3).
+  if (!f32 && it.rows_here > 32 && ((reinterpret_cast<uintptr_t>(obase) | (od.o_row_stride * 2)) & 15) == 0) {
+    const int lane4 = r & 3;
+    __nv_bfloat16* dst[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int rr = r - lane4 + k;
+      dst[k] = rr < it.rows_here ? obase + static_cast<long>((it.r0 + rr) >> psh) * od.o_row_stride +
+                                       static_cast<long>(it.q_head + (rr & ((1 << psh) - 1))) * ATTN_D + lane4 * 8
+                                 : nullptr;
+    }
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      float f[32];
+      columns(c, f);
+      uint4 u4[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        u4[q] = make_uint4(pack_bf16x2(f[q * 8], f[q * 8 + 1]), pack_bf16x2(f[q * 8 + 2], f[q * 8 + 3]), pack_bf16x2(f[q * 8 + 4], f[q * 8 + 5]),
+                           pack_bf16x2(f[q * 8 + 6], f[q * 8 + 7]));
+      swap_pieces<1>(u4[0], u4[1], lane4 & 1);
+      swap_pieces<1>(u4[2], u4[3], lane4 & 1);
+      swap_pieces<2>(u4[0], u4[2], lane4 >> 1);
+      swap_pieces<2>(u4[1], u4[3], lane4 >> 1);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (dst[k] != nullptr) *reinterpret_cast<uint4*>(dst[k] + c * 32) = u4[k];
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    float f[32];
+    columns(c, f);
     if (!valid_row) continue;
     if (f32) {
 #pragma unroll
@@ -492,6 +528,18 @@ __device__ __forceinline__ int seg_first_of(const AttnSeg& sg, int r) {
 // (16k tokens, 8 heads: 1038 us without, 917 with).
 #define PIN if (__builtin_expect(cnt == 0xFFFFFFFFu, 0)) break;
 
+// Persistent CTAs: the grid has one CTA per work item, and a CTA that is done with an item cancels one
+// that has not started yet and takes its place (cluster launch control), so that the hardware's own
+// dispatch order stays the schedule. The TMA warp runs ahead: it takes over the next item as soon as
+// the loads of this one are issued, its Q and first K / V tiles arrive while the softmax warps write
+// this item's output, and the MMA warp issues its first scores. TMEM, barriers and descriptors are
+// set up once. The producer hands an item over with what the others need of it (number of tiles, first segments), and
+// issues a CTA's first loads while tensor memory is being allocated: 512 causal tokens, 8 heads 21.3 -> 14.8 us,
+// 12 documents in 16k tokens 406 -> 365. One item per CTA -> this (B200, us): 64
+// sequences of 512 keys, one query, 32 heads 184 -> 143; 12 documents in 16k tokens 599 -> 546; window
+// 4096 in 16k tokens 1140 -> 1090; 4 x 2000 tokens 192 -> 182; causal 8k 609 -> 588, 16k 2010 -> 1978.
+// Launches that stage peers' blocks run one item per CTA (p.persist = 0): their CTAs must be able to
+// wait for each other's copies.
 template <bool FEW>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ FwdParams p) {
@@ -1205,6 +1253,7 @@ constexpr int FEW_MIN_KEY_TILES = 4;
 constexpr int MAX_SPLIT = 64;
 constexpr double TILE_US = 1.9;               // one 128-key tile of a 256-row CTA
 constexpr double CTA_US = 6.0;                // start, first loads, epilogue
+constexpr double FEW_FULL_TILE_US = 1.3;      // one 128-key tile of a FEW CTA with 128 rows
 constexpr double FEW_TILE_US = 0.75;          // one 128-key tile of a FEW CTA that has the memory to itself
 constexpr double FEW_BYTES_PER_US = 6.5e6;
 constexpr double COMBINE_US = 3.0;
@@ -1281,6 +1330,19 @@ static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_he
   }
   d.n_split = n_split > 0 ? (n_split < key_tiles ? n_split : key_tiles) : best_z;
   d.n_parts = d.n_split > 1 ? d.n_split : 0;
+  // Few items leave SMs idle, and the launch lasts as long as its longest item, whose two sub-tiles go through all keys. With
+  // items of 128 rows each sub-tile takes half of them: 1.0 us per key tile for 1.5 us (the issuing warp has one chain
+  // less to overlap with, so a launch that fills the device is slower that way: 1000 causal tokens, 32 heads over 8, 19.7 ->
+  // 21.1 us, and the rule asks for items that all run at once). It beats splitting too, unless the parts are many. Before -> now (B200,
+  // us): causal 1000 tokens, 8 heads 19.1 -> 15.1; 512 13.4 -> 11.2; 2000 tokens, 8 over 2 28.7 -> 23.6; 1000 tokens,
+  // 8 heads, not causal 18.7 -> 15.6. Left as it was: 512 of 2000 tokens, 8 heads (5 parts) 19.1, this 22.8; up to 3 tiles, equal.
+  const int few_q_tiles = static_cast<int>((rows + ATTN_TILE - 1) / ATTN_TILE);
+  if (!d.few && n_split == 0 && key_tiles >= FEW_MIN_KEY_TILES && few_q_tiles * per_head <= sms && CTA_US + key_tiles * FEW_FULL_TILE_US < best) {
+    d.few = true;
+    d.q_tiles = few_q_tiles;
+    d.n_split = 1;
+    d.n_parts = 0;
+  }
   return d;
 }
 
