@@ -7,6 +7,7 @@ import torch
 
 import ultraattn_b200 as ua
 from ultraattn_b200 import patterns as P
+from ultraattn_b200.api import local_backward
 from ultraattn_b200.ops import attention as A
 from ultraattn_b200.ops.flash_compat import flash_attn_func
 
@@ -85,6 +86,19 @@ def test_the_same_tensors_are_refused(monkeypatch):
                     (bf, bf.float(), bf)):
         a, b = _both(monkeypatch, lambda: flash_attn_func(q, k, v))
         assert a == b and isinstance(a[0], type)
+
+
+@pytest.mark.parametrize("B,Bk,Bv", [(2, 1, 1), (2, 2, 1), (2, 1, 2)])
+def test_missing_sequences_are_refused(B, Bk, Bv, monkeypatch):
+    """(on the host: without keys of a sequence its output would be zeros, and its gradients would be written behind dK and dV)"""
+    q, k, v = _rand(B, 300, 4, 128), _rand(Bk, 300, 2, 128, seed=1), _rand(Bv, 300, 2, 128, seed=2)
+    for f in (lambda: flash_attn_func(q, k, v), lambda: ua.attention(q, k, v, P.causal(1)), lambda: ua.attention(q, k, v, P.causal(2))):
+        a, b = _both(monkeypatch, f)
+        monkeypatch.undo()
+        assert a == b and a[0] is RuntimeError and "sequences" in a[1]
+    o, lse = torch.zeros_like(q), torch.zeros(B, 4, 300, device="cuda")
+    with pytest.raises((RuntimeError, AssertionError), match="sequences|no room for every key"):
+        local_backward(q, k, v, o, lse, q, None, dense=1)
 
 
 class _Sub(torch.Tensor):

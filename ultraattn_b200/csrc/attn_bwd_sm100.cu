@@ -1024,6 +1024,8 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
     UA_FAIL("ua_attn_bwd: too many sources (max %d)", ATTN_MAX_SRC);
   if (dense) n_tiles = static_cast<int>((k_src[0].tokens + ATTN_TILE - 1) / ATTN_TILE);
   if (n_tiles <= 0) return 0;
+  if (check_sources("ua_attn_bwd", batch, n_heads, n_kv_heads, q_src, n_q, k_src, v_src, n_kv)) return -1;
+  if (dense && v_src[0].tokens < k_src[0].tokens) UA_FAIL("ua_attn_bwd: %ld values for %ld keys", v_src[0].tokens, k_src[0].tokens);
   BwdParams p;
   memset(&p, 0, sizeof(p));
   for (int i = 0; i < n_q; ++i) {
@@ -1140,6 +1142,11 @@ struct UaLocalBwd {
 
 extern "C" int ua_attn_bwd_local(const UaLocalBwd* t, float softmax_scale, int* status, cudaStream_t stream) {
   const long batch = t->q.batch, tokens = t->q.tokens, heads = t->q.heads;
+  if (check_sources("ua_attn_bwd_local", batch, heads, t->k.heads, &t->q, 1, &t->k, &t->v, 1)) return -1;
+  // (dK and dV are as large as K and V: the launch has to write all of them)
+  if (t->k.batch != batch || t->v.batch != batch)
+    UA_FAIL("ua_attn_bwd_local: keys / values of %ld / %ld sequences for %ld of queries", t->k.batch, t->v.batch, batch);
+  if (t->dense && t->v.tokens < t->k.tokens) UA_FAIL("ua_attn_bwd_local: %ld values for %ld keys", t->v.tokens, t->k.tokens);
   if (ua_bwd_prepare(t->o, t->d_o.ptr, t->dvec, t->dq32, t->o_batch_stride, t->o_row_stride, t->d_o.batch_stride,
                      t->d_o.token_stride, static_cast<int>(batch), static_cast<int>(tokens), static_cast<int>(heads), stream))
     return -1;

@@ -1201,6 +1201,7 @@ extern "C" int ua_attn_fwd(const UaTensorSrc* q_src, int n_q, const UaTensorSrc*
   if (n_q > ATTN_MAX_SRC || n_kv > ATTN_MAX_SRC || n_out > ATTN_MAX_SRC)
     UA_FAIL("ua_attn_fwd: too many sources (max %d)", ATTN_MAX_SRC);
   if (n_tiles <= 0) return 0;
+  if (check_sources("ua_attn_fwd", batch, n_heads, n_kv_heads, q_src, n_q, k_src, v_src, n_kv)) return -1;
   FwdParams p;
   memset(&p, 0, sizeof(p));
   for (int i = 0; i < n_q; ++i)
@@ -1370,8 +1371,8 @@ extern "C" int ua_attn_fwd_dense(const UaDenseFwd* t, int causal, float softmax_
   const int batch = static_cast<int>(q->batch), sq = static_cast<int>(q->tokens), skv = static_cast<int>(k->tokens);
   const int n_heads = static_cast<int>(q->heads), n_kv_heads = static_cast<int>(k->heads);
   if (sq <= 0 || batch <= 0) return 0;
-  if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0)
-    UA_FAIL("ua_attn_fwd_dense: %d query heads do not divide into %d key/value heads", n_heads, n_kv_heads);
+  if (check_sources("ua_attn_fwd_dense", batch, n_heads, n_kv_heads, q, 1, k, v, 1)) return -1;
+  if (v->tokens < skv) UA_FAIL("ua_attn_fwd_dense: %ld values for %d keys", v->tokens, skv);
   const DensePlan d = plan_dense(batch, sq, skv, n_heads, n_kv_heads, causal, n_split, sm_count());
   if (d.n_parts > 0 && workspace == nullptr) UA_FAIL("ua_attn_fwd_dense: a split launch needs a workspace");
   FwdParams p;

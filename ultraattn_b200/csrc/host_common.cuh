@@ -47,6 +47,26 @@ inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, unsigned threa
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// What a launch over `batch` sequences reads has to be there. TMA returns zeros behind the end of a source, so
+// that a missing sequence or head would come out as zeros; and gradients are laid out like the keys, so that they would be
+// written behind their end.
+template <typename Src>
+inline int check_sources(const char* what, long batch, long heads, long kv_heads, const Src* q, int n_q, const Src* k,
+                         const Src* v, int n_kv) {
+  if (kv_heads <= 0 || heads % kv_heads != 0)
+    UA_FAIL("%s: %ld query heads do not divide into %ld key/value heads", what, heads, kv_heads);
+  for (int i = 0; i < n_q; ++i)
+    if (q[i].batch < batch || q[i].heads < heads)
+      UA_FAIL("%s: source %d has %ld sequences of %ld query heads, the launch %ld of %ld", what, i, q[i].batch, q[i].heads, batch, heads);
+  for (int i = 0; i < n_kv; ++i) {
+    if (k[i].batch < batch || v[i].batch < batch)
+      UA_FAIL("%s: keys / values of %ld / %ld sequences for %ld of queries", what, k[i].batch, v[i].batch, batch);
+    if (k[i].heads < kv_heads || v[i].heads < kv_heads)
+      UA_FAIL("%s: %ld / %ld heads of keys / values, not %ld", what, k[i].heads, v[i].heads, kv_heads);
+  }
+  return 0;
+}
+
 // Trace buffers registered by ua_set_kernel_trace: [0 = forward, 1 = backward][device].
 struct TraceSlot {
   unsigned long long* buf;
