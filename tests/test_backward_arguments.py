@@ -48,6 +48,23 @@ def test_one_call_backward_refuses_other_shapes(calls):
     assert len(calls) == 1
 
 
+def test_one_call_backward_refuses_plans_that_write_behind_the_gradients(calls, monkeypatch):
+    """A block pattern over more queries than keys; documents that end behind the buffer, also where the numbers of
+    tokens agree."""
+    from ultraattn_b200 import api, patterns as P
+    monkeypatch.setattr(A, "_native", lambda *t: True)
+    monkeypatch.setattr(_lib, "host", lambda: pytest.fail("the native route was taken"), raising=False)
+    shapes = dict(k=_bf16(1, 32, 2, 128), v=_bf16(1, 32, 2, 128), dk=_bf16(1, 32, 2, 128), dv=_bf16(1, 32, 2, 128))
+    t = dict(q=_bf16(1, 64, 4, 128), o=_bf16(1, 64, 4, 128), lse=torch.zeros(1, 4, 64), d_o=_bf16(1, 64, 4, 128))
+    for plan in (api.local_plans(P.causal(2), 64, "cpu")[1], api.varlen_plans([32, 64], True, "cpu")[1]):
+        with pytest.raises(AssertionError, match="behind the end"):
+            A.attn_bwd_local(plan=plan, dq=_bf16(1, 64, 4, 128), **t, **shapes)
+        assert A.local_backward(t["q"], shapes["k"], shapes["v"], t["o"], t["lse"], t["d_o"], plan) is None
+    fits = api.varlen_plans([0, 32], True, "cpu")[1]
+    A.attn_bwd_local(plan=fits, dq=_bf16(1, 64, 4, 128), **t, **shapes)
+    assert len(calls) == 1
+
+
 def test_returned_row_products_do_not_keep_the_workspace(calls):
     d = _local()
     assert d.shape == (1, 4, 64) and d.untyped_storage().nbytes() == 4 * d.numel()

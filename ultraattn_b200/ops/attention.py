@@ -414,7 +414,7 @@ def dense_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: boo
 def local_backward(q, k, v, o, lse, d_o, plan: "BwdPlan | None", dense: int = 0, softmax_scale=None):
     """(dQ, dK, dV) of :func:`attn_bwd_local`, in new tensors; None: not for these (see there). A plan has to write
     the gradient of every key."""
-    if not _native(q, k, v, o, lse, d_o):
+    if not _native(q, k, v, o, lse, d_o) or (not dense and plan.kv_end > k.shape[1]):
         return None
     tables = (0, 0, 0, 0) if dense else (plan.cols_t.data_ptr(), plan.segs_t.data_ptr(), plan.tiles_t.data_ptr(), plan.n_tiles)
     r = _lib.host().local_backward(q, k, v, o, lse, d_o, *tables, dense, 0 if dense else int(plan.skewed),
@@ -569,7 +569,8 @@ class BwdPlan:
                 tiles.append((_col_steps(c, t * TILE), ci, t))
         tiles = _launch_order(tiles)
         self.n_tiles = len(tiles)
-        self.kv_tokens = sum(c.kv_len for c in self.cols)      # gradient rows that the columns write
+        self.kv_tokens = sum(c.kv_len for c in self.cols)      # gradient rows that the columns write ...
+        self.kv_end = max((c.g_start + c.kv_len for c in self.cols), default=0)      # ... and where the last of them ends
         # (causal blocks: heaviest tile twice the average, strided ones 1.8; global + local 9, star and streaming 12 to 20)
         self.skewed = bool(tiles) and max(t[0] for t in tiles) * len(tiles) > 3 * sum(t[0] for t in tiles)
         self.total_steps = sum(c for c, _, _ in tiles)
@@ -724,6 +725,7 @@ def attn_bwd_local(q, k, v, o, lse, d_o, dq, dk, dv, plan: BwdPlan | None, dense
     # (the library takes the strides of lse, and how far dK / dV are written, from the shapes of q and k)
     assert lse.shape == (B, H, S), f"lse must be [batch, heads, tokens] of the queries {(B, H, S)}, not {tuple(lse.shape)}"
     assert all(n >= m for g in (dk, dv) for n, m in zip(g.shape, k.shape)), "dK / dV have no room for every key"
+    assert dense or plan.kv_end <= min(dk.shape[1], dv.shape[1]), "the plan has keys behind the end of dK / dV"
     assert o.shape == q.shape == d_o.shape == dq.shape and o.dtype == dq.dtype == dk.dtype == dv.dtype == torch.bfloat16
     so, sk, sv = _row_strides(o), _row_strides(dk), _row_strides(dv)
     _row_strides(d_o)
