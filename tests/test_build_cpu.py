@@ -1,9 +1,12 @@
 """The build: what an installed package brings along, and what happens without the optional parts."""
 import fnmatch
+import sysconfig
 import tomllib
 from pathlib import Path
 
-from ultraattn_b200 import build
+import pytest
+
+from ultraattn_b200 import _lib, build
 
 ROOT = Path(build.__file__).resolve().parents[1]
 
@@ -13,3 +16,53 @@ def test_an_installed_package_brings_every_source():
     files = [f"csrc/{f.name}" for f in build.CSRC.iterdir() if f.is_file()]
     assert len(files) > 10
     assert [f for f in files if not any(fnmatch.fnmatch(f, g) for g in globs)] == []
+
+
+@pytest.fixture
+def host_dir(monkeypatch, tmp_path):
+    _lib.load()
+    monkeypatch.setattr(build, "HOST_PATH", tmp_path / "ua_host.so")
+    monkeypatch.setattr(_lib, "_host", [])
+    return tmp_path
+
+
+def test_without_a_compiler_the_library_is_enough(host_dir, monkeypatch):
+    """The host extension is left out with a warning, once, and calls go through Python."""
+    monkeypatch.setenv("CXX", "no-such-compiler")
+    lib = _lib.load()
+    assert build._host_needs_build()
+    with pytest.warns(UserWarning, match="through Python"):
+        assert build.build_all() == build.LIB_PATH
+    assert not build._host_needs_build() and build.host_path() is None
+    assert _lib.host() is None and _lib.load() is lib
+    monkeypatch.setattr(build, "_host_tools", lambda: "a compiler has been installed")
+    assert build._host_needs_build()
+
+
+def test_an_extension_that_does_not_load_is_left_out(host_dir):
+    build.HOST_PATH.write_bytes(b"not a shared object")
+    build._host_stamp().write_text(build.host_digest())
+    with pytest.warns(UserWarning, match="through Python"):
+        assert _lib.host() is None
+
+
+def test_an_explicit_library_is_used_alone(host_dir, monkeypatch):
+    monkeypatch.setattr(build, "host_path", lambda: pytest.fail("looked for the extension of another library"))
+    monkeypatch.setenv("UA_LIB_PATH", str(build.LIB_PATH))
+    assert _lib.host() is None
+
+
+def test_an_extension_belongs_to_its_interpreter_flags_and_sources(host_dir, monkeypatch):
+    build.HOST_PATH.write_bytes(b"")
+    build._host_stamp().write_text(build.host_digest())
+    assert build.host_path() == build.HOST_PATH
+    get = sysconfig.get_config_var
+    for change in (lambda m: m.setattr(sysconfig, "get_config_var", lambda n: "cpython-399" if n == "SOABI" else get(n)),
+                   lambda m: m.setattr(build, "HOST_FLAGS", [*build.HOST_FLAGS, "-g"]), lambda m: m.setenv("CXX", "clang++"),
+                   lambda m: m.setattr(build, "_torch_dir", lambda: host_dir)):
+        (host_dir / "version.py").write_text("another PyTorch")
+        with monkeypatch.context() as m:
+            change(m)
+            assert build.host_path() is None
+    assert build.host_path() == build.HOST_PATH
+    assert build.source_digest() == build.STAMP_PATH.read_text().strip()          # (the kernel library depends on none of it)

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import ultraattn_b200 as ua
+from ultraattn_b200 import _lib
 from ultraattn_b200 import patterns as P
 from ultraattn_b200.api import local_backward
 from ultraattn_b200.ops import attention as A
@@ -99,6 +100,19 @@ def test_missing_sequences_are_refused(B, Bk, Bv, monkeypatch):
     o, lse = torch.zeros_like(q), torch.zeros(B, 4, 300, device="cuda")
     with pytest.raises((RuntimeError, AssertionError), match="sequences|no room for every key"):
         local_backward(q, k, v, o, lse, q, None, dense=1)
+
+
+def test_without_the_extension_calls_go_through_python(monkeypatch):
+    q, k, v = (_rand(1, 200, 2, 128, seed=i).requires_grad_() for i in range(3))
+    d_o = _rand(1, 200, 2, 128, seed=5)
+    out = []
+    for missing in (False, True):
+        if missing:
+            monkeypatch.setattr(_lib, "_host", [None])
+        o = flash_attn_func(q, k, v, causal=True)
+        out.append((o, *torch.autograd.grad(o, (q, k, v), d_o)))
+    A.check_status()
+    assert all(torch.equal(x, y) for i, (x, y) in enumerate(zip(*out)) if i != 1)          # (dQ is summed in arrival order)
 
 
 class _Sub(torch.Tensor):

@@ -13,7 +13,7 @@ from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_long, c_void_
 from . import build as _build
 
 _lib = None
-_host = None
+_host = []          # [the host extension, or None], once it has been looked for
 LAUNCHES = [0]      # kernels of this library launched so far (every wrapper reports here)
 
 
@@ -112,22 +112,31 @@ def load():
 
 
 def host():
-    """The native host part of single-device calls (csrc/host_ext.cpp), with the library's entry points."""
-    global _host
-    if _host is None:
-        import importlib.machinery
-        import importlib.util
-        import torch  # noqa: F401  (the extension's libraries)
+    """The native host part of single-device calls (csrc/host_ext.cpp), with the library's entry points. None: it could
+    not be built or loaded, or an explicit library is in use, whose argument blocks need not be those it was compiled
+    for; callers then go through Python."""
+    if not _host:
         lib = load()
-        path = str(_build.HOST_PATH)
-        loader = importlib.machinery.ExtensionFileLoader("ua_host", path)
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ua_host", path, loader=loader))
-        loader.exec_module(mod)
-        address = lambda name: ctypes.cast(getattr(lib, name), c_void_p).value
-        mod.init(address("ua_attn_fwd_dense_parts"), address("ua_attn_fwd_dense"), address("ua_attn_bwd_local"),
-                 address("ua_last_error"))
-        _host = mod
-    return _host
+        path = None if os.environ.get("UA_LIB_PATH") else _build.host_path()
+        mod = None
+        if path is not None:
+            import importlib.machinery
+            import importlib.util
+            import torch  # noqa: F401  (the extension's libraries)
+            loader = importlib.machinery.ExtensionFileLoader("ua_host", str(path))
+            try:
+                mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ua_host", str(path), loader=loader))
+                loader.exec_module(mod)
+            except ImportError as e:
+                import warnings
+                warnings.warn(f"ultraattn_b200: the host extension cannot be loaded; calls go through Python instead. {e}")
+                mod = None
+        if mod is not None:
+            address = lambda name: ctypes.cast(getattr(lib, name), c_void_p).value
+            mod.init(address("ua_attn_fwd_dense_parts"), address("ua_attn_fwd_dense"), address("ua_attn_bwd_local"),
+                     address("ua_last_error"))
+        _host.append(mod)
+    return _host[0]
 
 
 def stream_of(t) -> int:

@@ -393,8 +393,9 @@ _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
 def _native(*tensors) -> bool:
-    """Plain CUDA tensors, no debug mode: the native host part (csrc/host_ext.cpp) may be asked."""
-    return tensors[0].is_cuda and all(type(t) in _PLAIN for t in tensors) and not debug_bounds_enabled()
+    """Plain CUDA tensors, no debug mode, and the native host part (csrc/host_ext.cpp) is there: it may be asked."""
+    return (tensors[0].is_cuda and all(type(t) in _PLAIN for t in tensors) and not debug_bounds_enabled()
+            and _lib.host() is not None)
 
 
 def dense_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool, softmax_scale: float | None = None):
