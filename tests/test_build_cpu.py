@@ -1,5 +1,7 @@
 """The build: what an installed package brings along, and what happens without the optional parts."""
+import ctypes
 import fnmatch
+import re
 import sysconfig
 import tomllib
 from pathlib import Path
@@ -7,6 +9,7 @@ from pathlib import Path
 import pytest
 
 from ultraattn_b200 import _lib, build
+from ultraattn_b200.ops import attention as A
 
 ROOT = Path(build.__file__).resolve().parents[1]
 
@@ -66,3 +69,19 @@ def test_an_extension_belongs_to_its_interpreter_flags_and_sources(host_dir, mon
             assert build.host_path() is None
     assert build.host_path() == build.HOST_PATH
     assert build.source_digest() == build.STAMP_PATH.read_text().strip()          # (the kernel library depends on none of it)
+
+
+def test_argument_blocks_of_python_are_those_of_the_header():
+    text = re.sub(r"//.*", "", (build.CSRC / "arg_blocks.h").read_text())
+    fields = {}
+    for name, body in re.findall(r"struct (\w+) \{(.*?)\n\};", text, re.S):
+        fields[name] = []
+        for kind, names in re.findall(r"([\w ]+\**)[ ]((?:\*?\w+(?:, )?)+);", body):
+            for n in names.split(", "):
+                inner = fields.get(kind.strip(), [""])
+                fields[name] += [f"{n.lstrip('*')}.{i}".rstrip(".") for i in inner]
+    for mirror in (_lib.UaTensorSrc, _lib.UaOutDst):
+        assert [n for n, _ in mirror._fields_] == fields[mirror.__name__] and all(ctypes.sizeof(t) == 8 for _, t in mirror._fields_)
+    assert A._DENSE_FWD.size == 8 * len(fields["UaDenseFwd"]) and A._LOCAL_BWD.size == 8 * len(fields["UaLocalBwd"])
+    assert fields["UaLocalBwd"][28:] == ("o o_row_stride o_batch_stride lse dvec dq32 dq dk dv dkv_row_stride dkv_batch_stride cols segs "
+                                         "tiles n_tiles dense skewed").split()          # (attn_bwd_local packs them in this order)

@@ -46,6 +46,7 @@
 // dK/dV leave the CTA either as bf16 stores (the CTA is their only producer) or as fp32
 // red.add into an accumulator that may live in a peer GPU's memory (partial gradients of a
 // key/value block computed away from its owner).
+#include "arg_blocks.h"
 #include "attn_common.cuh"
 #include "host_common.cuh"
 #include "ptx.cuh"
@@ -969,15 +970,6 @@ extern "C" int ua_bwd_prof_read(long long* host64) {
 }
 #endif
 
-struct UaTensorSrc {
-  const void* ptr;
-  long tokens;
-  long heads;
-  long batch;
-  long token_stride;
-  long head_stride;
-  long batch_stride;
-};
 // query-side extras of one source
 struct UaBwdQSide {
   const float* lse;        // [batch, heads, tokens]
@@ -1122,23 +1114,6 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
 extern "C" int ua_bwd_prepare(const void* o, const void* d_o, float* dvec, float* dq, long o_bstride, long o_stride,
                               long do_bstride, long do_stride, int batch, int tokens, int heads, cudaStream_t stream);
 extern "C" int ua_cast_scale(const float* src, void* dst, long n, float scale, int accumulate, cudaStream_t stream);
-
-struct UaLocalBwd {
-  UaTensorSrc q, k, v, d_o;
-  const void* o;
-  long o_row_stride, o_batch_stride;
-  const float* lse;              // [batch, heads, tokens], contiguous; dvec alike
-  float* dvec;
-  float* dq32;                   // [batch, tokens, heads, 128] workspace
-  void* dq;                      // bf16, contiguous
-  void* dk;                      // bf16
-  void* dv;
-  long dkv_row_stride, dkv_batch_stride;
-  const void* cols;              // tables as in ua_attn_bwd, not read if dense
-  const void* segs;
-  const void* tiles;
-  long n_tiles, dense, skewed;
-};
 
 extern "C" int ua_attn_bwd_local(const UaLocalBwd* t, float softmax_scale, int* status, cudaStream_t stream) {
   const long batch = t->q.batch, tokens = t->q.tokens, heads = t->q.heads;

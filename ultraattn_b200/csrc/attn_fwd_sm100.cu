@@ -33,6 +33,7 @@
 //     key/value head and not once per query head;
 //   * split the keys over several CTAs when the rows alone leave SMs idle: every part writes its
 //     normalised fp32 O and lse, and combine_kernel merges them (see plan_dense).
+#include "arg_blocks.h"
 #include "attn_common.cuh"
 #include "host_common.cuh"
 #include "ptx.cuh"
@@ -1134,26 +1135,6 @@ extern "C" int ua_fwd_prof_read(long long* host64) {
 }
 #endif
 
-// Host-side description of one tensor source: [batch, tokens, heads, 128] bf16 with the given
-// strides (elements).
-struct UaTensorSrc {
-  const void* ptr;
-  long tokens;
-  long heads;
-  long batch;
-  long token_stride;
-  long head_stride;
-  long batch_stride;
-};
-struct UaOutDst {
-  void* o_ptr;
-  float* lse_ptr;
-  long o_row_stride;
-  long o_batch_stride;
-  long lse_head_stride;
-  long lse_batch_stride;
-};
-
 // rows_head / rows_tok: heads and tokens per 128-row tile (1 x 128, or a packed group of heads)
 static int encode_src(CUtensorMap* tm, const UaTensorSrc& t, uint32_t rows_head = 1) {
   uint64_t dims[4] = {ATTN_D, static_cast<uint64_t>(t.heads), static_cast<uint64_t>(t.tokens),
@@ -1355,12 +1336,6 @@ extern "C" int ua_attn_fwd_dense_parts(int batch, int sq, int skv, int n_heads, 
   if (batch <= 0 || sq <= 0 || skv <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return 0;
   return plan_dense(batch, sq, skv, n_heads, n_kv_heads, causal, n_split, sm_count()).n_parts;
 }
-
-// The tensors of a dense launch in one block, so that a caller marshals one argument.
-struct UaDenseFwd {
-  UaTensorSrc q, k, v;
-  UaOutDst out;
-};
 
 // All queries of `q` against all keys: O and lse of softmax(scale Q K^T) V; causal: key c is visible
 // to query r iff c <= r + skv - sq.

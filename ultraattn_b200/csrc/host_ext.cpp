@@ -10,35 +10,13 @@
 #include <ATen/ATen.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include "arg_blocks.h"
+
 namespace {
 
-// struct UaTensorSrc, UaDenseFwd and UaLocalBwd of the kernel library
-struct Src {
-  const void* ptr;
-  long tokens, heads, batch, token_stride, head_stride, batch_stride;
-};
-struct DenseFwd {
-  Src q, k, v;
-  void* o;
-  float* lse;
-  long o_row_stride, o_batch_stride, lse_head_stride, lse_batch_stride;
-};
-struct LocalBwd {
-  Src q, k, v, d_o;
-  const void* o;
-  long o_row_stride, o_batch_stride;
-  const float* lse;
-  float *dvec, *dq32;
-  void *dq, *dk, *dv;
-  long dkv_row_stride, dkv_batch_stride;
-  const void *cols, *segs, *tiles;
-  long n_tiles, dense, skewed;
-};
-static_assert(sizeof(DenseFwd) == 27 * 8 && sizeof(LocalBwd) == 45 * 8, "layout of the library's argument blocks");
-
 int (*fwd_dense_parts)(int, int, int, int, int, int, int);
-int (*fwd_dense)(const DenseFwd*, int, float, int, float*, int*, void*);
-int (*bwd_local)(const LocalBwd*, float, int*, void*);
+int (*fwd_dense)(const UaDenseFwd*, int, float, int, float*, int*, void*);
+int (*bwd_local)(const UaLocalBwd*, float, int*, void*);
 const char* (*last_error)();
 
 void init(uintptr_t parts, uintptr_t dense, uintptr_t local, uintptr_t error) {
@@ -57,8 +35,8 @@ bool takes(const at::Tensor& t, const at::Device& dev) {
 // ... whose heads lie side by side (an axis of one may have any stride)
 bool takes_rows(const at::Tensor& t, const at::Device& dev) { return takes(t, dev) && (t.stride(2) == D || t.size(2) == 1); }
 
-Src src(const at::Tensor& t) {
-  return Src{t.data_ptr(), t.size(1), t.size(2), t.size(0), t.stride(1), t.stride(2), t.stride(0)};
+UaTensorSrc src(const at::Tensor& t) {
+  return UaTensorSrc{t.data_ptr(), t.size(1), t.size(2), t.size(0), t.stride(1), t.stride(2), t.stride(0)};
 }
 
 void check(int rc, const char* what) {
@@ -79,8 +57,8 @@ py::object dense_forward(const at::Tensor& q, const at::Tensor& k, const at::Ten
                                     static_cast<int>(k.size(2)), causal, 0);
   at::Tensor ws;
   if (parts > 0) ws = at::empty({parts * B * S * H * (D + 1)}, f32);
-  const DenseFwd a{src(q), src(k), src(v), o.data_ptr(), static_cast<float*>(lse.data_ptr()), o.stride(1), o.stride(0), lse.stride(1),
-                   lse.stride(0)};
+  const UaDenseFwd a{src(q), src(k), src(v),
+                     {o.data_ptr(), static_cast<float*>(lse.data_ptr()), o.stride(1), o.stride(0), lse.stride(1), lse.stride(0)}};
   {
     py::gil_scoped_release nogil;
     check(fwd_dense(&a, causal, static_cast<float>(scale), 0, parts > 0 ? static_cast<float*>(ws.data_ptr()) : nullptr,
@@ -105,10 +83,10 @@ py::object local_backward(const at::Tensor& q, const at::Tensor& k, const at::Te
   if (!takes_rows(dk, dev) || dk.strides() != dv.strides()) return py::none();
   const auto f32 = q.options().dtype(at::kFloat);
   const at::Tensor dvec = at::empty({B, H, S}, f32), dq32 = at::empty({B * S * H * D}, f32);
-  const LocalBwd a{src(q), src(k), src(v), src(d_o), o.data_ptr(), o.stride(1), o.stride(0), static_cast<float*>(lse.data_ptr()),
-                   static_cast<float*>(dvec.data_ptr()), static_cast<float*>(dq32.data_ptr()), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                   dk.stride(1), dk.stride(0), reinterpret_cast<void*>(cols), reinterpret_cast<void*>(segs), reinterpret_cast<void*>(tiles),
-                   n_tiles, dense, skewed};
+  const UaLocalBwd a{src(q), src(k), src(v), src(d_o), o.data_ptr(), o.stride(1), o.stride(0), static_cast<float*>(lse.data_ptr()),
+                     static_cast<float*>(dvec.data_ptr()), static_cast<float*>(dq32.data_ptr()), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                     dk.stride(1), dk.stride(0), reinterpret_cast<void*>(cols), reinterpret_cast<void*>(segs), reinterpret_cast<void*>(tiles),
+                     n_tiles, dense, skewed};
   {
     py::gil_scoped_release nogil;
     check(bwd_local(&a, static_cast<float>(scale), reinterpret_cast<int*>(status), reinterpret_cast<void*>(stream)), "ua_attn_bwd_local");
