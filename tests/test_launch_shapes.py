@@ -70,3 +70,18 @@ def test_more_sequences_of_keys_than_of_queries_are_read_as_before():
     q, k = (1, 300, 4), (2, 300, 2)
     block = A._DENSE_FWD.pack(3, *_src(q, 1)[1:], *_src(k, 2), *_src(k, 3), 4 << 24, 5 << 24, 512, 300 * 512, 300, 1200)
     assert not _names_the_shapes(_refusal(_lib.load().ua_attn_fwd_dense(block, 1, 0.1, 1, None, None, None)))
+
+
+def test_a_given_split_stays_where_the_shares_of_the_keys_are_exact():
+    """(more parts than 2^16 for 2^18 key tiles: the products of the remainder and a part's number left 32 bits)"""
+    parts = _lib.load().ua_attn_fwd_dense_parts
+    keys = 128 << 18
+    assert parts(1, 1, keys, 1, 1, 0, 1000) == 1000 and parts(1, 1, 700, 1, 1, 0, 1000) == 6
+    for n_split in (65535, 65536, 70000, 200000):
+        z = parts(1, 1, keys, 1, 1, 0, n_split)
+        assert z == min(n_split, 65536)
+        for n in (1 << 18, (1 << 18) - 1, 3 * z - 1):               # r is largest, z - 1, where n + 1 is a multiple of z
+            q, r = divmod(n, z)
+            for split in (0, 1, z // 2, z - 1):
+                for at in (split, split + 1):
+                    assert r * at < 1 << 32 and q * at + r * at // z == n * at // z

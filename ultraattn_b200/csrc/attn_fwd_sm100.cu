@@ -242,7 +242,8 @@ __device__ __forceinline__ TileRange fwd_tiles(const FwdParams& p, const FwdItem
   TileRange tr = seg_tiles(sg, it.tok0, it.tok_last);
   if (p.n_split > 1) {
     const int n = tr.end - tr.first, base = tr.first;
-    // (n < 2^24 tiles; in 32 bits: a 64-bit division is a hundred instructions)
+    // (in 32 bits: a 64-bit division is a hundred instructions. q and r are n's quotient and remainder by n_split <= 2^16, so that
+    // no product here exceeds max(n, n_split^2 - n_split).)
     const unsigned q = static_cast<unsigned>(n) / p.n_split, r = static_cast<unsigned>(n) % p.n_split;
     tr.first = base + static_cast<int>(q * it.split + r * it.split / p.n_split);
     tr.end = base + static_cast<int>(q * (it.split + 1) + r * (it.split + 1) / p.n_split);
@@ -1233,6 +1234,7 @@ namespace ua {
 // Rates of the estimate below, measured on a B200 (us, bytes per us).
 constexpr int FEW_MIN_KEY_TILES = 4;
 constexpr int MAX_SPLIT = 64;
+constexpr int MAX_GIVEN_SPLIT = 1 << 16;      // (a caller's n_split; the shares of fwd_tiles are 32-bit products)
 constexpr double TILE_US = 1.9;               // one 128-key tile of a 256-row CTA
 constexpr double CTA_US = 6.0;                // start, first loads, epilogue
 constexpr double FEW_FULL_TILE_US = 1.3;      // one 128-key tile of a FEW CTA with 128 rows
@@ -1310,7 +1312,8 @@ static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_he
       best_z = z;
     }
   }
-  d.n_split = n_split > 0 ? (n_split < key_tiles ? n_split : key_tiles) : best_z;
+  const int most = key_tiles < MAX_GIVEN_SPLIT ? key_tiles : MAX_GIVEN_SPLIT;
+  d.n_split = n_split > 0 ? (n_split < most ? n_split : most) : best_z;
   d.n_parts = d.n_split > 1 ? d.n_split : 0;
   // Few items leave SMs idle, and the launch lasts as long as its longest item, whose two sub-tiles go through all keys. With
   // items of 128 rows each sub-tile takes half of them: 1.0 us per key tile for 1.5 us (the issuing warp has one chain
