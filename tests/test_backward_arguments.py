@@ -304,3 +304,27 @@ def test_plans_know_whether_a_few_tiles_hold_most_of_the_work():
     assert not any(skewed(p) for p in (P.causal(1), P.full(1), P.strided(32, 4, 2)))
     assert all(skewed(p) for p in (P.global_local(32, 1, 2), P.star(32, 1), P.streaming(32, 1, 2)))
     assert not A.BwdPlan([]).skewed
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S", [256, 300])
+@pytest.mark.parametrize("causal,scale", [(True, -0.05), (False, -0.05), (True, 0.05)])
+def test_backward_with_a_negative_scale(S, causal, scale):
+    """Masked scores, and rows behind the last one (300), are hidden after they are scaled, whatever the sign."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA GPU")
+    B, H, Hk = 1, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(5)
+    mk = lambda h: torch.randn(B, S, h, 128, device="cuda", dtype=torch.bfloat16, generator=g)
+    q, k, v, d_o = mk(H), mk(Hk), mk(Hk), mk(H)
+    qd, kd, vd = (t.double().requires_grad_() for t in (q, k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", qd, kd.repeat_interleave(2, 2)) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    o = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), vd.repeat_interleave(2, 2))
+    want = torch.autograd.grad(o, (qd, kd, vd), d_o.double())
+    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+    lse = torch.logsumexp(s, -1).detach().float().contiguous()
+    F._flash_attn_backward(d_o, q, k, v, o.detach().bfloat16().contiguous(), lse, dq, dk, dv, 0.0, scale, causal)
+    A.check_status()
+    assert all(_close(a, b) for a, b in zip((dq, dk, dv), want))

@@ -277,12 +277,13 @@ __device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, boo
   tmem_ld_x32(t_st + 32, reinterpret_cast<uint32_t(&)[32]>(sv[1]));
   tmem_wait_ld();
   if (masked) {
+    const float hidden = scale_log2 < 0.f ? INFINITY : -INFINITY;          // (-inf once it is scaled)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int a = min(max(r_first - h * 32, 0), 32), b = min(max(r_last + 1 - h * 32, 0), 32);
       const uint32_t seen = (b > 0 ? 0xFFFFFFFFu >> (32 - b) : 0u) & (a < 32 ? 0xFFFFFFFFu << a : 0u);
 #pragma unroll
-      for (int c = 0; c < 32; ++c) sv[h][c] = (seen >> c) & 1u ? sv[h][c] : -INFINITY;
+      for (int c = 0; c < 32; ++c) sv[h][c] = (seen >> c) & 1u ? sv[h][c] : hidden;
     }
   }
   const uint64_t sc2 = f2_pack(scale_log2, scale_log2);
@@ -735,9 +736,9 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
     };
     auto write_aug = [&](int stage, float lv, float dv) {
       if (lane < 16) {
-        // a row that attends to nothing (lse = -inf) or does not exist (+inf) gets a huge negative
-        // term: its probabilities come out as exactly 0
-        const float nl = (lv == INFINITY || lv == -INFINITY) ? -3.0e38f : -lv * inv_scale_log2;
+        // a row that attends to nothing (lse = -inf) or does not exist (+inf) gets a term that is hugely
+        // negative once it is scaled: its probabilities come out as exactly 0
+        const float nl = (lv == INFINITY || lv == -INFINITY) ? -copysignf(3.0e38f, inv_scale_log2) : -lv * inv_scale_log2;
         uint32_t a0, a1, b0, b1;
         split3(nl, a0, a1);
         split3(-dv, b0, b1);
