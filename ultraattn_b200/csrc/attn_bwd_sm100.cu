@@ -109,6 +109,8 @@ struct BwdParams {
   int kv_group;
   float scale;                      // softmax scale
   float scale_log2;
+  float hidden;             // what becomes -inf when it is scaled ...
+  float hidden_row;         // ... and hugely negative, of finite parts
   int* status;
   // dense launches (cols == nullptr): one column, one query segment, no tables
   BwdCol dense_col;
@@ -271,13 +273,12 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 
 // P^T of one thread's 64 queries: exp2(x * scale_log2) with x = S^T - lse / scale as it comes out
 // of the tensor core, packed to bf16 pairs. `masked` (tiles at a bound): queries outside [r_first, r_last] get 0.
-__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, bool masked, int r_first, int r_last, uint32_t (&pk)[32]) {
+__device__ __forceinline__ void bwd_phase_a(uint32_t t_st, float scale_log2, float hidden, bool masked, int r_first, int r_last, uint32_t (&pk)[32]) {
   float sv[2][32];
   tmem_ld_x32(t_st, reinterpret_cast<uint32_t(&)[32]>(sv[0]));
   tmem_ld_x32(t_st + 32, reinterpret_cast<uint32_t(&)[32]>(sv[1]));
   tmem_wait_ld();
   if (masked) {
-    const float hidden = scale_log2 < 0.f ? INFINITY : -INFINITY;          // (-inf once it is scaled)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int a = min(max(r_first - h * 32, 0), 32), b = min(max(r_last + 1 - h * 32, 0), 32);
@@ -738,7 +739,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
       if (lane < 16) {
         // a row that attends to nothing (lse = -inf) or does not exist (+inf) gets a term that is hugely
         // negative once it is scaled: its probabilities come out as exactly 0
-        const float nl = (lv == INFINITY || lv == -INFINITY) ? -copysignf(3.0e38f, inv_scale_log2) : -lv * inv_scale_log2;
+        const float nl = (lv == INFINITY || lv == -INFINITY) ? p.hidden_row : -lv * inv_scale_log2;
         uint32_t a0, a1, b0, b1;
         split3(nl, a0, a1);
         split3(-dv, b0, b1);
@@ -804,7 +805,7 @@ attn_bwd_kernel(const __grid_constant__ BwdParams p) {
         tc_fence_after_sync();
         uint32_t pk[32];                 // this thread's 64 probabilities, packed; kept for phase B
         const bool masked = !__all_sync(0xFFFFFFFFu, key_ok && r_first <= 0 && r_last >= 63);
-        bwd_phase_a(t_st, p.scale_log2, masked, key_ok ? r_first : 64, r_last, pk);
+        bwd_phase_a(t_st, p.scale_log2, p.hidden, masked, key_ok ? r_first : 64, r_last, pk);
         // packed P^T of this half goes to the first 32 columns of this half's own S^T columns
         // (the other warpgroup may still be reading its fp32 half)
         BWD_PROF(prof, pslot + 3);
@@ -1069,6 +1070,8 @@ extern "C" int ua_attn_bwd(const UaTensorSrc* q_src, const UaTensorSrc* do_src,
   p.kv_group = n_heads / n_kv_heads;
   p.scale = softmax_scale;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
+  p.hidden = softmax_scale < 0.f ? INFINITY : -INFINITY;
+  p.hidden_row = softmax_scale < 0.f ? 3.0e38f : -3.0e38f;
   p.status = status;
   p.stage.tasks = static_cast<const CopyTask*>(copy_tasks_dev);
   p.stage.n_tasks = n_copy_tasks;
@@ -1265,6 +1268,8 @@ extern "C" int ua_attn_bwd_dense_noalloc(const void* q, const void* k, const voi
   p.kv_group = n_heads / n_kv_heads;
   p.scale = softmax_scale;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
+  p.hidden = softmax_scale < 0.f ? INFINITY : -INFINITY;
+  p.hidden_row = softmax_scale < 0.f ? 3.0e38f : -3.0e38f;
   p.status = status;
   p.stage.tasks = nullptr;
   p.stage.n_tasks = 0;
