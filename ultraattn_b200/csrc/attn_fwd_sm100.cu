@@ -398,16 +398,14 @@ __device__ __forceinline__ void fwd_epilogue(FwdSmem<false>& s, uint32_t slot, u
         float f[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = (fnew == 0.f) ? 0.f : __uint_as_float(ov[q * 8 + i]) * fnew;
-        if (it.row.accumulate) {
-          const uint4 old = d4[q];
-          const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
+        const uint4 old = d4[q];
+        const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float lo = __uint_as_float(ow[i] << 16);
-            const float hi = __uint_as_float(ow[i] & 0xFFFF0000u);
-            f[2 * i] += w_old * lo;
-            f[2 * i + 1] += w_old * hi;
-          }
+        for (int i = 0; i < 4; ++i) {
+          const float lo = __uint_as_float(ow[i] << 16);
+          const float hi = __uint_as_float(ow[i] & 0xFFFF0000u);
+          f[2 * i] += w_old * lo;
+          f[2 * i + 1] += w_old * hi;
         }
         uint4 o;
         o.x = pack_bf16x2(f[0], f[1]);

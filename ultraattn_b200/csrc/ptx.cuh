@@ -418,19 +418,6 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t saddr, uint32_
   return d;
 }
 
-// Shared-memory matrix descriptor without swizzle for a K-major operand: 8-row x 16-byte core
-// matrices, `lbo_bytes` between the core matrices of consecutive 8-element K chunks, `sbo_bytes`
-// between consecutive 8-row groups.
-__device__ __forceinline__ uint64_t make_smem_desc_noswz(uint32_t saddr, uint32_t lbo_bytes,
-                                                         uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= static_cast<uint64_t>(1) << 46;  // descriptor version
-  return d;
-}
-
 // ----------------------------------------------------------------------------------------------
 // Register re-balancing between the warpgroups of a CTA (every warp of the warpgroup executes it)
 // ----------------------------------------------------------------------------------------------
@@ -500,7 +487,9 @@ __device__ __forceinline__ void umma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uin
       "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(B_HI)
       : "memory");
 }
-// words of make_smem_desc_sw128 / make_smem_desc_noswz
+// The words of make_smem_desc_sw128, and of a descriptor without swizzle for a K-major operand: 8-row x 16-byte core
+// matrices, `lbo_bytes` between the core matrices of consecutive 8-element K chunks, `sbo_bytes` between
+// consecutive 8-row groups.
 constexpr uint32_t desc_hi_sw128(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
 constexpr uint32_t desc_hi_noswz(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14); }
 __device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
