@@ -46,7 +46,7 @@ constexpr int FWD_QK_WARP = 9;         // issues S = Q K^T; owns the TMEM alloca
 constexpr int FWD_PV_WARP = 10;        // issues O += P V
 // three warpgroups (the last one: TMA, MMA and an idle warp), so that the register file can be
 // re-balanced by warpgroup: a softmax thread holds its row's 128 scores besides everything else (the assembler
-// allocates for the new number behind setmaxnreg); 2 x 216 + 72 <= 3 x 168.
+// allocates for the new number behind setmaxnreg); 2 x 216 + 72 <= 3 x 168. (FEW: 8 bytes of spills, 36 of reloads, by -Xptxas -v.)
 constexpr int FWD_THREADS = 384;
 constexpr int FWD_REGS_LAUNCH = 168, FWD_REGS_LOAD = 72, FWD_REGS_SOFTMAX = 216;
 static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setmaxnreg may only redistribute the launch-time pool");
@@ -60,10 +60,11 @@ static_assert(2 * FWD_REGS_SOFTMAX + FWD_REGS_LOAD <= 3 * FWD_REGS_LAUNCH, "setm
 // issuing warp (230), Q K^T (512 - 630), seen by the softmax warps (290), twice a pair: 2850.
 // The instructions of all roles are kept few and close together (one vote for all that is rare, errors reported by a call,
 // loops over segments not unrolled, 32-bit divisions, operand descriptors by addition): the instruction cache missed 99
-// times a pair before, 17 now, and every miss stops all four warps of a sub-tile; builds that differ in nothing but that
+// times a pair before, 22 now, and every miss stops all four warps of a sub-tile; builds that differ in nothing but that
 // (15 and 53 misses a pair) took 918 and 968 us for 16384 tokens, 8 heads. B200, us, before -> now: 8192 causal tokens, 32 heads
 // 510 -> 432; 16384 tokens, 8 heads 990 -> 847, 32 heads 3450 -> 3050 (1275 -> 1440 TFLOP/s); 512 queries behind 32768 keys, 32 / 8
-// heads 260 -> 222; 1000 causal tokens, 32 / 8 heads 26.6 -> 22.5. Part of the exponentials as a polynomial of degree 5 on the FMA
+// heads 260 -> 222; 1000 causal tokens, 32 / 8 heads 26.6 -> 22.5 (19 with early launches and the shorter
+// start of an item). Part of the exponentials as a polynomial of degree 5 on the FMA
 // pipe (1/8, 1/4, 3/8 of them, at the 914 us of the time): 924, 956, 1048 us. P handed over in two parts (96 + 32 keys): 2 %
 // slower in this form.
 constexpr int FWD_TILE_BYTES = ATTN_TILE * ATTN_D * 2;  // 32 KB: [2 d-halves][128 rows][128 B]
@@ -523,9 +524,9 @@ __device__ __forceinline__ int seg_end_of(const AttnSeg& sg, int r) {
 __device__ __forceinline__ int seg_first_of(const AttnSeg& sg, int r) {
   return (sg.causal & SEG_LOWER) ? max(0, r + sg.lo) : 0;
 }
-// A branch that is never taken (a CTA's 2^32nd score tile). The assembler moves arithmetic over everything that is not a
-// branch, and put the maxima in front of the arrival on s_free, which the other sub-tile's scores wait for
-// (16k tokens, 8 heads: 1038 us without, 917 with).
+// A branch that is never taken (a CTA's 2^32nd score tile), meant to keep the arrival on s_free, which the other sub-tile's
+// scores wait for, in front of the arithmetic behind it. What the compiler makes of it was not looked at; measured (nvcc
+// 12.9.86, 16k tokens, 8 heads): 1038 us without it, 917 with it. Another compiler may need it elsewhere, or not at all.
 #define PIN if (__builtin_expect(cnt == 0xFFFFFFFFu, 0)) break;
 
 // Persistent CTAs: the grid has one CTA per work item, and a CTA that is done with an item cancels one
@@ -560,8 +561,9 @@ attn_fwd_kernel(const __grid_constant__ FwdParams p) {
     for (int e = it.row.seg_begin; e < it.row.seg_end && !waits; ++e) waits = fwd_seg(p, e).wait_flag != 0;
     drain_stage_queue(p.stage, waits, it.linear, &s.stage_slot);
   }
-  // FEW: warps without a valid row have nothing to do (their scores are never read back). The
-  // launch has one row tile, so the number is the same for all its items.
+  // FEW: warps without a valid row have nothing to do (their scores are never read back). The number is the same for
+  // all items of a launch: with more than one row tile all four warps are at work, also in the last one, where those behind
+  // its rows see no key.
   const int act_warps = FEW ? (min(ATTN_TILE, p.dense_row.q_len << psh) + 31) / 32 : 4;
 
   // The producer sets the barriers up, looks up its first item and goes on to load it; the others meet at
@@ -1229,7 +1231,11 @@ extern "C" int ua_attn_fwd(const UaTensorSrc* q_src, int n_q, const UaTensorSrc*
 // ---- dense launches -------------------------------------------------------------------------------
 namespace ua {
 
-// Rates of the estimate below, measured on a B200 (us, bytes per us).
+// Rates of the estimate below (us, bytes per us). They are fitted to which cut was the fastest, with a kernel whose tiles were
+// slower, and are no times of the present one: a tile of a 256-row CTA takes 1.5 us now, one of a FEW CTA with 128 rows 1.0.
+// The choices still hold. Of 1, 2, 3, 4, 5, 6, 8 and 12 parts the chosen number was the fastest, or within 5 % of it, for 12 of 13
+// shapes between 1 query behind 8192 keys and 1000 causal tokens; 512 queries behind 2000 keys, 8 heads, take 19.4 us in the chosen 5
+// parts and 17.4 in 8.
 constexpr int FEW_MIN_KEY_TILES = 4;
 constexpr int MAX_SPLIT = 64;
 constexpr int MAX_GIVEN_SPLIT = 1 << 16;      // (a caller's n_split; the shares of fwd_tiles are 32-bit products)
@@ -1256,10 +1262,11 @@ struct DensePlan {
 // The estimate of one choice: CTAs of equal cost run in whole waves, unequal ones (causal, heaviest
 // first) fill up to about half a CTA of tail, whichever is shorter; plus what the extra fp32 parts
 // cost to write and merge.
-// Measured (us, unpacked and unsplit -> as planned here): 16 sequences, 1 query behind 8123 keys, 32 / 8
-// heads 528 -> 107 (cold L2; 82 is the time of the bytes); 1 sequence behind 8192 keys 138 -> 26; 512 queries
-// behind 32768 keys, 32 / 8 heads, 520 -> 292; 8192 causal tokens, 32 / 8 heads, 589 -> 517 (packing alone).
-// On the other side of the line: 1000 causal tokens, 32 / 8 heads, run 32 unsplit and 62 split in two.
+// Packing (us, kernel of the time, before -> after): 16 sequences, 1 query behind 8123 keys, 32 / 8 heads, 528 -> 107; 8192
+// causal tokens, 32 / 8 heads, 589 -> 517. Splitting (us, B200, cold L2, present kernel, one part -> as planned here): 1 query behind
+// 8192 keys, 32 / 8 heads, 64.5 -> 17.5 (10 parts); 512 queries behind 32768 keys 408 -> 217 (2). On the other side of the line: 16
+// sequences of 8123 keys, one query, take 82 us unsplit (the time of the bytes) and 86 in two parts, 1000 causal tokens, 32 / 8
+// heads, 25.5 and 44.7.
 static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_heads, int causal, int n_split, int sms) {
   DensePlan d{};
   const int group = n_heads / n_kv_heads;
@@ -1315,10 +1322,11 @@ static DensePlan plan_dense(int batch, int sq, int skv, int n_heads, int n_kv_he
   d.n_parts = d.n_split > 1 ? d.n_split : 0;
   // Few items leave SMs idle, and the launch lasts as long as its longest item, whose two sub-tiles go through all keys. With
   // items of 128 rows each sub-tile takes half of them: 1.0 us per key tile for 1.5 us (the issuing warp has one chain
-  // less to overlap with, so a launch that fills the device is slower that way: 1000 causal tokens, 32 heads over 8, 19.7 ->
-  // 21.1 us, and the rule asks for items that all run at once). It beats splitting too, unless the parts are many. Before -> now (B200,
+  // less to overlap with, so a launch that fills the device is slower that way: 1000 causal tokens, 32 heads over 8, by 7 %,
+  // and the rule asks for items that all run at once). It beats splitting too, unless the parts are many. Before -> now (B200,
   // us): causal 1000 tokens, 8 heads 19.1 -> 15.1; 512 13.4 -> 11.2; 2000 tokens, 8 over 2 28.7 -> 23.6; 1000 tokens,
-  // 8 heads, not causal 18.7 -> 15.6. Left as it was: 512 of 2000 tokens, 8 heads (5 parts) 19.1, this 22.8; up to 3 tiles, equal.
+  // 8 heads, not causal 18.7 -> 15.6. Left as it was: 512 of 2000 tokens, 8 heads (5 parts) 19.1, this 22.8; up to 3
+  // tiles, equal. (FEW_FULL_TILE_US is compared with the estimate above, so it is as much above its 1.0 us as TILE_US above 1.5.)
   const int few_q_tiles = static_cast<int>((rows + ATTN_TILE - 1) / ATTN_TILE);
   if (!d.few && n_split == 0 && key_tiles >= FEW_MIN_KEY_TILES && few_q_tiles * per_head <= sms && CTA_US + key_tiles * FEW_FULL_TILE_US < best) {
     d.few = true;
