@@ -16,6 +16,7 @@ input of the backward (orchestrated_attn/utils.py:148-188).
 """
 from __future__ import annotations
 
+import functools
 import math
 import struct
 from dataclasses import dataclass
@@ -570,8 +571,7 @@ class BwdPlan:
                 tiles.append((_col_steps(c, t * TILE), ci, t))
         tiles = _launch_order(tiles)
         self.n_tiles = len(tiles)
-        self.kv_tokens = sum(c.kv_len for c in self.cols)      # gradient rows that the columns write ...
-        self.kv_end = max((c.g_start + c.kv_len for c in self.cols), default=0)      # ... and where the last of them ends
+        self.kv_tokens = sum(c.kv_len for c in self.cols)      # gradient rows that the columns write
         # (causal blocks: heaviest tile twice the average, strided ones 1.8; global + local 9, star and streaming 12 to 20)
         self.skewed = bool(tiles) and max(t[0] for t in tiles) * len(tiles) > 3 * sum(t[0] for t in tiles)
         self.total_steps = sum(c for c, _, _ in tiles)
@@ -582,6 +582,11 @@ class BwdPlan:
         self.cols_t = torch.from_numpy(col_arr).to(self.device)
         self.segs_t = torch.from_numpy(seg_arr).to(self.device)
         self.tiles_t = torch.from_numpy(tile_arr).to(self.device)
+
+    @functools.cached_property
+    def kv_end(self) -> int:
+        """Where the last gradient row that the columns write ends (looked up when asked for: plans saved before have none)."""
+        return max((c.g_start + c.kv_len for c in self.cols), default=0)
 
 
 @dataclass
